@@ -28,7 +28,49 @@
 
 #define ATTN_MAX_D 512
 
-template <typename T>
+namespace {
+
+// The dot product of a lane's key row with the query, one fused multiply-add per element in ascending order.  VECTOR: 16 bytes
+// at a time, eight of them asked for before the first is used.
+template <typename T, bool VECTOR>
+__device__ __forceinline__ float row_dot(const float* q_row, const T* k_row, int head_dim) {
+    float dot = 0.0f;
+    if constexpr (VECTOR) {
+        constexpr int kCount = Vec16<T>::kCount, kDeep = 8;
+        int d = 0;
+        for (; d + kDeep * kCount <= head_dim; d += kDeep * kCount) {
+            uint4 raw[kDeep];
+#pragma unroll
+            for (int i = 0; i < kDeep; ++i) raw[i] = *reinterpret_cast<const uint4*>(k_row + d + i * kCount);
+#pragma unroll
+            for (int i = 0; i < kDeep; ++i) {
+                float k[kCount];
+                Vec16<T>::load(reinterpret_cast<const T*>(&raw[i]), k);
+#pragma unroll
+                for (int j = 0; j < kCount; ++j) dot = fmaf(q_row[d + i * kCount + j], k[j], dot);
+            }
+        }
+        for (; d < head_dim; d += kCount) {
+            float k[kCount];
+            Vec16<T>::load(k_row + d, k);
+#pragma unroll
+            for (int j = 0; j < kCount; ++j) dot = fmaf(q_row[d + j], k[j], dot);
+        }
+    } else {
+#pragma unroll 8
+        for (int d = 0; d < head_dim; ++d) dot = fmaf(q_row[d], Num<T>::load(k_row + d), dot);
+    }
+    return dot;
+}
+
+}  // namespace
+
+// COLUMNS: value elements per lane, the least power of two that covers the value size.  What bounds the kernel for few tokens is
+// the chain of dependent loads per 32 keys (table entry, key row, value rows); so the value rows of a round are asked for,
+// kAhead at a time, before the weights that multiply them are known, and the table entry of the next round with them.  With
+// 150 keys, heads of 32 and 4 tokens a launch took 52 us when the loads were issued one by one and the accumulator had 16
+// columns for every size.
+template <typename T, int COLUMNS, bool VECTOR>
 __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_pages,
                                          const T* __restrict__ v_pages, const int* __restrict__ block_tables,
                                          int max_blocks, const int* __restrict__ seq_of_token,
@@ -37,6 +79,7 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
                                          float scale, int window, const float* __restrict__ sinks,
                                          int chunk, const float* __restrict__ bias, int bias_len, int keep,
                                          const T* __restrict__ gate, int gate_stride, int* __restrict__ error_flag) {
+    constexpr int kAhead = COLUMNS >= 16 ? 2 : 32 / COLUMNS;      // value rows in flight: 32 registers per lane
     pdl_trigger();   // let the next kernel start launching
     pdl_wait();      // everything before this kernel in the stream is complete and visible
     extern __shared__ float q_shared[];  // [warps][head_dim]
@@ -54,32 +97,47 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
     for (int i = lane; i < head_dim; i += 32) q_row[i] = Num<T>::load(q_src + i);
     __syncwarp();
 
-    float accumulator[ATTN_MAX_D / 32];
+    float accumulator[COLUMNS];
 #pragma unroll
-    for (int i = 0; i < ATTN_MAX_D / 32; ++i) accumulator[i] = 0.0f;
+    for (int i = 0; i < COLUMNS; ++i) accumulator[i] = 0.0f;
     float running_max = -INFINITY, normaliser = 0.0f;
 
     int first = (window > 0 && position - window + 1 > 0) ? position - window + 1 : 0;
     if (chunk > 0) first = max(first, position / chunk * chunk);
     const int kept = min(keep, first);      // keys 0 .. kept - 1, then first .. position
     const int count = kept + position - first + 1;
+    auto key_of = [&](int index) { return index < kept ? index : first + index - kept; };
+    int next_page = lane < count ? table[key_of(lane) / page_size] : 0;
     for (int base = 0; base < count; base += 32) {
         const int index = base + lane;
-        const int key = index < kept ? index : first + index - kept;
+        const int key = key_of(index);
         const bool valid = index < count;
-        long long offset = 0;  // this lane's key's slot in the pages: its key row lies at offset * head_dim, its value row at offset * value_dim
+        int page = next_page;
+        if (index + 32 < count) next_page = table[key_of(index + 32) / page_size];
+        if (valid && (unsigned)page >= (unsigned)num_pages) {      // no page of the pool: report it, read page 0 instead
+            if (error_flag) atomicExch(error_flag, 5);
+            page = 0;
+        }
+        // this lane's key's slot in the pages: its key row lies at offset * head_dim, its value row at offset * value_dim
+        const long long offset = valid ? ((long long)page * n_kv_heads + kv_head) * page_size + key % page_size : 0;
+        const int in_chunk = min(32, count - base);
+        float ahead[kAhead][COLUMNS];
+        auto ask = [&](int j0) {      // value rows j0 .. j0 + kAhead - 1 of the round
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const long long row = __shfl_sync(0xffffffffu, offset, j0 + j);
+                const T* v_row = v_pages + row * value_dim;
+#pragma unroll
+                for (int i = 0; i < COLUMNS; ++i) {
+                    const int d = lane + 32 * i;
+                    ahead[j][i] = j0 + j < in_chunk && d < value_dim ? Num<T>::load(v_row + d) : 0.0f;
+                }
+            }
+        };
+        ask(0);
         float score = -INFINITY;
         if (valid) {
-            int page = table[key / page_size];
-            if ((unsigned)page >= (unsigned)num_pages) {      // no page of the pool: report it, read page 0 instead
-                if (error_flag) atomicExch(error_flag, 5);
-                page = 0;
-            }
-            offset = ((long long)page * n_kv_heads + kv_head) * page_size + key % page_size;
-            const T* k_row = k_pages + offset * head_dim;
-            float dot = 0.0f;
-            for (int d = 0; d < head_dim; ++d) dot += q_row[d] * Num<T>::load(k_row + d);
-            score = dot * scale;
+            score = row_dot<T, VECTOR>(q_row, k_pages + offset * head_dim, head_dim) * scale;
             if (bias) score += bias[(size_t)head * bias_len + min(position - key, bias_len - 1)];
         }
         const float chunk_max = warp_max(score);
@@ -88,16 +146,16 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
         const float weight = valid ? expf(score - new_max) : 0.0f;
         normaliser = normaliser * correction + warp_sum(weight);
 #pragma unroll
-        for (int i = 0; i < ATTN_MAX_D / 32; ++i) accumulator[i] *= correction;
-        const int in_chunk = min(32, count - base);
-        for (int j = 0; j < in_chunk; ++j) {
-            const float w = __shfl_sync(0xffffffffu, weight, j);
-            const long long row = __shfl_sync(0xffffffffu, offset, j);
-            const T* v_row = v_pages + row * value_dim;
+        for (int i = 0; i < COLUMNS; ++i) accumulator[i] *= correction;
+        for (int j0 = 0; j0 < in_chunk; j0 += kAhead) {
+            if (j0) ask(j0);
 #pragma unroll
-            for (int i = 0; i < ATTN_MAX_D / 32; ++i) {
-                const int d = lane + 32 * i;
-                if (d < value_dim) accumulator[i] += w * Num<T>::load(v_row + d);
+            for (int j = 0; j < kAhead; ++j) {
+                const float w = __shfl_sync(0xffffffffu, weight, j0 + j);
+                if (j0 + j < in_chunk) {
+#pragma unroll
+                    for (int i = 0; i < COLUMNS; ++i) accumulator[i] = fmaf(w, ahead[j][i], accumulator[i]);
+                }
             }
         }
         running_max = new_max;
@@ -108,12 +166,12 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
         const float correction = expf(running_max - new_max);
         normaliser = normaliser * correction + expf(sink - new_max);
 #pragma unroll
-        for (int i = 0; i < ATTN_MAX_D / 32; ++i) accumulator[i] *= correction;
+        for (int i = 0; i < COLUMNS; ++i) accumulator[i] *= correction;
     }
     T* dst = out + (size_t)token * n_q_heads * value_dim + (size_t)head * value_dim;
     const float inverse = 1.0f / normaliser;
 #pragma unroll
-    for (int i = 0; i < ATTN_MAX_D / 32; ++i) {
+    for (int i = 0; i < COLUMNS; ++i) {
         const int d = lane + 32 * i;
         if (d < value_dim) {
             float value = accumulator[i] * inverse;
@@ -153,9 +211,20 @@ LLM_EXPORT int llm_attention_generic(const void* q, int q_stride, const void* k_
     const int warps = 4;
     dim3 grid(n_tokens, (n_q_heads + warps - 1) / warps);
     const size_t shared = (size_t)warps * head_dim * sizeof(float);
-    LLM_DISPATCH_DTYPE(dtype, (llm_launch(attention_generic_kernel<T>, grid, warps * 32, shared, stream, 
-                                  (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages, block_tables,
-                                  max_blocks, seq_of_token, positions, (T*)out, n_q_heads, n_kv_heads, head_dim,
-                                  value_dim, page_size, num_pages, scale, window, sinks, chunk, bias, bias_len, keep, (const T*)gate, gate_stride, error_flag)));
+    // key rows in 16-byte pieces where every row starts on such a boundary
+    const int count = dtype == LLM_F32 ? 4 : 8;
+    const bool vector = head_dim % count == 0 && aligned16(k_pages);
+#define LLM_GENERIC(COLUMNS)                                                                                                       \
+    LLM_DISPATCH_DTYPE(dtype, llm_launch(vector ? attention_generic_kernel<T, COLUMNS, true> : attention_generic_kernel<T, COLUMNS, false>, \
+                                         grid, warps * 32, shared, stream, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages,     \
+                                         block_tables, max_blocks, seq_of_token, positions, (T*)out, n_q_heads, n_kv_heads, head_dim,       \
+                                         value_dim, page_size, num_pages, scale, window, sinks, chunk, bias, bias_len, keep,                \
+                                         (const T*)gate, gate_stride, error_flag))
+    if (value_dim <= 32) LLM_GENERIC(1);
+    else if (value_dim <= 64) LLM_GENERIC(2);
+    else if (value_dim <= 128) LLM_GENERIC(4);
+    else if (value_dim <= 256) LLM_GENERIC(8);
+    else LLM_GENERIC(16);
+#undef LLM_GENERIC
     return llm_check_launch("attention_generic");
 }

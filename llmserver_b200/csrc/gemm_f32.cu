@@ -64,9 +64,111 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
     }
 }
 
+// The same product for few rows (M <= 32), where a launch is the latency of its loads and not arithmetic: a block owns 32
+// columns, the columns are a warp's lanes and the rows are dealt to four warps, ROWS each.  W goes through shared memory in
+// pieces of 128 along K, three of them in flight, the first three asked for before the kernel in front has ended (weights do
+// not depend on it).  Every output is still one thread's running sum over ascending k, so the results are those of the kernel
+// above bit for bit.
+namespace {
+constexpr int kColumns = 32, kPiece = 128, kPitch = kPiece + 4, kDeep = 3, kFewThreads = 128, kFewRows = 32;
+
+__device__ __forceinline__ void copy16(float* to, const float* from, bool present) {
+    const int bytes = present ? 16 : 0;      // 0: the 16 bytes are filled with zeros and nothing is read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+}  // namespace
+
+template <int ROWS>
+__global__ void __launch_bounds__(kFewThreads) gemm_f32_few_rows_kernel(const float* __restrict__ a, const float* __restrict__ w,
+                                                                        float* __restrict__ c, int m_total, int n_total, int k_total,
+                                                                        int lda, int ldw, int ldc) {
+    pdl_trigger();   // let the next kernel start launching
+    extern __shared__ __align__(16) float stages[];      // [kDeep]{ W [kColumns][kPitch], rows [4 ROWS][kPitch] }
+    constexpr int kStage = (kColumns + 4 * ROWS) * kPitch, kVectors = kPiece / 4;
+    const int n0 = blockIdx.x * kColumns;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int pieces = (k_total + kPiece - 1) / kPiece;
+
+    auto load_w = [&](int piece) {
+        float* to = stages + piece % kDeep * kStage;
+        const int k = piece * kPiece + lane * 4;
+#pragma unroll
+        for (int column = warp; column < kColumns; column += kFewThreads / kVectors) {
+            const bool present = n0 + column < n_total && k < k_total;
+            copy16(to + column * kPitch + lane * 4, present ? w + (size_t)(n0 + column) * ldw + k : w, present);
+        }
+    };
+    auto load_rows = [&](int piece) {
+        float* to = stages + piece % kDeep * kStage + kColumns * kPitch;
+        const int k = piece * kPiece + lane * 4;
+#pragma unroll
+        for (int row = warp; row < 4 * ROWS; row += kFewThreads / kVectors) {
+            const bool present = row < m_total && k < k_total;
+            copy16(to + row * kPitch + lane * 4, present ? a + (size_t)row * lda + k : a, present);
+        }
+    };
+
+    for (int piece = 0; piece < kDeep && piece < pieces; ++piece) load_w(piece);
+    pdl_wait();      // everything before this kernel in the stream is complete and visible
+#pragma unroll
+    for (int piece = 0; piece < kDeep; ++piece) {
+        if (piece < pieces) load_rows(piece);
+        copy_commit();
+    }
+    float sums[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) sums[r] = 0.0f;
+    for (int piece = 0; piece < pieces; ++piece) {
+        copy_wait<kDeep - 1>();
+        __syncthreads();
+        const float* column = stages + piece % kDeep * kStage + lane * kPitch;
+        const float* rows = stages + piece % kDeep * kStage + (kColumns + warp * ROWS) * kPitch;
+#pragma unroll 8
+        for (int k = 0; k < kPiece; k += 4) {      // past the end of K both factors are zero
+            const float4 right = *reinterpret_cast<const float4*>(column + k);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                const float4 left = *reinterpret_cast<const float4*>(rows + r * kPitch + k);
+                sums[r] = fmaf(left.w, right.w, fmaf(left.z, right.z, fmaf(left.y, right.y, fmaf(left.x, right.x, sums[r]))));
+            }
+        }
+        __syncthreads();
+        if (piece + kDeep < pieces) {
+            load_w(piece + kDeep);
+            load_rows(piece + kDeep);
+        }
+        copy_commit();
+    }
+    if (n0 + lane < n_total) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+            if (warp * ROWS + r < m_total) c[(size_t)(warp * ROWS + r) * ldc + n0 + lane] = sums[r];
+    }
+}
+
+template <int ROWS>
+static int few_rows_launch(const float* a, const float* w, float* c, int m, int n, int k, int lda, int ldw, int ldc, cudaStream_t stream) {
+    const size_t shared = (size_t)kDeep * (kColumns + 4 * ROWS) * kPitch * sizeof(float);
+    if (int status = llm_raise_shared_limit(reinterpret_cast<const void*>(gemm_f32_few_rows_kernel<ROWS>), shared, "gemm_f32")) return status;
+    llm_launch(gemm_f32_few_rows_kernel<ROWS>, dim3((unsigned)((n + kColumns - 1) / kColumns)), kFewThreads, shared, stream, a, w, c, m, n, k,
+               lda, ldw, ldc);
+    return llm_check_launch("gemm_f32");
+}
+
 LLM_EXPORT int llm_gemm_f32(const float* a, const float* w, float* c, int m, int n, int k, int lda, int ldw, int ldc,
                             cudaStream_t stream) {
     if (m == 0 || n == 0) return LLM_OK;
+    // few rows whose 16-byte pieces are aligned and whole; any other product runs in tiles of 64 x 64
+    if (m <= kFewRows && k > 0 && k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && aligned16(a) && aligned16(w)) {
+        if (m <= 4) return few_rows_launch<1>(a, w, c, m, n, k, lda, ldw, ldc, stream);
+        if (m <= 8) return few_rows_launch<2>(a, w, c, m, n, k, lda, ldw, ldc, stream);
+        if (m <= 16) return few_rows_launch<4>(a, w, c, m, n, k, lda, ldw, ldc, stream);
+        return few_rows_launch<8>(a, w, c, m, n, k, lda, ldw, ldc, stream);
+    }
     const int blocks_m = (m + BM - 1) / BM;
     if ((n + BN - 1) / BN > 65535) {
         llm_set_error("gemm_f32: at most %d output columns per launch, got %d", 65535 * BN, n);
