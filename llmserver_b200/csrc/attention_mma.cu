@@ -22,7 +22,7 @@
 // utils/attention.py:75-96.  Probabilities are rounded to bfloat16 for the P V product; the normaliser
 // is summed in 32-bit from the unrounded values.
 //
-// The cp.async kernels also come in a form for models whose attention weights have to stay 32-bit and whose softmax
+// The kernels also come in a form for models whose attention weights have to stay 32-bit and whose softmax
 // has a sink (llm_attention_mma_sinks): values may have another size than keys (each 64 or 128), every probability
 // enters the P V product as the sum of two bfloat16 numbers (its rounding and the rounding of what that left over:
 // 16 significant bits, two MMAs instead of one), and exp(sink) joins the denominator once per row.  That form also
@@ -71,15 +71,16 @@ struct AttnParams {
     int* error_flag;         // 3: a bounded wait of the TMA decode kernel ran out; 5: a block-table entry names no page
                              // of the pool; 6: a context needs more splits than max_splits (may be null)
     const float* sinks = nullptr;   // [Hq] or null: one more term exp(sinks[h]) in head h's softmax denominator (a score
-                                    // without key or value, neither scaled nor masked); cp.async kernels only
+                                    // without key or value, neither scaled nor masked); PRECISE kernels only
     int chunk = 0;                  // > 0: a query at position p sees keys (p / chunk) * chunk .. p only
     const float* bias = nullptr;    // [Hq, bias_len], times log2(e): added to the score of the key n positions back, n
     int bias_len = 0;               // at most bias_len - 1 (farther keys: the last entry); BIAS kernels only
     int bias_stride = 0;            // floats between two heads' staged rows; 0: the bias is not staged
     int bias_offset = 0;            // where the staged rows lie in the kernel's shared memory (bytes)
-    int keep = 0;                   // with a window: keys 0 .. keep - 1 stay visible; cp.async kernels only
+    int keep = 0;                   // with a window: keys 0 .. keep - 1 stay visible; PRECISE kernels only
     const __nv_bfloat16* gate = nullptr;    // row of token n from gate + n * gate_stride on, [Hq * DV]: results are multiplied
-    int gate_stride = 0;                    // by its sigmoid; cp.async kernels and their merge only
+    int gate_stride = 0;                    // by its sigmoid; PRECISE kernels and their merge only
+    int by_length = 0;              // TMA decode kernel: blocks take the sequences longest first (up to kThreads of them)
 };
 
 // The first key that the query at `position` may see.
@@ -699,10 +700,34 @@ __global__ void __launch_bounds__(kThreads) attention_decode_kernel(const AttnPa
 // halves x {K, V} copies of page_size x 128 bytes; no thread computes addresses per 16 bytes.  Needs a
 // page size of 8, 16, 32 or 64 tokens (whole pages per tile, whole swizzle atoms per page).
 // ------------------------------------------------------------------------------------------------
+//
+// PRECISE: the form whose weights keep 16 significant bits through the P V product (see warp_tile), with sinks, chunks, kept
+// first keys and an output gate.  A cache of keys that are also the values is copied once, in a ring of twice as many
+// stages.  24 sequences of 517 to 4003 keys with sinks (32 / 8 heads of 128) took 196 us a layer on the cp.async kernel, which
+// keeps two tiles per block in flight and whose every thread computes addresses; a step of four such layers with experts
+// went from 3076 to 2630 us.
 constexpr int kDecodeStages = 3;
+constexpr int kMaxDecodeStages = 2 * kDecodeStages;
 constexpr int kDecodeThreads = kThreads + 32;   // four consumer warps and one producer warp
 
-template <int D>
+// The sequence that the blocks at `place` along the grid take: the one with that many longer ones before it (equal lengths in
+// the order of their numbers).  With more than a wave of blocks the longest sequences then start first and the short ones
+// fill the end, whatever the order in which the requests lie in the batch.  Every thread of the block calls this.
+__device__ __forceinline__ int longest_first(const AttnParams& p, int place, int* lengths, int* answer) {
+    const int mine = threadIdx.x;
+    if (mine < p.n_seqs) lengths[mine] = p.context_len[mine];
+    __syncthreads();
+    if (mine < p.n_seqs) {
+        const int length = lengths[mine];
+        int before = 0;
+        for (int other = 0; other < p.n_seqs; ++other) before += lengths[other] > length || (lengths[other] == length && other < mine);
+        if (before == place) *answer = mine;
+    }
+    __syncthreads();
+    return *answer;
+}
+
+template <int D, bool PRECISE = false>
 __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                               const __grid_constant__ CUtensorMap map_v,
                                                                               const AttnParams p) {
@@ -715,20 +740,22 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
     const bool early = p.old_keys_settled != 0;
     if (!early) pdl_wait();
     extern __shared__ __align__(16) unsigned char shared_raw[];
-    __shared__ __align__(8) uint64_t full_bar[kDecodeStages];
-    __shared__ __align__(8) uint64_t empty_bar[kDecodeStages];
-    __shared__ int failed;
+    __shared__ __align__(8) uint64_t full_bar[kMaxDecodeStages];
+    __shared__ __align__(8) uint64_t empty_bar[kMaxDecodeStages];
+    __shared__ int failed, place_of, lengths[kThreads];
     using Layout = typename std::conditional<D == 128, PageLayout, TmaLayout<D, kTileKeys>>::type;
     constexpr int kHalves = D / 64;
     constexpr uint32_t kTileBytes = kTileKeys * D * 2;          // one of K or V
-    constexpr uint32_t kStageBytes = 2 * kTileBytes;
+    const bool one_copy = PRECISE && p.k_pages == p.v_pages;     // what is cached is key and value
+    const uint32_t stage_bytes = one_copy ? kTileBytes : 2 * kTileBytes;
+    const int n_stages = one_copy ? 2 * kDecodeStages : kDecodeStages;
 
     const uint32_t raw = tma::smem_u32(shared_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;                 // swizzle atoms need 1024-byte alignment
     unsigned char* stages = shared_raw + (base - raw);
-    __nv_bfloat16* q_tile = reinterpret_cast<__nv_bfloat16*>(stages + kDecodeStages * kStageBytes);   // [16][D]
+    __nv_bfloat16* q_tile = reinterpret_cast<__nv_bfloat16*>(stages + kDecodeStages * 2 * kTileBytes);   // [16][D]
 
-    const int seq = blockIdx.z, kv_head = blockIdx.y, split = blockIdx.x;
+    const int seq = p.by_length ? longest_first(p, blockIdx.z, lengths, &place_of) : blockIdx.z, kv_head = blockIdx.y, split = blockIdx.x;
     const int token = p.q_start[seq];
     if (p.q_start[seq + 1] - token != 1) {
         if (early) pdl_wait();
@@ -737,10 +764,18 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
     const int group = p.n_q_heads / p.n_kv_heads;
     const int context = p.context_len[seq];
     const int position = context - 1;
-    const int low_key = p.window > 0 ? max(0, position - p.window + 1) : 0;
-    const int first_key = (low_key / kTileKeys) * kTileKeys;
-    const int split_len = split_length(p, context - first_key);
-    const int n_splits = (context - first_key + split_len - 1) / split_len;
+    // the keys in front of the window's first tile are walked through as one run of tiles, kept ones first (PRECISE)
+    const int low_key = PRECISE ? first_visible(p, position) : p.window > 0 ? max(0, position - p.window + 1) : 0;
+    Walk walk;
+    if constexpr (PRECISE) {
+        walk = walk_of(p, low_key);
+    } else {
+        walk.kept_tiles = 0;
+        walk.first_key = (low_key / kTileKeys) * kTileKeys;
+    }
+    const int span = walk_span(walk, context);
+    const int split_len = split_length(p, span);
+    const int n_splits = (span + split_len - 1) / split_len;
     if (n_splits > p.max_splits && split == 0 && kv_head == 0 && threadIdx.x == 0 && p.error_flag) atomicExch(p.error_flag, 6);
     if (context <= 0 && split == 0) {       // nothing to attend to
         if (early) pdl_wait();
@@ -757,15 +792,14 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
         }
         return;
     }
-    const int split_begin = first_key + split * split_len;
-    const int split_end = min(split_begin + split_len, context);
-    const int n_tiles = (split_end - split_begin + kTileKeys - 1) / kTileKeys;
+    const int first_tile = split * split_len / kTileKeys;      // of the walk; splits are whole tiles
+    const int n_tiles = (min(split_len, span - split * split_len) + kTileKeys - 1) / kTileKeys;
     const int* table = p.block_tables + (size_t)seq * p.max_blocks;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         failed = 0;
-        for (int s = 0; s < kDecodeStages; ++s) {
+        for (int s = 0; s < n_stages; ++s) {
             tma::mbar_init(tma::smem_u32(&full_bar[s]), 1);
             tma::mbar_init(tma::smem_u32(&empty_bar[s]), 4);      // one arrival per consumer warp
         }
@@ -781,11 +815,12 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
         // (head_dim 128: one 5-D box per page and operand instead of one per column half)
         constexpr int kBoxesPerPage = D == 128 ? 1 : kHalves;
         const int pages_per_tile = kTileKeys / p.page_size;
-        const int copies = pages_per_tile * kBoxesPerPage * 2;
-        const int my_page = lane / (kBoxesPerPage * 2), my_half = (lane / 2) % kBoxesPerPage, my_v = lane & 1;
+        const int operands = one_copy ? 1 : 2;
+        const int copies = pages_per_tile * kBoxesPerPage * operands;
+        const int my_page = lane / (kBoxesPerPage * operands), my_half = (lane / operands) % kBoxesPerPage, my_v = lane & (operands - 1);
         bool waited = !early;
         for (int t = 0; t < n_tiles; ++t) {
-            const int s = t % kDecodeStages;
+            const int s = t % n_stages;
             // the tile that may hold the sequence's newest key (the last tile of the last split) is written by the
             // kernel in front of this one
             if (!waited && split == n_splits - 1 && t == n_tiles - 1) {
@@ -793,25 +828,25 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
                 waited = true;
             }
             bool ok = true;
-            if (t >= kDecodeStages) ok = tma::mbar_wait(tma::smem_u32(&empty_bar[s]), ((t / kDecodeStages) - 1) & 1);
+            if (t >= n_stages) ok = tma::mbar_wait(tma::smem_u32(&empty_bar[s]), ((t / n_stages) - 1) & 1);
             if (!ok) {
                 failed = 1;
                 break;
             }
             const uint32_t bar = tma::smem_u32(&full_bar[s]);
-            if (lane == 0) tma::mbar_expect_tx(bar, 2u * kTileBytes);
+            if (lane == 0) tma::mbar_expect_tx(bar, stage_bytes);
             __syncwarp();
             if (lane < copies) {
-                const int key = split_begin + t * kTileKeys + my_page * p.page_size;
+                const int key = walk_key(walk, first_tile + t) + my_page * p.page_size;
                 // an entry that names no page of the pool lies outside the tensor map's extent and is copied as zeros
                 const int page = table[min(key / p.page_size, p.max_blocks - 1)];
                 if ((unsigned)page >= (unsigned)p.num_pages && p.error_flag) atomicExch(p.error_flag, 5);
                 const int y = (page * p.n_kv_heads + kv_head) * p.page_size;
                 if (D == 128) {
-                    const uint32_t dst = base + s * kStageBytes + (my_v ? kTileBytes : 0u) + (uint32_t)(my_page * p.page_size) * 256u;
+                    const uint32_t dst = base + s * stage_bytes + (my_v ? kTileBytes : 0u) + (uint32_t)(my_page * p.page_size) * 256u;
                     tc5::tma_load_5d(dst, my_v ? &map_v : &map_k, bar, 0, 0, 0, 0, page * p.n_kv_heads + kv_head);
                 } else {
-                    const uint32_t dst = base + s * kStageBytes + (my_v ? kTileBytes : 0u) + my_half * (kTileKeys * 128u) +
+                    const uint32_t dst = base + s * stage_bytes + (my_v ? kTileBytes : 0u) + my_half * (kTileKeys * 128u) +
                                          (uint32_t)(my_page * p.page_size) * 128u;
                     tma::load_2d(dst, my_v ? &map_v : &map_k, bar, my_half * 64, y);
                 }
@@ -864,13 +899,27 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
 
     bool ok = true;
     for (int it = 0; it < n_tiles; ++it) {
-        const int s = it % kDecodeStages;
-        if (ok && !tma::mbar_wait(tma::smem_u32(&full_bar[s]), (it / kDecodeStages) & 1)) ok = false;
-        const __nv_bfloat16* k_tile = reinterpret_cast<const __nv_bfloat16*>(stages + s * kStageBytes);
-        const __nv_bfloat16* v_tile = k_tile + kTileKeys * D;
-        const int key_index = split_begin + it * kTileKeys + warp * 16;
-        if (key_index < split_end)
-            warp_tile<D, 2, Layout>(q_frag, k_tile, v_tile, warp * 16, key_index, row_low, row_high, p.scale_log2, o_acc, row_max, row_sum);
+        const int s = it % n_stages;
+        if (ok && !tma::mbar_wait(tma::smem_u32(&full_bar[s]), (it / n_stages) & 1)) ok = false;
+        const __nv_bfloat16* k_tile = reinterpret_cast<const __nv_bfloat16*>(stages + s * stage_bytes);
+        const __nv_bfloat16* v_tile = one_copy ? k_tile : k_tile + kTileKeys * D;
+        const int key_index = walk_key(walk, first_tile + it) + warp * 16;
+        if constexpr (PRECISE) {
+            // rows behind the context hold whatever lay in the page: a weight of zero does not erase a value that is not finite
+            // (only the sequence's last tile has such rows, and its stage is not filled again)
+            if (key_index < context && key_index + 16 > context) {
+                __nv_bfloat16* rows = const_cast<__nv_bfloat16*>(v_tile);
+                for (int c = lane; c < 16 * (D / 8); c += 32) {
+                    const int row = warp * 16 + c / (D / 8);
+                    if (key_index - warp * 16 + row >= context)
+                        *reinterpret_cast<uint4*>(rows + Layout::at(row, c % (D / 8))) = make_uint4(0, 0, 0, 0);
+                }
+                __syncwarp();
+            }
+        }
+        if (key_index < context)
+            warp_tile<D, 2, Layout, D, PRECISE>(q_frag, k_tile, v_tile, warp * 16, key_index, row_low, row_high, p.scale_log2, o_acc, row_max,
+                                                row_sum, nullptr, 0, PRECISE ? p.keep : 0);
         __syncwarp();
         if (lane == 0) tma::mbar_arrive(tma::smem_u32(&empty_bar[s]));     // this warp is done with the stage
     }
@@ -907,13 +956,21 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
         float weights[4], best = -INFINITY, denominator = 0.0f;
 #pragma unroll
         for (int w = 0; w < 4; ++w) best = fmaxf(best, merge[((size_t)w * 16 + r) * (D + 2) + D]);
+        const int head = kv_head * group + r;
+        if constexpr (PRECISE) {
+            // the sink counts once per row: the first split takes it in, as one more score without a value
+            if (p.sinks != nullptr && split == 0) {
+                const float sink = p.sinks[head] * kLog2e;
+                best = fmaxf(best, sink);
+                denominator = exp2f(sink - best);
+            }
+        }
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
             const float* row = merge + ((size_t)w * 16 + r) * (D + 2);
             weights[w] = row[D] == -INFINITY ? 0.0f : exp2f(row[D] - best);
             denominator += row[D + 1] * weights[w];
         }
-        const int head = kv_head * group + r;
         const size_t slot = ((size_t)(p.slot_by_seq ? seq : token) * p.n_q_heads + head) * p.max_splits + split;
         for (int d = 2 * lane; d < D; d += 64) {
             float numerator[2] = {0.0f, 0.0f};
@@ -924,8 +981,15 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
                 numerator[1] += pair.y * weights[w];
             }
             if (n_splits == 1) {
+                float result[2] = {numerator[0] / denominator, numerator[1] / denominator};
+                if constexpr (PRECISE) {
+                    if (p.gate) {
+                        result[0] = gated(p, result[0], token, head * D + d);
+                        result[1] = gated(p, result[1], token, head * D + d + 1);
+                    }
+                }
                 *reinterpret_cast<__nv_bfloat162*>(p.out + (size_t)token * p.n_q_heads * D + (size_t)head * D + d) =
-                    __floats2bfloat162_rn(numerator[0] / denominator, numerator[1] / denominator);
+                    __floats2bfloat162_rn(result[0], result[1]);
             } else if (in_cluster) {
                 *reinterpret_cast<float2*>(mine + r * (D + 2) + d) = make_float2(numerator[0] / denominator, numerator[1] / denominator);
             } else {
@@ -982,7 +1046,11 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
                 cluster_arrive();
                 arrived = true;
             }
-            p.out[(size_t)token * p.n_q_heads * D + (size_t)(kv_head * group + r) * D + d] = __float2bfloat16_rn(numerator / denominator);
+            float result = numerator / denominator;
+            if constexpr (PRECISE) {
+                if (p.gate) result = gated(p, result, token, (kv_head * group + r) * D + d);
+            }
+            p.out[(size_t)token * p.n_q_heads * D + (size_t)(kv_head * group + r) * D + d] = __float2bfloat16_rn(result);
         }
         if (!arrived) cluster_arrive();
         cluster_wait();      // nobody leaves while another rank may still read its shared memory
@@ -1056,26 +1124,14 @@ int launch_decode_cp_async(const AttnParams& given, cudaStream_t stream) {
     return llm_check_launch("attention_decode");
 }
 
-// The form with 32-bit-grade attention weights, sinks and a value size of its own: the cp.async kernels, splits merged
-// by the merge kernel.
-template <int D, int DV, bool BIAS>
-int launch_precise(const AttnParams& p, int run_portions, int total_tiles, int run_decode, cudaStream_t stream) {
-    int status = LLM_OK;
-    if (run_portions && total_tiles > 0) status = launch_portions<D, DV, true, BIAS>(p, total_tiles, stream);
-    if (status != LLM_OK || !run_decode) return status;
-    if (p.max_splits > 1 && (p.partial_out == nullptr || p.partial_ml == nullptr)) {
-        llm_set_error("attention_decode: %d splits need the scratch buffers for partial results", p.max_splits);
-        return LLM_REFUSED;
-    }
-    status = launch_decode_cp_async<D, DV, true, BIAS>(p, stream);
-    if (status != LLM_OK || p.max_splits <= 1) return status;
-    dim3 merge_grid(p.n_q_heads, p.n_seqs);
-    llm_launch(attention_decode_merge_kernel<DV>, merge_grid, DV < 128 ? DV : 128, 0, stream, p);
-    return llm_check_launch("attention_decode_merge");
-}
-
-template <int D>
-int launch_decode_tma(const AttnParams& p, cudaStream_t stream) {
+template <int D, bool PRECISE>
+int launch_decode_tma(const AttnParams& given, cudaStream_t stream) {
+    AttnParams p = given;
+    auto* kernel = attention_decode_tma_kernel<D, PRECISE>;
+    // Two blocks share an SM.  Beyond one wave of them the order in which sequences start decides how raggedly the last wave
+    // ends: 61 sequences of 301 to 4077 keys that lie shortest first, a decode step of the 8B shape 7.51 ms as they lie and
+    // 6.70 ms longest first (more splits instead: 7.3 ms with two parts, 7.8 with three).  Within a wave all start at once.
+    p.by_length = p.n_seqs <= kThreads && (long long)p.max_splits * p.n_kv_heads * p.n_seqs > 2 * llm_sm_count();
     // rows of the page pool seen as a [pages * kv_heads * page_size, D] matrix: the real extent, so that a block-table
     // entry that names no page of the pool is copied as zeros and nothing outside the pool is read
     const uint64_t rows = (uint64_t)p.num_pages * p.n_kv_heads * p.page_size;
@@ -1089,19 +1145,19 @@ int launch_decode_tma(const AttnParams& p, cudaStream_t stream) {
         described = tma::make_map_bf16(&map_k, p.k_pages, rows, D, (uint32_t)p.page_size) &&
                     tma::make_map_bf16(&map_v, p.v_pages, rows, D, (uint32_t)p.page_size);
     }
-    if (!described) return launch_decode_cp_async<D>(p, stream);
+    if (!described) return launch_decode_cp_async<D, D, PRECISE>(p, stream);
     const size_t shared = (size_t)kDecodeStages * 2 * kTileKeys * D * 2 + (size_t)16 * D * 2 + 1024;
-    if (int limit_status = llm_raise_shared_limit(reinterpret_cast<const void*>(attention_decode_tma_kernel<D>), shared, "attention_decode_tma")) return limit_status;
+    if (int limit_status = llm_raise_shared_limit(reinterpret_cast<const void*>(kernel), shared, "attention_decode_tma")) return limit_status;
     dim3 grid(p.max_splits, p.n_kv_heads, p.n_seqs);
     if (!p.cluster_merge) {
-        llm_launch(attention_decode_tma_kernel<D>, grid, kDecodeThreads, shared, stream, map_k, map_v, p);
+        llm_launch(kernel, grid, kDecodeThreads, shared, stream, map_k, map_v, p);
         return llm_check_launch("attention_decode_tma");
     }
     // the splits of a (sequence, kv head) pair as one cluster along x
     if (p.max_splits > 8) {
         static bool allowed = false;
         if (!allowed) {
-            cudaError_t status = cudaFuncSetAttribute(attention_decode_tma_kernel<D>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (status != cudaSuccess) {
                 llm_set_error("attention_decode_tma: clusters of %d are not allowed: %s", p.max_splits, cudaGetErrorString(status));
                 return (int)status;
@@ -1128,7 +1184,7 @@ int launch_decode_tma(const AttnParams& p, cudaStream_t stream) {
     ++count;
     config.attrs = attribute;
     config.numAttrs = count;
-    cudaError_t status = cudaLaunchKernelEx(&config, attention_decode_tma_kernel<D>, map_k, map_v, p);
+    cudaError_t status = cudaLaunchKernelEx(&config, kernel, map_k, map_v, p);
     if (status != cudaSuccess) {
         llm_set_error("attention_decode_tma (cluster of %d): %s", p.max_splits, cudaGetErrorString(status));
         return (int)status;
@@ -1136,7 +1192,7 @@ int launch_decode_tma(const AttnParams& p, cudaStream_t stream) {
     return llm_check_launch("attention_decode_tma");
 }
 
-template <int D>
+template <int D, bool PRECISE = false>
 int launch_decode(const AttnParams& p, cudaStream_t stream) {
     const bool whole_pages = p.page_size >= 8 && p.page_size <= kTileKeys && kTileKeys % p.page_size == 0 && p.page_size % 8 == 0;
     const bool by_tma = whole_pages && aligned16(p.k_pages) && aligned16(p.v_pages);
@@ -1148,10 +1204,29 @@ int launch_decode(const AttnParams& p, cudaStream_t stream) {
         llm_set_error("attention_decode: %d splits need the scratch buffers for partial results", p.max_splits);
         return LLM_REFUSED;
     }
-    int status = by_tma ? launch_decode_tma<D>(q, stream) : launch_decode_cp_async<D>(q, stream);
+    int status = by_tma ? launch_decode_tma<D, PRECISE>(q, stream) : launch_decode_cp_async<D, D, PRECISE>(q, stream);
     if (status != LLM_OK || p.max_splits <= 1 || q.cluster_merge) return status;
     dim3 merge_grid(p.n_q_heads, p.n_seqs);
     llm_launch(attention_decode_merge_kernel<D>, merge_grid, D < 128 ? D : 128, 0, stream, p);
+    return llm_check_launch("attention_decode_merge");
+}
+
+// The form with 32-bit-grade attention weights, sinks and a value size of its own: values as wide as keys run the TMA decode
+// kernel, other sizes and scores with a bias the cp.async kernel with the merge kernel behind it.
+template <int D, int DV, bool BIAS>
+int launch_precise(const AttnParams& p, int run_portions, int total_tiles, int run_decode, cudaStream_t stream) {
+    int status = LLM_OK;
+    if (run_portions && total_tiles > 0) status = launch_portions<D, DV, true, BIAS>(p, total_tiles, stream);
+    if (status != LLM_OK || !run_decode) return status;
+    if constexpr (D == DV && !BIAS) return launch_decode<D, true>(p, stream);
+    if (p.max_splits > 1 && (p.partial_out == nullptr || p.partial_ml == nullptr)) {
+        llm_set_error("attention_decode: %d splits need the scratch buffers for partial results", p.max_splits);
+        return LLM_REFUSED;
+    }
+    status = launch_decode_cp_async<D, DV, true, BIAS>(p, stream);
+    if (status != LLM_OK || p.max_splits <= 1) return status;
+    dim3 merge_grid(p.n_q_heads, p.n_seqs);
+    llm_launch(attention_decode_merge_kernel<DV>, merge_grid, DV < 128 ? DV : 128, 0, stream, p);
     return llm_check_launch("attention_decode_merge");
 }
 
@@ -1386,7 +1461,7 @@ LLM_EXPORT int llm_attention_mma_sinks(const void* q, int q_stride, const void* 
                                        int page_size, int num_pages, float scale, int window, const float* sinks,
                                        int chunk, const float* bias, int bias_len, int keep, const void* gate, int gate_stride,
                                        int run_portions, int total_tiles, int run_decode, int split_len, int max_splits,
-                                       float* partial_out, float* partial_ml, int* error_flag, cudaStream_t stream) {
+                                       float* partial_out, float* partial_ml, int old_keys_settled, int* error_flag, cudaStream_t stream) {
     if (!llm_attention_mma_sinks_supports(head_dim, value_dim, n_q_heads, n_kv_heads)) {
         llm_set_error("attention_mma_sinks: keys of %d and values of %d with %d/%d heads are not supported (64 or 128 each, "
                       "group <= 16)", head_dim, value_dim, n_q_heads, n_kv_heads);
@@ -1409,8 +1484,8 @@ LLM_EXPORT int llm_attention_mma_sinks(const void* q, int q_stride, const void* 
     p.max_blocks = max_blocks;
     p.num_pages = num_pages;
     p.slot_by_seq = 0;
-    p.cluster_merge = 0;
-    p.old_keys_settled = 0;
+    p.cluster_merge = decode_cluster_merge_enabled() ? 1 : 0;
+    p.old_keys_settled = old_keys_settled;
     p.q_start = q_start;
     p.context_len = context_len;
     p.out = (__nv_bfloat16*)out;

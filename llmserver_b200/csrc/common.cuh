@@ -17,6 +17,7 @@ enum : int { LLM_OK = 0, LLM_REFUSED = -1 };
 // Records a human-readable reason for the last refusal; read back with llm_last_error().
 void llm_set_error(const char* format, ...);
 int llm_check_launch(const char* what);
+extern "C" int llm_sm_count();      // of the current device
 
 // Programmatic dependent launch: a kernel launched with the attribute below may start while the kernel
 // before it in the stream is still running; it calls pdl_wait() before it touches anything that kernel

@@ -201,6 +201,12 @@ def key_span(window, chunk, keep=0):
     return int(window) + -(-int(keep) // TILE) * TILE if window else None
 
 
+def decode_by_tma(k_pages, v_pages) -> bool:
+    """Whether the decode kernel copies these pages by TMA (whole pages per tile of 64 keys, whole swizzle atoms per page)."""
+    page_size = k_pages.shape[2]
+    return 8 <= page_size <= TILE and TILE % page_size == 0 and k_pages.data_ptr() % 16 == 0 and v_pages.data_ptr() % 16 == 0
+
+
 def try_attention_precise(qkv, q_stride, batch, block_tables, k_pages, v_pages, n_q_heads, n_kv_heads, head_dim, value_dim,
                           scale, window, sinks, chunk=0, bias_log2=None, keep=0, gate=None, gate_column=0):
     """The tensor-core kernels in the form that keeps attention weights at 16 significant bits through the P V product,
@@ -220,11 +226,13 @@ def try_attention_precise(qkv, q_stride, batch, block_tables, k_pages, v_pages, 
         check(bias_log2, "distance bias", torch.float32)
         if bias_log2.dim() != 2 or bias_log2.shape[0] != n_q_heads:
             raise ValueError(f"the distance bias must be [{n_q_heads}, distances], got {tuple(bias_log2.shape)}")
-    # the cp.async decode kernel keeps two tiles in flight per block: three blocks an SM (its shared memory allows them)
-    # and splits without the cluster's bound keep more bytes in flight
-    run_portions, tiles, run_decode, split_len, max_splits = plan(batch, n_q_heads // n_kv_heads, n_kv_heads, qkv.device,
-                                                                  blocks_per_sm=PRECISE_DECODE_BLOCKS_PER_SM, cluster=False,
-                                                                  span=key_span(window, chunk, keep))
+    # Values as wide as keys and no bias: single tokens run the TMA decode kernel (two blocks an SM, splits merged in a
+    # cluster).  The cp.async decode kernel, which takes the rest, keeps two tiles in flight per block: three blocks an SM
+    # (its shared memory allows them) and splits without the cluster's bound keep more bytes in flight.
+    by_tma = value_dim == head_dim and bias_log2 is None and decode_by_tma(k_pages, v_pages)
+    run_portions, tiles, run_decode, split_len, max_splits = plan(
+        batch, n_q_heads // n_kv_heads, n_kv_heads, qkv.device, span=key_span(window, chunk, keep),
+        **({} if by_tma else {"blocks_per_sm": PRECISE_DECODE_BLOCKS_PER_SM, "cluster": False}))
     from . import _gate_rows
     gate_pointer, gate_stride = _gate_rows(gate, gate_column, batch.n_tokens, n_q_heads * value_dim, torch.bfloat16)
     keep = int(keep) if window else 0
@@ -266,7 +274,7 @@ def try_attention_precise(qkv, q_stride, batch, block_tables, k_pages, v_pages, 
          0 if sinks is None else sinks.data_ptr(), int(chunk), 0 if bias_log2 is None else bias_log2.data_ptr(),
          0 if bias_log2 is None else bias_log2.shape[1], keep, gate_pointer, gate_stride, int(run_portions), tiles, int(run_decode), split_len, max_splits,
          0 if partial_out is None else partial_out.data_ptr(), 0 if partial_ml is None else partial_ml.data_ptr(),
-         wait_error_flag(qkv.device).data_ptr(), stream_handle())
+         int(EARLY_KEYS and getattr(batch, "keys_settled", False)), wait_error_flag(qkv.device).data_ptr(), stream_handle())
     return out
 
 

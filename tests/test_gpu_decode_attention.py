@@ -1,0 +1,75 @@
+"""The TMA decode kernel's form with 16-bit-grade weights (sinks, chunks, kept first keys, gates) against the kernel for every
+size, and the order in which its blocks take sequences."""
+import pytest
+import torch
+
+from test_gpu_serving_sizes import DEVICE, HostBatch, paged_case, plain_rows, relative_error
+
+pytestmark = pytest.mark.gpu
+
+MANY = [1, 63, 64, 65, 127, 128, 129, 700, 4096, 2, 1025, 2047, 2048, 2049, 191, 192, 193]
+
+
+def decode_batch(contexts):
+    batch = HostBatch([1] * len(contexts), contexts)
+    batch.max_q_len, batch.keys_settled = 1, True
+    batch.positions, batch.seq_of_token = batch.context_len - 1, torch.arange(len(contexts), dtype=torch.int32, device=DEVICE)
+    return batch
+
+
+# no limit, windows on and off a tile's edge, with kept first keys, chunks, a gate, sinks
+FORMS = [dict(), dict(sinks=True), dict(window=1024, gate=True), dict(window=100, keep=5, sinks=True), dict(window=129, keep=70, gate=True),
+         dict(chunk=128), dict(chunk=1000, sinks=True, gate=True)]
+
+
+@pytest.mark.parametrize("form", FORMS, ids=lambda form: "-".join(form) or "plain")
+@pytest.mark.parametrize("heads,kv_heads,dim,page_size,contexts", [
+    (4, 4, 128, 16, [1]), (16, 1, 128, 16, [3000]), (32, 8, 128, 16, [900, 64, 2500]), (10, 2, 64, 8, MANY), (8, 8, 128, 64, MANY),
+    (32, 8, 128, 32, MANY * 4), (16, 1, 64, 16, MANY * 7)])
+@pytest.mark.parametrize("shared", [False, True])
+def test_precise_decode_attention(form, heads, kv_heads, dim, page_size, contexts, shared):
+    """From one block to more than a wave of them (sequences then start longest first; 119 sequences are just what that rule
+    takes), values of their own and values that are the keys.  Rows of the pages behind a context hold NaN: nothing of
+    them may reach a result.  The bound: weights of 16 bits against 32, and one rounding of the output to bfloat16."""
+    from llmserver_b200 import ops
+    from llmserver_b200.ops import attention_bf16
+    from llmserver_b200.ops.library import check_wait_errors
+    batch = decode_batch(contexts)
+    qkv, q_stride, k_pages, v_pages, tables = paged_case(len(contexts) + dim, [1] * len(contexts), contexts, heads, kv_heads, dim, page_size, 2.0)
+    for row, context in enumerate(contexts):
+        last = int(tables[row, (context - 1) // page_size])
+        for pages in (k_pages, v_pages):
+            pages[last, :, (context - 1) % page_size + 1:] = float("nan")
+    if shared:
+        v_pages = k_pages
+    assert attention_bf16.decode_by_tma(k_pages, v_pages)
+    given = dict(window=form.get("window", 0), chunk=form.get("chunk", 0), keep=form.get("keep", 0),
+                 sinks=torch.linspace(-2.0, 3.0, heads, device=DEVICE) if form.get("sinks") else None,
+                 gate=torch.randn((len(contexts), heads * dim), device=DEVICE).to(torch.bfloat16) if form.get("gate") else None)
+    got = ops.attention(qkv, batch, tables, k_pages, v_pages, heads, kv_heads, dim, dim ** -0.5, precise=True, q_stride=q_stride, **given)
+    want = ops.attention_generic(qkv, q_stride, k_pages, v_pages, tables, batch.seq_of_token, batch.positions, heads, kv_heads, dim,
+                                 dim ** -0.5, **given)
+    torch.cuda.synchronize()
+    check_wait_errors()
+    got, want = got.double(), want.double()
+    assert torch.isfinite(got).all()
+    # both are rounded to bfloat16 once: they differ by at most one step of 2^-8 where the 32-bit results straddle a boundary,
+    # beside 2^-16 of weight error on sums whose size is the row's largest value
+    error = (got - want).abs() / torch.maximum(want.abs(), 0.05 * want.abs().amax(dim=-1, keepdim=True))
+    assert error.max() <= 2.0 ** -7, f"{float(error.max()):.2e}"
+
+
+@pytest.mark.parametrize("n_seqs", [127, 128, 129])
+def test_longest_first_takes_every_sequence_once(n_seqs):
+    """Up to 128 sequences are taken longest first; among them equal lengths, in an order that is neither rising nor falling."""
+    from llmserver_b200.ops import attention_bf16
+    heads, kv_heads, dim, page_size = 8, 4, 128, 16
+    contexts = [1 + (37 * row) % 50 * 20 for row in range(n_seqs)]
+    batch = decode_batch(contexts)
+    qkv, q_stride, k_pages, v_pages, tables = paged_case(n_seqs, [1] * n_seqs, contexts, heads, kv_heads, dim, page_size)
+    out = attention_bf16.try_attention(qkv, q_stride, batch, tables, k_pages, v_pages, heads, kv_heads, dim, dim ** -0.5, 0)
+    worst = 0.0
+    for row, context in enumerate(contexts):
+        want = plain_rows(qkv, k_pages, v_pages, tables[row], context, context - 1, [0], heads, kv_heads, dim, page_size, dim ** -0.5, row)
+        worst = max(worst, relative_error(out[row:row + 1], want))
+    assert worst <= 2e-2, f"relative error {worst:.3e}"
