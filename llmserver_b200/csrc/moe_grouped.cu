@@ -51,7 +51,8 @@ __device__ __forceinline__ int tile_at(int row, int chunk) { return row * kBlock
 // plan[0] = number of row tiles; then per tile (expert, first row, rows); see llm_moe_plan for the other outputs.
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ chosen, int n_pairs, int experts,
                                                         int* __restrict__ offsets, int* __restrict__ pair_of_row,
-                                                        int* __restrict__ row_of_pair, int* __restrict__ tiles, int max_tiles) {
+                                                        int* __restrict__ row_of_pair, int* __restrict__ tiles, int max_tiles,
+                                                        int tile_rows) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ int plan_shared[];     // [experts] counts, then cursors; [experts + 1] offsets
@@ -67,10 +68,10 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
         for (int e = 0; e < experts; ++e) {
             start[e] = total;
             offsets[e] = total;
-            for (int row = 0; row < count[e] && tile < max_tiles; row += kBlockRows, ++tile) {
+            for (int row = 0; row < count[e] && tile < max_tiles; row += tile_rows, ++tile) {
                 tiles[1 + 3 * tile] = e;
                 tiles[2 + 3 * tile] = total + row;
-                tiles[3 + 3 * tile] = min(kBlockRows, count[e] - row);
+                tiles[3 + 3 * tile] = min(tile_rows, count[e] - row);
             }
             total += count[e];
         }
@@ -286,13 +287,12 @@ __global__ void moe_combine_rows_kernel(const float* __restrict__ down, const in
 }
 
 // Sorts the pairs by expert.  chosen: int32 [n_pairs]; offsets: int32 [experts + 1]; pair_of_row, row_of_pair: int32
-// [n_pairs]; tiles: int32 [1 + 3 * max_tiles] with max_tiles >= ceil(n_pairs / 128) + experts.
+// [n_pairs]; tiles: int32 [1 + 3 * max_tiles] with max_tiles >= ceil(n_pairs / tile_rows) + experts.
 LLM_EXPORT int llm_moe_plan(const int* chosen, int n_pairs, int experts, int* offsets, int* pair_of_row, int* row_of_pair,
-                            int* tiles, int max_tiles, cudaStream_t stream) {
+                            int* tiles, int max_tiles, int tile_rows, cudaStream_t stream) {
     if (n_pairs == 0) return LLM_OK;
-    if (max_tiles < (n_pairs + kBlockRows - 1) / kBlockRows + experts) {
-        llm_set_error("moe_plan: room for %d tiles, %d pairs of %d experts may need %d", max_tiles, n_pairs, experts,
-                      (n_pairs + kBlockRows - 1) / kBlockRows + experts);
+    if (tile_rows <= 0 || max_tiles < (n_pairs + tile_rows - 1) / tile_rows + experts) {
+        llm_set_error("moe_plan: room for %d tiles of %d rows, %d pairs of %d experts may need more", max_tiles, tile_rows, n_pairs, experts);
         return LLM_REFUSED;
     }
     const size_t shared = (size_t)(2 * experts + 1) * sizeof(int);
@@ -300,7 +300,7 @@ LLM_EXPORT int llm_moe_plan(const int* chosen, int n_pairs, int experts, int* of
         llm_set_error("moe_plan: %d experts are too many", experts);
         return LLM_REFUSED;
     }
-    llm_launch(moe_plan_kernel, 1, 1024, shared, stream, chosen, n_pairs, experts, offsets, pair_of_row, row_of_pair, tiles, max_tiles);
+    llm_launch(moe_plan_kernel, 1, 1024, shared, stream, chosen, n_pairs, experts, offsets, pair_of_row, row_of_pair, tiles, max_tiles, tile_rows);
     return llm_check_launch("moe_plan");
 }
 

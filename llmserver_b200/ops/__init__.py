@@ -19,7 +19,7 @@ from .stream import STREAM_ROWS, RowScaled, StreamSink
 __all__ = ["KernelError", "embedding", "add_rmsnorm", "rmsnorm", "silu_mul", "sample", "qk_norm_rope_kv_write",
            "attention_generic", "rope_kv_write_split", "normed_add_rmsnorm", "scaled_add_rmsnorm", "moe_route", "moe_select", "indexed_linear", "moe_combine", "moe_plan", "moe_grouped",
            "moe_grouped_supported", "moe_combine_rows", "ExpertPlan",
-           "clamped_glu", "gemm_f32", "linear", "linear_wide", "qkv_projection", "gate_up_silu", "interleave_gate_up", "require_device", "library", "launch_count",
+           "clamped_glu", "clamped_gate_up", "gemm_f32", "linear", "linear_wide", "qkv_projection", "gate_up_silu", "interleave_gate_up", "require_device", "library", "launch_count",
            "RowScaled", "StreamSink", "STREAM_ROWS", "unscaled_rows_supported", "norm_rope_units", "rotate_units", "attention_diff", "gla_supported",
            "gla_recurrent", "head_linear", "relu_squared", "tanh_narrow", "softcap_", "scaled_sum", "token_shift_mix",
            "short_conv_units", "matrix_recurrence_supported", "wkv_recurrent", "delta_rule_recurrent", "retention_recurrent", "ssd_recurrent", "decay_recurrence_supported",
@@ -145,9 +145,22 @@ def gate_up_silu(x, weight: torch.Tensor, group: int = 0) -> torch.Tensor:
     if x.dtype == torch.bfloat16 and group == GATE_UP_GROUP:
         from . import gemm_bf16
         fused = gemm_bf16.gate_up_silu_fused(x, weight)
+        if fused is None:
+            fused = gemm_bf16.gated_by_pairs(x, weight, group, float("inf"), 1.0, 0.0)
         if fused is not None:
             return fused
     return silu_mul(linear(x, weight), group=group)
+
+
+def clamped_gate_up(x: torch.Tensor, weight: torch.Tensor, limit: float, alpha: float) -> torch.Tensor:
+    """``clamped_glu`` of x W^T for W [2 I, H], gate rows first: as one kernel where the product can finish its rows, else the
+    product followed by ``clamped_glu``."""
+    if x.dtype == torch.bfloat16:
+        from . import gemm_bf16
+        fused = gemm_bf16.gated_by_pairs(x, weight, 0, limit, alpha, 1.0)
+        if fused is not None:
+            return fused
+    return clamped_glu(linear(x, weight), limit, alpha)
 
 
 def sample(logits: torch.Tensor, temperatures: Optional[torch.Tensor] = None, seeds: Optional[torch.Tensor] = None,
@@ -1207,27 +1220,29 @@ class ExpertPlan:
     order holds, ``row_of_pair`` the inverse, ``offsets[e]`` the first row of expert e, ``tiles`` the row tiles the
     grouped product walks (count first, then (expert, first row, rows) per tile)."""
 
-    def __init__(self, pairs, offsets, pair_of_row, row_of_pair, tiles, max_tiles):
+    def __init__(self, pairs, offsets, pair_of_row, row_of_pair, tiles, max_tiles, tile_rows):
         self.pairs, self.offsets, self.pair_of_row, self.row_of_pair = pairs, offsets, pair_of_row, row_of_pair
-        self.tiles, self.max_tiles = tiles, max_tiles
+        self.tiles, self.max_tiles, self.tile_rows = tiles, max_tiles, tile_rows
 
 
-MOE_TILE_ROWS = 128
+MOE_TILE_ROWS = 128         # of the tiled products, which one SM each makes
+MOE_PAIR_TILE_ROWS = 256    # of the product that pairs of SMs make
 
 
-def moe_plan(chosen: torch.Tensor, experts: int) -> ExpertPlan:
+def moe_plan(chosen: torch.Tensor, experts: int, tile_rows: int = MOE_TILE_ROWS) -> ExpertPlan:
     """Sorts the pairs of ``chosen`` (int32 [N, top]) by expert on the device; nothing comes back to the host.  Pairs that
-    chose an identity output (``experts`` or beyond) get no row: their ``row_of_pair`` is -1."""
+    chose an identity output (``experts`` or beyond) get no row: their ``row_of_pair`` is -1.  ``tile_rows``: the most rows
+    of a tile, MOE_TILE_ROWS or MOE_PAIR_TILE_ROWS; the plan's products run the kernel that makes such tiles."""
     check(chosen, "chosen experts", torch.int32)
     pairs = chosen.numel()
-    max_tiles = -(-pairs // MOE_TILE_ROWS) + experts
+    max_tiles = -(-pairs // tile_rows) + experts
     offsets = torch.empty((experts + 1,), dtype=torch.int32, device=chosen.device)
     pair_of_row = torch.empty((pairs,), dtype=torch.int32, device=chosen.device)
     row_of_pair = torch.empty((pairs,), dtype=torch.int32, device=chosen.device)
     tiles = torch.empty((1 + 3 * max_tiles,), dtype=torch.int32, device=chosen.device)
     call("llm_moe_plan", chosen.data_ptr(), pairs, experts, offsets.data_ptr(), pair_of_row.data_ptr(), row_of_pair.data_ptr(),
-         tiles.data_ptr(), max_tiles, stream_handle())
-    return ExpertPlan(pairs, offsets, pair_of_row, row_of_pair, tiles, max_tiles)
+         tiles.data_ptr(), max_tiles, int(tile_rows), stream_handle())
+    return ExpertPlan(pairs, offsets, pair_of_row, row_of_pair, tiles, max_tiles, int(tile_rows))
 
 
 # "tcgen05" (default): the tiled product with its accumulator in tensor memory; "mma": the mma.sync kernel
@@ -1266,14 +1281,15 @@ def moe_grouped(x: torch.Tensor, weight: torch.Tensor, plan: ExpertPlan, gather_
     out = torch.empty((plan.pairs, rows), dtype=torch.bfloat16 if gated or squared_relu else torch.float32, device=x.device)
     form = 1 if gated else 2 if squared_relu else 0
     limit, alpha, up_shift = _gate_constants(gated)
-    tensor_memory = MOE_GROUPED_KERNEL != "mma" and library().llm_moe_grouped_tc_supports(rows, inner, int(bool(gated))) and (gated or rows % 4 == 0)
+    by_pairs = plan.tile_rows == MOE_PAIR_TILE_ROWS
+    tensor_memory = by_pairs or MOE_GROUPED_KERNEL != "mma" and library().llm_moe_grouped_tc_supports(rows, inner, int(bool(gated))) and (gated or rows % 4 == 0)
     if gather_div is not None and (tensor_memory or pair_scale is not None):
         ordered = torch.empty((plan.pairs, inner), dtype=torch.bfloat16, device=x.device)
         call("llm_moe_gather_rows", x.data_ptr(), plan.pair_of_row.data_ptr(), int(gather_div), ordered.data_ptr(), plan.pairs,
              inner, pointer(pair_scale), stream_handle())
         x, gather_div = ordered, None
     if tensor_memory:
-        call("llm_moe_grouped_tc", x.data_ptr(), plan.pairs, weight.data_ptr(), weight.shape[0], plan.tiles.data_ptr(), out.data_ptr(),
+        call("llm_moe_grouped_pair" if by_pairs else "llm_moe_grouped_tc", x.data_ptr(), plan.pairs, weight.data_ptr(), weight.shape[0], plan.tiles.data_ptr(), out.data_ptr(),
              rows, inner, plan.max_tiles, form, limit, alpha, up_shift, wait_error_flag(x.device).data_ptr(),
              stream_handle())
         return out

@@ -6,7 +6,8 @@ cuBLAS: utils/attention.py:119-124,181; utils/layers.py:205-217; utils/model.py:
 * up to 64 rows (decode steps, the output head): this package's tcgen05 / TMA kernel
   (``csrc/gemm_tcgen05.cu``), which streams the weights once and can write float32 directly, or the
   library product, whichever a one-time measurement per shape finds faster;
-* more rows (prompt portions): the library product (cuBLAS through PyTorch).
+* more rows (prompt portions): the library product (cuBLAS through PyTorch); gated feed-forwards of many rows run a product
+  of this package that pairs of SMs make and whose epilogue applies the gate (``csrc/gemm_pair_tcgen05.cu``).
 """
 from __future__ import annotations
 
@@ -406,6 +407,31 @@ def qkv_rope_fused(x: torch.Tensor, weight: torch.Tensor, q_weight, k_weight, in
 
 
 FUSE_GATE_UP_SILU = os.environ.get("LLMSERVER_B200_FUSE_GATE_UP_SILU", "1") != "0"
+# From these many rows and up to this inner size the gated product that pairs of SMs make (with the activation in its epilogue) is
+# the faster way.  Both sides are limited by the power cap there, and the library's product alone needs a little less of it: what
+# the fused form saves is the activation's pass over memory, whose share shrinks with the inner size.  Whole prompts (library
+# product and activation kernel against pairs, ms): 8B shape (4096) 14.45 / 14.53 at 1024 rows, 20.56 / 20.46 at 1500, 27.40 /
+# 26.82 at 2048, 56.59 / 54.46 at 4096, 119.7 / 118.9 at 8192; 14B shape (5120) 59.8 / 59.3 at 2400, 99.0 / 99.8 at 4096,
+# 140.7 / 141.2 at 6000.
+PAIR_MIN_ROWS, PAIR_MAX_INNER = 1536, 4096
+
+
+def gated_by_pairs(x, weight: torch.Tensor, group: int, limit: float, alpha: float, up_shift: float) -> Optional[torch.Tensor]:
+    """The gated activation min(g, limit) * sigmoid(alpha * min(g, limit)) * (clamp(u) + up_shift) of many rows, in the epilogue
+    of the product that pairs of SMs make (``csrc/gemm_pair_tcgen05.cu``).  ``weight`` [2 I, H]: gate rows first (``group`` 0)
+    or gate and up rows in turn.  None when that product does not take the case or is not the faster way."""
+    if isinstance(x, RowScaled) or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16:
+        return None
+    rows, inner = x.shape
+    features = weight.shape[0] // 2
+    if not (rows >= PAIR_MIN_ROWS and inner <= PAIR_MAX_INNER and x.is_contiguous() and weight.is_contiguous() and weight.shape[1] == inner
+            and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and library().llm_gemm_pair_supports(features, inner, group)):
+        return None
+    out = torch.empty((rows, features), dtype=torch.bfloat16, device=x.device)
+    call("llm_gemm_pair_gated", x.data_ptr(), weight.data_ptr(), out.data_ptr(), rows, features, inner, group, float(limit), float(alpha),
+         float(up_shift), error_flag(x.device).data_ptr(), stream_handle())
+    return out
 
 
 def gate_up_silu_fused(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tensor]:

@@ -52,7 +52,10 @@ SIGNATURES = {
     "llm_indexed_linear": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _I, _I, _P, _F, _I, _I, _S],
     "llm_moe_combine": [_P, _P, _P, _P, _P, _I, _I, _I, _P, _I, _P, _I, _S],
     "llm_clamped_glu": [_P, _P, _I, _I, _F, _F, _I, _S],
-    "llm_moe_plan": [_P, _I, _I, _P, _P, _P, _P, _I, _S],
+    "llm_moe_plan": [_P, _I, _I, _P, _P, _P, _P, _I, _I, _S],
+    "llm_gemm_pair_supports": [_I, _I, _I],
+    "llm_gemm_pair_gated": [_P, _P, _P, _I, _I, _I, _I, _F, _F, _F, _P, _S],
+    "llm_moe_grouped_pair": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _F, _F, _F, _P, _S],
     "llm_moe_grouped_supports": [_I, _I, _I],
     "llm_moe_grouped": [_P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _F, _F, _F, _S],
     "llm_moe_grouped_tc_supports": [_I, _I, _I],

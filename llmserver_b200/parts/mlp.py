@@ -160,7 +160,7 @@ class ClampedGLU(FeedForward):
         self.limit, self.alpha = float(params["limit"]), float(params.get("alpha", 1.702))
 
     def forward(self, x):
-        return ops.linear(ops.clamped_glu(ops.linear(x, self.gate_up), self.limit, self.alpha), self.down)
+        return ops.linear(ops.clamped_gate_up(x, self.gate_up, self.limit, self.alpha), self.down)
 
 
 @FEED_FORWARDS.register("squared_relu")

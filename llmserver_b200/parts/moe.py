@@ -155,6 +155,10 @@ class RoutedExperts(FeedForward):
                         and self.gate_up.shape[2] % 64 == 0 and self.down.shape[2] % 64 == 0)
 
     GROUPED_FROM = 16     # tokens from which pairs are sorted and multiplied tile by tile
+    # (token, expert) pairs per expert from which pairs of SMs make tiles of 256 rows: the tiles of 128 rows that single SMs make
+    # read W once per 128 rows.  Prompts of 64 experts of 1792 with 6 per token: 3.47 ms on tiles of 128 and 4.12 on tiles of 256
+    # at 1024 tokens (96 pairs per expert fit one tile of 128), 5.43 and 5.00 at 2048 (192), 9.66 and 9.37 at 4096 (384)
+    PAIR_TILES_FROM = 160
 
     def forward(self, x):
         tokens = x.shape[0]
@@ -170,13 +174,12 @@ class RoutedExperts(FeedForward):
         elif self.shared_gate_up is not None and self.params.get("activation") == "silu":
             shared = ops.linear(ops.gate_up_silu(x, self.shared_gate_up, self.shared_group), self.shared_down)
         elif self.shared_gate_up is not None:
-            shared = ops.linear(ops.clamped_glu(ops.linear(x, self.shared_gate_up), self.shared_limit, self.alpha),
-                                self.shared_down)
+            shared = ops.linear(ops.clamped_gate_up(x, self.shared_gate_up, self.shared_limit, self.alpha), self.shared_down)
         on_input = weights.view(-1) if self.weight_on_input else None
         if self.weight_on_input:
             weights = self._ones(weights)       # the weights act on the way in; on the way out the outputs are summed
         if self.grouped and tokens >= self.GROUPED_FROM:
-            plan = ops.moe_plan(chosen, self.experts)
+            plan = ops.moe_plan(chosen, self.experts, ops.MOE_PAIR_TILE_ROWS if tokens * self.top >= self.PAIR_TILES_FROM * self.experts else ops.MOE_TILE_ROWS)
             hidden = ops.moe_grouped(x, self.gate_up, plan, gather_div=self.top, gated=self.gate, pair_scale=on_input,
                                      squared_relu=self.squared_relu)
             down = ops.moe_grouped(hidden, self.down, plan)
