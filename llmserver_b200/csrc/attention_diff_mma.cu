@@ -15,6 +15,9 @@
 // in shared memory; one warp per row merges the splits, subtracts the maps, normalises the head, applies the gate and
 // stores.
 //
+// Maps of 64 with values of 128 run the tcgen05 prompt kernel and the TMA decode kernel instead (llm_attention_diff_prefill,
+// llm_attention_diff_decode) wherever those take the pages and the group, with attention_diff_combine_kernel behind them.
+//
 // Sizes: units of 64 or 128 elements per map, values of 64 or 128; any group, window, page size (pages need not
 // align with tiles: every key's page is looked up).  Other sizes run attention_diff.cu.
 #include "common.cuh"
@@ -444,7 +447,45 @@ int launch_diff(const DiffParams& p, int n_seqs, int max_q_len, cudaStream_t str
     return llm_check_launch("attention_diff_mma");
 }
 
+// One warp per (token, head): o = a_1 - lambda a_2 of the maps that the tcgen05 prompt kernel and the TMA decode kernel leave as
+// 32-bit numbers, the head norm, the gate, one rounding.  Four elements a lane; it reads 8 bytes per byte that it writes.
+__global__ void attention_diff_combine_kernel(const float* __restrict__ maps, DiffParams p, int total) {
+    pdl_trigger();
+    pdl_wait();
+    const int index = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (index >= total) return;
+    const float4 one = *reinterpret_cast<const float4*>(maps + (size_t)index * 256 + lane * 4);
+    const float4 two = *reinterpret_cast<const float4*>(maps + (size_t)index * 256 + 128 + lane * 4);
+    const float o[4] = {one.x - p.lambda * two.x, one.y - p.lambda * two.y, one.z - p.lambda * two.z, one.w - p.lambda * two.w};
+    float factor = rsqrtf(warp_sum(o[0] * o[0] + o[1] * o[1] + o[2] * o[2] + o[3] * o[3]) / 128.0f + p.eps) * p.out_scale;
+    if (p.gate) {
+        const float g = __bfloat162float(p.gate[(size_t)(index / p.n_q_heads) * p.gate_stride + index % p.n_q_heads]);
+        factor *= 1.0f / (1.0f + __expf(-g));
+    }
+    uint2 packed;
+    packed.x = pack_pair(o[0] * factor, o[1] * factor);
+    packed.y = pack_pair(o[2] * factor, o[3] * factor);
+    *reinterpret_cast<uint2*>(p.out + (size_t)index * 128 + lane * 4) = packed;
+}
+
 }  // namespace
+
+// out[n, h] = rms-normalised (maps[n, h, 0] - lambda maps[n, h, 1]) * out_scale * sigmoid(gate[n, h]); maps float32 [N, heads, 2,
+// 128], out bfloat16 [N, heads * 128], gate (may be null) bfloat16 with rows gate_stride apart.
+LLM_EXPORT int llm_attention_diff_combine(const float* maps, const void* gate, int gate_stride, void* out, int n_tokens, int n_q_heads,
+                                          float lambda, float eps, float out_scale, cudaStream_t stream) {
+    if (n_tokens == 0) return LLM_OK;
+    if (!aligned16(maps) || !aligned16(out) || (long long)n_tokens * n_q_heads > 0x7fffffffLL) {
+        llm_set_error("attention_diff_combine: maps and output must be 16-byte aligned (%d tokens, %d heads)", n_tokens, n_q_heads);
+        return LLM_REFUSED;
+    }
+    DiffParams p = {};
+    p.gate = (const __nv_bfloat16*)gate; p.gate_stride = gate_stride; p.out = (__nv_bfloat16*)out; p.n_q_heads = n_q_heads;
+    p.lambda = lambda; p.eps = eps; p.out_scale = out_scale;
+    const int total = n_tokens * n_q_heads;
+    llm_launch(attention_diff_combine_kernel, dim3((total + 7) / 8), 256, 0, stream, maps, p, total);
+    return llm_check_launch("attention_diff_combine");
+}
 
 LLM_EXPORT int llm_attention_diff_mma_supports(int dim, int value_dim, int n_q_heads, int n_kv_heads) {
     return (dim == 64 || dim == 128) && (value_dim == 64 || value_dim == 128) && n_kv_heads > 0 && n_q_heads % n_kv_heads == 0;

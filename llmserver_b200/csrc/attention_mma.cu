@@ -80,6 +80,8 @@ struct AttnParams {
     int keep = 0;                   // with a window: keys 0 .. keep - 1 stay visible; PRECISE kernels only
     const __nv_bfloat16* gate = nullptr;    // row of token n from gate + n * gate_stride on, [Hq * DV]: results are multiplied
     int gate_stride = 0;                    // by its sigmoid; PRECISE kernels and their merge only
+    float* maps_out = nullptr;      // DIFF: [N, Hq, D], 32-bit, in place of `out`
+    float cap_log2 = 0.0f, cap_slope = 0.0f;    // CAP: cap * log2(e) (0: scores are not capped), 2 * scale / cap * log2(e)
     int by_length = 0;              // TMA decode kernel: blocks take the sequences longest first (up to kThreads of them)
 };
 
@@ -289,12 +291,13 @@ __device__ __forceinline__ void load_kv_tile(__nv_bfloat16* k_tile, __nv_bfloat1
 //
 // DV: the size of a value row (V tiles are laid out by VLayout).  PRECISE: each probability enters the P V product as
 // two bfloat16 numbers, its rounding and the rounding of the rest, so the weights keep 16 significant bits.
-template <int D, int NT, class Layout = XorLayout<D>, int DV = D, bool PRECISE = false, class VLayout = Layout, bool BIAS = false>
+template <int D, int NT, class Layout = XorLayout<D>, int DV = D, bool PRECISE = false, class VLayout = Layout, bool BIAS = false, bool CAP = false>
 __device__ __forceinline__ void warp_tile(const uint32_t (&q_frag)[D / 16][4], const __nv_bfloat16* k_tile,
                                           const __nv_bfloat16* v_tile, int key_row, int key_index,
                                           const int (&row_low)[2], const int (&row_high)[2], float scale_log2,
                                           float (&o_acc)[DV / 8][4], float (&row_max)[2], float (&row_sum)[2],
-                                          const float* const* bias_row = nullptr, int bias_last = 0, int keep = 0) {
+                                          const float* const* bias_row = nullptr, int bias_last = 0, int keep = 0,
+                                          float cap_log2 = 0.0f, float cap_slope = 0.0f) {
     const int lane = threadIdx.x & 31;
     const int matrix = lane >> 3, matrix_row = lane & 7;
     float s_acc[NT][4];
@@ -327,6 +330,8 @@ __device__ __forceinline__ void warp_tile(const uint32_t (&q_frag)[D / 16][4], c
             const int key = key_index + n * 8 + 2 * t + (i & 1);
             const bool seen = (key >= row_low[h] || key < keep) && key <= row_high[h];
             if (BIAS) s_acc[n][i] = seen ? fmaf(s_acc[n][i], scale_log2, bias_row[h][min(row_high[h] - key, bias_last)]) : -INFINITY;
+            else if (CAP && cap_log2 > 0.0f)      // cap * tanh(s / cap) as cap * (1 - 2 / (exp(2 s / cap) + 1))
+                s_acc[n][i] = seen ? fmaf(__fdividef(-2.0f, exp2f(s_acc[n][i] * cap_slope) + 1.0f), cap_log2, cap_log2) : -INFINITY;
             else s_acc[n][i] = seen ? s_acc[n][i] * scale_log2 : -INFINITY;
             tile_max[h] = fmaxf(tile_max[h], s_acc[n][i]);
         }
@@ -727,7 +732,12 @@ __device__ __forceinline__ int longest_first(const AttnParams& p, int place, int
     return *answer;
 }
 
-template <int D, bool PRECISE = false>
+// DIFF: the heads of differential attention are [map 1 | map 2] of D / 2 elements each in Q and in the K rows, and every map of a
+// head is a row of the tile: its own half of the query, zeros in the other half, so that one product over whole K rows gives the
+// row's own map.  `n_q_heads` then counts maps (two per head), and results leave as 32-bit numbers for the kernel that subtracts
+// the maps.  64 sequences over a window of 1024 keys (32 / 8 heads) took 101 us in blocks of warps that each load keys of their own; a
+// decode step with two such layers went from 1193 to 1111 us.
+template <int D, bool PRECISE = false, bool DIFF = false>
 __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                               const __grid_constant__ CUtensorMap map_v,
                                                                               const AttnParams p) {
@@ -779,7 +789,12 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
     if (n_splits > p.max_splits && split == 0 && kv_head == 0 && threadIdx.x == 0 && p.error_flag) atomicExch(p.error_flag, 6);
     if (context <= 0 && split == 0) {       // nothing to attend to
         if (early) pdl_wait();
-        zero_output<D>(p, token, kv_head, group);
+        if constexpr (DIFF) {
+            for (int index = threadIdx.x; index < group * D; index += blockDim.x)
+                p.maps_out[(size_t)token * p.n_q_heads * D + (size_t)(kv_head * group) * D + index] = 0.0f;
+        } else {
+            zero_output<D>(p, token, kv_head, group);
+        }
     }
     // every thread of a cluster whose splits merge in shared memory meets at the same two cluster barriers, also the
     // blocks beyond the sequence's last split and the producer warps, which have nothing to add
@@ -867,8 +882,12 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
         for (int c = threadIdx.x; c < 16 * kChunks; c += kThreads) {
             const int row = c / kChunks, chunk = c % kChunks;
             uint4 value = make_uint4(0, 0, 0, 0);
-            if (row < group)
+            if (DIFF) {
+                if (row < group && chunk / (kChunks / 2) == (row & 1))
+                    value = *reinterpret_cast<const uint4*>(p.q + (size_t)token * p.q_stride + (size_t)(kv_head * group + row) * (D / 2) + chunk % (kChunks / 2) * 8);
+            } else if (row < group) {
                 value = *reinterpret_cast<const uint4*>(p.q + (size_t)token * p.q_stride + (size_t)(kv_head * group + row) * D + chunk * 8);
+            }
             *reinterpret_cast<uint4*>(q_tile + swizzled<D>(row, chunk)) = value;
         }
     }
@@ -905,21 +924,23 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
         const __nv_bfloat16* v_tile = one_copy ? k_tile : k_tile + kTileKeys * D;
         const int key_index = walk_key(walk, first_tile + it) + warp * 16;
         if constexpr (PRECISE) {
-            // rows behind the context hold whatever lay in the page: a weight of zero does not erase a value that is not finite
-            // (only the sequence's last tile has such rows, and its stage is not filled again)
-            if (key_index < context && key_index + 16 > context) {
+            // rows behind the context, and rows of pages that a window has given back, hold whatever lay in the page: a weight
+            // of zero does not erase a value that is not finite
+            const bool hidden_rows = key_index + 16 > context || (key_index < low_key && key_index + 16 > p.keep);
+            if (key_index < context && hidden_rows) {
                 __nv_bfloat16* rows = const_cast<__nv_bfloat16*>(v_tile);
                 for (int c = lane; c < 16 * (D / 8); c += 32) {
-                    const int row = warp * 16 + c / (D / 8);
-                    if (key_index - warp * 16 + row >= context)
+                    const int row = warp * 16 + c / (D / 8), key = key_index - warp * 16 + row;
+                    if (key >= context || (key < low_key && key >= p.keep))
                         *reinterpret_cast<uint4*>(rows + Layout::at(row, c % (D / 8))) = make_uint4(0, 0, 0, 0);
                 }
+                tma::fence_proxy_async();      // the stage may be filled again
                 __syncwarp();
             }
         }
         if (key_index < context)
-            warp_tile<D, 2, Layout, D, PRECISE>(q_frag, k_tile, v_tile, warp * 16, key_index, row_low, row_high, p.scale_log2, o_acc, row_max,
-                                                row_sum, nullptr, 0, PRECISE ? p.keep : 0);
+            warp_tile<D, 2, Layout, D, PRECISE, Layout, false, DIFF>(q_frag, k_tile, v_tile, warp * 16, key_index, row_low, row_high, p.scale_log2, o_acc, row_max,
+                                                                     row_sum, nullptr, 0, PRECISE ? p.keep : 0, p.cap_log2, p.cap_slope);
         __syncwarp();
         if (lane == 0) tma::mbar_arrive(tma::smem_u32(&empty_bar[s]));     // this warp is done with the stage
     }
@@ -988,8 +1009,9 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
                         result[1] = gated(p, result[1], token, head * D + d + 1);
                     }
                 }
-                *reinterpret_cast<__nv_bfloat162*>(p.out + (size_t)token * p.n_q_heads * D + (size_t)head * D + d) =
-                    __floats2bfloat162_rn(result[0], result[1]);
+                const size_t at = (size_t)token * p.n_q_heads * D + (size_t)head * D + d;
+                if constexpr (DIFF) *reinterpret_cast<float2*>(p.maps_out + at) = make_float2(result[0], result[1]);
+                else *reinterpret_cast<__nv_bfloat162*>(p.out + at) = __floats2bfloat162_rn(result[0], result[1]);
             } else if (in_cluster) {
                 *reinterpret_cast<float2*>(mine + r * (D + 2) + d) = make_float2(numerator[0] / denominator, numerator[1] / denominator);
             } else {
@@ -1050,7 +1072,9 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
             if constexpr (PRECISE) {
                 if (p.gate) result = gated(p, result, token, (kv_head * group + r) * D + d);
             }
-            p.out[(size_t)token * p.n_q_heads * D + (size_t)(kv_head * group + r) * D + d] = __float2bfloat16_rn(result);
+            const size_t at = (size_t)token * p.n_q_heads * D + (size_t)(kv_head * group + r) * D + d;
+            if constexpr (DIFF) p.maps_out[at] = result;
+            else p.out[at] = __float2bfloat16_rn(result);
         }
         if (!arrived) cluster_arrive();
         cluster_wait();      // nobody leaves while another rank may still read its shared memory
@@ -1083,7 +1107,9 @@ __global__ void attention_decode_merge_kernel(const AttnParams p) {
         }
         float value = numerator / denominator;
         if (p.gate) value = gated(p, value, token, head * D + d);
-        p.out[(size_t)token * p.n_q_heads * D + (size_t)head * D + d] = __float2bfloat16_rn(value);
+        const size_t at = (size_t)token * p.n_q_heads * D + (size_t)head * D + d;
+        if (p.maps_out) p.maps_out[at] = value;
+        else p.out[at] = __float2bfloat16_rn(value);
     }
 }
 
@@ -1124,10 +1150,10 @@ int launch_decode_cp_async(const AttnParams& given, cudaStream_t stream) {
     return llm_check_launch("attention_decode");
 }
 
-template <int D, bool PRECISE>
+template <int D, bool PRECISE, bool DIFF>
 int launch_decode_tma(const AttnParams& given, cudaStream_t stream) {
     AttnParams p = given;
-    auto* kernel = attention_decode_tma_kernel<D, PRECISE>;
+    auto* kernel = attention_decode_tma_kernel<D, PRECISE, DIFF>;
     // Two blocks share an SM.  Beyond one wave of them the order in which sequences start decides how raggedly the last wave
     // ends: 61 sequences of 301 to 4077 keys that lie shortest first, a decode step of the 8B shape 7.51 ms as they lie and
     // 6.70 ms longest first (more splits instead: 7.3 ms with two parts, 7.8 with three).  Within a wave all start at once.
@@ -1144,6 +1170,10 @@ int launch_decode_tma(const AttnParams& given, cudaStream_t stream) {
     } else {
         described = tma::make_map_bf16(&map_k, p.k_pages, rows, D, (uint32_t)p.page_size) &&
                     tma::make_map_bf16(&map_v, p.v_pages, rows, D, (uint32_t)p.page_size);
+    }
+    if (!described && DIFF) {
+        llm_set_error("attention_diff_decode: cannot describe the cache pages to TMA");
+        return LLM_REFUSED;
     }
     if (!described) return launch_decode_cp_async<D, D, PRECISE>(p, stream);
     const size_t shared = (size_t)kDecodeStages * 2 * kTileKeys * D * 2 + (size_t)16 * D * 2 + 1024;
@@ -1192,7 +1222,7 @@ int launch_decode_tma(const AttnParams& given, cudaStream_t stream) {
     return llm_check_launch("attention_decode_tma");
 }
 
-template <int D, bool PRECISE = false>
+template <int D, bool PRECISE = false, bool DIFF = false>
 int launch_decode(const AttnParams& p, cudaStream_t stream) {
     const bool whole_pages = p.page_size >= 8 && p.page_size <= kTileKeys && kTileKeys % p.page_size == 0 && p.page_size % 8 == 0;
     const bool by_tma = whole_pages && aligned16(p.k_pages) && aligned16(p.v_pages);
@@ -1204,7 +1234,11 @@ int launch_decode(const AttnParams& p, cudaStream_t stream) {
         llm_set_error("attention_decode: %d splits need the scratch buffers for partial results", p.max_splits);
         return LLM_REFUSED;
     }
-    int status = by_tma ? launch_decode_tma<D, PRECISE>(q, stream) : launch_decode_cp_async<D, D, PRECISE>(q, stream);
+    if (DIFF && !by_tma) {
+        llm_set_error("attention_diff_decode: pages of %d tokens are not supported", p.page_size);
+        return LLM_REFUSED;
+    }
+    int status = by_tma ? launch_decode_tma<D, PRECISE, DIFF>(q, stream) : launch_decode_cp_async<D, D, PRECISE>(q, stream);
     if (status != LLM_OK || p.max_splits <= 1 || q.cluster_merge) return status;
     dim3 merge_grid(p.n_q_heads, p.n_seqs);
     llm_launch(attention_decode_merge_kernel<D>, merge_grid, D < 128 ? D : 128, 0, stream, p);
@@ -1523,4 +1557,50 @@ LLM_EXPORT int llm_attention_mma_sinks(const void* q, int q_stride, const void* 
     if (bias) LLM_PRECISE(true);
     LLM_PRECISE(false);
 #undef LLM_PRECISE
+}
+
+// Both maps of differential attention for a step of single tokens: maps_out (float32 [N, n_q_heads, 2, 128]) gets
+// softmax(cap(q_m . k_m * scale)) V of each head and map.  A head of the queries and of the K pages is [map 1 | map 2] of 64
+// elements each, values have 128; groups of up to 8 heads; pages as the TMA decode kernel takes them.  partial_out holds
+// [N, 2 n_q_heads, max_splits, 128] floats.  The other arguments as for llm_attention_mma.
+LLM_EXPORT int llm_attention_diff_decode(const void* q, int q_stride, const void* k_pages, const void* v_pages, const int* block_tables,
+                                         int max_blocks, const int* q_start, const int* context_len, float* maps_out, int n_seqs,
+                                         int n_q_heads, int n_kv_heads, int page_size, int num_pages, float scale, float cap, int window,
+                                         int split_len, int max_splits, float* partial_out, float* partial_ml, int old_keys_settled,
+                                         int* error_flag, cudaStream_t stream) {
+    if (n_kv_heads <= 0 || n_q_heads % n_kv_heads || n_q_heads / n_kv_heads > 8 || n_seqs > 65535 || n_kv_heads > 65535 || num_pages <= 0 ||
+        split_len == 0 || (split_len > 0 && split_len % kTileKeys) || max_splits <= 0 || -split_len > max_splits || cap < 0.0f ||
+        !aligned16(q) || q_stride % 8) {
+        llm_set_error("attention_diff_decode: %d/%d heads, splits of %d (at most %d) are not supported", n_q_heads, n_kv_heads, split_len, max_splits);
+        return LLM_REFUSED;
+    }
+    AttnParams p = {};
+    p.q = (const __nv_bfloat16*)q;
+    p.q_stride = q_stride;
+    p.k_pages = (const __nv_bfloat16*)k_pages;
+    p.v_pages = (const __nv_bfloat16*)v_pages;
+    p.block_tables = block_tables;
+    p.max_blocks = max_blocks;
+    p.num_pages = num_pages;
+    p.q_start = q_start;
+    p.context_len = context_len;
+    p.n_seqs = n_seqs;
+    p.n_q_heads = 2 * n_q_heads;      // maps
+    p.n_kv_heads = n_kv_heads;
+    p.page_size = page_size;
+    p.scale_log2 = scale * kLog2e;
+    p.window = window;
+    p.split_len = split_len;
+    p.max_splits = max_splits;
+    p.partial_out = partial_out;
+    p.partial_ml = partial_ml;
+    p.old_keys_settled = old_keys_settled;
+    p.cluster_merge = decode_cluster_merge_enabled() ? 1 : 0;
+    p.error_flag = error_flag;
+    p.maps_out = maps_out;
+    if (cap > 0.0f) {
+        p.cap_log2 = cap * kLog2e;
+        p.cap_slope = 2.0f * scale / cap * kLog2e;
+    }
+    return launch_decode<128, true, true>(p, stream);
 }

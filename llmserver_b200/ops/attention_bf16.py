@@ -278,7 +278,9 @@ def try_attention_precise(qkv, q_stride, batch, block_tables, k_pages, v_pages, 
     return out
 
 
-DIFF_KERNEL = os.environ.get("LLMSERVER_B200_DIFF_ATTENTION", "mma")      # "generic": always the kernel that takes every size
+# "tcgen05": maps of 64 with values of 128 on the tcgen05 prompt kernel and the TMA decode kernel; "mma": the tiled mma.sync kernel
+# for all sizes that it takes; "generic": always the kernel that takes every size
+DIFF_KERNEL = os.environ.get("LLMSERVER_B200_DIFF_ATTENTION", "tcgen05")
 # row tiles per block of the tiled kernel: 0 = by the step (2, and 2 key splits, with prompt portions; 1 and 4 key splits
 # for single tokens); 1, 2 or 4 force an arrangement
 DIFF_ROW_TILES = int(os.environ.get("LLMSERVER_B200_DIFF_ROW_TILES", "0"))
@@ -290,15 +292,20 @@ def try_attention_diff(qkv, gate_column, batch, block_tables, k_pages, v_pages, 
     rows of the packed projection 16-byte aligned); False when it does not (the caller then runs the kernel that takes
     every size).  Prompt portions and single tokens go in one launch."""
     row_width = qkv.shape[1]
-    if DIFF_KERNEL != "mma" or row_width % 8 or not library().llm_attention_diff_mma_supports(dim, value_dim, n_q_heads, n_kv_heads):
+    if DIFF_KERNEL == "generic" or row_width % 8 or not library().llm_attention_diff_mma_supports(dim, value_dim, n_q_heads, n_kv_heads):
         return False
     check(qkv, "qkv", torch.bfloat16)
     gate = 0 if gate_column is None else qkv.data_ptr() + gate_column * qkv.element_size()
+    group = n_q_heads // n_kv_heads
+    if DIFF_KERNEL == "tcgen05" and DIFF_ROW_TILES == 0 and dim == 64 and value_dim == 128 and group <= 8 and scale > 0.0 and \
+            qkv.data_ptr() % 16 == 0 and decode_by_tma(k_pages, v_pages):
+        _attention_diff_maps(qkv, gate, batch, block_tables, k_pages, v_pages, n_q_heads, n_kv_heads, scale, cap, window, lam, eps, out_scale, out)
+        return True
     # A step of single tokens has few (sequence, key/value head) pairs: several blocks then share a pair's keys, four
     # warp splits each, and leave partial results that a merge kernel adds up.  The count is a function of the batch's
     # host-side shape (so a captured graph keeps it): about four key tiles of 16 per warp, at most 16 blocks a pair,
     # and no more blocks than fill the GPU twice.
-    block_splits, partials, group = 1, None, n_q_heads // n_kv_heads
+    block_splits, partials = 1, None
     if batch.max_q_len == 1 and group <= 16 and DIFF_ROW_TILES in (0, 1):
         span = min(int(window), batch.max_context) if window else batch.max_context
         wanted = -(-span // (16 * 4 * 4))
@@ -318,3 +325,40 @@ def try_attention_diff(qkv, gate_column, batch, block_tables, k_pages, v_pages, 
          wait_error_flag(qkv.device).data_ptr(), DIFF_ROW_TILES, block_splits, 0 if partials is None else partials.data_ptr(),
          stream_handle())
     return True
+
+
+def _attention_diff_maps(qkv, gate, batch, block_tables, k_pages, v_pages, n_q_heads, n_kv_heads, scale, cap, window, lam, eps,
+                         out_scale, out) -> None:
+    """Differential attention as attention with each of the maps (32-bit results), then one kernel that subtracts them: prompt portions
+    (and single tokens beside them) on the tcgen05 kernel, steps of single tokens on the TMA decode kernel."""
+    row_width, group, page_size = qkv.shape[1], n_q_heads // n_kv_heads, k_pages.shape[2]
+    window, flag = int(window or 0), wait_error_flag(qkv.device).data_ptr()
+    maps = torch.empty((batch.n_tokens, n_q_heads, 2, 128), dtype=torch.float32, device=qkv.device)
+    if batch.max_q_len == 1:
+        _, _, _, split_len, max_splits = plan(batch, group, n_kv_heads, qkv.device, span=window or None)
+        partial_out = partial_ml = None
+        if max_splits > 1:
+            key = ("attention_diff_scratch", n_q_heads, max_splits)
+            if key not in batch.scratch:
+                batch.scratch[key] = (torch.empty((batch.n_tokens, 2 * n_q_heads, max_splits, 128), dtype=torch.float32, device=qkv.device),
+                                      torch.empty((batch.n_tokens, 2 * n_q_heads, max_splits, 2), dtype=torch.float32, device=qkv.device))
+            partial_out, partial_ml = batch.scratch[key]
+        call("llm_attention_diff_decode", qkv.data_ptr(), row_width, k_pages.data_ptr(), v_pages.data_ptr(), block_tables.data_ptr(),
+             block_tables.shape[-1], batch.q_start.data_ptr(), batch.context_len.data_ptr(), maps.data_ptr(), batch.n_seqs, n_q_heads,
+             n_kv_heads, page_size, k_pages.shape[0], float(scale), float(cap or 0.0), window, split_len, max_splits,
+             0 if partial_out is None else partial_out.data_ptr(), 0 if partial_ml is None else partial_ml.data_ptr(),
+             int(EARLY_KEYS and getattr(batch, "keys_settled", False)), flag, stream_handle())
+    else:
+        # as for the other portions, but a row tile is two blocks, one per map
+        tile_counts = [-(-length // (PREFILL_TILE // group)) for length in batch.q_lens]
+        paired = sum((count + 1) // 2 for count in tile_counts)
+        slots = _block_slots(qkv.device, False)
+        cost_paired = 2.0 * -(-paired * 2 * n_kv_heads // slots)
+        cost_single = 1.3 * max(sum(tile_counts) * 2 * n_kv_heads / slots, 1.0)
+        pairing = cost_paired < cost_single if FORCE_PAIRING is None else FORCE_PAIRING
+        call("llm_attention_diff_prefill", qkv.data_ptr(), row_width, batch.n_tokens, k_pages.data_ptr(), v_pages.data_ptr(),
+             block_tables.data_ptr(), block_tables.shape[-1], batch.q_start.data_ptr(), batch.context_len.data_ptr(), maps.data_ptr(),
+             batch.n_seqs, n_q_heads, n_kv_heads, page_size, k_pages.shape[0], float(scale), float(cap or 0.0), window, int(pairing),
+             paired if pairing else sum(tile_counts), flag, stream_handle())
+    call("llm_attention_diff_combine", maps.data_ptr(), gate, row_width, out.data_ptr(), batch.n_tokens, n_q_heads, float(lam), float(eps),
+         float(out_scale), stream_handle())
