@@ -1,10 +1,10 @@
-// y[M, N] = x[M, K] * W[N, K]^T in bfloat16 with 32-bit accumulation, for few rows (M <= 64: decode steps
-// and the output head), written for the fifth-generation tensor cores: TMA loads into 128-byte-swizzled
+// y[M, N] = x[M, K] * W[N, K]^T in bfloat16 with 32-bit accumulation, for few rows (M <= 128: decode steps, short
+// prompts and the output head), written for the fifth-generation tensor cores: TMA loads into 128-byte-swizzled
 // shared tiles, tcgen05.mma with the accumulator in tensor memory, tcgen05.ld for the epilogue.
 //
 // With few rows the product is a stream of W through the SM: every weight is read once and used M times.
 // So the roles of the operands are swapped for the hardware: a CTA owns 128 rows of W as the MMA's
-// M = 128 dimension and the (padded) token rows as its N dimension (16..64), walks its share of K in
+// M = 128 dimension and the (padded) token rows as its N dimension (16..128), walks its share of K in
 // blocks of 64 through a ring of shared-memory stages, and ends with a 128 x M tile of y^T in tensor
 // memory, which the epilogue writes transposed.  When N / 128 tiles are too few to fill 148 SMs, K is
 // split across a thread-block cluster; the partial tiles are added through distributed shared memory in
@@ -46,8 +46,9 @@ namespace {
 
 constexpr int kBlockRows = 128;     // rows of W per CTA (UMMA M)
 constexpr int kAtomK = 64;          // one 128-byte swizzle atom of bfloat16
-constexpr int kAtoms = 2;           // atoms per pipeline stage
-constexpr int kBlockK = kAtomK * kAtoms;
+constexpr int kMaxRows = 128;       // tokens per launch
+constexpr int kTwoAtomRows = 64;    // up to this many tokens a pipeline stage holds two atoms of K, beyond (where a token atom is as
+                                    // large as a weight atom) one: three stages of 32 KiB then leave room for two blocks per SM
 constexpr int kThreads = 256;       // at most: four warps up to 16 tokens, eight beyond (two have a role in the main
                                     // loop, all work in the epilogue, whose time per token is instruction issue)
 constexpr int kMaxStages = 12;
@@ -342,6 +343,9 @@ __device__ __forceinline__ void stream_finish(const GemmParams& p, int m, int la
     }
 }
 
+// MANY: more than 16 tokens, eight warps; a warp finishes several tokens.  What it does for the second and later ones costs the
+// steps of few tokens 0.5 us a launch (a batch-8 step of the 8B shape 3.64 against 3.55 ms), so they run a form without it.
+template <int kAtoms, bool MANY>
 __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                 const __grid_constant__ CUtensorMap map_x,
                                                                 const GemmParams p) {
@@ -349,20 +353,21 @@ __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_con
     // them + this + 1 KiB that the system reserves = 75 KiB, and three blocks share an SM (225 of 227 KiB): two of this
     // kernel and one of the next, whose weights are then on their way while this kernel still runs.  With 2 KiB more
     // only two fit: a decode step of the 8B shape then took 4.23 ms instead of 3.67.
+    constexpr int kBlockK = kAtomK * kAtoms;
     extern __shared__ __align__(1024) unsigned char shared_raw[];
     __shared__ __align__(8) uint64_t full_bar[kMaxStages];
     __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
     __shared__ __align__(8) uint64_t accum_bar;
     __shared__ uint32_t tmem_base_slot;
     __shared__ int failed;
-    __shared__ float row_scale[64];                 // RowScale: 1 / rms of each token's stream row
+    __shared__ float row_scale[kMaxRows];                 // RowScale: 1 / rms of each token's stream row
 
     // the dynamic region is aligned to 1024 bytes by hand (the swizzle atoms need it)
     const uint32_t raw = smem_u32(shared_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* aligned = shared_raw + (base - raw);
     const uint32_t a_bytes = kBlockRows * kAtomK * 2;                 // 16 KiB per atom of W
-    const uint32_t b_bytes = (uint32_t)p.token_pad * kAtomK * 2;      // 2..8 KiB per atom of tokens
+    const uint32_t b_bytes = (uint32_t)p.token_pad * kAtomK * 2;      // 2..16 KiB per atom of tokens
     const uint32_t b_pitch = (b_bytes + 1023u) & ~1023u;
     const uint32_t b_offset = kAtoms * a_bytes;                       // token atoms follow the W atoms of a stage
     const uint32_t stage_bytes = b_offset + kAtoms * b_pitch;
@@ -396,8 +401,9 @@ __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_con
                 tma_load_2d(base + i * stage_bytes + atom * a_bytes, &map_w, bar, (kb_begin + i) * kBlockK + atom * kAtomK, n0);
         }
     }
-    if (warp == 1) {   // this warp owns the tensor-memory allocation (64 columns: up to 64 token columns of float)
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(64));
+    const uint32_t tmem_cols = p.token_pad > 64 ? 128 : 64;      // one column of floats per token
+    if (warp == 1) {   // this warp owns the tensor-memory allocation
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(tmem_cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -456,14 +462,27 @@ __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_con
         }
         umma_commit(smem_u32(&accum_bar));            // the accumulator is complete once all MMAs are done
     } else if (warp >= 2 && p.scale.parts != nullptr) {
-        // ---- the two warps without a role in the main loop add the sums of squares, in an order that depends on
+        // ---- the warps without a role in the main loop add the sums of squares, in an order that depends on
         // the number of parts only, and leave 1 / rms per token for the epilogue
         pdl_wait();
-        for (int m = warp - 2; m < p.m; m += n_warps - 2) {
-            float squares = 0.0f;
-            for (int i = lane; i < p.scale.n_parts; i += 32) squares += p.scale.parts[(size_t)i * p.scale.stride + m];
-            squares = warp_sum(squares);
-            if (lane == 0) row_scale[m] = rsqrtf(squares / (float)p.k + p.scale.eps);
+        if (MANY) {      // a lane per token: its parts are independent loads, where a warp per token waits for memory token by token
+            const int m = (warp - 2) * 32 + lane;
+            if (m < p.m) {
+                float squares[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+                for (int i = 0; i < p.scale.n_parts; i += 4)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (i + c < p.scale.n_parts) squares[c] += p.scale.parts[(size_t)(i + c) * p.scale.stride + m];
+                row_scale[m] = rsqrtf(((squares[0] + squares[1]) + (squares[2] + squares[3])) / (float)p.k + p.scale.eps);
+            }
+        } else {
+            for (int m = warp - 2; m < p.m; m += n_warps - 2) {
+                float squares = 0.0f;
+                for (int i = lane; i < p.scale.n_parts; i += 32) squares += p.scale.parts[(size_t)i * p.scale.stride + m];
+                squares = warp_sum(squares);
+                if (lane == 0) row_scale[m] = rsqrtf(squares / (float)p.k + p.scale.eps);
+            }
         }
     }
 
@@ -531,7 +550,7 @@ __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_con
     // given back now, so that nothing but the rows' results stands between a warp and its exit
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(64));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols));
     }
 
     // Lane i finishes elements 4 i .. 4 i + 3 of the tile for its warp's tokens, one token after the other.
@@ -539,7 +558,11 @@ __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_con
     const uint32_t parts_address = smem_u32(parts_tile);
     bool arrived = false;
     for (int m = first_token; m < p.m; m += token_step) {
-        if (m != first_token) token_inputs(p, m, tile, n4, info, before);
+        // MANY: the next token's inputs are asked for before this one's are used (three dependent loads for a page)
+        RopeRow next_info;
+        float next_before[4];
+        if (MANY) token_inputs(p, m + token_step, tile, n4, next_info, next_before);
+        else if (m != first_token) token_inputs(p, m, tile, n4, info, before);
         // the ranks' parts of the token, all asked for before the first is used, added in the order of the ranks
         float4 parts[kMaxSplit];
 #pragma unroll
@@ -579,6 +602,11 @@ __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_con
             if (p.out_is_f32) store4_f32(reinterpret_cast<float*>(p.out) + (size_t)m * p.ldc + n4, total, p.n - n4, p.vector_out != 0);
             else store4_bf16(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)m * p.ldc + n4, total, p.n - n4, p.vector_out != 0);
         }
+        if (MANY) {
+            info = next_info;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) before[c] = next_before[c];
+        }
     }
     if (p.split > 1) {          // nobody leaves while a peer may still read its shared memory
         if (!arrived) cluster_arrive();
@@ -595,7 +623,7 @@ bool make_map(CUtensorMap* map, const void* pointer, int rows, int k, int box_ro
 
 // 1 when the kernel takes the sizes, else 0 (the caller then uses the library product).
 LLM_EXPORT int llm_gemm_small_m_supports(int m, int n, int k) {
-    return m >= 1 && m <= 64 && n >= 1 && k >= 8 && k % 8 == 0;
+    return m >= 1 && m <= kMaxRows && n >= 1 && k >= 8 && k % 8 == 0;
 }
 
 static RowScale row_scale_of(const float* parts, int n_parts, int stride, float eps) {
@@ -612,7 +640,7 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
                           int silu_gate, const RowScale& scale, const StreamEpilogue* stream_out = nullptr) {
     if (m == 0 || n == 0) return LLM_OK;
     if (!llm_gemm_small_m_supports(m, n, k) || !aligned16(x) || !aligned16(w)) {
-        llm_set_error("gemm_small_m: takes 1..64 rows, K a multiple of 8 and 16-byte aligned operands (got m %d, n %d, k %d)", m, n, k);
+        llm_set_error("gemm_small_m: takes 1..128 rows, K a multiple of 8 and 16-byte aligned operands (got m %d, n %d, k %d)", m, n, k);
         return LLM_REFUSED;
     }
     GemmParams p;
@@ -632,7 +660,7 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
     }
     p.silu_gate = silu_gate;
     p.scale = scale;
-    if (scale.parts != nullptr && (scale.stride < m || m > 64)) {
+    if (scale.parts != nullptr && (scale.stride < m || m > kMaxRows)) {
         llm_set_error("gemm_small_m: the sums of squares have room for %d tokens, the product has %d", scale.stride, m);
         return LLM_REFUSED;
     }
@@ -646,7 +674,8 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
                    (rope == nullptr || (aligned16(rope->k_pages) && aligned16(rope->v_pages)));
     p.vector_stream = p.stream.on && aligned16(p.stream.residual) && (p.stream.scaled == nullptr || aligned16(p.stream.scaled)) && n % 4 == 0;
     const int tiles = (n + kBlockRows - 1) / kBlockRows;
-    const int total_kb = (k + kBlockK - 1) / kBlockK;
+    const int atoms = m > kTwoAtomRows ? 1 : 2;
+    const int total_kb = (k + kAtomK * atoms - 1) / (kAtomK * atoms);
     // K is split across a cluster so that the tiles fill the machine; each rank keeps >= 4 K blocks.  The
     // caller may name the split (it times a few once per shape); 0 asks for about one wave of 148 SMs.
     int split = requested_split > 0 ? requested_split : 148 / tiles;
@@ -656,7 +685,7 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
     p.split = split;
     const size_t a_bytes = (size_t)kBlockRows * kAtomK * 2;
     const size_t b_bytes = ((size_t)p.token_pad * kAtomK * 2 + 1023) & ~(size_t)1023;
-    const size_t stage_bytes = kAtoms * (a_bytes + b_bytes);
+    const size_t stage_bytes = atoms * (a_bytes + b_bytes);
     // The ring of stages (about 100 KiB: two CTAs fit on an SM) lets a CTA that was launched early, while the kernels
     // before it still run, request that many bytes of weights before it has to wait for its input.
     static int ring_kib = -1;
@@ -676,12 +705,13 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
     if (shared < reduce_bytes) shared = reduce_bytes;
     shared += 1024;   // room to align the region to 1024 bytes
 
+    auto* kernel = atoms == 1 ? gemm_small_m_kernel<1, true> : m > 16 ? gemm_small_m_kernel<2, true> : gemm_small_m_kernel<2, false>;
     CUtensorMap map_w, map_x;
     if (!make_map(&map_w, w, n, k, kBlockRows) || !make_map(&map_x, x, m, k, p.token_pad)) {
         llm_set_error("gemm_small_m: cuTensorMapEncodeTiled failed (m %d, n %d, k %d)", m, n, k);
         return LLM_REFUSED;
     }
-    if (int limit_status = llm_raise_shared_limit(reinterpret_cast<const void*>(gemm_small_m_kernel), (size_t)226 * 1024, "gemm_small_m")) return limit_status;
+    if (int limit_status = llm_raise_shared_limit(reinterpret_cast<const void*>(kernel), (size_t)226 * 1024, "gemm_small_m")) return limit_status;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)(tiles * split), 1, 1);
     config.blockDim = dim3(m > 16 ? kThreads : kThreads / 2, 1, 1);
@@ -703,7 +733,7 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
     }
     config.attrs = attribute;
     config.numAttrs = count;
-    cudaError_t status = cudaLaunchKernelEx(&config, gemm_small_m_kernel, map_w, map_x, p);
+    cudaError_t status = cudaLaunchKernelEx(&config, kernel, map_w, map_x, p);
     if (status != cudaSuccess) {
         llm_set_error("gemm_small_m launch: %s", cudaGetErrorString(status));
         return (int)status;
@@ -745,11 +775,11 @@ LLM_EXPORT int llm_gemm_into_stream(const void* x, const void* w, float* residua
                           row_scale_of(nullptr, 0, 0, 0.0f), &e);
 }
 
-// 1 when the fused q/k/v projection takes the sizes: heads of 128 (a head is a tile of the product), up to 64 tokens
+// 1 when the fused q/k/v projection takes the sizes: heads of 128 (a head is a tile of the product), up to 128 tokens
 // (each costs a block-wide reduction in the epilogue of the block that finishes it: with many tokens the caller
 // measures whether the fused form still wins), and what llm_gemm_small_m itself needs.
 LLM_EXPORT int llm_gemm_qkv_rope_supports(int m, int n_q_heads, int n_kv_heads, int head_dim, int k) {
-    return head_dim == kBlockRows && m >= 1 && m <= 64 && n_q_heads >= 1 && n_kv_heads >= 1 &&
+    return head_dim == kBlockRows && m >= 1 && m <= kMaxRows && n_q_heads >= 1 && n_kv_heads >= 1 &&
            llm_gemm_small_m_supports(m, (n_q_heads + 2 * n_kv_heads) * head_dim, k);
 }
 
@@ -765,7 +795,7 @@ LLM_EXPORT int llm_gemm_qkv_rope(const void* x, const void* w, void* qkv, int m,
                                  int scale_n_parts, int scale_stride, float scale_eps, int* error_flag,
                                  cudaStream_t stream) {
     if (!llm_gemm_qkv_rope_supports(m, n_q_heads, n_kv_heads, head_dim, k)) {
-        llm_set_error("gemm_qkv_rope: takes heads of 128 and 1..64 tokens (got head_dim %d, m %d, k %d)", head_dim, m, k);
+        llm_set_error("gemm_qkv_rope: takes heads of 128 and 1..128 tokens (got head_dim %d, m %d, k %d)", head_dim, m, k);
         return LLM_REFUSED;
     }
     if (positions == nullptr || seq_of_token == nullptr || block_tables == nullptr || page_error == nullptr ||

@@ -14,13 +14,13 @@ import torch
 
 from .library import (KernelError, call, check, declare, dtype_code, launch_count, library, pointer,
                       require_device, stream_handle, wait_error_flag)
-from .stream import STREAM_ROWS, RowScaled, StreamSink
+from .stream import STREAM_MANY_ROWS, STREAM_ROWS, RowScaled, StreamSink
 
 __all__ = ["KernelError", "embedding", "add_rmsnorm", "rmsnorm", "silu_mul", "sample", "qk_norm_rope_kv_write",
            "attention_generic", "rope_kv_write_split", "normed_add_rmsnorm", "scaled_add_rmsnorm", "moe_route", "moe_select", "indexed_linear", "moe_combine", "moe_plan", "moe_grouped",
            "moe_grouped_supported", "moe_combine_rows", "ExpertPlan",
            "clamped_glu", "clamped_gate_up", "gemm_f32", "linear", "linear_wide", "qkv_projection", "gate_up_silu", "interleave_gate_up", "require_device", "library", "launch_count",
-           "RowScaled", "StreamSink", "STREAM_ROWS", "unscaled_rows_supported", "norm_rope_units", "rotate_units", "attention_diff", "gla_supported",
+           "RowScaled", "StreamSink", "STREAM_ROWS", "STREAM_MANY_ROWS", "unscaled_rows_supported", "norm_rope_units", "rotate_units", "attention_diff", "gla_supported",
            "gla_recurrent", "head_linear", "relu_squared", "tanh_narrow", "softcap_", "scaled_sum", "token_shift_mix",
            "short_conv_units", "matrix_recurrence_supported", "wkv_recurrent", "delta_rule_recurrent", "retention_recurrent", "ssd_recurrent", "decay_recurrence_supported",
            "gelu_mul", "grouped_rmsnorm", "conv_norm_kv", "streams_norm", "unit_linear_wide", "gated_scan"]
@@ -1393,7 +1393,7 @@ def qkv_projection(x, weight: torch.Tensor, q_weight: Optional[torch.Tensor], k_
     epilogue (bfloat16, heads of 128, up to 64 tokens, the whole head rotating in halves; from 17 tokens on only where
     that is measured to be faster), else as two.  ``x`` may be a ``RowScaled``."""
     whole_head = rotary_dim is None or rotary_dim == head_dim
-    if x.dtype == torch.bfloat16 and whole_head and not interleaved and x.shape[0] <= 64:
+    if x.dtype == torch.bfloat16 and whole_head and not interleaved and x.shape[0] <= (128 if isinstance(x, RowScaled) else 64):
         from . import gemm_bf16
         fused = gemm_bf16.qkv_rope_fused(x, weight, q_weight, k_weight, inv_freq, positions, seq_of_token, block_tables,
                                          k_pages, v_pages, n_q_heads, n_kv_heads, head_dim, eps, write_cache, error_flag)

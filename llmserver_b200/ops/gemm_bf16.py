@@ -17,9 +17,10 @@ from typing import Optional
 import torch
 
 from .library import KernelError, call, check_wait_errors, library, stream_handle, wait_error_flag
-from .stream import NO_SCALE, STREAM_ROWS, RowScaled, StreamSink, rows_of, scale_args_of
+from .stream import NO_SCALE, STREAM_MANY_ROWS, STREAM_ROWS, RowScaled, StreamSink, rows_of, scale_args_of
 
-SMALL_M = 64
+SMALL_M = 64        # up to these many rows products without a fused epilogue may run this package's kernel
+FUSED_M = 128       # up to these many rows the kernel takes products (its fused epilogues among them)
 _use_small_m = os.environ.get("LLMSERVER_B200_SMALL_M_GEMM", "1") != "0"
 error_flag = wait_error_flag        # the kernels of this package share one flag per device
 check_errors = check_wait_errors
@@ -32,7 +33,7 @@ def small_m_supported(rows: int, cols: int, inner: int) -> bool:
 # (row bucket, N, K, out dtype) -> split of K to use with this package's kernel, or 0 for the library product.
 _choice = {}
 SPLITS = (1, 2, 3, 4, 6, 8)
-ROW_BUCKETS = (1, 2, 4, 8, 16, 32, 48, 64)
+ROW_BUCKETS = (1, 2, 4, 8, 16, 32, 48, 64, 96, 128)
 _tunings = 0
 
 
@@ -45,7 +46,7 @@ def _row_bucket(rows: int) -> int:
     for bucket in ROW_BUCKETS:
         if rows <= bucket:
             return bucket
-    return SMALL_M
+    return FUSED_M
 
 
 # The choices can be kept in a file (LLMSERVER_B200_GEMM_PLAN): what is in the file is used as it is, what is
@@ -248,7 +249,7 @@ def linear_into_stream(x: torch.Tensor, weight: torch.Tensor, sink: StreamSink) 
     cols = weight.shape[0]
     residual = sink.residual
     if not (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.is_contiguous() and weight.is_contiguous()
-            and rows <= STREAM_ROWS and small_m_supported(rows, cols, inner) and residual.dtype == torch.float32
+            and rows <= STREAM_MANY_ROWS and small_m_supported(rows, cols, inner) and residual.dtype == torch.float32
             and residual.is_contiguous() and tuple(residual.shape) == (rows, cols)):
         return False
     norm_weight = sink.norm_weight
@@ -259,7 +260,7 @@ def linear_into_stream(x: torch.Tensor, weight: torch.Tensor, sink: StreamSink) 
     scaled = parts = None
     if norm_weight is not None:
         scaled = torch.empty((rows, cols), dtype=torch.bfloat16, device=x.device)
-        parts = torch.empty((library().llm_gemm_into_stream_parts(cols), max(STREAM_ROWS, rows)), dtype=torch.float32, device=x.device)
+        parts = torch.empty((library().llm_gemm_into_stream_parts(cols), -(-rows // 16) * 16), dtype=torch.float32, device=x.device)
     call("llm_gemm_into_stream", x.data_ptr(), weight.data_ptr(), residual.data_ptr(), rows, cols, inner, split,
          0 if norm_weight is None else norm_weight.data_ptr(), int(norm_weight is not None and norm_weight.dtype == torch.float32),
          0 if scaled is None else scaled.data_ptr(), 0 if parts is None else parts.data_ptr(), 0 if parts is None else parts.shape[1],
@@ -277,7 +278,7 @@ def linear_bf16(x, weight: torch.Tensor, out: Optional[torch.Tensor] = None,
         rows, inner = x.shape
         cols = weight.shape[0]
         out_dtype = out_dtype or torch.bfloat16
-        if not (rows <= SMALL_M and unscaled_rows_supported(weight) and x.x.is_contiguous()):
+        if not (rows <= FUSED_M and unscaled_rows_supported(weight) and x.x.is_contiguous()):
             raise KernelError(f"linear_bf16: no product kernel takes unscaled rows for {rows} rows and a weight {tuple(weight.shape)}")
         if out is None:
             out = torch.empty((rows, cols), dtype=out_dtype, device=x.device)
@@ -368,7 +369,7 @@ def qkv_rope_fused(x: torch.Tensor, weight: torch.Tensor, q_weight, k_weight, in
     norms, the rotation and the cache write (see ``ops.qk_norm_rope_kv_write`` for the arithmetic).  Returns the packed
     [N, (Hq + 2 Hkv) D] tensor whose Q heads are finished (its K and V heads are not written: they went to the pages),
     or None when the fused kernel does not take the case; the caller then runs the two kernels one after the other."""
-    scale, x = scale_args_of(x), rows_of(x)
+    scaled, scale, x = isinstance(x, RowScaled), scale_args_of(x), rows_of(x)
     rows, inner = x.shape
     if not (FUSE_QKV_ROPE and _use_small_m and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and x.is_contiguous() and weight.is_contiguous() and k_pages.dtype == torch.bfloat16
@@ -390,8 +391,9 @@ def qkv_rope_fused(x: torch.Tensor, weight: torch.Tensor, q_weight, k_weight, in
              k_pages.data_ptr(), v_pages.data_ptr(), n_q_heads, n_kv_heads, head_dim, k_pages.shape[2], k_pages.shape[0],
              float(eps), int(write_cache), page_error.data_ptr(), *scale, error_flag(x.device).data_ptr(), stream_handle())
 
-    if rows <= 16:
-        split = _plan_for(x, weight, torch.bfloat16, own_kernel_only=True)      # few rows: always this package's kernel
+    if rows <= 16 or scaled:
+        # few rows, and rows that the library's product does not take as they are: always this package's kernel
+        split = _plan_for(x, weight, torch.bfloat16, own_kernel_only=True)
     else:
         def apart() -> None:      # what the caller would run instead (it writes the same values to the same places)
             from . import qk_norm_rope_kv_write
@@ -438,10 +440,10 @@ def gate_up_silu_fused(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.
     """silu(gate) * up in the epilogue of the product for few rows; ``weight`` is the fused [2 I, H] matrix with gate
     and up rows interleaved in groups of 64.  None when the product kernel does not take the case (the caller then
     runs the product and the activation kernel)."""
-    scale, x = scale_args_of(x), rows_of(x)
+    scaled, scale, x = isinstance(x, RowScaled), scale_args_of(x), rows_of(x)
     rows, inner = x.shape
     cols = weight.shape[0]
-    if not (FUSE_GATE_UP_SILU and rows <= SMALL_M and cols % 128 == 0 and x.is_contiguous() and weight.is_contiguous()
+    if not (FUSE_GATE_UP_SILU and rows <= (FUSED_M if scaled else SMALL_M) and cols % 128 == 0 and x.is_contiguous() and weight.is_contiguous()
             and weight.dtype == torch.bfloat16 and small_m_supported(rows, cols, inner)):
         return None
     out = torch.empty((rows, cols // 2), dtype=torch.bfloat16, device=x.device)
@@ -453,7 +455,7 @@ def gate_up_silu_fused(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.
     # up to 16 rows this package's kernel, whatever a measurement of the bare products says (whole steps are faster with
     # it there, and the activation kernel goes away); with more rows whichever is measured faster: the fused kernel, or
     # the library's product followed by the activation kernel
-    if rows <= 16:
+    if rows <= 16 or scaled:
         split = _plan_for(x, weight, torch.bfloat16, own_kernel_only=True)
     else:
         def apart() -> None:

@@ -108,7 +108,7 @@ class RMSNorm(Norm):
                                unscaled=unscaled)
 
     def _few_rows(self, residual) -> bool:
-        return self.runtime.dtype == torch.bfloat16 and residual.shape[0] <= ops.STREAM_ROWS
+        return self.runtime.dtype == torch.bfloat16 and residual.shape[0] <= (ops.STREAM_MANY_ROWS if ops.STREAM_ROWS else 0)
 
     def sink(self, residual, consumer):
         if not self._few_rows(residual) or (consumer is not None and not getattr(consumer, "takes_unscaled", False)):

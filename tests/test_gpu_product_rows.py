@@ -1,0 +1,79 @@
+"""The product kernel for few rows at 65 to 128 rows (one K atom per stage, twice the tensor memory) and its fused epilogues from 17
+rows on, where a warp finishes several tokens and a lane adds a token's sums of squares."""
+import pytest
+import torch
+
+from test_gpu_kernels import DEVICE, close, rand
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows", [17, 63, 64, 65, 96, 97, 127, 128])
+@pytest.mark.parametrize("cols,inner,split", [(130, 72, 1), (256, 64, 1), (1000, 520, 2), (4096, 1024, 8)])
+def test_product(rows, cols, inner, split):
+    from llmserver_b200.ops import gemm_bf16
+    from llmserver_b200.ops.library import call, check_wait_errors, stream_handle
+    x, w = rand((rows, inner), torch.bfloat16, 12), rand((cols, inner), torch.bfloat16, 13, 0.05)
+    for out_dtype in (torch.float32, torch.bfloat16):
+        out = torch.full((rows, cols), float("nan"), dtype=out_dtype, device=DEVICE)
+        call("llm_gemm_small_m", x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, cols, inner, cols, int(out_dtype == torch.float32), split,
+             *gemm_bf16.NO_SCALE, gemm_bf16.error_flag(DEVICE).data_ptr(), stream_handle())
+        torch.cuda.synchronize()
+        check_wait_errors()
+        close(out, x.double() @ w.double().T, out_dtype, f"{rows, cols, inner, split}", factor=4.0 if out_dtype == torch.float32 else 1.0)
+
+
+@pytest.mark.parametrize("rows", [16, 17, 33, 64, 65, 119, 128])
+def test_stream_and_scaled_rows(rows):
+    """x W^T added to the stream, the sums of squares it leaves, and the gated product that divides by them: against the same in 64
+    bits.  A stream of 640 columns leaves five sums per token."""
+    from llmserver_b200 import ops
+    from llmserver_b200.ops import gemm_bf16
+    from llmserver_b200.ops.library import check_wait_errors
+    width, inner, features, eps = 640, 512, 320, 1e-6
+    x, w = rand((rows, inner), torch.bfloat16, 1), rand((width, inner), torch.bfloat16, 2, inner ** -0.5)
+    stream, norm = rand((rows, width), torch.float32, 3, 2.0), rand((width,), torch.bfloat16, 4, 0.1) + 1
+    gate, up = rand((features, width), torch.bfloat16, 5, width ** -0.5), rand((features, width), torch.bfloat16, 6, width ** -0.5)
+    want = stream.double() + x.double() @ w.double().T
+    sink = ops.StreamSink(stream, norm, eps)
+    assert gemm_bf16.linear_into_stream(x, w, sink) and sink.added
+    close(stream, want, torch.float32, "the stream", factor=4.0)
+    normed = want / torch.sqrt((want * want).mean(-1, keepdim=True) + eps) * norm.double()
+    g, u = normed @ gate.double().T, normed @ up.double().T
+    out = ops.gate_up_silu(sink.scaled, ops.interleave_gate_up(gate, up), ops.GATE_UP_GROUP)
+    torch.cuda.synchronize()
+    check_wait_errors()
+    close(out, g * torch.sigmoid(g) * u, torch.bfloat16, "the gated product of scaled rows")
+
+
+@pytest.mark.parametrize("rows", [17, 40, 64, 65, 128])
+def test_fused_heads(rows):
+    """The q/k/v epilogue for the tokens of several sequences, each warp finishing several: queries and cache rows as the two
+    kernels that it stands for leave them (which round the product to bfloat16 first)."""
+    from llmserver_b200 import ops
+    from llmserver_b200.ops import gemm_bf16
+    heads, kv_heads, dim, inner, page_size = 4, 2, 128, 256, 16
+    width = (heads + 2 * kv_heads) * dim
+    x, w = rand((rows, inner), torch.bfloat16, 1), rand((width, inner), torch.bfloat16, 2, inner ** -0.5)
+    q_norm, k_norm = rand((dim,), torch.bfloat16, 3, 0.1) + 1, rand((dim,), torch.bfloat16, 4, 0.1) + 1
+    inv_freq = (1e6 ** (-torch.arange(0, dim, 2) / dim)).float().to(DEVICE)
+    seq = (torch.arange(rows) % 3).to(torch.int32).to(DEVICE)
+    positions = (torch.arange(rows) // 3 * 7 % 300 + torch.arange(rows) // 3).to(torch.int32).to(DEVICE)
+    tables = (torch.randperm(90, generator=torch.Generator().manual_seed(1)).view(3, 30)).to(torch.int32).to(DEVICE)
+    parts = torch.empty((1, 128), dtype=torch.float32, device=DEVICE)
+    parts[0, :rows] = (x.float() ** 2).sum(-1)
+    normed = (x.float() / torch.sqrt((x.float() ** 2).mean(-1, keepdim=True) + 1e-6)).to(torch.bfloat16)
+    results = []
+    for fused in (True, False):
+        k_pages = torch.zeros((90, kv_heads, page_size, dim), dtype=torch.bfloat16, device=DEVICE)
+        v_pages, error = torch.zeros_like(k_pages), torch.zeros(1, dtype=torch.int32, device=DEVICE)
+        if fused:
+            out = gemm_bf16.qkv_rope_fused(ops.RowScaled(x, parts, 1e-6), w, q_norm, k_norm, inv_freq, positions, seq, tables, k_pages,
+                                           v_pages, heads, kv_heads, dim, 1e-6, True, error)
+        else:
+            out = torch.matmul(normed, w.t())
+            ops.qk_norm_rope_kv_write(out, q_norm, k_norm, inv_freq, positions, seq, tables, k_pages, v_pages, heads, kv_heads, dim, 1e-6, True, error)
+        assert int(error) == 0
+        results.append((out[:, :heads * dim], k_pages, v_pages))
+    for name, got, want in zip(("queries", "keys", "values"), *results):
+        close(got, want, torch.bfloat16, name, factor=2.0)      # either side is rounded where the other is not
