@@ -11,7 +11,10 @@
 // so an encoding that stretches its frequencies (and scales cos and sin to make up for it) needs nothing but its
 // own inv_freq and magnitude.  Angles, cos, sin and the products are 32-bit; each value is rounded once.
 // There is no per-head norm here; `llm_qk_norm_rope_kv_write` is the kernel for equal sizes with one.
+//
+// bfloat16 heads of 64 or 128 that turn as a whole, halves paired, are moved in 16-byte pieces (unit_pieces.cuh).
 #include "common.cuh"
+#include "unit_pieces.cuh"
 
 template <typename T>
 __global__ void rope_kv_write_split_kernel(T* __restrict__ qkv, const float* __restrict__ inv_freq, float magnitude,
@@ -90,6 +93,29 @@ LLM_EXPORT int llm_rope_kv_write_split(void* qkv, const float* inv_freq, float m
     if (key_dim <= 0 || value_dim <= 0 || n_q_heads <= 0 || n_kv_heads <= 0 || page_size <= 0 || num_pages <= 0) {
         llm_set_error("rope_kv_write_split: sizes must be positive");
         return LLM_REFUSED;
+    }
+    if (dtype == LLM_BF16 && (rotary_dim == 0 || (rotary_dim == key_dim && !interleaved))) {
+        UnitPieces p = {};
+        p.qkv = (__nv_bfloat16*)qkv;
+        p.row_width = (n_q_heads + n_kv_heads) * key_dim + n_kv_heads * value_dim;
+        p.inv_freq = rotary_dim > 0 ? inv_freq : nullptr;
+        p.magnitude = magnitude;
+        p.positions = positions;
+        p.seq_of_token = seq_of_token;
+        p.block_tables = block_tables;
+        p.max_blocks = max_blocks;
+        p.k_pages = (__nv_bfloat16*)k_pages;
+        p.v_pages = (__nv_bfloat16*)v_pages;
+        p.n_kv_heads = n_kv_heads;
+        p.maps = 1;
+        p.q_cols = n_q_heads * key_dim;
+        p.dim = key_dim;
+        p.value_dim = value_dim;
+        p.page_size = page_size;
+        p.num_pages = num_pages;
+        p.write_cache = write_cache;
+        p.error_flag = error_flag;
+        if (unit_pieces_take(p)) return unit_pieces_launch(p, n_tokens, stream);
     }
     const int total_heads = n_q_heads + 2 * n_kv_heads;
     const int warps = n_tokens >= 256 ? 8 : 4;
