@@ -20,9 +20,23 @@
 namespace {
 constexpr int kChunk = 8;        // elements a thread handles at a time in the vector form
 constexpr int kMaxChunks = 4;    // per thread
+
+// Pieces per thread and threads per block of the vector forms, for a row of `chunks` pieces: up to 320 threads where four pieces
+// each suffice (512 threads leave most of a block idle for the last pieces of a width of 5120, and more pieces per thread keep
+// more bytes in flight), up to 512 for wider rows.
+inline int turns_of(int chunks) {
+    const int turns = (chunks + 319) / 320;
+    return turns < 1 ? 1 : turns > kMaxChunks ? kMaxChunks : turns;
+}
+inline int threads_of(int chunks) {
+    const int turns = turns_of(chunks), threads = ((chunks + turns - 1) / turns + 31) / 32 * 32;
+    return threads < 32 ? 32 : threads > 512 ? 512 : threads;
+}
 }
 
-template <typename T, typename W>
+// CHUNKS: pieces of eight elements per thread.  Bound by memory: 8192 rows of 5120 (503 MB) took 115 us in blocks of 512 threads
+// that fetched, added and stored piece after piece, and take 80 with all of a thread's pieces asked for at once.
+template <typename T, typename W, int CHUNKS>
 __global__ void add_rmsnorm_vec_kernel(float* __restrict__ residual, const T* __restrict__ delta,
                                        const W* __restrict__ weight, T* __restrict__ out,
                                        const int* __restrict__ rows, int width, float eps, int write_residual,
@@ -35,16 +49,25 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ residual, const T* __
     float* res = residual + (size_t)r * width;
     const T* del = delta ? delta + (size_t)r * width : nullptr;
     const int chunks = width / kChunk;
-    float values[kMaxChunks][kChunk];
+    // all of a thread's pieces are asked for before the first sum is stored
+    float values[CHUNKS][kChunk];
+    Raw8<T> added_raw[CHUNKS];
     float sum_squares = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kMaxChunks; ++i) {
+    for (int i = 0; i < CHUNKS; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
         if (c < chunks) {
             load8<float>(res + c * kChunk, values[i]);
+            if (del) added_raw[i].fetch(del + c * kChunk);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < CHUNKS; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        if (c < chunks) {
             if (del) {
                 float added[kChunk];
-                load8<T>(del + c * kChunk, added);
+                added_raw[i].widen(added);
 #pragma unroll
                 for (int j = 0; j < kChunk; ++j) values[i][j] += added[j];
                 if (write_residual) store8<float>(res + c * kChunk, values[i]);
@@ -58,7 +81,7 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ residual, const T* __
     if (squares_out && threadIdx.x == 0) squares_out[o] = total;
     T* dst = out + (size_t)o * width;
 #pragma unroll
-    for (int i = 0; i < kMaxChunks; ++i) {
+    for (int i = 0; i < CHUNKS; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
         if (c < chunks) {
             float scale[kChunk], scaled[kChunk];
@@ -131,15 +154,16 @@ LLM_EXPORT int llm_add_rmsnorm(float* residual, const void* delta, const void* w
     if (n_rows == 0) return LLM_OK;
     const int chunks = width / kChunk;
     // the block size depends on the width only, so a row is summed in the same order in every call
-    int threads = ((chunks + 31) / 32) * 32;
-    if (threads > 512) threads = 512;
+    const int turns = turns_of(chunks), threads = threads_of(chunks);
     const bool vector_form = width % kChunk == 0 && width >= kChunk && aligned16(residual) && aligned16(out) &&
                              aligned16(delta) && aligned16(weight) && chunks <= threads * kMaxChunks;
     if (vector_form) {
         LLM_DISPATCH_DTYPE_WEIGHT(dtype, weight_dtype,
-                                  (llm_launch(add_rmsnorm_vec_kernel<T, W>, n_rows, threads, 0, stream, 
-                                      residual, (const T*)delta, (const W*)weight, (T*)out, rows, width, eps,
-                                      write_residual, squares_out)));
+                                  llm_launch(turns == 1   ? add_rmsnorm_vec_kernel<T, W, 1>
+                                             : turns == 2 ? add_rmsnorm_vec_kernel<T, W, 2>
+                                                          : add_rmsnorm_vec_kernel<T, W, kMaxChunks>,
+                                             n_rows, threads, 0, stream, residual, (const T*)delta, (const W*)weight, (T*)out, rows, width, eps,
+                                             write_residual, squares_out));
         return llm_check_launch("add_rmsnorm");
     }
     LLM_DISPATCH_DTYPE_WEIGHT(dtype, weight_dtype,
@@ -210,7 +234,8 @@ __global__ void normed_add_rmsnorm_kernel(float* __restrict__ residual, const T*
 
 // The same with 16-byte accesses and the row held in registers between the passes (widths that are a multiple of 8,
 // up to blockDim * 32); the order of each sum depends on the width only.
-template <typename T, typename W>
+// The stream's row is asked for together with the delta's, not behind the sum over it.
+template <typename T, typename W, int CHUNKS>
 __global__ void normed_add_rmsnorm_vec_kernel(float* __restrict__ residual, const T* __restrict__ delta,
                                               const W* __restrict__ post_weight, float post_eps, const float* __restrict__ extra,
                                               const W* __restrict__ weight, T* __restrict__ out, const int* __restrict__ rows,
@@ -222,13 +247,18 @@ __global__ void normed_add_rmsnorm_vec_kernel(float* __restrict__ residual, cons
     const int r = rows ? rows[o] : o;
     float* res = residual + (size_t)r * width;
     const int chunks = width / kChunk;
-    float values[kMaxChunks][kChunk];
+    float values[CHUNKS][kChunk], stream[CHUNKS][kChunk];
+#pragma unroll
+    for (int i = 0; i < CHUNKS; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        if (c < chunks) load8<float>(res + c * kChunk, stream[i]);
+    }
     float inverse_post = 0.0f;
     if (delta) {
         const T* del = delta + (size_t)r * width;
         float sum_squares = 0.0f;
 #pragma unroll
-        for (int i = 0; i < kMaxChunks; ++i) {
+        for (int i = 0; i < CHUNKS; ++i) {
             const int c = threadIdx.x + i * blockDim.x;
             if (c < chunks) {
                 load8<T>(del + c * kChunk, values[i]);
@@ -246,28 +276,26 @@ __global__ void normed_add_rmsnorm_vec_kernel(float* __restrict__ residual, cons
     }
     float sum_squares = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kMaxChunks; ++i) {
+    for (int i = 0; i < CHUNKS; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
         if (c < chunks) {
-            float stream[kChunk];
-            load8<float>(res + c * kChunk, stream);
             if (delta) {
                 float scale[kChunk];
                 load8<W>(post_weight + c * kChunk, scale);
 #pragma unroll
-                for (int j = 0; j < kChunk; ++j) stream[j] += values[i][j] * inverse_post * scale[j];
+                for (int j = 0; j < kChunk; ++j) stream[i][j] += values[i][j] * inverse_post * scale[j];
             }
             if (extra) {
                 float more[kChunk];
                 load8<float>(extra + (size_t)r * width + c * kChunk, more);
 #pragma unroll
-                for (int j = 0; j < kChunk; ++j) stream[j] += more[j];
+                for (int j = 0; j < kChunk; ++j) stream[i][j] += more[j];
             }
-            if (write_residual && (delta || extra)) store8<float>(res + c * kChunk, stream);
+            if (write_residual && (delta || extra)) store8<float>(res + c * kChunk, stream[i]);
 #pragma unroll
             for (int j = 0; j < kChunk; ++j) {
-                values[i][j] = stream[j];
-                sum_squares += stream[j] * stream[j];
+                values[i][j] = stream[i][j];
+                sum_squares += stream[i][j] * stream[i][j];
             }
         }
     }
@@ -275,7 +303,7 @@ __global__ void normed_add_rmsnorm_vec_kernel(float* __restrict__ residual, cons
     T* dst = out + (size_t)o * width;
     if (!weight) {
 #pragma unroll
-        for (int i = 0; i < kMaxChunks; ++i) {
+        for (int i = 0; i < CHUNKS; ++i) {
             const int c = threadIdx.x + i * blockDim.x;
             if (c < chunks) store8<T>(dst + c * kChunk, values[i]);
         }
@@ -283,7 +311,7 @@ __global__ void normed_add_rmsnorm_vec_kernel(float* __restrict__ residual, cons
     }
     const float inverse = rsqrtf(block_sum(sum_squares, scratch) / (float)width + eps);
 #pragma unroll
-    for (int i = 0; i < kMaxChunks; ++i) {
+    for (int i = 0; i < CHUNKS; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
         if (c < chunks) {
             float scale[kChunk], scaled[kChunk];
@@ -305,15 +333,16 @@ LLM_EXPORT int llm_normed_add_rmsnorm(float* residual, const void* delta, const 
         return LLM_REFUSED;
     }
     const int chunks = width / kChunk;
-    int threads = ((chunks + 31) / 32) * 32;      // depends on the width only
-    if (threads > 512) threads = 512;
+    const int turns = turns_of(chunks), threads = threads_of(chunks);      // depend on the width only
     const bool vector_form = width % kChunk == 0 && width >= kChunk && chunks <= threads * kMaxChunks && aligned16(residual) &&
                              aligned16(delta) && aligned16(post_weight) && aligned16(extra) && aligned16(weight) && aligned16(out) && aligned16(delta_bias);
     if (vector_form) {
         LLM_DISPATCH_DTYPE_WEIGHT(dtype, weight_dtype,
-                                  (llm_launch(normed_add_rmsnorm_vec_kernel<T, W>, n_rows, threads, 0, stream, residual,
-                                      (const T*)delta, (const W*)post_weight, post_eps, extra, (const W*)weight, (T*)out, rows,
-                                      width, eps, write_residual, delta_bias)));
+                                  llm_launch(turns == 1   ? normed_add_rmsnorm_vec_kernel<T, W, 1>
+                                             : turns == 2 ? normed_add_rmsnorm_vec_kernel<T, W, 2>
+                                                          : normed_add_rmsnorm_vec_kernel<T, W, kMaxChunks>,
+                                             n_rows, threads, 0, stream, residual, (const T*)delta, (const W*)post_weight, post_eps, extra,
+                                             (const W*)weight, (T*)out, rows, width, eps, write_residual, delta_bias));
         return llm_check_launch("normed_add_rmsnorm");
     }
     const size_t shared = (size_t)width * sizeof(float);
