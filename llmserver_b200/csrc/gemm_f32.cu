@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
 
 // The same product for few rows (M <= 32), where a launch is the latency of its loads and not arithmetic: a block owns 32
 // columns, the columns are a warp's lanes and the rows are dealt to four warps, ROWS each.  W goes through shared memory in
-// pieces of 128 along K, three of them in flight, the first three asked for before the kernel in front has ended (weights do
-// not depend on it).  Every output is still one thread's running sum over ascending k, so the results are those of the kernel
+// pieces of 128 along K, three of them in flight; where the caller says that W is a weight, which the
+// kernel in front does not write, the first three are asked for before that kernel has ended.  Every output is still one thread's running sum over ascending k, so the results are those of the kernel
 // above bit for bit.
 namespace {
 constexpr int kColumns = 32, kPiece = 128, kPitch = kPiece + 4, kDeep = 3, kFewThreads = 128, kFewRows = 32;
@@ -85,8 +85,9 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 template <int ROWS>
 __global__ void __launch_bounds__(kFewThreads) gemm_f32_few_rows_kernel(const float* __restrict__ a, const float* __restrict__ w,
                                                                         float* __restrict__ c, int m_total, int n_total, int k_total,
-                                                                        int lda, int ldw, int ldc) {
+                                                                        int lda, int ldw, int ldc, int w_settled) {
     pdl_trigger();   // let the next kernel start launching
+    if (!w_settled) pdl_wait();
     extern __shared__ __align__(16) float stages[];      // [kDeep]{ W [kColumns][kPitch], rows [4 ROWS][kPitch] }
     constexpr int kStage = (kColumns + 4 * ROWS) * kPitch, kVectors = kPiece / 4;
     const int n0 = blockIdx.x * kColumns;
@@ -151,23 +152,24 @@ __global__ void __launch_bounds__(kFewThreads) gemm_f32_few_rows_kernel(const fl
 }
 
 template <int ROWS>
-static int few_rows_launch(const float* a, const float* w, float* c, int m, int n, int k, int lda, int ldw, int ldc, cudaStream_t stream) {
+static int few_rows_launch(const float* a, const float* w, float* c, int m, int n, int k, int lda, int ldw, int ldc, int w_settled, cudaStream_t stream) {
     const size_t shared = (size_t)kDeep * (kColumns + 4 * ROWS) * kPitch * sizeof(float);
     if (int status = llm_raise_shared_limit(reinterpret_cast<const void*>(gemm_f32_few_rows_kernel<ROWS>), shared, "gemm_f32")) return status;
     llm_launch(gemm_f32_few_rows_kernel<ROWS>, dim3((unsigned)((n + kColumns - 1) / kColumns)), kFewThreads, shared, stream, a, w, c, m, n, k,
-               lda, ldw, ldc);
+               lda, ldw, ldc, w_settled);
     return llm_check_launch("gemm_f32");
 }
 
+// w_settled: the caller vouches that no kernel which may still be running writes w (it is a model's weight).
 LLM_EXPORT int llm_gemm_f32(const float* a, const float* w, float* c, int m, int n, int k, int lda, int ldw, int ldc,
-                            cudaStream_t stream) {
+                            int w_settled, cudaStream_t stream) {
     if (m == 0 || n == 0) return LLM_OK;
     // few rows whose 16-byte pieces are aligned and whole; any other product runs in tiles of 64 x 64
     if (m <= kFewRows && k > 0 && k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && aligned16(a) && aligned16(w)) {
-        if (m <= 4) return few_rows_launch<1>(a, w, c, m, n, k, lda, ldw, ldc, stream);
-        if (m <= 8) return few_rows_launch<2>(a, w, c, m, n, k, lda, ldw, ldc, stream);
-        if (m <= 16) return few_rows_launch<4>(a, w, c, m, n, k, lda, ldw, ldc, stream);
-        return few_rows_launch<8>(a, w, c, m, n, k, lda, ldw, ldc, stream);
+        if (m <= 4) return few_rows_launch<1>(a, w, c, m, n, k, lda, ldw, ldc, w_settled, stream);
+        if (m <= 8) return few_rows_launch<2>(a, w, c, m, n, k, lda, ldw, ldc, w_settled, stream);
+        if (m <= 16) return few_rows_launch<4>(a, w, c, m, n, k, lda, ldw, ldc, w_settled, stream);
+        return few_rows_launch<8>(a, w, c, m, n, k, lda, ldw, ldc, w_settled, stream);
     }
     const int blocks_m = (m + BM - 1) / BM;
     if ((n + BN - 1) / BN > 65535) {

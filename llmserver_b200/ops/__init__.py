@@ -1332,8 +1332,9 @@ def clamped_glu(gate_up: torch.Tensor, limit: float, alpha: float) -> torch.Tens
     return out
 
 
-def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """x [M, K] times weight [N, K] transposed, all float32, FMA only (no tensor cores, no TF32)."""
+def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, settled: bool = False) -> torch.Tensor:
+    """x [M, K] times weight [N, K] transposed, all float32, FMA only (no tensor cores, no TF32).  ``settled``: ``weight`` is a
+    model's weight, which no kernel that may still be running writes; the kernel then reads it ahead."""
     check(x, "x", torch.float32)
     check(weight, "weight", torch.float32, x.shape[-1])
     rows, inner = x.shape
@@ -1342,7 +1343,7 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] 
         out = torch.empty((rows, cols), dtype=torch.float32, device=x.device)
     check(out, "gemm output", torch.float32, cols)
     call("llm_gemm_f32", x.data_ptr(), weight.data_ptr(), out.data_ptr(), rows, cols, inner, inner, inner, cols,
-         stream_handle())
+         int(settled), stream_handle())
     return out
 
 
@@ -1358,7 +1359,7 @@ def linear(x, weight: torch.Tensor, out: Optional[torch.Tensor] = None,
     if x.device.type != "cuda":
         raise KernelError("linear: there is no CPU path")
     if x.dtype == torch.float32:
-        result = gemm_f32(x, weight, out)
+        result = gemm_f32(x, weight, out, settled=True)
         return result
     from . import gemm_bf16
     if sink is not None and out is None and not isinstance(x, RowScaled) and gemm_bf16.linear_into_stream(x, weight, sink):
@@ -1371,7 +1372,7 @@ def linear_wide(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     widened): a product with few output columns whose values decide something, a router's logits for instance.  Up
     to 64 rows: this package's kernel; more: the library's product with a 32-bit result in one launch."""
     if x.dtype == torch.float32:
-        return gemm_f32(x, weight)
+        return gemm_f32(x, weight, settled=True)
     from . import gemm_bf16
     if x.shape[0] <= gemm_bf16.SMALL_M:
         return gemm_bf16.linear_bf16(x, weight, out_dtype=torch.float32)

@@ -345,7 +345,7 @@ def _attention_diff_maps(qkv, gate, batch, block_tables, k_pages, v_pages, n_q_h
             partial_out, partial_ml = batch.scratch[key]
         call("llm_attention_diff_decode", qkv.data_ptr(), row_width, k_pages.data_ptr(), v_pages.data_ptr(), block_tables.data_ptr(),
              block_tables.shape[-1], batch.q_start.data_ptr(), batch.context_len.data_ptr(), maps.data_ptr(), batch.n_seqs, n_q_heads,
-             n_kv_heads, page_size, k_pages.shape[0], float(scale), float(cap or 0.0), window, split_len, max_splits,
+             n_kv_heads, page_size, k_pages.shape[0], float(scale), max(float(cap or 0.0), 0.0), window, split_len, max_splits,
              0 if partial_out is None else partial_out.data_ptr(), 0 if partial_ml is None else partial_ml.data_ptr(),
              int(EARLY_KEYS and getattr(batch, "keys_settled", False)), flag, stream_handle())
     else:
@@ -358,7 +358,7 @@ def _attention_diff_maps(qkv, gate, batch, block_tables, k_pages, v_pages, n_q_h
         pairing = cost_paired < cost_single if FORCE_PAIRING is None else FORCE_PAIRING
         call("llm_attention_diff_prefill", qkv.data_ptr(), row_width, batch.n_tokens, k_pages.data_ptr(), v_pages.data_ptr(),
              block_tables.data_ptr(), block_tables.shape[-1], batch.q_start.data_ptr(), batch.context_len.data_ptr(), maps.data_ptr(),
-             batch.n_seqs, n_q_heads, n_kv_heads, page_size, k_pages.shape[0], float(scale), float(cap or 0.0), window, int(pairing),
+             batch.n_seqs, n_q_heads, n_kv_heads, page_size, k_pages.shape[0], float(scale), max(float(cap or 0.0), 0.0), window, int(pairing),
              paired if pairing else sum(tile_counts), flag, stream_handle())
     call("llm_attention_diff_combine", maps.data_ptr(), gate, row_width, out.data_ptr(), batch.n_tokens, n_q_heads, float(lam), float(eps),
          float(out_scale), stream_handle())

@@ -65,7 +65,7 @@ SIGNATURES = {
     "llm_moe_gather_rows": [_P, _P, _I, _P, _I, _I, _P, _S],
     "llm_moe_grouped_tc": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _F, _F, _F, _P, _S],
     "llm_moe_combine_rows": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _P, _I, _S],
-    "llm_gemm_f32": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _S],
+    "llm_gemm_f32": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _S],
     "llm_attention_mma_supports": [_I, _I, _I],
     "llm_attention_mma_sinks_supports": [_I, _I, _I, _I],
     "llm_attention_mma_sinks": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P, _S],

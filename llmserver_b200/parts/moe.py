@@ -179,7 +179,8 @@ class RoutedExperts(FeedForward):
         if self.weight_on_input:
             weights = self._ones(weights)       # the weights act on the way in; on the way out the outputs are summed
         if self.grouped and tokens >= self.GROUPED_FROM:
-            plan = ops.moe_plan(chosen, self.experts, ops.MOE_PAIR_TILE_ROWS if tokens * self.top >= self.PAIR_TILES_FROM * self.experts else ops.MOE_TILE_ROWS)
+            by_pairs = tokens * self.top >= self.PAIR_TILES_FROM * self.experts and ops.MOE_GROUPED_KERNEL != "mma"
+            plan = ops.moe_plan(chosen, self.experts, ops.MOE_PAIR_TILE_ROWS if by_pairs else ops.MOE_TILE_ROWS)
             hidden = ops.moe_grouped(x, self.gate_up, plan, gather_div=self.top, gated=self.gate, pair_scale=on_input,
                                      squared_relu=self.squared_relu)
             down = ops.moe_grouped(hidden, self.down, plan)
