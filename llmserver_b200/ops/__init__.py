@@ -145,7 +145,7 @@ def gate_up_silu(x, weight: torch.Tensor, group: int = 0) -> torch.Tensor:
     if x.dtype == torch.bfloat16 and group == GATE_UP_GROUP:
         from . import gemm_bf16
         fused = gemm_bf16.gate_up_silu_fused(x, weight)
-        if fused is None:
+        if fused is None and x.shape[0] >= gemm_bf16.PAIR_MIN_ROWS:
             fused = gemm_bf16.gated_by_pairs(x, weight, group, float("inf"), 1.0, 0.0)
         if fused is not None:
             return fused

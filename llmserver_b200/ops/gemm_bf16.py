@@ -313,9 +313,10 @@ def linear_bf16(x, weight: torch.Tensor, out: Optional[torch.Tensor] = None,
                 out = torch.empty((rows, cols), dtype=out_dtype, device=x.device)
             _small_m(x, weight, out, max(split, 0))
             return out
+    # (mm, which matmul of two matrices ends in: prompts of a few hundred tokens are bound by what their launches cost on the host)
     if out is not None:
-        return torch.matmul(x, weight.t(), out=out)
-    return torch.matmul(x, weight.t())
+        return torch.mm(x, weight.t(), out=out)
+    return torch.mm(x, weight.t())
 
 
 def _float32_by_library(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]) -> torch.Tensor:

@@ -155,14 +155,16 @@ def call(name: str, *args) -> None:
         raise KernelError(f"{name} failed ({status}): {library().llm_last_error().decode()}")
 
 
+# (the call behind torch.cuda.current_device, without its check that CUDA has been initialised: tensors on the device exist by then)
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device_index = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def stream_handle() -> int:
     """The raw handle of PyTorch's current stream on the current device (asked for at every launch: it is
     another stream while a CUDA graph is being captured)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_device_index())
     return torch.cuda.current_stream().cuda_stream
 
 
