@@ -376,6 +376,8 @@ __global__ void __launch_bounds__(kThreads) gemm_pair_kernel(const __grid_consta
     __syncwarp();
     tc5::fence_before();
     __syncthreads();
+    if (failed)                  // a wait ran out: copies that may still be in flight get time to land
+        for (int i = 0; i < 200; ++i) __nanosleep(1000);
     pair_sync();                 // nobody signals a block that has left, and the pair frees its tensor memory together
     tc5::fence_after();
     if (failed && threadIdx.x == 0 && p.error_flag) atomicExch(p.error_flag, 7);
