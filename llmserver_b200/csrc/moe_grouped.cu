@@ -63,7 +63,47 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
     for (int p = threadIdx.x; p < n_pairs; p += blockDim.x)
         if (chosen[p] < experts) atomicAdd(count + chosen[p], 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (experts <= (int)blockDim.x) {
+        // a thread per expert: the rows and the tiles in front of its own by a scan over the block (one thread that walked all
+        // experts and wrote their tiles made a plan over 64 experts 19.7 us long for 12288 pairs and 8.1 for 144; it takes 14.0
+        // and 3.4, most of the rest the atomics that count and place the pairs)
+        __shared__ int warp_rows[32], warp_tiles[32];
+        const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+        const int rows = e < experts ? count[e] : 0, mine = (rows + tile_rows - 1) / tile_rows;
+        int row_sum = rows, tile_sum = mine;
+#pragma unroll
+        for (int offset = 1; offset < 32; offset <<= 1) {
+            const int r = __shfl_up_sync(0xffffffffu, row_sum, offset), t = __shfl_up_sync(0xffffffffu, tile_sum, offset);
+            if (lane >= offset) {
+                row_sum += r;
+                tile_sum += t;
+            }
+        }
+        if (lane == 31) {
+            warp_rows[warp] = row_sum;
+            warp_tiles[warp] = tile_sum;
+        }
+        __syncthreads();
+        int first = row_sum - rows, tile = tile_sum - mine;
+        for (int w = 0; w < warp; ++w) {
+            first += warp_rows[w];
+            tile += warp_tiles[w];
+        }
+        if (e < experts) {
+            start[e] = first;
+            offsets[e] = first;
+            for (int k = 0; k < mine && tile + k < max_tiles; ++k) {
+                tiles[1 + 3 * (tile + k)] = e;
+                tiles[2 + 3 * (tile + k)] = first + k * tile_rows;
+                tiles[3 + 3 * (tile + k)] = min(tile_rows, rows - k * tile_rows);
+            }
+            if (e == experts - 1) {
+                start[experts] = first + rows;
+                offsets[experts] = first + rows;
+                tiles[0] = min(tile + mine, max_tiles);
+            }
+        }
+    } else if (threadIdx.x == 0) {
         int total = 0, tile = 0;
         for (int e = 0; e < experts; ++e) {
             start[e] = total;
