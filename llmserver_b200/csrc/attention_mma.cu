@@ -1150,32 +1150,29 @@ int launch_decode_cp_async(const AttnParams& given, cudaStream_t stream) {
     return llm_check_launch("attention_decode");
 }
 
+// Describes the page pool to TMA: its real extent, so that a block-table entry that names no page of the pool is copied as zeros
+// and nothing outside the pool is read.  False where the driver refuses (a pool of more than 2^32 rows, for one).
+template <int D>
+bool describe_pages(const AttnParams& p, CUtensorMap* map_k, CUtensorMap* map_v) {
+    if (D == 128) {
+        tma::EncodeTiled encode = tma::encode_tiled();
+        const long long page_heads = (long long)p.num_pages * p.n_kv_heads;
+        return encode != nullptr && tc5::make_page_map(map_k, encode, p.k_pages, p.page_size, page_heads) &&
+               tc5::make_page_map(map_v, encode, p.v_pages, p.page_size, page_heads);
+    }
+    const uint64_t rows = (uint64_t)p.num_pages * p.n_kv_heads * p.page_size;
+    return tma::make_map_bf16(map_k, p.k_pages, rows, D, (uint32_t)p.page_size) &&
+           tma::make_map_bf16(map_v, p.v_pages, rows, D, (uint32_t)p.page_size);
+}
+
 template <int D, bool PRECISE, bool DIFF>
-int launch_decode_tma(const AttnParams& given, cudaStream_t stream) {
+int launch_decode_tma(const AttnParams& given, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t stream) {
     AttnParams p = given;
     auto* kernel = attention_decode_tma_kernel<D, PRECISE, DIFF>;
     // Two blocks share an SM.  Beyond one wave of them the order in which sequences start decides how raggedly the last wave
     // ends: 61 sequences of 301 to 4077 keys that lie shortest first, a decode step of the 8B shape 7.51 ms as they lie and
     // 6.70 ms longest first (more splits instead: 7.3 ms with two parts, 7.8 with three).  Within a wave all start at once.
     p.by_length = p.n_seqs <= kThreads && (long long)p.max_splits * p.n_kv_heads * p.n_seqs > 2 * llm_sm_count();
-    // rows of the page pool seen as a [pages * kv_heads * page_size, D] matrix: the real extent, so that a block-table
-    // entry that names no page of the pool is copied as zeros and nothing outside the pool is read
-    const uint64_t rows = (uint64_t)p.num_pages * p.n_kv_heads * p.page_size;
-    CUtensorMap map_k, map_v;
-    bool described;
-    if (D == 128) {
-        tma::EncodeTiled encode = tma::encode_tiled();
-        described = encode != nullptr && tc5::make_page_map(&map_k, encode, p.k_pages, p.page_size, (long long)p.num_pages * p.n_kv_heads) &&
-                    tc5::make_page_map(&map_v, encode, p.v_pages, p.page_size, (long long)p.num_pages * p.n_kv_heads);
-    } else {
-        described = tma::make_map_bf16(&map_k, p.k_pages, rows, D, (uint32_t)p.page_size) &&
-                    tma::make_map_bf16(&map_v, p.v_pages, rows, D, (uint32_t)p.page_size);
-    }
-    if (!described && DIFF) {
-        llm_set_error("attention_diff_decode: cannot describe the cache pages to TMA");
-        return LLM_REFUSED;
-    }
-    if (!described) return launch_decode_cp_async<D, D, PRECISE>(p, stream);
     const size_t shared = (size_t)kDecodeStages * 2 * kTileKeys * D * 2 + (size_t)16 * D * 2 + 1024;
     if (int limit_status = llm_raise_shared_limit(reinterpret_cast<const void*>(kernel), shared, "attention_decode_tma")) return limit_status;
     dim3 grid(p.max_splits, p.n_kv_heads, p.n_seqs);
@@ -1225,7 +1222,8 @@ int launch_decode_tma(const AttnParams& given, cudaStream_t stream) {
 template <int D, bool PRECISE = false, bool DIFF = false>
 int launch_decode(const AttnParams& p, cudaStream_t stream) {
     const bool whole_pages = p.page_size >= 8 && p.page_size <= kTileKeys && kTileKeys % p.page_size == 0 && p.page_size % 8 == 0;
-    const bool by_tma = whole_pages && aligned16(p.k_pages) && aligned16(p.v_pages);
+    CUtensorMap map_k, map_v;
+    const bool by_tma = whole_pages && aligned16(p.k_pages) && aligned16(p.v_pages) && describe_pages<D>(p, &map_k, &map_v);
     AttnParams q = p;
     // up to 8 splits (the portable cluster size) or exactly 16 (allowed on request) merge inside the kernel; others, or the cp.async kernel, go through the
     // scratch buffers and the merge kernel
@@ -1235,10 +1233,10 @@ int launch_decode(const AttnParams& p, cudaStream_t stream) {
         return LLM_REFUSED;
     }
     if (DIFF && !by_tma) {
-        llm_set_error("attention_diff_decode: pages of %d tokens are not supported", p.page_size);
+        llm_set_error("attention_diff_decode: %d pages of %d tokens are not supported", p.num_pages, p.page_size);
         return LLM_REFUSED;
     }
-    int status = by_tma ? launch_decode_tma<D, PRECISE, DIFF>(q, stream) : launch_decode_cp_async<D, D, PRECISE>(q, stream);
+    int status = by_tma ? launch_decode_tma<D, PRECISE, DIFF>(q, map_k, map_v, stream) : launch_decode_cp_async<D, D, PRECISE>(q, stream);
     if (status != LLM_OK || p.max_splits <= 1 || q.cluster_merge) return status;
     dim3 merge_grid(p.n_q_heads, p.n_seqs);
     llm_launch(attention_decode_merge_kernel<D>, merge_grid, D < 128 ? D : 128, 0, stream, p);

@@ -73,3 +73,34 @@ def test_longest_first_takes_every_sequence_once(n_seqs):
         want = plain_rows(qkv, k_pages, v_pages, tables[row], context, context - 1, [0], heads, kv_heads, dim, page_size, dim ** -0.5, row)
         worst = max(worst, relative_error(out[row:row + 1], want))
     assert worst <= 2e-2, f"relative error {worst:.3e}"
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("precise", [False, True])
+@pytest.mark.parametrize("contexts", [[900], [3000, 700]])
+def test_pages_that_tma_cannot_describe(monkeypatch, dim, precise, contexts):
+    """A pool said to have 2^31 - 1 pages (every table entry names one of those that exist) has more rows than a tensor map can: the
+    step runs the other kernel, whose splits do not merge in a cluster, and its results are written all the same."""
+    from llmserver_b200 import ops
+    from llmserver_b200.ops import attention_bf16
+    from llmserver_b200.ops.library import check_wait_errors
+    heads, kv_heads, page_size = 16, 4, 16
+    batch = decode_batch(contexts)
+    qkv, q_stride, k_pages, v_pages, tables = paged_case(3, [1] * len(contexts), contexts, heads, kv_heads, dim, page_size)
+    torch.full((len(contexts), heads * dim), float("nan"), dtype=torch.bfloat16, device=DEVICE)      # what the allocator hands out next
+    launch, launched = attention_bf16.call, []
+
+    def call(name, *args):
+        launched.append(name)
+        place = {"llm_attention_mma": 14, "llm_attention_mma_sinks": 15}[name]
+        assert args[place] == k_pages.shape[0]
+        launch(name, *args[:place], 2 ** 31 - 1, *args[place + 1:])
+
+    monkeypatch.setattr(attention_bf16, "call", call)
+    got = ops.attention(qkv, batch, tables, k_pages, v_pages, heads, kv_heads, dim, dim ** -0.5, precise=precise, q_stride=q_stride)
+    torch.cuda.synchronize()
+    check_wait_errors()
+    assert launched == ["llm_attention_mma_sinks" if precise else "llm_attention_mma"]
+    for row, context in enumerate(contexts):
+        want = plain_rows(qkv, k_pages, v_pages, tables[row], context, context - 1, [0], heads, kv_heads, dim, page_size, dim ** -0.5, row)
+        assert relative_error(got[row:row + 1], want) <= 2e-2      # of bfloat16 weights and results, as in the test above
