@@ -11,7 +11,8 @@
 //   gated   W holds gate rows and up rows; the tile's 256 rows of W are 128 gate rows and the same features' 128 up rows,
 //           fetched as four boxes of 64 rows, so either arrangement of the matrix can be read: gate rows in front of all up
 //           rows, or groups of 64 in turn.  A thread finds gate and up of an output in columns j and 128 + j of its own row
-//           and writes min(g, limit) * sigmoid(alpha * min(g, limit)) * (clamp(u) + up_shift), rounded once to bfloat16;
+//           and writes min(g, limit) * sigmoid(alpha * min(g, limit)) * (clamp(u) + up_shift), rounded once to bfloat16 (with the exact
+//           division: the hardware's gives 0 for gates between -87.3 and -88.7, where the result is still a number);
 //   plain   the 32-bit sums are written as they are;
 //   squared relu    max(sum, 0)^2 rounded once to bfloat16.
 //
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(kThreads) gemm_pair_kernel(const __grid_consta
                                 g = fminf(g, p.limit);
                                 u = fminf(fmaxf(u, -p.limit), p.limit);
                             }
-                            y[h] = __fdividef(g, 1.0f + __expf(-p.alpha * g)) * (u + p.up_shift);
+                            y[h] = g / (1.0f + __expf(-p.alpha * g)) * (u + p.up_shift);
                         }
                         words[e / 2] = tc5::pack2(y[0], y[1]);
                     }

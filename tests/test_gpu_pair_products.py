@@ -40,6 +40,28 @@ def test_gated_product(rows, features, inner, interleave):
         assert error.max() <= 2.0 ** -8, f"{float(error.max()):.2e}"
 
 
+@pytest.mark.parametrize("by_pairs", [False, True])
+def test_gate_over_its_range(by_pairs):
+    """Products of one term each, so that gates and values are the weights themselves: gates from -88.5, whose exponential is still a
+    number, to 88.  The bound: the hardware's exponential is off by up to 2 + 1.17 |x| units in the last place at x, beside one rounding to 8 bits."""
+    from llmserver_b200 import ops
+    from llmserver_b200.ops.library import check_wait_errors
+    features, inner, tokens = 256, 64, 256
+    gate = torch.cat([torch.arange(-88.5, -80.0, 0.5), torch.linspace(-80.0, 88.0, features - 17)]).to(torch.bfloat16).to(DEVICE)
+    up = torch.linspace(-8.0, 8.0, features).to(torch.bfloat16).to(DEVICE)
+    weight = torch.zeros((1, 2 * features, inner), dtype=torch.bfloat16, device=DEVICE)
+    weight[0, :features, 0], weight[0, features:, 0] = gate, up
+    x = torch.zeros((tokens, inner), dtype=torch.bfloat16, device=DEVICE)
+    x[:, 0] = 1.0
+    plan = ops.moe_plan(torch.zeros((tokens, 1), dtype=torch.int32, device=DEVICE), 1, ops.MOE_PAIR_TILE_ROWS if by_pairs else ops.MOE_TILE_ROWS)
+    got = ops.moe_grouped(x, weight, plan, gather_div=1, gated=(100.0, 1.0)).double()
+    torch.cuda.synchronize()
+    check_wait_errors()
+    g, u = gate.double(), up.double()
+    want = g * torch.sigmoid(g) * (u + 1.0)
+    assert ((got - want).abs() <= (2.0 ** -8 + 106 * 2.0 ** -23) * want.abs()).all(), f"{got[0, :20]} {want[:20]}"
+
+
 def test_gated_product_keeps_nan():
     """Without a limit a NaN in the gate stays one (a minimum with infinity would drop it)."""
     from llmserver_b200.ops import gemm_bf16
@@ -87,7 +109,5 @@ def test_expert_products_on_tiles_of_256_rows(tokens, experts, top, features, in
     check_wait_errors()
     few, many = got[ops.MOE_TILE_ROWS], got[ops.MOE_PAIR_TILE_ROWS]
     assert torch.equal(many[1], few[1])
-    # the gate's division is the exact one in one kernel and the hardware's in the other: one step of 2^-8 where a rounding flips
-    assert ((many[0].double() - few[0].double()).abs() <= 2.0 ** -7 * few[0].double().abs() + 1e-6).all()
-    scale = few[2].abs().max()
-    assert ((many[2] - few[2]).abs() <= 2.0 ** -8 * scale).all()
+    assert torch.equal(many[0], few[0])
+    assert torch.equal(many[2], few[2])
