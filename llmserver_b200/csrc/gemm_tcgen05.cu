@@ -468,13 +468,19 @@ __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_con
         if (MANY) {      // a lane per token: its parts are independent loads, where a warp per token waits for memory token by token
             const int m = (warp - 2) * 32 + lane;
             if (m < p.m) {
-                float squares[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-                for (int i = 0; i < p.scale.n_parts; i += 4)
+                // what the lanes of a warp hold below, and their sum in the order of warp_sum: the same bits for the same parts
+                float squares[32];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c)
+                for (int c = 0; c < 32; ++c) squares[c] = 0.0f;
+                for (int i = 0; i < p.scale.n_parts; i += 32)
+#pragma unroll
+                    for (int c = 0; c < 32; ++c)
                         if (i + c < p.scale.n_parts) squares[c] += p.scale.parts[(size_t)(i + c) * p.scale.stride + m];
-                row_scale[m] = rsqrtf(((squares[0] + squares[1]) + (squares[2] + squares[3])) / (float)p.k + p.scale.eps);
+#pragma unroll
+                for (int half = 16; half > 0; half >>= 1)
+#pragma unroll
+                    for (int c = 0; c < half; ++c) squares[c] += squares[c + half];
+                row_scale[m] = rsqrtf(squares[0] / (float)p.k + p.scale.eps);
             }
         } else {
             for (int m = warp - 2; m < p.m; m += n_warps - 2) {

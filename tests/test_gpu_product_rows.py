@@ -77,3 +77,27 @@ def test_fused_heads(rows):
         results.append((out[:, :heads * dim], k_pages, v_pages))
     for name, got, want in zip(("queries", "keys", "values"), *results):
         close(got, want, torch.bfloat16, name, factor=2.0)      # either side is rounded where the other is not
+
+
+@pytest.mark.parametrize("n_parts", [1, 5, 32, 40, 64, 200])
+def test_a_row_is_divided_alike_in_every_step(n_parts):
+    """The sums of squares that a row's scale is made of are added in the order that their number gives, whether the step has up to
+    16 rows, up to 64 or more: the same row and parts give the same bits."""
+    from llmserver_b200 import ops
+    from llmserver_b200.ops import gemm_bf16
+    from llmserver_b200.ops.library import call, check_wait_errors, stream_handle
+    cols, inner = 256, 512
+    w = rand((cols, inner), torch.bfloat16, 2, inner ** -0.5)
+    x = rand((16, inner), torch.bfloat16, 1)
+    parts = rand((n_parts, 16), torch.float32, 3).abs() * torch.logspace(-3, 1, n_parts, device=DEVICE)[:, None]
+    results = []
+    for rows in (16, 17, 64, 65, 128):
+        many = x.repeat(8, 1)[:rows].contiguous()
+        scaled = ops.RowScaled(many, parts.repeat(1, 8).contiguous(), 1e-6)
+        out = torch.empty((rows, cols), dtype=torch.float32, device=DEVICE)
+        call("llm_gemm_small_m", many.data_ptr(), w.data_ptr(), out.data_ptr(), rows, cols, inner, cols, 1, 1, *scaled.scale_args(),
+             gemm_bf16.error_flag(DEVICE).data_ptr(), stream_handle())
+        torch.cuda.synchronize()
+        check_wait_errors()
+        results.append(out[:16])
+    assert all(torch.equal(result, results[0]) for result in results)
