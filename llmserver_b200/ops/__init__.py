@@ -14,13 +14,13 @@ import torch
 
 from .library import (KernelError, call, check, declare, dtype_code, launch_count, library, pointer,
                       require_device, stream_handle, wait_error_flag)
-from .stream import STREAM_MANY_ROWS, STREAM_ROWS, RowScaled, StreamSink
+from .stream import STREAM_MANY_ROWS, STREAM_ROWS, RowScaled, StreamSink, stream_rows
 
 __all__ = ["KernelError", "embedding", "add_rmsnorm", "rmsnorm", "silu_mul", "sample", "qk_norm_rope_kv_write",
            "attention_generic", "rope_kv_write_split", "normed_add_rmsnorm", "scaled_add_rmsnorm", "moe_route", "moe_select", "indexed_linear", "moe_combine", "moe_plan", "moe_grouped",
            "moe_grouped_supported", "moe_combine_rows", "ExpertPlan",
            "clamped_glu", "clamped_gate_up", "gemm_f32", "linear", "linear_wide", "qkv_projection", "gate_up_silu", "interleave_gate_up", "require_device", "library", "launch_count",
-           "RowScaled", "StreamSink", "STREAM_ROWS", "STREAM_MANY_ROWS", "unscaled_rows_supported", "norm_rope_units", "rotate_units", "attention_diff", "gla_supported",
+           "RowScaled", "StreamSink", "STREAM_ROWS", "STREAM_MANY_ROWS", "stream_rows", "unscaled_rows_supported", "norm_rope_units", "rotate_units", "attention_diff", "gla_supported",
            "gla_recurrent", "head_linear", "relu_squared", "tanh_narrow", "softcap_", "scaled_sum", "token_shift_mix",
            "short_conv_units", "matrix_recurrence_supported", "wkv_recurrent", "delta_rule_recurrent", "retention_recurrent", "ssd_recurrent", "decay_recurrence_supported",
            "gelu_mul", "grouped_rmsnorm", "conv_norm_kv", "streams_norm", "unit_linear_wide", "gated_scan"]

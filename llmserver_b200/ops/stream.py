@@ -17,11 +17,28 @@ import torch
 # LLMSERVER_B200_STREAM_EPILOGUES=0 switches it off: the stand-alone add + norm kernel then runs at every row count.
 STREAM_ROWS = (min(max(int(os.environ.get("LLMSERVER_B200_STREAM_ROWS", "16")), 0), 128)
                if os.environ.get("LLMSERVER_B200_STREAM_EPILOGUES", "1") != "0" else 0)
-# Where neither variable says otherwise it runs this way up to all rows that the product kernel takes.  Steps that are not
-# replayed (prompts) are bound by what their launches cost on the host, and this way has five a layer instead of nine: 8B shape,
-# ms, with the stand-alone kernels from 17 rows on and without: prompts of 20 tokens 5.47 / 3.87, 64 5.49 / 4.12, 119 5.44 / 4.81;
-# replayed decode steps of 24 sequences 5.77 / 5.68, 40 6.06 / 5.95, 64 6.97 / 6.80.
+# The most rows that may run this way at all; ``stream_rows`` says how many do.
 STREAM_MANY_ROWS = STREAM_ROWS if "LLMSERVER_B200_STREAM_ROWS" in os.environ else 128 if STREAM_ROWS else 0
+STREAM_DEVICE_ROWS, STREAM_LAUNCH_WIDTH = 64, 4096
+
+
+def stream_rows(width: int, decode: bool) -> int:
+    """Up to how many rows a step over a stream of ``width`` columns runs this way where the environment does not say; ``decode``: it
+    is a step of single tokens, which graphs replay.
+
+    Up to 64 rows every step: the products are level with the library's and four launches a layer fall away.  Beyond, a token tile is
+    as large as a weight tile and the library's products are faster on the device, which decides wherever launches are replayed or
+    the matrices are wide; only steps that the host's launches bound gain.  Stand-alone kernels from 17 rows on / none, ms:
+    replayed decode steps, contexts of 301 to 2000: width 2048 2.33 / 2.24 at 24 rows, 2.94 / 2.95 at 64, 3.93 / 4.07 at 96, 4.72 / 4.98
+    at 128; 8B shape 4.75 / 4.70 at 24, 5.55 / 5.43 at 48, 5.63 / 5.40 at 61, 7.04 / 7.23 at 96, 8.09 / 8.51 at 128; 14B shape (5120) 6.68 /
+    6.42 at 24, 7.91 / 7.94 at 64, 9.90 / 9.76 at 96, 11.19 / 11.43 at 128; 32B shape (5120) 15.66 / 15.50 at 64.  Prompts: width 2048 4.33 /
+    3.16 at 128 tokens; 8B 5.38 / 3.92 at 20, 6.18 / 4.38 at 64, 5.39 / 4.83 at 100, 5.34 / 5.13 at 128; 14B 6.02 / 5.61 at 20, 6.52 / 6.31
+    at 64, 6.94 / 6.95 at 100, 7.13 / 7.21 at 128; 32B 13.6 / 13.1 at 40, 14.4 / 14.1 at 64, 15.2 / 16.0 at 100, 15.8 / 16.9 at 128."""
+    if STREAM_MANY_ROWS <= STREAM_ROWS:
+        return STREAM_MANY_ROWS
+    return STREAM_DEVICE_ROWS if decode or width > STREAM_LAUNCH_WIDTH else STREAM_MANY_ROWS
+
+
 NO_SCALE = (0, 0, 0, 0.0)
 
 

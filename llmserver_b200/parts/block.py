@@ -4,6 +4,7 @@ from __future__ import annotations
 from .base import Block
 import torch
 
+from .. import ops
 from ..weights.declare import MIXING, NORM, WeightDecl
 from .norm import NormedDelta, ScaledDelta, StreamsDelta, add_and_read
 from .registry import BLOCKS
@@ -29,17 +30,24 @@ class PreNormBlock(Block):
         # With few rows, parts that can do so add their results to the stream themselves and prepare the next norm's
         # input (``sink``), and take a norm's output before its division (``unscaled``); see ``ops.stream``.  Parts
         # and norms that cannot are called as ever.
-        normed = _add_norm(self.mixer_norm, residual, delta, self.mixer)
-        sink = self.feed_forward_norm.sink(residual, self.feed_forward) if self.mixer.feeds_stream else None
+        normed = _add_norm(self.mixer_norm, residual, delta, self.mixer, batch)
+        sink = _sink(self.feed_forward_norm, residual, self.feed_forward, batch) if self.mixer.feeds_stream else None
         mixed = self.mixer.forward(normed, batch, cache, sink=sink) if sink is not None else self.mixer.forward(normed, batch, cache)
-        normed = _add_norm(self.feed_forward_norm, residual, sink if sink is not None and sink.added else mixed, self.feed_forward)
-        sink = after[0].sink(residual, after[1]) if after is not None and self.feed_forward.feeds_stream else None
+        normed = _add_norm(self.feed_forward_norm, residual, sink if sink is not None and sink.added else mixed, self.feed_forward, batch)
+        sink = _sink(after[0], residual, after[1], batch) if after is not None and self.feed_forward.feeds_stream else None
         out = self.feed_forward.forward(normed, sink=sink) if sink is not None else self.feed_forward.forward(normed)
         return residual, (sink if sink is not None and sink.added else out)
 
 
-def _add_norm(norm, residual, delta, consumer):
-    if getattr(consumer, "takes_unscaled", False) and norm.sink(residual, consumer) is not None:
+def _sink(norm, residual, consumer, batch):
+    """What ``norm`` offers the part in front of it, in steps of so few rows that its products are the faster ones."""
+    if residual.shape[0] > ops.stream_rows(residual.shape[-1], decode=batch.max_q_len == 1):
+        return None
+    return norm.sink(residual, consumer)
+
+
+def _add_norm(norm, residual, delta, consumer, batch):
+    if getattr(consumer, "takes_unscaled", False) and _sink(norm, residual, consumer, batch) is not None:
         return norm.add_norm(residual, delta, unscaled=True)
     return norm.add_norm(residual, delta)
 
