@@ -1557,10 +1557,10 @@ LLM_EXPORT int llm_attention_mma_sinks(const void* q, int q_stride, const void* 
 #undef LLM_PRECISE
 }
 
-// Both maps of differential attention for a step of single tokens: maps_out (float32 [N, n_q_heads, 2, 128]) gets
+// Both maps of differential attention for the single tokens of a step: maps_out (float32 [N, n_q_heads, 2, 128]) gets
 // softmax(cap(q_m . k_m * scale)) V of each head and map.  A head of the queries and of the K pages is [map 1 | map 2] of 64
 // elements each, values have 128; groups of up to 8 heads; pages as the TMA decode kernel takes them.  partial_out holds
-// [N, 2 n_q_heads, max_splits, 128] floats.  The other arguments as for llm_attention_mma.
+// [n_seqs, 2 n_q_heads, max_splits, 128] floats.  The other arguments as for llm_attention_mma.
 LLM_EXPORT int llm_attention_diff_decode(const void* q, int q_stride, const void* k_pages, const void* v_pages, const int* block_tables,
                                          int max_blocks, const int* q_start, const int* context_len, float* maps_out, int n_seqs,
                                          int n_q_heads, int n_kv_heads, int page_size, int num_pages, float scale, float cap, int window,
@@ -1592,6 +1592,7 @@ LLM_EXPORT int llm_attention_diff_decode(const void* q, int q_stride, const void
     p.max_splits = max_splits;
     p.partial_out = partial_out;
     p.partial_ml = partial_ml;
+    p.slot_by_seq = 1;
     p.old_keys_settled = old_keys_settled;
     p.cluster_merge = decode_cluster_merge_enabled() ? 1 : 0;
     p.error_flag = error_flag;

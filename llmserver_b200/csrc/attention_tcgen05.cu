@@ -651,13 +651,13 @@ LLM_EXPORT int llm_attention_prefill_tcgen05_precise(const void* q, int q_stride
                                   total_pairs, error_flag, sinks, true, chunk, bias, bias_len, keep, gate, gate_stride, stream);
 }
 
-// Both maps of differential attention for every token of the step: maps_out (float32 [n_tokens, n_q_heads, 2, 128], 16-byte aligned)
-// gets softmax(cap(q_m . k_m * scale)) V of each head and map.  A head of the queries and of the K pages is [map 1 | map 2] of
+// Both maps of differential attention: maps_out (float32 [n_tokens, n_q_heads, 2, 128], 16-byte aligned) gets
+// softmax(cap(q_m . k_m * scale)) V of each head and map, of every token or, with skip_single, of the sequences with more than one.  A head of the queries and of the K pages is [map 1 | map 2] of
 // 64 elements each, values have 128.  `cap` 0: scores are not capped.  The other arguments as above.
 LLM_EXPORT int llm_attention_diff_prefill(const void* q, int q_stride, int n_tokens, const void* k_pages, const void* v_pages,
                                           const int* block_tables, int max_blocks, const int* q_start, const int* context_len,
                                           float* maps_out, int n_seqs, int n_q_heads, int n_kv_heads, int page_size, int num_pages,
-                                          float scale, float cap, int window, int pairing, int total_pairs, int* error_flag,
+                                          float scale, float cap, int window, int skip_single, int pairing, int total_pairs, int* error_flag,
                                           cudaStream_t stream) {
     if (total_pairs <= 0) return LLM_OK;
     if (num_pages <= 0 || !llm_attention_prefill_tcgen05_supports(kDim, n_q_heads, n_kv_heads, page_size) || !aligned16(q) || q_stride % 8 ||
@@ -686,6 +686,7 @@ LLM_EXPORT int llm_attention_diff_prefill(const void* q, int q_stride, int n_tok
     p.page_size = page_size;
     p.scale_log2 = scale * kLog2e;
     p.window = window;
+    p.skip_single = skip_single;
     p.pairing = pairing;
     p.error_flag = error_flag;
     p.maps_out = maps_out;

@@ -330,27 +330,17 @@ def try_attention_diff(qkv, gate_column, batch, block_tables, k_pages, v_pages, 
 def _attention_diff_maps(qkv, gate, batch, block_tables, k_pages, v_pages, n_q_heads, n_kv_heads, scale, cap, window, lam, eps,
                          out_scale, out) -> None:
     """Differential attention as attention with each of the maps (32-bit results), then one kernel that subtracts them: prompt portions
-    (and single tokens beside them) on the tcgen05 kernel, steps of single tokens on the TMA decode kernel."""
+    on the tcgen05 kernel, single tokens, alone or beside portions, on the TMA decode kernel."""
     row_width, group, page_size = qkv.shape[1], n_q_heads // n_kv_heads, k_pages.shape[2]
     window, flag = int(window or 0), wait_error_flag(qkv.device).data_ptr()
     maps = torch.empty((batch.n_tokens, n_q_heads, 2, 128), dtype=torch.float32, device=qkv.device)
-    if batch.max_q_len == 1:
-        _, _, _, split_len, max_splits = plan(batch, group, n_kv_heads, qkv.device, span=window or None)
-        partial_out = partial_ml = None
-        if max_splits > 1:
-            key = ("attention_diff_scratch", n_q_heads, max_splits)
-            if key not in batch.scratch:
-                batch.scratch[key] = (torch.empty((batch.n_tokens, 2 * n_q_heads, max_splits, 128), dtype=torch.float32, device=qkv.device),
-                                      torch.empty((batch.n_tokens, 2 * n_q_heads, max_splits, 2), dtype=torch.float32, device=qkv.device))
-            partial_out, partial_ml = batch.scratch[key]
-        call("llm_attention_diff_decode", qkv.data_ptr(), row_width, k_pages.data_ptr(), v_pages.data_ptr(), block_tables.data_ptr(),
-             block_tables.shape[-1], batch.q_start.data_ptr(), batch.context_len.data_ptr(), maps.data_ptr(), batch.n_seqs, n_q_heads,
-             n_kv_heads, page_size, k_pages.shape[0], float(scale), max(float(cap or 0.0), 0.0), window, split_len, max_splits,
-             0 if partial_out is None else partial_out.data_ptr(), 0 if partial_ml is None else partial_ml.data_ptr(),
-             int(EARLY_KEYS and getattr(batch, "keys_settled", False)), flag, stream_handle())
-    else:
-        # as for the other portions, but a row tile is two blocks, one per map
-        tile_counts = [-(-length // (PREFILL_TILE // group)) for length in batch.q_lens]
+    run_portions, _, run_decode, split_len, max_splits = plan(batch, group, n_kv_heads, qkv.device, span=window or None)
+    if run_portions:
+        # As for the other portions, but a row tile is two blocks, one per map.  A single token in a tile of its own would fill `group`
+        # of 128 rows, read its cache once per map and walk it in one block: a step with 48 of them behind 900 to 4001 keys
+        # beside a prompt of 256 takes 2.57 ms that way and 2.41 with them on the decode kernel; 21 behind 140 to 2300 beside
+        # 2000 tokens 4.12 and 4.18 (the launches show where the portions fill the GPU).
+        tile_counts = [-(-length // (PREFILL_TILE // group)) for length in batch.q_lens if length > 1]
         paired = sum((count + 1) // 2 for count in tile_counts)
         slots = _block_slots(qkv.device, False)
         cost_paired = 2.0 * -(-paired * 2 * n_kv_heads // slots)
@@ -358,7 +348,20 @@ def _attention_diff_maps(qkv, gate, batch, block_tables, k_pages, v_pages, n_q_h
         pairing = cost_paired < cost_single if FORCE_PAIRING is None else FORCE_PAIRING
         call("llm_attention_diff_prefill", qkv.data_ptr(), row_width, batch.n_tokens, k_pages.data_ptr(), v_pages.data_ptr(),
              block_tables.data_ptr(), block_tables.shape[-1], batch.q_start.data_ptr(), batch.context_len.data_ptr(), maps.data_ptr(),
-             batch.n_seqs, n_q_heads, n_kv_heads, page_size, k_pages.shape[0], float(scale), max(float(cap or 0.0), 0.0), window, int(pairing),
-             paired if pairing else sum(tile_counts), flag, stream_handle())
+             batch.n_seqs, n_q_heads, n_kv_heads, page_size, k_pages.shape[0], float(scale), max(float(cap or 0.0), 0.0), window,
+             int(run_decode), int(pairing), paired if pairing else sum(tile_counts), flag, stream_handle())
+    if run_decode:
+        partial_out = partial_ml = None
+        if max_splits > 1:
+            key = ("attention_diff_scratch", n_q_heads, max_splits)
+            if key not in batch.scratch:
+                batch.scratch[key] = (torch.empty((batch.n_seqs, 2 * n_q_heads, max_splits, 128), dtype=torch.float32, device=qkv.device),
+                                      torch.empty((batch.n_seqs, 2 * n_q_heads, max_splits, 2), dtype=torch.float32, device=qkv.device))
+            partial_out, partial_ml = batch.scratch[key]
+        call("llm_attention_diff_decode", qkv.data_ptr(), row_width, k_pages.data_ptr(), v_pages.data_ptr(), block_tables.data_ptr(),
+             block_tables.shape[-1], batch.q_start.data_ptr(), batch.context_len.data_ptr(), maps.data_ptr(), batch.n_seqs, n_q_heads,
+             n_kv_heads, page_size, k_pages.shape[0], float(scale), max(float(cap or 0.0), 0.0), window, split_len, max_splits,
+             0 if partial_out is None else partial_out.data_ptr(), 0 if partial_ml is None else partial_ml.data_ptr(),
+             int(EARLY_KEYS and getattr(batch, "keys_settled", False)), flag, stream_handle())
     call("llm_attention_diff_combine", maps.data_ptr(), gate, row_width, out.data_ptr(), batch.n_tokens, n_q_heads, float(lam), float(eps),
          float(out_scale), stream_handle())

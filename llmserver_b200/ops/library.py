@@ -36,7 +36,7 @@ SIGNATURES = {
     "llm_scaled_add_rmsnorm": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _F, _I, _I, _I, _S],
     "llm_attention_diff": [_P, _I, _P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _I, _F, _F, _F, _P, _I, _S],
     "llm_attention_diff_mma_supports": [_I, _I, _I, _I],
-    "llm_attention_diff_prefill": [_P, _I, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _I, _I, _P, _S],
+    "llm_attention_diff_prefill": [_P, _I, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _I, _I, _I, _P, _S],
     "llm_attention_diff_decode": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _I, _I, _P, _P, _I, _P, _S],
     "llm_attention_diff_combine": [_P, _P, _I, _P, _I, _I, _F, _F, _F, _S],
     "llm_attention_diff_mma": [_P, _I, _P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _I, _F, _F, _F, _P, _I, _I, _P, _S],

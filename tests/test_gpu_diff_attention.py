@@ -80,3 +80,15 @@ MANY = [1, 63, 64, 65, 127, 128, 129, 700, 3000, 2, 1025, 1087, 1088, 1089]
 def test_single_tokens(heads, kv_heads, page_size, contexts, window, cap):
     """From one block to more than a wave of them; contexts of one split, of several, and beyond the window."""
     both(heads, kv_heads, page_size, window, cap, [1] * len(contexts), contexts, True)
+
+
+def test_single_tokens_beside_portions_run_the_decode_kernel(monkeypatch):
+    """In one block of the prompt kernel a token would walk all of its context; results as in the tests above."""
+    from llmserver_b200.ops import attention_bf16
+    launch, launched = attention_bf16.call, []
+    monkeypatch.setattr(attention_bf16, "call", lambda name, *args: (launched.append(name), launch(name, *args))[1])
+    for q_lens, contexts in (([1, 40, 1], [3000, 700, 64]), ([200, 1], [200, 2500]), ([64], [64]), ([1, 1], [9, 900])):
+        del launched[:]
+        both(8, 2, 16, 0, 30.0, q_lens, contexts, True)
+        kernels = [name for name in launched if "diff" in name]
+        assert ("llm_attention_diff_decode" in kernels) == (1 in q_lens) and ("llm_attention_diff_prefill" in kernels) == (max(q_lens) > 1)
