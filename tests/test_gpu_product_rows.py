@@ -101,3 +101,52 @@ def test_a_row_is_divided_alike_in_every_step(n_parts):
         check_wait_errors()
         results.append(out[:16])
     assert all(torch.equal(result, results[0]) for result in results)
+
+
+def test_steps_of_more_than_64_rows(tiny_folders, monkeypatch):
+    """A prompt of 100 tokens runs without stand-alone norms (but for the first layer's input and the final norm); a step that decodes
+    96 requests runs with them, eagerly and replayed; all against the plain implementation."""
+    from helpers import assert_close, plain_logits, tokens_for
+    from llmserver_b200 import ops
+    from llmserver_b200.cache import CacheManager
+    from llmserver_b200.engine.step import StepFunction
+    from llmserver_b200.models import load_model
+    from llmserver_b200.sampling import SamplingRow
+    folder, rows = tiny_folders["e"], 96
+    model = load_model(folder, "bfloat16", "cuda:0")
+    cache = CacheManager(model.cache_needs(), 16, 3 * rows + 16, num_slots=rows, prefix_sharing=False)
+    cache.materialize(model.runtime.device, model.runtime.dtype)
+    step = StepFunction(model, cache)
+    step.enable_graphs(64, rows)
+    norm, calls = ops.add_rmsnorm, []
+    monkeypatch.setattr(ops, "add_rmsnorm", lambda *args, **kwargs: (calls.append(1), norm(*args, **kwargs))[1])
+    vocab, layers = model.spec.vocab_size, len(model.spec.schedule)
+    tokens = tokens_for(vocab, 100, 3)
+    step.admit("prompt")
+    got = step.run([("prompt", tokens, list(range(100)))])
+    assert len(calls) == 2
+    assert_close(got.float().cpu().numpy(), plain_logits(folder, tokens), "bfloat16", "a prompt of 100 tokens")
+    step.release("prompt")
+    prompts = [tokens_for(vocab, 3 + row % 30, 100 + row) for row in range(rows)]
+    for row, prompt in enumerate(prompts):
+        step.admit(row)
+        step.run([(row, prompt, [])])
+    want = {row: plain_logits(folder, prompts[row] + [row])[-1:] for row in (0, 1, 50, 95)}
+    for turn in range(4):      # the third replays
+        del calls[:]
+        entries = [(row, [row], [0]) for row in range(rows)]
+        if turn == 0:
+            logits = step.run(entries)
+        else:
+            step.run_and_sample(entries, [SamplingRow()] * rows)
+            graph = step.graphs.graphs.get(rows)
+            logits = graph.logits if graph is not None else None
+        if turn != 3:
+            assert len(calls) == 2 * layers + 1
+        for row in range(rows):
+            step.computed[row] -= 1      # the same step again
+        if logits is not None:
+            for row, expected in want.items():
+                assert_close(logits[row:row + 1].float().cpu().numpy(), expected, "bfloat16", f"turn {turn}, row {row}")
+    assert step.graph_steps > 0
+    step.check_errors()
