@@ -453,7 +453,7 @@ int launch_form(int form, const void* a, int n_rows, const void* w, long long w_
 
 }  // namespace
 
-// `interleave`: rows of gate and up in turn (0: all gate rows in front); groups of 64 need features in whole tiles of 128.
+// `interleave`: rows of gate and up in turn (0: all gate rows in front); groups of 64 need a multiple of 64 features.
 LLM_EXPORT int llm_gemm_pair_supports(int out_cols, int inner, int interleave) {
     return inner >= 64 && inner % 8 == 0 && out_cols > 0 && out_cols % 8 == 0 && (interleave == 0 || (interleave == kBox && out_cols % kBox == 0));
 }

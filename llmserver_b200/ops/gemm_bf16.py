@@ -410,13 +410,33 @@ def qkv_rope_fused(x: torch.Tensor, weight: torch.Tensor, q_weight, k_weight, in
 
 
 FUSE_GATE_UP_SILU = os.environ.get("LLMSERVER_B200_FUSE_GATE_UP_SILU", "1") != "0"
-# From these many rows and up to this inner size the gated product that pairs of SMs make (with the activation in its epilogue) is
-# the faster way.  Both sides are limited by the power cap there, and the library's product alone needs a little less of it: what
-# the fused form saves is the activation's pass over memory, whose share shrinks with the inner size.  Whole prompts (library
-# product and activation kernel against pairs, ms): 8B shape (4096) 14.45 / 14.53 at 1024 rows, 20.56 / 20.46 at 1500, 27.40 /
-# 26.82 at 2048, 56.59 / 54.46 at 4096, 119.7 / 118.9 at 8192; 14B shape (5120) 59.8 / 59.3 at 2400, 99.0 / 99.8 at 4096,
-# 140.7 / 141.2 at 6000.
+# Where the gated product that pairs of SMs make (with the activation in its epilogue) is the faster way.  It has tiles of 256 rows by
+# 128 features and does not split K, so it takes whole waves of tiles: with few tiles, or a last wave that is mostly empty, the
+# library's product wins by more than the activation kernel costs.  The library's product is the faster of the two per tile, and
+# the activation's share shrinks with the inner size.  Library product and activation kernel / pairs, us (148 SMs = 74 pairs; clamped
+# gate, weights from HBM): inner 1024: 1024 features 11.5 / 12.4 at 1536 rows (48 tiles), 13.7 / 13.1 at 2048 (64), 16.9 / 18.5 at 3000
+# (96), 21.6 / 19.5 at 4096 (128); 6144 features 41 / 34 at 1536 (288), 97 / 81 at 4096 (768).  Inner 2048: 128 features 8.0 / 16.5 at 1536
+# (6), 1024 features 18.5 / 19.4 at 2048 (64), 1536 features 19.5 / 19.0 at 1536 (72), 25.2 / 30.3 at 2048 (96), 46.2 / 43.9 at 4096 (192);
+# 12288 features 115 / 109 at 1536 (576), 307 / 278 at 4096 (1536).  Inner 4096: 1536 features 41.5 / 52.8 at 2048 (96), 53.4 / 55.2 at 3000
+# (144), 6144 features 103 / 106 at 1536 (288), 145 / 155 at 2048 (384), 199 / 205 at 3000 (576), 286 / 282 at 4096 (768), 12288 features
+# 201 / 207 at 1536 (576), 291 / 288 at 2048 (768), 413 / 417 at 3000 (1152), 604 / 572 at 4096 (1536).  Both sides are
+# limited by the power cap in long prompts; whole prompts (ms): 8B shape (inner 4096, 12288 features) 14.45 / 14.53 at 1024 rows, 27.40 / 26.82
+# at 2048, 56.59 / 54.46 at 4096, 119.7 / 118.9 at 8192; 14B shape (5120) 59.8 / 59.3 at 2400, 99.0 / 99.8 at 4096, 140.7 / 141.2 at 6000.
 PAIR_MIN_ROWS, PAIR_MAX_INNER = 1536, 4096
+PAIR_NARROW_INNER = 2048        # up to this inner size one wave of tiles may do, beyond it takes PAIR_WIDE_WAVES
+PAIR_WIDE_WAVES = 10
+
+
+def pair_tiles_fill(rows: int, features: int, inner: int, pairs: int) -> bool:
+    """Whether the tiles of a gated product fill the pairs of SMs: the last of several waves to more than half, so that all are
+    filled to 0.85, a lone wave to 0.95."""
+    if pairs < 1 or rows < PAIR_MIN_ROWS or inner > PAIR_MAX_INNER:
+        return False
+    tiles = -(-rows // 256) * -(-features // 128)
+    waves = -(-tiles // pairs)
+    if inner > PAIR_NARROW_INNER and waves < PAIR_WIDE_WAVES:
+        return False
+    return tiles >= (0.95 if waves == 1 else 0.85) * waves * pairs
 
 
 def gated_by_pairs(x, weight: torch.Tensor, group: int, limit: float, alpha: float, up_shift: float) -> Optional[torch.Tensor]:
@@ -427,8 +447,8 @@ def gated_by_pairs(x, weight: torch.Tensor, group: int, limit: float, alpha: flo
         return None
     rows, inner = x.shape
     features = weight.shape[0] // 2
-    if not (rows >= PAIR_MIN_ROWS and inner <= PAIR_MAX_INNER and x.is_contiguous() and weight.is_contiguous() and weight.shape[1] == inner
-            and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+    if not (pair_tiles_fill(rows, features, inner, library().llm_sm_count() // 2) and x.is_contiguous() and weight.is_contiguous()
+            and weight.shape[1] == inner and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
             and library().llm_gemm_pair_supports(features, inner, group)):
         return None
     out = torch.empty((rows, features), dtype=torch.bfloat16, device=x.device)

@@ -66,22 +66,23 @@ def test_gated_product_keeps_nan():
     """Without a limit a NaN in the gate stays one (a minimum with infinity would drop it)."""
     from llmserver_b200.ops import gemm_bf16
     from llmserver_b200 import ops
-    x, gate, up = rand((2000, 256), torch.bfloat16, 1), rand((128, 256), torch.bfloat16, 2), rand((128, 256), torch.bfloat16, 3)
+    x, gate, up = rand((2000, 256), torch.bfloat16, 1), rand((1152, 256), torch.bfloat16, 2), rand((1152, 256), torch.bfloat16, 3)
     x[1700, 3] = float("nan")
     out = gemm_bf16.gated_by_pairs(x, ops.interleave_gate_up(gate, up), 64, math.inf, 1.0, 0.0)
     assert torch.isnan(out[1700]).all() and torch.isfinite(out[:1700]).all() and torch.isfinite(out[1701:]).all()
 
 
 def test_which_products_are_fused():
-    """Few rows, a large inner size, operands that are no bfloat16 rows in one piece: the caller's two kernels."""
+    """Few rows, few features, a large inner size, operands that are no bfloat16 rows in one piece: the caller's two kernels."""
     from llmserver_b200.ops import gemm_bf16
-    weight = rand((256, 512), torch.bfloat16, 2)
+    weight = rand((2 * 1536, 512), torch.bfloat16, 2)      # 72 tiles at the fewest rows: a wave of 74 pairs
     take = lambda x, w=weight: gemm_bf16.gated_by_pairs(x, w, 0, math.inf, 1.0, 0.0)  # noqa: E731
     assert take(rand((gemm_bf16.PAIR_MIN_ROWS, 512), torch.bfloat16, 1)) is not None
     assert take(rand((gemm_bf16.PAIR_MIN_ROWS - 1, 512), torch.bfloat16, 1)) is None
+    assert take(rand((gemm_bf16.PAIR_MIN_ROWS, 512), torch.bfloat16, 1), weight[:256]) is None
     assert take(rand((2000, 1024), torch.bfloat16, 1)[:, :512]) is None
     wide = gemm_bf16.PAIR_MAX_INNER + 64
-    assert take(rand((2000, wide), torch.bfloat16, 1), rand((256, wide), torch.bfloat16, 2)) is None
+    assert take(rand((2000, wide), torch.bfloat16, 1), rand((3072, wide), torch.bfloat16, 2)) is None
 
 
 @pytest.mark.parametrize("tokens,experts,top,features,inner", [(5, 4, 2, 64, 64), (300, 3, 2, 136, 128), (700, 5, 3, 320, 192), (2048, 16, 4, 256, 256)])
