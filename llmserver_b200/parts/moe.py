@@ -156,9 +156,15 @@ class RoutedExperts(FeedForward):
 
     GROUPED_FROM = 16     # tokens from which pairs are sorted and multiplied tile by tile
     # (token, expert) pairs per expert from which pairs of SMs make tiles of 256 rows: the tiles of 128 rows that single SMs make
-    # read W once per 128 rows.  Prompts of 64 experts of 1792 with 6 per token: 3.47 ms on tiles of 128 and 4.12 on tiles of 256
-    # at 1024 tokens (96 pairs per expert fit one tile of 128), 5.43 and 5.00 at 2048 (192), 9.66 and 9.37 at 4096 (384)
+    # read W once per 128 rows.  Prompts of 64 experts of 1792 with 6 per token, ms on tiles of 128 / of 256: 3.47 / 4.12 at 1024
+    # tokens (96 pairs per expert fit one tile of 128), 5.14 / 4.82 at 1707 (160), 5.47 / 5.02 at 2048 (192), 6.88 / 6.87 at 2730 (256),
+    # 8.28 / 8.78 at 3413 (320: a second tile of 256 holds 64 rows), 9.46 / 9.42 at 4096 (384).
     PAIR_TILES_FROM = 160
+
+    @classmethod
+    def pair_tiles(cls, pairs: int, experts: int) -> bool:
+        """Whether runs of ``pairs`` / ``experts`` rows go in tiles of 256: not where the second tile of a run is less than half full."""
+        return pairs >= cls.PAIR_TILES_FROM * experts and not 256 * experts < pairs < 384 * experts
 
     def forward(self, x):
         tokens = x.shape[0]
@@ -179,7 +185,7 @@ class RoutedExperts(FeedForward):
         if self.weight_on_input:
             weights = self._ones(weights)       # the weights act on the way in; on the way out the outputs are summed
         if self.grouped and tokens >= self.GROUPED_FROM:
-            by_pairs = tokens * self.top >= self.PAIR_TILES_FROM * self.experts and ops.MOE_GROUPED_KERNEL != "mma"
+            by_pairs = self.pair_tiles(tokens * self.top, self.experts) and ops.MOE_GROUPED_KERNEL != "mma"
             plan = ops.moe_plan(chosen, self.experts, ops.MOE_PAIR_TILE_ROWS if by_pairs else ops.MOE_TILE_ROWS)
             hidden = ops.moe_grouped(x, self.gate_up, plan, gather_div=self.top, gated=self.gate, pair_scale=on_input,
                                      squared_relu=self.squared_relu)

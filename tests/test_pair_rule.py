@@ -1,4 +1,5 @@
-"""Which gated products of many rows go to pairs of SMs: the fill of their waves of tiles of 256 rows by 128 features."""
+"""Which products of many rows go to pairs of SMs: gated ones by the fill of their waves of tiles of 256 rows by 128 features, experts'
+by how their runs fill tiles of 256 rows."""
 import pytest
 
 PAIRS = 74
@@ -16,3 +17,10 @@ def test_pair_tiles_fill(rows, features, inner, want):
     from llmserver_b200.ops import gemm_bf16
     assert gemm_bf16.pair_tiles_fill(rows, features, inner, PAIRS) is want
     assert not gemm_bf16.pair_tiles_fill(rows, features, inner, 0)
+
+
+@pytest.mark.parametrize("experts", [1, 64])
+def test_expert_tiles(experts):
+    from llmserver_b200.parts.moe import RoutedExperts
+    large = {per: RoutedExperts.pair_tiles(per * experts, experts) for per in (1, 128, 159, 160, 192, 256, 257, 320, 383, 384, 512, 4096)}
+    assert large == {per: per in (160, 192, 256, 384, 512, 4096) for per in large}
