@@ -5,9 +5,11 @@ cuBLAS: utils/attention.py:119-124,181; utils/layers.py:205-217; utils/model.py:
 
 * up to 64 rows (decode steps, the output head): this package's tcgen05 / TMA kernel
   (``csrc/gemm_tcgen05.cu``), which streams the weights once and can write float32 directly, or the
-  library product, whichever a one-time measurement per shape finds faster;
+  library product, whichever a one-time measurement per shape finds faster; steps that add to the residual stream in their
+  products (``ops/stream.py``: up to 64 rows, short prompts up to 128) always run this package's kernel;
 * more rows (prompt portions): the library product (cuBLAS through PyTorch); gated feed-forwards of many rows run a product
-  of this package that pairs of SMs make and whose epilogue applies the gate (``csrc/gemm_pair_tcgen05.cu``).
+  of this package that pairs of SMs make and whose epilogue applies the gate (``csrc/gemm_pair_tcgen05.cu``) where its tiles
+  fill whole waves.
 """
 from __future__ import annotations
 
@@ -177,9 +179,19 @@ def _small_m(x, weight, out, split: int, scale: tuple = NO_SCALE) -> None:
          int(out.dtype == torch.float32), split, *scale, error_flag(x.device).data_ptr(), stream_handle())
 
 
+def _split_beyond_64_rows(cols: int) -> int:
+    """The split of K beyond 64 rows, where only prompts run this package's kernel: the most parts that make clusters of a power of two
+    and at most two blocks per SM.  Measuring it stopped the first such prompt for 0.15 to 0.2 s and found no better one (8B shape, ms,
+    measured / this: 4.61 / 4.63 at 70 tokens, 4.83 / 4.82 at 100, 5.08 / 5.10 at 128; with clusters of 6 for q/k/v 5.29 at 100, with one
+    block per SM 5.11)."""
+    tiles = -(-cols // 128)
+    return max([split for split in (1, 2, 4, 8) if tiles * split <= 2 * library().llm_sm_count()], default=1)
+
+
 def _plan_for(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, own_kernel_only: bool = False) -> int:
     """``own_kernel_only``: the best split of this package's kernel, the library's product not considered (for the
-    products that finish their result in the kernel's epilogue, which the library's cannot; kept under a key of its own).
+    products that finish their result in the kernel's epilogue, which the library's cannot; kept under a key of its own;
+    beyond 64 rows the split follows from the shape unless a plan file names another).
 
     Measures, once per (rows bucket, shape), this package's kernel with a few splits of K and the
     library product, each as a model step runs it, and remembers the fastest: a split (> 0) or 0 for the library.  All candidates read
@@ -197,6 +209,8 @@ def _plan_for(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, own
         load_plan()
         if key in _choice:
             return _choice[key]
+    if own_kernel_only and rows > SMALL_M:
+        return _split_beyond_64_rows(cols)
     if torch.cuda.is_current_stream_capturing():
         return -1
     if out_dtype == torch.float32 or own_kernel_only:
@@ -330,7 +344,7 @@ def _float32_by_library(x: torch.Tensor, weight: torch.Tensor, out: Optional[tor
 
 
 def _plan_fused(kind: str, rows: int, cols: int, inner: int, fused, apart, device) -> int:
-    """For 17 to 64 rows: the split with which the fused kernel ``fused(split)`` is fastest inside a step, or 0 when
+    """For 17 to 64 rows that are normalised already: the split with which the fused kernel ``fused(split)`` is fastest inside a step, or 0 when
     the library's product followed by the kernel of its own (``apart()``) is faster.  Measured once per (kind, row
     bucket, shape), kept with the other choices (and in the plan file).  While a graph is being captured nothing can
     be measured: an unknown shape then runs apart."""

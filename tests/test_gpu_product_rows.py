@@ -150,3 +150,16 @@ def test_steps_of_more_than_64_rows(tiny_folders, monkeypatch):
                 assert_close(logits[row:row + 1].float().cpu().numpy(), expected, "bfloat16", f"turn {turn}, row {row}")
     assert step.graph_steps > 0
     step.check_errors()
+
+
+def test_prompts_of_more_than_64_tokens_time_nothing():
+    """The splits of products that only prompts run at these rows follow from the shape: the first such prompt does not stop for them."""
+    from llmserver_b200 import ops
+    from llmserver_b200.ops import gemm_bf16
+    x, w = rand((100, 1032), torch.bfloat16, 1), rand((392, 1032), torch.bfloat16, 2, 1032 ** -0.5)
+    stream = rand((100, 392), torch.float32, 3)
+    want = stream.double() + x.double() @ w.double().T
+    before = gemm_bf16.tunings()
+    assert gemm_bf16.linear_into_stream(x, w, ops.StreamSink(stream))
+    assert gemm_bf16.tunings() == before
+    close(stream, want, torch.float32, "the stream", factor=4.0)
