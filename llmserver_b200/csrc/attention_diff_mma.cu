@@ -448,7 +448,7 @@ int launch_diff(const DiffParams& p, int n_seqs, int max_q_len, cudaStream_t str
 }
 
 // One warp per (token, head): o = a_1 - lambda a_2 of the maps that the tcgen05 prompt kernel and the TMA decode kernel leave as
-// 32-bit numbers, the head norm, the gate, one rounding.  Four elements a lane; it reads 8 bytes per byte that it writes.
+// 32-bit numbers, the head norm, the gate, one rounding.  Four elements a lane; it reads 4 bytes per byte that it writes.
 __global__ void attention_diff_combine_kernel(const float* __restrict__ maps, DiffParams p, int total) {
     pdl_trigger();
     pdl_wait();

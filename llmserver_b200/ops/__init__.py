@@ -1391,8 +1391,8 @@ def qkv_projection(x, weight: torch.Tensor, q_weight: Optional[torch.Tensor], k_
                    head_dim: int, eps: float, write_cache: bool, error_flag: torch.Tensor, rotary_dim: Optional[int] = None,
                    interleaved: bool = False) -> torch.Tensor:
     """qkv = x W^T followed by ``qk_norm_rope_kv_write``: as one kernel where the product kernel can finish heads in its
-    epilogue (bfloat16, heads of 128, up to 64 tokens, the whole head rotating in halves; from 17 tokens on only where
-    that is measured to be faster), else as two.  ``x`` may be a ``RowScaled``."""
+    epilogue (bfloat16, heads of 128, the whole head rotating in halves; up to 16 tokens, up to 64 where that is measured to
+    be faster, and up to 128 for a ``RowScaled``, which only that kernel takes), else as two."""
     whole_head = rotary_dim is None or rotary_dim == head_dim
     if x.dtype == torch.bfloat16 and whole_head and not interleaved and x.shape[0] <= (128 if isinstance(x, RowScaled) else 64):
         from . import gemm_bf16
