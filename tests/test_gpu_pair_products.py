@@ -62,6 +62,21 @@ def test_gate_over_its_range(by_pairs):
     assert ((got - want).abs() <= (2.0 ** -8 + 106 * 2.0 ** -23) * want.abs()).all(), f"{got[0, :20]} {want[:20]}"
 
 
+@pytest.mark.parametrize("by_pairs", [False, True])
+def test_gates_that_are_not_finite(by_pairs):
+    """A gate beyond the type's range has its limit: itself upwards, 0 downwards as far as the exponential is infinite and the gate a number."""
+    from llmserver_b200 import ops
+    gate = torch.tensor([-3e38, -1000.0, -89.0, 0.0, 1000.0, 3e38, float("inf"), float("nan")]).to(torch.bfloat16).to(DEVICE)
+    weight = torch.zeros((1, 16, 64), dtype=torch.bfloat16, device=DEVICE)
+    weight[0, :8, 0] = gate
+    x = torch.zeros((256, 64), dtype=torch.bfloat16, device=DEVICE)
+    x[:, 0] = 1.0
+    plan = ops.moe_plan(torch.zeros((256, 1), dtype=torch.int32, device=DEVICE), 1, ops.MOE_PAIR_TILE_ROWS if by_pairs else ops.MOE_TILE_ROWS)
+    got = ops.moe_grouped(x, weight, plan, gather_div=1, gated=(math.inf, 1.0)).float()
+    assert (got[:, :4] == 0.0).all() and torch.equal(got[:, 4:7], gate[4:7].float().expand(256, 3))
+    assert not by_pairs or torch.isnan(got[:, 7]).all()      # the tiles of 128 rows take the limit of a gate that is no number
+
+
 def test_gated_product_keeps_nan():
     """Without a limit a NaN in the gate stays one (a minimum with infinity would drop it)."""
     from llmserver_b200.ops import gemm_bf16
