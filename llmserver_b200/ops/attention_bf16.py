@@ -339,7 +339,7 @@ def _attention_diff_maps(qkv, gate, batch, block_tables, k_pages, v_pages, n_q_h
         # As for the other portions, but a row tile is two blocks, one per map.  A single token in a tile of its own would fill `group`
         # of 128 rows, read its cache once per map and walk it in one block: a step with 48 of them behind 900 to 4001 keys
         # beside a prompt of 256 takes 2.57 ms that way and 2.41 with them on the decode kernel; 21 behind 140 to 2300 beside
-        # 2000 tokens 4.12 and 4.18 (the launches show where the portions fill the GPU).
+        # 2000 tokens, whose tiles fill the GPU, 4.19 and 4.17.
         tile_counts = [-(-length // (PREFILL_TILE // group)) for length in batch.q_lens if length > 1]
         paired = sum((count + 1) // 2 for count in tile_counts)
         slots = _block_slots(qkv.device, False)
