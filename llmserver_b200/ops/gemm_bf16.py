@@ -184,8 +184,8 @@ def _split_beyond_64_rows(cols: int) -> int:
     and at most two blocks per SM.  Measuring it stopped the first such prompt for 0.15 to 0.2 s and found no better one (8B shape, ms,
     measured / this: 4.61 / 4.63 at 70 tokens, 4.83 / 4.82 at 100, 5.08 / 5.10 at 128; with clusters of 6 for q/k/v 5.29 at 100, with one
     block per SM 5.11)."""
-    tiles = -(-cols // 128)
-    return max([split for split in (1, 2, 4, 8) if tiles * split <= 2 * library().llm_sm_count()], default=1)
+    blocks = 2 * library().llm_sm_count()
+    return max([split for split in (1, 2, 4, 8) if -(-cols // 128) * split <= blocks], default=1)
 
 
 def _plan_for(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, own_kernel_only: bool = False) -> int:
@@ -210,7 +210,8 @@ def _plan_for(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, own
         if key in _choice:
             return _choice[key]
     if own_kernel_only and rows > SMALL_M:
-        return _split_beyond_64_rows(cols)
+        _choice[key] = _split_beyond_64_rows(cols)
+        return _choice[key]
     if torch.cuda.is_current_stream_capturing():
         return -1
     if out_dtype == torch.float32 or own_kernel_only:
@@ -461,7 +462,7 @@ def gated_by_pairs(x, weight: torch.Tensor, group: int, limit: float, alpha: flo
         return None
     rows, inner = x.shape
     features = weight.shape[0] // 2
-    if not (pair_tiles_fill(rows, features, inner, library().llm_sm_count() // 2) and x.is_contiguous() and weight.is_contiguous()
+    if not (rows >= PAIR_MIN_ROWS and pair_tiles_fill(rows, features, inner, library().llm_sm_count() // 2) and x.is_contiguous() and weight.is_contiguous()
             and weight.shape[1] == inner and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
             and library().llm_gemm_pair_supports(features, inner, group)):
         return None

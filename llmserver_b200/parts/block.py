@@ -22,6 +22,7 @@ class PreNormBlock(Block):
     KNOWN_PARAMS = ("mixer_prefix", "feed_forward_prefix", "mixer_norm_prefix", "feed_forward_norm_prefix")
 
     passes_stream = True
+    stream_bounds = None        # (rows of other steps, of decode steps) up to which products add to the stream; set by the first step
 
     def entry(self):
         return self.mixer_norm, self.mixer
@@ -30,24 +31,21 @@ class PreNormBlock(Block):
         # With few rows, parts that can do so add their results to the stream themselves and prepare the next norm's
         # input (``sink``), and take a norm's output before its division (``unscaled``); see ``ops.stream``.  Parts
         # and norms that cannot are called as ever.
-        normed = _add_norm(self.mixer_norm, residual, delta, self.mixer, batch)
-        sink = _sink(self.feed_forward_norm, residual, self.feed_forward, batch) if self.mixer.feeds_stream else None
+        if self.stream_bounds is None:
+            self.stream_bounds = ops.stream_rows(residual.shape[-1], False), ops.stream_rows(residual.shape[-1], True)
+        inside = batch.n_tokens <= self.stream_bounds[batch.max_q_len == 1]
+        normed = _add_norm(self.mixer_norm, residual, delta, self.mixer, inside)
+        sink = self.feed_forward_norm.sink(residual, self.feed_forward) if inside and self.mixer.feeds_stream else None
         mixed = self.mixer.forward(normed, batch, cache, sink=sink) if sink is not None else self.mixer.forward(normed, batch, cache)
-        normed = _add_norm(self.feed_forward_norm, residual, sink if sink is not None and sink.added else mixed, self.feed_forward, batch)
-        sink = _sink(after[0], residual, after[1], batch) if after is not None and self.feed_forward.feeds_stream else None
+        normed = _add_norm(self.feed_forward_norm, residual, sink if sink is not None and sink.added else mixed, self.feed_forward, inside)
+        sink = after[0].sink(residual, after[1]) if inside and after is not None and self.feed_forward.feeds_stream else None
         out = self.feed_forward.forward(normed, sink=sink) if sink is not None else self.feed_forward.forward(normed)
         return residual, (sink if sink is not None and sink.added else out)
 
 
-def _sink(norm, residual, consumer, batch):
-    """What ``norm`` offers the part in front of it, in steps of so few rows that its products are the faster ones."""
-    if residual.shape[0] > ops.stream_rows(residual.shape[-1], decode=batch.max_q_len == 1):
-        return None
-    return norm.sink(residual, consumer)
-
-
-def _add_norm(norm, residual, delta, consumer, batch):
-    if getattr(consumer, "takes_unscaled", False) and _sink(norm, residual, consumer, batch) is not None:
+def _add_norm(norm, residual, delta, consumer, inside):
+    """``inside``: the step has so few rows that it adds to the stream in its products."""
+    if inside and getattr(consumer, "takes_unscaled", False) and norm.sink(residual, consumer) is not None:
         return norm.add_norm(residual, delta, unscaled=True)
     return norm.add_norm(residual, delta)
 

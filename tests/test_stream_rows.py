@@ -30,7 +30,7 @@ class Consumer:
 def inside(rows, width, max_q_len):
     norms = [RecordingNorm() for _ in range(3)]
     block = PreNormBlock({}, {"mixer": Consumer(), "feed_forward": Consumer(), "mixer_norm": norms[0], "feed_forward_norm": norms[1]})
-    block.forward(torch.empty((rows, width)), None, SimpleNamespace(max_q_len=max_q_len), None, after=(norms[2], None))
+    block.forward(torch.empty((rows, width)), None, SimpleNamespace(n_tokens=rows, max_q_len=max_q_len), None, after=(norms[2], None))
     taken = {norm.asked > 0 for norm in norms} | set(norms[0].unscaled + norms[1].unscaled)
     assert len(taken) == 1, "one way for the whole block"
     return taken.pop()
