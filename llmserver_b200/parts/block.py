@@ -45,6 +45,8 @@ class PreNormBlock(Block):
 
 def _add_norm(norm, residual, delta, consumer, inside):
     """``inside``: the step has so few rows that it adds to the stream in its products."""
+    if isinstance(delta, ops.StreamSink) and delta.scaled is not None:      # prepared for this consumer, which was asked then
+        return norm.add_norm(residual, delta, unscaled=True)
     if inside and getattr(consumer, "takes_unscaled", False) and norm.sink(residual, consumer) is not None:
         return norm.add_norm(residual, delta, unscaled=True)
     return norm.add_norm(residual, delta)
