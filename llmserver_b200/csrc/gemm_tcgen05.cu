@@ -49,6 +49,7 @@ constexpr int kAtomK = 64;          // one 128-byte swizzle atom of bfloat16
 constexpr int kMaxRows = 128;       // tokens per launch
 constexpr int kTwoAtomRows = 64;    // up to this many tokens a pipeline stage holds two atoms of K, beyond (where a token atom is as
                                     // large as a weight atom) one: three stages of 32 KiB then leave room for two blocks per SM
+constexpr int kThreeBlocksKib = 74; // ring of a block that shares its SM with two others
 constexpr int kThreads = 256;       // at most: four warps up to 16 tokens, eight beyond (two have a role in the main
                                     // loop, all work in the epilogue, whose time per token is instruction issue)
 constexpr int kMaxStages = 12;
@@ -247,21 +248,23 @@ __device__ __forceinline__ RopeRow rope_row(const GemmParams& p, int m, int tile
 
 // What finishing token m needs beside the product: its position and page (q/k/v epilogue) or the stream's values at
 // columns n4 .. n4 + 3 (stream epilogue).  Nothing for a token that does not exist.
-__device__ __forceinline__ void token_inputs(const GemmParams& p, int m, int tile, int n4, RopeRow& info, float (&before)[4]) {
+__device__ __forceinline__ RopeRow rope_inputs(const GemmParams& p, int m, int tile) {
+    RopeRow info;
     info.position = info.page = 0;
+    if (m < p.m && p.rope.on) info = rope_row(p, m, tile);
+    return info;
+}
+__device__ __forceinline__ void stream_inputs(const GemmParams& p, int m, int n4, float (&before)[4]) {
 #pragma unroll
     for (int c = 0; c < 4; ++c) before[c] = 0.0f;
-    if (m >= p.m) return;
-    if (p.rope.on) info = rope_row(p, m, tile);
-    if (p.stream.on) {
-        if (p.vector_stream && n4 + 3 < p.n) {
-            const float4 v = *reinterpret_cast<const float4*>(p.stream.residual + (size_t)m * p.n + n4);
-            before[0] = v.x, before[1] = v.y, before[2] = v.z, before[3] = v.w;
-        } else {
+    if (m >= p.m || !p.stream.on) return;
+    if (p.vector_stream && n4 + 3 < p.n) {
+        const float4 v = *reinterpret_cast<const float4*>(p.stream.residual + (size_t)m * p.n + n4);
+        before[0] = v.x, before[1] = v.y, before[2] = v.z, before[3] = v.w;
+    } else {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (n4 + c < p.n) before[c] = p.stream.residual[(size_t)m * p.n + n4 + c];
-        }
+        for (int c = 0; c < 4; ++c)
+            if (n4 + c < p.n) before[c] = p.stream.residual[(size_t)m * p.n + n4 + c];
     }
 }
 
@@ -343,10 +346,159 @@ __device__ __forceinline__ void stream_finish(const GemmParams& p, int m, int la
     }
 }
 
-// MANY: more than 16 tokens, eight warps; a warp finishes several tokens.  What it does for the second and later ones costs the
+// ---- The same for steps of more than 16 tokens, where a block finishes many tokens and their time is instruction issue: half a
+// warp takes a token, lane i of the half (0..15) elements 4 i .. 4 i + 3 and 64 + 4 i .. 64 + 4 i + 3 of the tile's 128.  Rotation
+// partners and gate/up pairs lie in one thread, an angle is formed once, sums over a token take four shuffles for two tokens, and
+// every sum has the order that it has above (lane i there adds lane i + 16 first).  Figures: gemm_small_m_kernel.
+constexpr int kHalfTile = kBlockRows / 2;
+
+__device__ __forceinline__ float half_warp_sum(float v) {
+#pragma unroll
+    for (int offset = 8; offset > 0; offset >>= 1) v += __shfl_xor_sync(0xffffffffu, v, offset);
+    return v;
+}
+
+// The ranks' parts of a token's eight elements, all asked for before the first is used, added in the order of the ranks.
+template <int SPLIT>
+__device__ __forceinline__ void sum_ranks(uint32_t address, float (&v)[8]) {
+    float4 low[SPLIT], high[SPLIT];
+#pragma unroll
+    for (int peer = 0; peer < SPLIT; ++peer) {
+        low[peer] = load_peer4(address, (uint32_t)peer);
+        high[peer] = load_peer4(address + kHalfTile * 4u, (uint32_t)peer);
+    }
+    v[0] = low[0].x, v[1] = low[0].y, v[2] = low[0].z, v[3] = low[0].w;
+    v[4] = high[0].x, v[5] = high[0].y, v[6] = high[0].z, v[7] = high[0].w;
+#pragma unroll
+    for (int peer = 1; peer < SPLIT; ++peer) {
+        v[0] += low[peer].x, v[1] += low[peer].y, v[2] += low[peer].z, v[3] += low[peer].w;
+        v[4] += high[peer].x, v[5] += high[peer].y, v[6] += high[peer].z, v[7] += high[peer].w;
+    }
+}
+__device__ __forceinline__ void sum_of_parts(int split, const float* here, uint32_t address, float (&v)[8]) {
+    if (split == 1) {
+        const float4 low = *reinterpret_cast<const float4*>(here), high = *reinterpret_cast<const float4*>(here + kHalfTile);
+        v[0] = low.x, v[1] = low.y, v[2] = low.z, v[3] = low.w;
+        v[4] = high.x, v[5] = high.y, v[6] = high.z, v[7] = high.w;
+    } else if (split == 2) {
+        sum_ranks<2>(address, v);
+    } else if (split == 4) {
+        sum_ranks<4>(address, v);
+    } else if (split == 8) {
+        sum_ranks<8>(address, v);
+    } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) v[c] = 0.0f;
+        for (int peer = 0; peer < split; ++peer) {
+            const float4 low = load_peer4(address, (uint32_t)peer), high = load_peer4(address + kHalfTile * 4u, (uint32_t)peer);
+            v[0] += low.x, v[1] += low.y, v[2] += low.z, v[3] += low.w;
+            v[4] += high.x, v[5] += high.y, v[6] += high.z, v[7] += high.w;
+        }
+    }
+}
+
+__device__ __forceinline__ void four_of(const float (&v)[8], int first, float (&four)[4]) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) four[c] = v[first + c];
+}
+
+// What rope_finish, silu_finish and stream_finish do, for this lane's eight elements; `present`: the token exists (the lanes of a
+// half warp without one take part in the shuffles only).
+__device__ __forceinline__ void rope_finish8(const GemmParams& p, int m, bool present, int r4, int tile, float (&value)[8],
+                                             const float (&weight)[8], const float (&frequency)[4], RopeRow info) {
+    const RopeEpilogue& e = p.rope;
+    const bool is_q = tile < e.n_q_heads;
+    const bool is_k = !is_q && tile < e.n_q_heads + e.n_kv_heads;
+    if (is_q || is_k) {
+        if ((is_q ? e.q_weight : e.k_weight) != nullptr) {
+            const float squares = half_warp_sum((value[0] * value[0] + value[1] * value[1] + value[2] * value[2] + value[3] * value[3]) +
+                                                (value[4] * value[4] + value[5] * value[5] + value[6] * value[6] + value[7] * value[7]));
+            const float inverse = rsqrtf(squares / (float)kBlockRows + e.eps);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) value[c] = value[c] * inverse * weight[c];
+        }
+        if (e.inv_freq != nullptr) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float angle = (float)info.position * frequency[c];
+                const float cs = cosf(angle), sn = sinf(angle);
+                const float first = value[c], second = value[4 + c];
+                value[c] = first * cs - second * sn;
+                value[4 + c] = second * cs + first * sn;
+            }
+        }
+    }
+    if (!present) return;
+    __nv_bfloat16* dst;
+    if (is_q) {
+        dst = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)m * p.ldc + (size_t)tile * kBlockRows;
+    } else {
+        if (!e.write_cache) return;
+        const int kv_head = is_k ? tile - e.n_q_heads : tile - e.n_q_heads - e.n_kv_heads;
+        if (info.page < 0) {
+            if (r4 == 0) atomicExch(e.page_error, 1 + m);
+            return;
+        }
+        dst = (is_k ? e.k_pages : e.v_pages) +
+              (((size_t)info.page * e.n_kv_heads + kv_head) * e.page_size + info.position % e.page_size) * kBlockRows;
+    }
+    float four[4];
+    four_of(value, 0, four);
+    store4_bf16(dst + r4, four, 4, p.vector_out != 0);
+    four_of(value, 4, four);
+    store4_bf16(dst + kHalfTile + r4, four, 4, p.vector_out != 0);
+}
+
+__device__ __forceinline__ void silu_finish8(const GemmParams& p, int m, int r4, int tile, const float (&value)[8]) {
+    float result[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) result[c] = __fdividef(value[c], 1.0f + __expf(-value[c])) * value[4 + c];
+    const int column = tile * kHalfTile + r4;
+    store4_bf16(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)m * p.ldc + column, result, p.n / 2 - column, p.vector_out != 0);
+}
+
+__device__ __forceinline__ void stream_finish8(const GemmParams& p, int m, bool present, int r4, int tile, const float (&value)[8],
+                                               const float (&before)[8], const float (&weight)[8]) {
+    const StreamEpilogue& e = p.stream;
+    float squares[2];
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+        const int n4 = tile * kBlockRows + part * kHalfTile + r4, valid = p.n - n4;
+        float updated[4], scaled[4];
+        squares[part] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            updated[c] = c < valid ? before[4 * part + c] + value[4 * part + c] : 0.0f;
+            scaled[c] = updated[c] * weight[4 * part + c];
+            squares[part] += updated[c] * updated[c];
+        }
+        if (present && valid > 0) {
+            store4_f32(e.residual + (size_t)m * p.n + n4, updated, valid, p.vector_stream != 0);
+            if (e.next_weight != nullptr) store4_bf16(e.scaled + (size_t)m * p.n + n4, scaled, valid, p.vector_stream != 0);
+        }
+    }
+    if (e.next_weight != nullptr) {
+        const float total = half_warp_sum(squares[0] + squares[1]);
+        if (present && r4 == 0) e.parts[(size_t)tile * e.stride + m] = total;
+    }
+}
+
+// MANY: more than 16 tokens, eight warps; a half warp finishes several tokens.  What it does for the second and later ones costs the
 // steps of few tokens 0.5 us a launch (a batch-8 step of the 8B shape 3.64 against 3.55 ms), so they run a form without it.
-template <int kAtoms, bool MANY>
-__global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_constant__ CUtensorMap map_w,
+//
+// PER_SM (MANY): how many blocks share an SM.  Two have room for a ring of 100 KiB and for registers that hold the parts of eight
+// ranks at once.  Where a launch has more than two blocks per SM, three of them with a shorter ring of single atoms (and 80 registers)
+// are faster than a second wave: gate/up projection of the 8B shape in two parts (384 blocks), one behind the other with weights
+// from HBM, at 24 / 61 / 119 tokens 33.9 / 35.6 / 40.0 us against 40.3 / 43.8 / 50.0 with two an SM and 35.8 / 37.4 / 41.5 unsplit; output
+// head of 151936 rows at 20 / 64 tokens 190 / 199 us against 206 / 218 (190 is what its bytes take).
+//
+// What bounds a product of 17 to 128 tokens beside its weights' bytes is the epilogue.  Leaving the token tiles out after the first
+// ring changes nothing up to 128 tokens (48.7 against 48.8 us for gate/up at 119), finishing 16 tokens only takes a warp-per-token
+// epilogue from 48.8 to 39.2 us.  A warp per token / half a warp per token, us: gate/up 40.8 / 37.4 at 61 tokens and 47.9 / 41.5 at 119,
+// q/k/v 14.3 / 14.3 and 17.5 / 17.1, down projection 22.5 / 22.4 and 25.9 / 26.6 (eight ranks: the parts that cross
+// distributed shared memory are the same), output head 226 / 218 at 64.
+template <int kAtoms, bool MANY, int PER_SM>
+__global__ void __launch_bounds__(kThreads, PER_SM) gemm_small_m_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                 const __grid_constant__ CUtensorMap map_x,
                                                                 const GemmParams p) {
     // Static shared memory has to stay within 1 KiB.  Up to 16 tokens a block takes 72 KiB of stages + 1 KiB to align
@@ -498,25 +650,53 @@ __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_con
     // What the epilogue needs beside the product is asked for now, while the product is still being made: the norm
     // weights and frequencies of this lane's four elements, and for the first token this warp will finish its
     // position and page (a chain of three dependent loads) or the stream's values.
-    const int r4 = 4 * lane, n4 = n0 + r4;
-    const int token_step = n_warps * p.split;         // between two tokens of one warp (rows are dealt round-robin to
-    const int first_token = (int)rank + p.split * warp;   // the ranks, a rank's rows round-robin to its warps)
-    float weight[4] = {1.0f, 1.0f, 1.0f, 1.0f}, frequency[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const int half = MANY ? lane >> 4 : 0;                // MANY: which of the warp's two tokens this lane works on
+    const int r4 = 4 * (MANY ? lane & 15 : lane), n4 = n0 + r4;
+    // Tokens are dealt round-robin to the ranks, a rank's round-robin to its warps (MANY: half warps).
+    const int token_step = (MANY ? 2 : 1) * n_warps * p.split;
+    const int first_token = (int)rank + p.split * (MANY ? 2 * warp + half : warp);
+    constexpr int kFours = MANY ? 2 : 1;                  // groups of four elements of a token that a lane has: r4 .., 64 + r4 ..
+    float weight[4 * kFours], frequency[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int c = 0; c < 4 * kFours; ++c) weight[c] = 1.0f;
     RopeRow info;
-    float before[4];
+    float before[4 * kFours];
+    auto take4 = [](float (&all)[4 * kFours], int part, const float (&four)[4]) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) all[4 * part + c] = four[c];
+    };
     if (p.rope.on) {
         const bool is_q = tile < p.rope.n_q_heads, is_k = !is_q && tile < p.rope.n_q_heads + p.rope.n_kv_heads;
         if (is_q || is_k) {
-            load_weights4(is_q ? p.rope.q_weight : p.rope.k_weight, p.rope.weight_is_f32, r4, kBlockRows, weight);
+#pragma unroll
+            for (int part = 0; part < kFours; ++part) {
+                float four[4];
+                load_weights4(is_q ? p.rope.q_weight : p.rope.k_weight, p.rope.weight_is_f32, r4 + part * kHalfTile, kBlockRows, four);
+                take4(weight, part, four);
+            }
             if (p.rope.inv_freq != nullptr) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) frequency[c] = p.rope.inv_freq[(r4 + c) & (kBlockRows / 2 - 1)];
             }
         }
     } else if (p.stream.on) {
-        load_weights4(p.stream.next_weight, p.stream.weight_is_f32, n4, p.n, weight);
+#pragma unroll
+        for (int part = 0; part < kFours; ++part) {
+            float four[4];
+            load_weights4(p.stream.next_weight, p.stream.weight_is_f32, n4 + part * kHalfTile, p.n, four);
+            take4(weight, part, four);
+        }
     }
-    token_inputs(p, first_token, tile, n4, info, before);
+    auto inputs = [&](int m, RopeRow& row, float (&values)[4 * kFours]) {
+        row = rope_inputs(p, m, tile);
+#pragma unroll
+        for (int part = 0; part < kFours; ++part) {
+            float four[4];
+            stream_inputs(p, m, n4 + part * kHalfTile, four);
+            take4(values, part, four);
+        }
+    };
+    inputs(first_token, info, before);
     bool ready = true;
     if (n_kb > 0) ready = mbar_wait(smem_u32(&accum_bar), 0);
     if (!ready) failed = 1;
@@ -559,59 +739,94 @@ __global__ void __launch_bounds__(kThreads) gemm_small_m_kernel(const __grid_con
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols));
     }
 
-    // Lane i finishes elements 4 i .. 4 i + 3 of the tile for its warp's tokens, one token after the other.
+    // Lane i finishes its elements of the tile for its tokens, one token after the other.
     const bool scaled = p.scale.parts != nullptr;
     const uint32_t parts_address = smem_u32(parts_tile);
     bool arrived = false;
-    for (int m = first_token; m < p.m; m += token_step) {
-        // MANY: the next token's inputs are asked for before this one's are used (three dependent loads for a page)
-        RopeRow next_info;
-        float next_before[4];
-        if (MANY) token_inputs(p, m + token_step, tile, n4, next_info, next_before);
-        else if (m != first_token) token_inputs(p, m, tile, n4, info, before);
-        // the ranks' parts of the token, all asked for before the first is used, added in the order of the ranks
-        float4 parts[kMaxSplit];
-#pragma unroll
-        for (int peer = 0; peer < kMaxSplit; ++peer) {
-            if (peer >= p.split) {
-                parts[peer] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            } else if (p.split > 1) {
-                parts[peer] = load_peer4(parts_address + (uint32_t)(m * kBlockRows + r4) * 4u, (uint32_t)peer);
-            } else {
-                parts[peer] = *reinterpret_cast<const float4*>(parts_tile + m * kBlockRows + r4);
+    if constexpr (MANY) {
+        for (int m = first_token; m - p.split * half < p.m; m += token_step) {      // (the warp's first token decides)
+            const bool present = m < p.m;
+            const int there = present ? m : p.m - 1;
+            // the next token's inputs are asked for before this one's are used (three dependent loads for a page)
+            RopeRow next_info;
+            float next_before[8];
+            inputs(m + token_step, next_info, next_before);
+            float total[8];
+            const int place = there * kBlockRows + r4;
+            sum_of_parts(p.split, parts_tile + place, parts_address + (uint32_t)place * 4u, total);
+            if (p.split > 1 && m - p.split * half + token_step >= p.m) {      // the warp's last tokens: their parts are here
+                __syncwarp();
+                cluster_arrive();
+                arrived = true;
             }
-        }
-        float total[4] = {parts[0].x, parts[0].y, parts[0].z, parts[0].w};
+            if (scaled) {
+                const float s = row_scale[there];
 #pragma unroll
-        for (int peer = 1; peer < kMaxSplit; ++peer) {      // absent peers add 0
-            total[0] += parts[peer].x;
-            total[1] += parts[peer].y;
-            total[2] += parts[peer].z;
-            total[3] += parts[peer].w;
-        }
-        if (p.split > 1 && m + token_step >= p.m) {      // this warp's last token: its parts are here (they were added)
-            cluster_arrive();
-            arrived = true;
-        }
-        if (scaled) {
-            const float s = row_scale[m];
+                for (int c = 0; c < 8; ++c) total[c] *= s;
+            }
+            if (p.stream.on) {
+                stream_finish8(p, m, present, r4, tile, total, before, weight);
+            } else if (p.rope.on) {
+                rope_finish8(p, m, present, r4, tile, total, weight, frequency, info);
+            } else if (p.silu_gate) {
+                if (present) silu_finish8(p, m, r4, tile, total);
+            } else if (present) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) total[c] *= s;
-        }
-        if (p.stream.on) {
-            stream_finish(p, m, lane, tile, n4, total, before, weight);
-        } else if (p.rope.on) {
-            rope_finish(p, m, lane, tile, total, weight, frequency, info);
-        } else if (p.silu_gate) {
-            silu_finish(p, m, lane, tile, total);
-        } else if (n4 < p.n) {
-            if (p.out_is_f32) store4_f32(reinterpret_cast<float*>(p.out) + (size_t)m * p.ldc + n4, total, p.n - n4, p.vector_out != 0);
-            else store4_bf16(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)m * p.ldc + n4, total, p.n - n4, p.vector_out != 0);
-        }
-        if (MANY) {
+                for (int part = 0; part < 2; ++part) {
+                    const int column = n4 + part * kHalfTile;
+                    float four[4];
+                    four_of(total, 4 * part, four);
+                    if (column >= p.n) continue;
+                    if (p.out_is_f32) store4_f32(reinterpret_cast<float*>(p.out) + (size_t)m * p.ldc + column, four, p.n - column, p.vector_out != 0);
+                    else store4_bf16(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)m * p.ldc + column, four, p.n - column, p.vector_out != 0);
+                }
+            }
             info = next_info;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) before[c] = next_before[c];
+            for (int c = 0; c < 8; ++c) before[c] = next_before[c];
+        }
+    } else {
+        for (int m = first_token; m < p.m; m += token_step) {
+            if (m != first_token) inputs(m, info, before);
+            // the ranks' parts of the token, all asked for before the first is used, added in the order of the ranks
+            float4 parts[kMaxSplit];
+#pragma unroll
+            for (int peer = 0; peer < kMaxSplit; ++peer) {
+                if (peer >= p.split) {
+                    parts[peer] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                } else if (p.split > 1) {
+                    parts[peer] = load_peer4(parts_address + (uint32_t)(m * kBlockRows + r4) * 4u, (uint32_t)peer);
+                } else {
+                    parts[peer] = *reinterpret_cast<const float4*>(parts_tile + m * kBlockRows + r4);
+                }
+            }
+            float total[4] = {parts[0].x, parts[0].y, parts[0].z, parts[0].w};
+#pragma unroll
+            for (int peer = 1; peer < kMaxSplit; ++peer) {      // absent peers add 0
+                total[0] += parts[peer].x;
+                total[1] += parts[peer].y;
+                total[2] += parts[peer].z;
+                total[3] += parts[peer].w;
+            }
+            if (p.split > 1 && m + token_step >= p.m) {      // this warp's last token: its parts are here (they were added)
+                cluster_arrive();
+                arrived = true;
+            }
+            if (scaled) {
+                const float s = row_scale[m];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) total[c] *= s;
+            }
+            if (p.stream.on) {
+                stream_finish(p, m, lane, tile, n4, total, before, weight);
+            } else if (p.rope.on) {
+                rope_finish(p, m, lane, tile, total, weight, frequency, info);
+            } else if (p.silu_gate) {
+                silu_finish(p, m, lane, tile, total);
+            } else if (n4 < p.n) {
+                if (p.out_is_f32) store4_f32(reinterpret_cast<float*>(p.out) + (size_t)m * p.ldc + n4, total, p.n - n4, p.vector_out != 0);
+                else store4_bf16(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)m * p.ldc + n4, total, p.n - n4, p.vector_out != 0);
+            }
         }
     }
     if (p.split > 1) {          // nobody leaves while a peer may still read its shared memory
@@ -680,14 +895,21 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
                    (rope == nullptr || (aligned16(rope->k_pages) && aligned16(rope->v_pages)));
     p.vector_stream = p.stream.on && aligned16(p.stream.residual) && (p.stream.scaled == nullptr || aligned16(p.stream.scaled)) && n % 4 == 0;
     const int tiles = (n + kBlockRows - 1) / kBlockRows;
-    const int atoms = m > kTwoAtomRows ? 1 : 2;
-    const int total_kb = (k + kAtomK * atoms - 1) / (kAtomK * atoms);
     // K is split across a cluster so that the tiles fill the machine; each rank keeps >= 4 K blocks.  The
     // caller may name the split (it times a few once per shape); 0 asks for about one wave of 148 SMs.
     int split = requested_split > 0 ? requested_split : 148 / tiles;
+    const bool many = m > 16;
+    int atoms = m > kTwoAtomRows ? 1 : 2;
+    int total_kb = (k + kAtomK * atoms - 1) / (kAtomK * atoms);
     if (split > total_kb / 2) split = total_kb / 2;
     if (split > kMaxSplit) split = kMaxSplit;
     if (split < 1) split = 1;
+    // more than two blocks per SM: three, of single atoms (see gemm_small_m_kernel)
+    const bool three = many && m <= kTwoAtomRows && (long long)tiles * split > 2 * llm_sm_count();
+    if (three) {
+        atoms = 1;
+        total_kb = (k + kAtomK - 1) / kAtomK;
+    }
     p.split = split;
     const size_t a_bytes = (size_t)kBlockRows * kAtomK * 2;
     const size_t b_bytes = ((size_t)p.token_pad * kAtomK * 2 + 1023) & ~(size_t)1023;
@@ -701,7 +923,8 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
         if (ring_kib < 32) ring_kib = 32;
         if (ring_kib > 200) ring_kib = 200;
     }
-    int stages = (int)(((size_t)ring_kib * 1024) / stage_bytes);
+    int stages = (int)(((size_t)(three && ring_kib > kThreeBlocksKib ? kThreeBlocksKib : ring_kib) * 1024) / stage_bytes);
+    if (stages < 1) stages = 1;
     if (stages > kMaxStages) stages = kMaxStages;
     const int my_kb = (total_kb + split - 1) / split;
     if (stages > my_kb) stages = my_kb < 1 ? 1 : my_kb;
@@ -711,7 +934,7 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
     if (shared < reduce_bytes) shared = reduce_bytes;
     shared += 1024;   // room to align the region to 1024 bytes
 
-    auto* kernel = atoms == 1 ? gemm_small_m_kernel<1, true> : m > 16 ? gemm_small_m_kernel<2, true> : gemm_small_m_kernel<2, false>;
+    auto* kernel = three ? gemm_small_m_kernel<1, true, 3> : atoms == 1 ? gemm_small_m_kernel<1, true, 2> : many ? gemm_small_m_kernel<2, true, 2> : gemm_small_m_kernel<2, false, 0>;
     CUtensorMap map_w, map_x;
     if (!make_map(&map_w, w, n, k, kBlockRows) || !make_map(&map_x, x, m, k, p.token_pad)) {
         llm_set_error("gemm_small_m: cuTensorMapEncodeTiled failed (m %d, n %d, k %d)", m, n, k);

@@ -23,6 +23,36 @@ def test_product(rows, cols, inner, split):
         close(out, x.double() @ w.double().T, out_dtype, f"{rows, cols, inner, split}", factor=4.0 if out_dtype == torch.float32 else 1.0)
 
 
+@pytest.mark.parametrize("rows", [16, 17, 18, 47, 64, 65])
+@pytest.mark.parametrize("tiles,inner,split", [(296, 136, 1), (297, 136, 1), (149, 520, 2), (99, 264, 3), (38, 1032, 8)])
+def test_three_blocks_an_sm(rows, tiles, inner, split):
+    """Launches around two blocks per SM of 148, beyond which 17 to 64 rows run three of them with stages of one atom, K split or not:
+    plain sums, the gated form and the sums added to a stream, each with a last tile that is not full (the gated form's are)."""
+    from llmserver_b200.ops import gemm_bf16
+    from llmserver_b200.ops.library import call, check_wait_errors, stream_handle
+    cols = tiles * 128 - 126
+    x, w = rand((rows, inner), torch.bfloat16, 1), rand((tiles * 128, inner), torch.bfloat16, 2, inner ** -0.5)
+    flag, exact = gemm_bf16.error_flag(DEVICE).data_ptr(), x.double() @ w.double().T
+    out = torch.full((rows, cols), float("nan"), dtype=torch.float32, device=DEVICE)
+    call("llm_gemm_small_m", x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, cols, inner, cols, 1, split, *gemm_bf16.NO_SCALE, flag, stream_handle())
+    close(out, exact[:, :cols], torch.float32, "sums", factor=4.0)
+    gated = torch.full((rows, tiles * 64), float("nan"), dtype=torch.bfloat16, device=DEVICE)
+    call("llm_gemm_gate_up_silu", x.data_ptr(), w.data_ptr(), gated.data_ptr(), rows, tiles * 128, inner, tiles * 64, split, *gemm_bf16.NO_SCALE, flag,
+         stream_handle())
+    pairs = exact.view(rows, tiles, 2, 64)
+    close(gated, (pairs[:, :, 0] * torch.sigmoid(pairs[:, :, 0]) * pairs[:, :, 1]).flatten(1), torch.bfloat16, "gates")
+    stream, norm = rand((rows, cols), torch.float32, 3), rand((cols,), torch.bfloat16, 4)
+    want = stream.double() + exact[:, :cols]
+    scaled, parts = torch.zeros((rows, cols), dtype=torch.bfloat16, device=DEVICE), torch.zeros((tiles, 128), dtype=torch.float32, device=DEVICE)
+    call("llm_gemm_into_stream", x.data_ptr(), w.data_ptr(), stream.data_ptr(), rows, cols, inner, split, norm.data_ptr(), 0, scaled.data_ptr(),
+         parts.data_ptr(), 128, flag, stream_handle())
+    torch.cuda.synchronize()
+    check_wait_errors()
+    close(stream, want, torch.float32, "stream", factor=4.0)
+    close(scaled, want * norm.double(), torch.bfloat16, "the next norm's input")
+    close(parts[:, :rows].sum(0), (want * want).sum(-1), torch.float32, "sums of squares", factor=4.0)
+
+
 @pytest.mark.parametrize("rows", [16, 17, 33, 64, 65, 119, 128])
 def test_stream_and_scaled_rows(rows):
     """x W^T added to the stream, the sums of squares it leaves, and the gated product that divides by them: against the same in 64
