@@ -61,8 +61,8 @@ struct AttnParams {
     int skip_single;         // portions kernel: leave sequences with one token to the decode kernel
     int split_len;           // decode kernel: keys per split (multiple of 64); negative: -split_len equal parts per sequence
     int max_splits;
-    float* partial_out;      // [N, Hq, max_splits, D]
-    float* partial_ml;       // [N, Hq, max_splits, 2]
+    float* partial_out;      // [N, Hq, max_splits, D]; with slot_by_seq [S, Hq, max_splits, D]
+    float* partial_ml;       // [N, Hq, max_splits, 2]; the same
     int old_keys_settled;    // TMA decode kernel: every key but each sequence's newest was written before the kernel in
                              // front of this one started (by an earlier step), so their copies need not wait for it
     int cluster_merge;       // TMA decode kernel: the splits of a sequence form a thread-block cluster and merge their
@@ -83,6 +83,9 @@ struct AttnParams {
     float* maps_out = nullptr;      // DIFF: [N, Hq, D], 32-bit, in place of `out`
     float cap_log2 = 0.0f, cap_slope = 0.0f;    // CAP: cap * log2(e) (0: scores are not capped), 2 * scale / cap * log2(e)
     int by_length = 0;              // TMA decode kernel: blocks take the sequences longest first (up to kThreads of them)
+    int balance = 0;                // TMA decode kernel: > 0: long sequences are divided into more parts than short ones, so that no
+                                    // more than this many parts per kv head are made (see part_of_block)
+    int* part_counters = nullptr;   // balance: [S, Hkv], zero before and after: parts of a sequence that have left their result
 };
 
 // The first key that the query at `position` may see.
@@ -732,12 +735,78 @@ __device__ __forceinline__ int longest_first(const AttnParams& p, int place, int
     return *answer;
 }
 
+// The tiles that the single token of sequence `s` walks; -1 for portions of prompts.
+template <bool PRECISE>
+__device__ __forceinline__ int decode_tiles(const AttnParams& p, int s) {
+    const int context = p.context_len[s];
+    if (p.q_start[s + 1] - p.q_start[s] != 1) return -1;
+    if (context <= 0) return 0;
+    const int position = context - 1;
+    const int low = PRECISE ? first_visible(p, position) : p.window > 0 ? max(0, position - p.window + 1) : 0;
+    const int kept = PRECISE ? walk_of(p, low).kept_tiles : 0;
+    return kept + (context - low / kTileKeys * kTileKeys + kTileKeys - 1) / kTileKeys;
+}
+
+// Parts by length: which sequence the blocks at `place` along the grid take, which of its parts, and how many it has.  A part has
+// at most as many tiles as make the parts of all sequences fit one wave of blocks (the shortest such length, growing by eighths).
+// With equal numbers of parts the blocks of the longest sequence end last, while most SMs have nothing left to copy: a block
+// copies a tile in 0.84 us when it is nearly alone and in 1.45 us when a wave is at work.  Sequences so short that a
+// block of theirs ends within the first quarter are not counted (the padding rows of a replayed step among them).  Every
+// warp finds the same: it depends on the lengths alone.  False: no part is left for this place.
+template <bool PRECISE>
+__device__ __forceinline__ bool part_of_block(const AttnParams& p, int place, int& seq, int& part, int& parts) {
+    constexpr int kEach = kThreads / 32;
+    const int lane = threadIdx.x & 31;
+    int tiles[kEach], total = 0;
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) {
+        const int s = lane + 32 * i;
+        tiles[i] = s < p.n_seqs ? decode_tiles<PRECISE>(p, s) : -1;
+        total += max(tiles[i], 0);
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    int length = max(3, (total + p.balance - 1) / p.balance);
+    for (int round = 0; round < 32; ++round) {
+        int counted = 0;
+#pragma unroll
+        for (int i = 0; i < kEach; ++i)
+            if (4 * tiles[i] > length) counted += min((tiles[i] + length - 1) / length, p.max_splits);
+        if (__reduce_add_sync(0xffffffffu, counted) <= p.balance) break;
+        length += max(1, length >> 3);
+    }
+    int before = 0;      // parts of the sequences in front of this group of 32
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) {
+        const int mine = tiles[i] < 0 ? 0 : max(1, min((tiles[i] + length - 1) / length, p.max_splits));
+        int sum = mine;
+#pragma unroll
+        for (int offset = 1; offset < 32; offset <<= 1) {
+            const int other = __shfl_up_sync(0xffffffffu, sum, offset);
+            if (lane >= offset) sum += other;
+        }
+        const int first = before + sum - mine;
+        const unsigned found = __ballot_sync(0xffffffffu, place >= first && place < first + mine);
+        if (found) {
+            const int source = __ffs(found) - 1;
+            seq = source + 32 * i;
+            part = place - __shfl_sync(0xffffffffu, first, source);
+            parts = __shfl_sync(0xffffffffu, mine, source);
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    return false;
+}
+
 // DIFF: the heads of differential attention are [map 1 | map 2] of D / 2 elements each in Q and in the K rows, and every map of a
 // head is a row of the tile: its own half of the query, zeros in the other half, so that one product over whole K rows gives the
 // row's own map.  `n_q_heads` then counts maps (two per head), and results leave as 32-bit numbers for the kernel that subtracts
 // the maps.  64 sequences over a window of 1024 keys (32 / 8 heads) took 101 us in blocks of warps that each load keys of their own; a
 // decode step with two such layers went from 1193 to 1111 us.
-template <int D, bool PRECISE = false, bool DIFF = false>
+//
+// BALANCE: parts by length (part_of_block), each a block of its own, and the part that comes last adds them; a form of its own,
+// because the others run at 8 sequences 0.4 % slower a step with its code inside.
+template <int D, bool PRECISE = false, bool DIFF = false, bool BALANCE = false>
 __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                               const __grid_constant__ CUtensorMap map_v,
                                                                               const AttnParams p) {
@@ -765,7 +834,13 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
     unsigned char* stages = shared_raw + (base - raw);
     __nv_bfloat16* q_tile = reinterpret_cast<__nv_bfloat16*>(stages + kDecodeStages * 2 * kTileBytes);   // [16][D]
 
-    const int seq = p.by_length ? longest_first(p, blockIdx.z, lengths, &place_of) : blockIdx.z, kv_head = blockIdx.y, split = blockIdx.x;
+    int seq, kv_head, split, parts = 0;
+    if constexpr (BALANCE) {
+        kv_head = blockIdx.x;
+        if (!part_of_block<PRECISE>(p, blockIdx.y, seq, split, parts)) return;      // (others wait for the kernel in front)
+    } else {
+        seq = p.by_length ? longest_first(p, blockIdx.z, lengths, &place_of) : blockIdx.z, kv_head = blockIdx.y, split = blockIdx.x;
+    }
     const int token = p.q_start[seq];
     if (p.q_start[seq + 1] - token != 1) {
         if (early) pdl_wait();
@@ -784,7 +859,13 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
         walk.first_key = (low_key / kTileKeys) * kTileKeys;
     }
     const int span = walk_span(walk, context);
-    const int split_len = split_length(p, span);
+    int split_len;
+    if constexpr (BALANCE) {
+        const int tiles = (span + kTileKeys - 1) / kTileKeys;
+        split_len = max((tiles + parts - 1) / parts, 3) * kTileKeys;
+    } else {
+        split_len = split_length(p, span);
+    }
     const int n_splits = (span + split_len - 1) / split_len;
     if (n_splits > p.max_splits && split == 0 && kv_head == 0 && threadIdx.x == 0 && p.error_flag) atomicExch(p.error_flag, 6);
     if (context <= 0 && split == 0) {       // nothing to attend to
@@ -798,7 +879,7 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
     }
     // every thread of a cluster whose splits merge in shared memory meets at the same two cluster barriers, also the
     // blocks beyond the sequence's last split and the producer warps, which have nothing to add
-    const bool meets_cluster = p.cluster_merge && n_splits > 1;
+    const bool meets_cluster = !BALANCE && p.cluster_merge && n_splits > 1;
     if (split >= n_splits) {
         if (early) pdl_wait();
         if (meets_cluster) {
@@ -1028,6 +1109,54 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
             }
         }
     }
+    if constexpr (BALANCE) {
+        if (n_splits == 1) return;
+        // The part that comes last adds all of them, in their order and with the merge kernel's arithmetic: what the others left
+        // lies in L2.  (Clusters with a rank for every part that there could be keep the places of ranks without a part
+        // until the whole cluster ends: 32 sequences of 3072 keys in clusters of two, one rank idle, 6.86 ms a step against 5.56.)
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        int* counter = p.part_counters + (size_t)seq * p.n_kv_heads + kv_head;
+        if (threadIdx.x == 0)      // releases what the barrier has put in front of it, acquires what the other parts released
+            asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(place_of) : "l"(counter) : "memory");
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (place_of != n_splits - 1) return;
+        if (threadIdx.x == 0) *counter = 0;
+        constexpr int kMaxParts = 8;
+        for (int index = 2 * threadIdx.x; index < group * D; index += 2 * kThreads) {
+            const int r = index / D, d = index % D, head = kv_head * group + r;
+            const size_t slot0 = ((size_t)(p.slot_by_seq ? seq : token) * p.n_q_heads + head) * p.max_splits;
+            float2 statistics[kMaxParts], outputs[kMaxParts];
+#pragma unroll
+            for (int s = 0; s < kMaxParts; ++s) {
+                statistics[s] = s < n_splits ? __ldcg(reinterpret_cast<const float2*>(p.partial_ml + (slot0 + s) * 2)) : make_float2(-INFINITY, 0.0f);
+                outputs[s] = s < n_splits ? __ldcg(reinterpret_cast<const float2*>(p.partial_out + (slot0 + s) * D + d)) : make_float2(0.0f, 0.0f);
+            }
+            float best = -INFINITY;
+#pragma unroll
+            for (int s = 0; s < kMaxParts; ++s) best = fmaxf(best, statistics[s].x);
+            float numerator[2] = {0.0f, 0.0f}, denominator = 0.0f;
+#pragma unroll
+            for (int s = 0; s < kMaxParts; ++s) {
+                if (s < n_splits) {
+                    const float weight = statistics[s].y * exp2f(statistics[s].x - best);
+                    numerator[0] += outputs[s].x * weight;
+                    numerator[1] += outputs[s].y * weight;
+                    denominator += weight;
+                }
+            }
+            float result[2] = {numerator[0] / denominator, numerator[1] / denominator};
+            if constexpr (PRECISE) {
+                if (p.gate) {
+                    result[0] = gated(p, result[0], token, head * D + d);
+                    result[1] = gated(p, result[1], token, head * D + d + 1);
+                }
+            }
+            const size_t at = (size_t)token * p.n_q_heads * D + (size_t)head * D + d;
+            if constexpr (DIFF) *reinterpret_cast<float2*>(p.maps_out + at) = make_float2(result[0], result[1]);
+            else *reinterpret_cast<__nv_bfloat162*>(p.out + at) = __floats2bfloat162_rn(result[0], result[1]);
+        }
+        return;
+    }
     if (in_cluster) {
         // The splits of this (sequence, kv head) are the ranks 0 .. n_splits - 1 of one cluster (ranks beyond have left
         // already; a cluster barrier waits for threads that have not exited).  Every rank takes a share of the group's
@@ -1168,7 +1297,7 @@ bool describe_pages(const AttnParams& p, CUtensorMap* map_k, CUtensorMap* map_v)
 template <int D, bool PRECISE, bool DIFF>
 int launch_decode_tma(const AttnParams& given, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t stream) {
     AttnParams p = given;
-    auto* kernel = attention_decode_tma_kernel<D, PRECISE, DIFF>;
+    auto* kernel = p.balance > 0 ? attention_decode_tma_kernel<D, PRECISE, DIFF, !DIFF> : attention_decode_tma_kernel<D, PRECISE, DIFF>;
     // Two blocks share an SM.  Beyond one wave of them the order in which sequences start decides how raggedly the last wave
     // ends: 61 sequences of 301 to 4077 keys that lie shortest first, a decode step of the 8B shape 7.51 ms as they lie and
     // 6.70 ms longest first (more splits instead: 7.3 ms with two parts, 7.8 with three).  Within a wave all start at once.
@@ -1176,6 +1305,7 @@ int launch_decode_tma(const AttnParams& given, const CUtensorMap& map_k, const C
     const size_t shared = (size_t)kDecodeStages * 2 * kTileKeys * D * 2 + (size_t)16 * D * 2 + 1024;
     if (int limit_status = llm_raise_shared_limit(reinterpret_cast<const void*>(kernel), shared, "attention_decode_tma")) return limit_status;
     dim3 grid(p.max_splits, p.n_kv_heads, p.n_seqs);
+    if (p.balance > 0) grid = dim3(p.n_kv_heads, p.balance + p.n_seqs);      // the parts that are counted and those that are not
     if (!p.cluster_merge) {
         llm_launch(kernel, grid, kDecodeThreads, shared, stream, map_k, map_v, p);
         return llm_check_launch("attention_decode_tma");
@@ -1227,8 +1357,16 @@ int launch_decode(const AttnParams& p, cudaStream_t stream) {
     AttnParams q = p;
     // up to 8 splits (the portable cluster size) or exactly 16 (allowed on request) merge inside the kernel; others, or the cp.async kernel, go through the
     // scratch buffers and the merge kernel
-    q.cluster_merge = by_tma && p.cluster_merge && p.max_splits > 1 && (p.max_splits <= 8 || p.max_splits == 16);
-    if (p.max_splits > 1 && !q.cluster_merge && (p.partial_out == nullptr || p.partial_ml == nullptr)) {
+    // More parts allowed than the equal parts asked for: the longer sequences get more of them than the others, where that can be done.
+    if (p.split_len < 0 && p.max_splits > -p.split_len && p.part_counters != nullptr) {
+        q.slot_by_seq = 1;
+        if (by_tma && !DIFF && p.cluster_merge && p.n_seqs <= kThreads && p.max_splits <= 8 && p.partial_out != nullptr && p.partial_ml != nullptr)
+            q.balance = 2 * llm_sm_count() / p.n_kv_heads;
+        else
+            q.max_splits = -p.split_len;
+    }
+    q.cluster_merge = by_tma && p.cluster_merge && q.balance == 0 && q.max_splits > 1 && (q.max_splits <= 8 || q.max_splits == 16);
+    if (q.max_splits > 1 && !q.cluster_merge && (p.partial_out == nullptr || p.partial_ml == nullptr)) {
         llm_set_error("attention_decode: %d splits need the scratch buffers for partial results", p.max_splits);
         return LLM_REFUSED;
     }
@@ -1237,9 +1375,9 @@ int launch_decode(const AttnParams& p, cudaStream_t stream) {
         return LLM_REFUSED;
     }
     int status = by_tma ? launch_decode_tma<D, PRECISE, DIFF>(q, map_k, map_v, stream) : launch_decode_cp_async<D, D, PRECISE>(q, stream);
-    if (status != LLM_OK || p.max_splits <= 1 || q.cluster_merge) return status;
+    if (status != LLM_OK || q.max_splits <= 1 || q.cluster_merge || q.balance > 0) return status;
     dim3 merge_grid(p.n_q_heads, p.n_seqs);
-    llm_launch(attention_decode_merge_kernel<D>, merge_grid, D < 128 ? D : 128, 0, stream, p);
+    llm_launch(attention_decode_merge_kernel<D>, merge_grid, D < 128 ? D : 128, 0, stream, q);
     return llm_check_launch("attention_decode_merge");
 }
 
@@ -1291,7 +1429,7 @@ LLM_EXPORT int llm_attention_mma(const void* q, int q_stride, const void* k_page
                                  const int* block_tables, int max_blocks, const int* q_start, const int* context_len,
                                  void* out, int n_seqs, int n_q_heads, int n_kv_heads, int head_dim, int page_size,
                                  int num_pages, float scale, int window, int run_portions, int total_tiles, int run_decode,
-                                 int split_len, int max_splits, float* partial_out, float* partial_ml,
+                                 int split_len, int max_splits, float* partial_out, float* partial_ml, int* part_counters,
                                  int old_keys_settled, int* error_flag, cudaStream_t stream) {
     if (!llm_attention_mma_supports(head_dim, n_q_heads, n_kv_heads)) {
         llm_set_error("attention_mma: head_dim %d with %d/%d heads is not supported (head_dim 64 or 128, group <= 16)",
@@ -1335,6 +1473,7 @@ LLM_EXPORT int llm_attention_mma(const void* q, int q_stride, const void* k_page
     p.max_splits = max_splits;
     p.partial_out = partial_out;
     p.partial_ml = partial_ml;
+    p.part_counters = part_counters;
     p.error_flag = error_flag;
     int status = LLM_OK;
     if (run_portions && total_tiles > 0)
@@ -1493,7 +1632,8 @@ LLM_EXPORT int llm_attention_mma_sinks(const void* q, int q_stride, const void* 
                                        int page_size, int num_pages, float scale, int window, const float* sinks,
                                        int chunk, const float* bias, int bias_len, int keep, const void* gate, int gate_stride,
                                        int run_portions, int total_tiles, int run_decode, int split_len, int max_splits,
-                                       float* partial_out, float* partial_ml, int old_keys_settled, int* error_flag, cudaStream_t stream) {
+                                       float* partial_out, float* partial_ml, int* part_counters, int old_keys_settled, int* error_flag,
+                                       cudaStream_t stream) {
     if (!llm_attention_mma_sinks_supports(head_dim, value_dim, n_q_heads, n_kv_heads)) {
         llm_set_error("attention_mma_sinks: keys of %d and values of %d with %d/%d heads are not supported (64 or 128 each, "
                       "group <= 16)", head_dim, value_dim, n_q_heads, n_kv_heads);
@@ -1532,6 +1672,7 @@ LLM_EXPORT int llm_attention_mma_sinks(const void* q, int q_stride, const void* 
     p.max_splits = max_splits;
     p.partial_out = partial_out;
     p.partial_ml = partial_ml;
+    p.part_counters = part_counters;
     p.error_flag = error_flag;
     p.sinks = sinks;
     if (chunk < 0 || (bias && bias_len <= 0) || keep < 0 || (keep > 0 && chunk > 0)) {

@@ -21,6 +21,14 @@ MAX_CLUSTER_SPLITS = 8
 # 8B shape), clusters of 16 (beyond the portable size, which the hardware allows on request) get each block's keys in
 # flight at once: 3.21 against 3.25 ms per batch-1 step.  With more pairs they are slower (batch 2: 3.49 against 3.30).
 WIDE_CLUSTER_SPLITS = 16
+# Up to a wave of (sequence, kv head) pairs, and where equal parts would be at most two, the TMA kernel divides sequences by their
+# lengths (up to this many sequences, of up to MAX_CLUSTER_SPLITS parts each), on the device: a replayed step is planned for contexts
+# that it does not know.  Equal parts / by length, ms a step of the 8B shape: 24 sequences of 517 to 4003 keys 5.74 / 4.87, 12 of 100 to
+# 4000 4.13 / 3.75, 16 of 301 to 4077 4.20 / 4.03; equal contexts of 3072 keys, 32 sequences 5.55 / 5.51, 16 sequences 4.26 / 4.32 (merging
+# through L2 instead of a cluster).  With four equal parts the cluster stays ahead: 8 sequences of 3072 3.53 / 3.61, of 301 to 4077
+# 3.52 / 3.44.
+UNEVEN_SPLITS, UNEVEN_SEQUENCES = 2, 128
+
 
 
 # "tcgen05": the 256-row kernel for long portions and the 128-row kernel otherwise; "tcgen05-128" / "tcgen05-256":
@@ -74,13 +82,14 @@ def supported(head_dim: int, n_q_heads: int, n_kv_heads: int) -> bool:
 
 
 def plan(batch, group: int, n_kv_heads: int, device=None, blocks_per_sm: int = DECODE_BLOCKS_PER_SM, cluster: bool = None,
-         span: int = None):
+         span: int = None, by_length: bool = False):
     """Launch shape of a batch, derived once per step from its host-side lengths (and the number of SMs: the split
     count fixes the order of the partial sums, so it is a function of the batch and the GPU model only).
     ``blocks_per_sm``: decode blocks an SM holds at a time; ``cluster``: whether splits merge inside a cluster (which
-    bounds their number) or through the merge kernel; ``span``: the most keys a query sees, where that is bounded."""
+    bounds their number) or through the merge kernel; ``span``: the most keys a query sees, where that is bounded; ``by_length``: the
+    caller's kernel can give longer sequences more parts than others."""
     cluster = CLUSTER_MERGE if cluster is None else cluster
-    key = ("attention_mma", group, n_kv_heads, blocks_per_sm, cluster, span)
+    key = ("attention_mma", group, n_kv_heads, blocks_per_sm, cluster, span, by_length)
     cached = batch.scratch.get(key)
     if cached is not None:
         return cached
@@ -121,6 +130,8 @@ def plan(batch, group: int, n_kv_heads: int, device=None, blocks_per_sm: int = D
         # every sequence is divided into this many equal parts (a negative split length says so to the kernel): the
         # longest gets the planned splits, shorter ones the same number of shorter blocks
         split_len, max_splits = -splits, splits
+        if by_length and cluster and pairs <= wave_blocks and splits <= UNEVEN_SPLITS and 1 < singles and batch.n_seqs <= UNEVEN_SEQUENCES:
+            max_splits = MAX_CLUSTER_SPLITS      # more than the equal parts: what says "by length" to the kernel
         forced = os.environ.get("LLMSERVER_B200_DECODE_SPLIT")
         if forced:
             split_len = int(forced)
@@ -128,6 +139,18 @@ def plan(batch, group: int, n_kv_heads: int, device=None, blocks_per_sm: int = D
     cached = (run_portions, tiles, run_decode, split_len, max_splits)
     batch.scratch[key] = cached
     return cached
+
+
+def _part_counters(batch, n_kv_heads: int, split_len: int, max_splits: int, device) -> int:
+    """Where the parts of a (sequence, kv head) pair are counted when sequences are divided by their lengths: zero before and after
+    every launch, shared by the layers of a step.  0 when parts are equal."""
+    if not 0 < -split_len < max_splits:
+        return 0
+    key = ("attention_part_counters", n_kv_heads)
+    counters = batch.scratch.get(key)
+    if counters is None:
+        counters = batch.scratch[key] = torch.zeros(batch.n_seqs * n_kv_heads, dtype=torch.int32, device=device)
+    return counters.data_ptr()
 
 
 # A decode row's older keys were cached by earlier steps, which lie behind the step's batch copy; the decode kernel may
@@ -143,7 +166,7 @@ def try_attention(qkv, q_stride, batch, block_tables, k_pages, v_pages, n_q_head
     check(k_pages, "k pages", torch.bfloat16, head_dim)
     check(v_pages, "v pages", torch.bfloat16, head_dim)
     check(block_tables, "block_tables", torch.int32)
-    run_portions, tiles, run_decode, split_len, max_splits = plan(batch, n_q_heads // n_kv_heads, n_kv_heads, qkv.device)
+    run_portions, tiles, run_decode, split_len, max_splits = plan(batch, n_q_heads // n_kv_heads, n_kv_heads, qkv.device, by_length=True)
     out = torch.empty((batch.n_tokens, n_q_heads * head_dim), dtype=torch.bfloat16, device=qkv.device)
     partial_out = partial_ml = None
     if run_decode and max_splits > 1:
@@ -151,8 +174,9 @@ def try_attention(qkv, q_stride, batch, block_tables, k_pages, v_pages, n_q_head
         key = ("attention_mma_scratch", n_q_heads, head_dim, max_splits)
         scratch = batch.scratch.get(key)
         if scratch is None:
-            scratch = (torch.empty((batch.n_tokens, n_q_heads, max_splits, head_dim), dtype=torch.float32, device=qkv.device),
-                       torch.empty((batch.n_tokens, n_q_heads, max_splits, 2), dtype=torch.float32, device=qkv.device))
+            rows = batch.n_seqs if 0 < -split_len < max_splits else batch.n_tokens      # parts by length have a place per sequence
+            scratch = (torch.empty((rows, n_q_heads, max_splits, head_dim), dtype=torch.float32, device=qkv.device),
+                       torch.empty((rows, n_q_heads, max_splits, 2), dtype=torch.float32, device=qkv.device))
             batch.scratch[key] = scratch
         partial_out, partial_ml = scratch
     page_size = k_pages.shape[2]
@@ -184,8 +208,8 @@ def try_attention(qkv, q_stride, batch, block_tables, k_pages, v_pages, n_q_head
          block_tables.shape[-1], batch.q_start.data_ptr(), batch.context_len.data_ptr(), out.data_ptr(), batch.n_seqs,
          n_q_heads, n_kv_heads, head_dim, page_size, k_pages.shape[0], float(scale), int(window), int(run_portions), tiles,
          int(run_decode), split_len, max_splits, 0 if partial_out is None else partial_out.data_ptr(),
-         0 if partial_ml is None else partial_ml.data_ptr(), int(EARLY_KEYS and getattr(batch, "keys_settled", False)), flag,
-         stream_handle())
+         0 if partial_ml is None else partial_ml.data_ptr(), _part_counters(batch, n_kv_heads, split_len, max_splits, qkv.device),
+         int(EARLY_KEYS and getattr(batch, "keys_settled", False)), flag, stream_handle())
     return out
 
 
@@ -232,7 +256,7 @@ def try_attention_precise(qkv, q_stride, batch, block_tables, k_pages, v_pages, 
     by_tma = value_dim == head_dim and bias_log2 is None and decode_by_tma(k_pages, v_pages)
     run_portions, tiles, run_decode, split_len, max_splits = plan(
         batch, n_q_heads // n_kv_heads, n_kv_heads, qkv.device, span=key_span(window, chunk, keep),
-        **({} if by_tma else {"blocks_per_sm": PRECISE_DECODE_BLOCKS_PER_SM, "cluster": False}))
+        **({"by_length": True} if by_tma else {"blocks_per_sm": PRECISE_DECODE_BLOCKS_PER_SM, "cluster": False}))
     from . import _gate_rows
     gate_pointer, gate_stride = _gate_rows(gate, gate_column, batch.n_tokens, n_q_heads * value_dim, torch.bfloat16)
     keep = int(keep) if window else 0
@@ -242,8 +266,9 @@ def try_attention_precise(qkv, q_stride, batch, block_tables, k_pages, v_pages, 
         key = ("attention_mma_scratch", n_q_heads, value_dim, max_splits)
         scratch = batch.scratch.get(key)
         if scratch is None:
-            scratch = (torch.empty((batch.n_tokens, n_q_heads, max_splits, value_dim), dtype=torch.float32, device=qkv.device),
-                       torch.empty((batch.n_tokens, n_q_heads, max_splits, 2), dtype=torch.float32, device=qkv.device))
+            rows = batch.n_seqs if 0 < -split_len < max_splits else batch.n_tokens
+            scratch = (torch.empty((rows, n_q_heads, max_splits, value_dim), dtype=torch.float32, device=qkv.device),
+                       torch.empty((rows, n_q_heads, max_splits, 2), dtype=torch.float32, device=qkv.device))
             batch.scratch[key] = scratch
         partial_out, partial_ml = scratch
     page_size = k_pages.shape[2]
@@ -274,6 +299,7 @@ def try_attention_precise(qkv, q_stride, batch, block_tables, k_pages, v_pages, 
          0 if sinks is None else sinks.data_ptr(), int(chunk), 0 if bias_log2 is None else bias_log2.data_ptr(),
          0 if bias_log2 is None else bias_log2.shape[1], keep, gate_pointer, gate_stride, int(run_portions), tiles, int(run_decode), split_len, max_splits,
          0 if partial_out is None else partial_out.data_ptr(), 0 if partial_ml is None else partial_ml.data_ptr(),
+         _part_counters(batch, n_kv_heads, split_len, max_splits, qkv.device),
          int(EARLY_KEYS and getattr(batch, "keys_settled", False)), wait_error_flag(qkv.device).data_ptr(), stream_handle())
     return out
 

@@ -75,6 +75,59 @@ def test_longest_first_takes_every_sequence_once(n_seqs):
     assert worst <= 2e-2, f"relative error {worst:.3e}"
 
 
+# (contexts, tokens of prompt portions in front of them): lengths around a tile and around the shortest part, one much longer than
+# all others, equal ones, a sequence without tokens, rows of a padded step, as many sequences as are divided by length
+UNEVEN = [([4000] + [1] * 20, 0), ([64 * k + k % 3 - 1 for k in range(1, 34)], 0), ([3000] * 17, 0), ([2500, 0, 70, 900, 0] * 4, 0),
+          ([1 + 31 * k for k in range(128)], 0), ([700, 4096, 33, 1900, 128, 129, 191, 192, 193, 2000] * 2, 150)]
+
+
+@pytest.mark.parametrize("form", [None, dict(), dict(sinks=True, gate=True), dict(window=300, keep=70)], ids=["narrow", "precise", "sinks-gate", "window"])
+@pytest.mark.parametrize("case", range(len(UNEVEN)))
+@pytest.mark.parametrize("heads,dim", [(32, 128), (10, 64)])
+def test_parts_by_length(form, case, heads, dim):
+    """Sequences of unequal length on up to a wave of blocks: the longer ones are divided into more parts, and the part that comes
+    last adds them.  Three launches on the same counters give the same bits, and what the kernel for every size gives but for
+    the rounding of weights."""
+    from llmserver_b200 import ops
+    from llmserver_b200.ops import attention_bf16
+    from llmserver_b200.ops.library import check_wait_errors
+    contexts, portion = UNEVEN[case]
+    kv_heads, page_size = (2 if len(contexts) > 37 else 8) if dim == 128 else 2, 16
+    q_lens = [1] * len(contexts) + ([portion] if portion else [])
+    contexts = contexts + ([portion + 77] if portion else [])
+    batch = HostBatch(q_lens, contexts)
+    batch.max_q_len = max(q_lens)
+    batch.seq_of_token = torch.repeat_interleave(torch.arange(len(q_lens), dtype=torch.int32), torch.tensor(q_lens)).to(DEVICE)
+    batch.positions = torch.cat([torch.arange(context - count, context) for context, count in zip(contexts, q_lens)]).clamp_min(0).to(torch.int32).to(DEVICE)
+    qkv, q_stride, k_pages, v_pages, tables = paged_case(case, q_lens, [max(c, 1) for c in contexts], heads, kv_heads, dim, page_size, 2.0)
+    given = dict(window=0) if form is None else dict(
+        window=form.get("window", 0), keep=form.get("keep", 0), sinks=torch.linspace(-2.0, 3.0, heads, device=DEVICE) if form.get("sinks") else None,
+        gate=torch.randn((batch.n_tokens, heads * dim), device=DEVICE).to(torch.bfloat16) if form.get("gate") else None)
+    planned = attention_bf16.plan(batch, heads // kv_heads, kv_heads, torch.device(DEVICE), by_length=True,
+                                  span=attention_bf16.key_span(given["window"], 0, given.get("keep", 0)))
+    singles = sum(count == 1 for count in q_lens)
+    assert (0 < -planned[3] < planned[4]) == (296 // (singles * kv_heads) <= attention_bf16.UNEVEN_SPLITS), planned
+    results = []
+    for _ in range(3):
+        if form is None:
+            results.append(attention_bf16.try_attention(qkv, q_stride, batch, tables, k_pages, v_pages, heads, kv_heads, dim, dim ** -0.5, 0))
+        else:
+            results.append(ops.attention(qkv, batch, tables, k_pages, v_pages, heads, kv_heads, dim, dim ** -0.5, precise=True, q_stride=q_stride, **given))
+    want = ops.attention_generic(qkv, q_stride, k_pages, v_pages, tables, batch.seq_of_token, batch.positions, heads, kv_heads, dim, dim ** -0.5, **given)
+    torch.cuda.synchronize()
+    check_wait_errors()
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
+    got, want = results[0].double(), want.double()
+    for row, context in enumerate(contexts[:singles]):
+        if context == 0:
+            assert not got[row].any()
+            want[row] = 0
+    assert torch.isfinite(got).all()
+    # as above; weights of 8 bits (narrow) are off by 2^-9 each, at most that much of the row's largest value
+    error = (got - want).abs() / torch.maximum(want.abs(), 0.05 * want.abs().amax(dim=-1, keepdim=True).clamp_min(1e-30))
+    assert error.max() <= (2.0 ** -7 if form is not None else 2.0 ** -7 + 20 * 2.0 ** -9), f"{float(error.max()):.2e}"
+
+
 @pytest.mark.parametrize("dim", [64, 128])
 @pytest.mark.parametrize("precise", [False, True])
 @pytest.mark.parametrize("contexts", [[900], [3000, 700]])
