@@ -25,6 +25,7 @@
 // blocks as there are segments; sums are then grouped by segment, so results agree with the one-pass form to rounding,
 // not bit for bit (the 32-bit path keeps the one-pass form).
 #include "common.cuh"
+#include "tcgen05.cuh"      // two-wide 32-bit arithmetic
 
 #define GLA_TOKENS 16
 
@@ -183,6 +184,230 @@ __global__ void __launch_bounds__(RR == 128 ? 256 : 512, RR <= 16 ? 2 : 1) gla_r
     }
 }
 
+// The same passes for bfloat16 steps and heads of 64 key channels, where a thread owns a tile of S: 8 rows of 8 columns, so that what
+// it reads of shared memory for a token (q, k and alpha of its rows, v of its columns: eight 16-byte loads) serves 192
+// multiply-adds, made two at a time (fma.rn.f32x2 over pairs of rows).  A warp holds 32 columns of S: lane = row group + 8 * column
+// group, row group r has rows 4 r .. 4 r + 3 and 32 + 4 r .. 32 + 4 r + 3 (so that the eight groups of a load are 128 contiguous
+// bytes), and the row groups' parts of o are added by seven shuffles, each of which halves the columns that a lane still holds.
+// What bounds the kernel above for long portions is its staging: a thread's loads of a batch of tokens wait for one another (up to
+// 16 in a row).  Here all of a batch is asked for at once, 16 bytes at a time.  2048 tokens of 32 heads of 64 / 128, us, the
+// kernel above / this: states of the segments 153 / 76, outputs 232 / 156 (tiles with loads one after the other: 148 and 254).
+constexpr int kTileDim = 64;
+
+// Eight bfloat16 numbers, times `scale`, as 32-bit numbers in shared memory.
+__device__ __forceinline__ void spread8(const float4& raw, float scale, float* dst) {
+    const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    float v[8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float2 both = __bfloat1622float2(pairs[c]);
+        v[2 * c] = both.x * scale;
+        v[2 * c + 1] = both.y * scale;
+    }
+    *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+
+template <typename W, int VDIM, int MODE>
+__global__ void __launch_bounds__(VDIM) gla_tiles_kernel(GlaArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    typedef __nv_bfloat16 T;
+    extern __shared__ float4 gla_shared_raw[];
+    float* shared = reinterpret_cast<float*>(gla_shared_raw);
+    const int seq = blockIdx.x, head = blockIdx.y;
+    int begin = a.q_start[seq], end = a.q_start[seq + 1];
+    if (begin >= end) return;
+    bool last_segment = true;
+    size_t segment_index = 0;
+    if (MODE != GLA_ONE_PASS) {
+        const int segments = (end - begin + a.segment - 1) / a.segment;
+        const int segment = blockIdx.z;
+        if (segment >= segments) return;
+        last_segment = segment == segments - 1;
+        if (MODE == GLA_LOCAL && last_segment) return;      // nobody needs the state a zero start leaves behind the last one
+        begin += segment * a.segment;
+        end = min(end, begin + a.segment);
+        segment_index = ((size_t)seq * a.max_segments + segment) * a.heads + head;
+    }
+    float* q_s = shared;                                   // [GLA_TOKENS][64]
+    float* k_s = q_s + GLA_TOKENS * kTileDim;
+    float* alpha_s = k_s + GLA_TOKENS * kTileDim;
+    float* v_s = alpha_s + GLA_TOKENS * kTileDim;          // [GLA_TOKENS][VDIM]
+    float* o_s = v_s + GLA_TOKENS * VDIM;                  // [GLA_TOKENS][VDIM]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kWarps = VDIM / 32;
+    const int row_group = lane & 7, column0 = warp * 32 + (lane >> 3) * 8;
+    const T* proj = (const T*)a.proj;
+
+    uint64_t S[4][8];                                       // [pair of rows][column]
+    uint64_t decay[MODE == GLA_LOCAL ? 4 : 1];               // pass A: the product of the segment's decays
+    float* state = a.state + ((size_t)a.state_slots[seq] * a.heads + head) * kTileDim * VDIM;
+    float* segment_state = a.segment_state + segment_index * kTileDim * VDIM;
+    const float* source = MODE == GLA_OUTPUT ? segment_state : state;
+    auto row_of = [&](int pair) { return 4 * row_group + (pair >> 1) * 32 + (pair & 1) * 2; };
+#pragma unroll
+    for (int pair = 0; pair < 4; ++pair) {
+        if (MODE == GLA_LOCAL) {
+            decay[pair] = tc5::pair_of(1.0f, 1.0f);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) S[pair][c] = 0;
+        } else {
+            const float* first = source + (size_t)row_of(pair) * VDIM + column0;
+#pragma unroll
+            for (int c = 0; c < 8; c += 4) {
+                const float4 low = *reinterpret_cast<const float4*>(first + c), high = *reinterpret_cast<const float4*>(first + VDIM + c);
+                S[pair][c] = tc5::pair_of(low.x, high.x);
+                S[pair][c + 1] = tc5::pair_of(low.y, high.y);
+                S[pair][c + 2] = tc5::pair_of(low.z, high.z);
+                S[pair][c + 3] = tc5::pair_of(low.w, high.w);
+            }
+        }
+    }
+    const int my_column = column0 + row_group;      // the one of its eight that a lane holds when the row groups' parts have been added
+
+    for (int first = begin; first < end; first += GLA_TOKENS) {
+        const int count = min(GLA_TOKENS, end - first);
+        __syncthreads();      // what the tokens before left in shared memory has been read
+        // Everything a batch of tokens needs is asked for before the first of it is used, 16 bytes at a time.
+        constexpr int kNarrow = GLA_TOKENS * kTileDim / 8, kWide = GLA_TOKENS * kTileDim / 4, kValues = GLA_TOKENS * VDIM / 8;
+        constexpr int kNarrowEach = (kNarrow + VDIM - 1) / VDIM, kWideEach = (kWide + VDIM - 1) / VDIM, kValuesEach = (kValues + VDIM - 1) / VDIM;
+        float4 q_raw[kNarrowEach], k_raw[kNarrowEach], z_raw[kWideEach], v_raw[kValuesEach];
+#pragma unroll
+        for (int u = 0; u < kNarrowEach; ++u) {
+            const int e = threadIdx.x + u * VDIM, t = e / (kTileDim / 8), i = e % (kTileDim / 8) * 8;
+            if (e < kNarrow && t < count) {
+                const T* row = proj + (size_t)(first + t) * a.row_width + head * kTileDim + i;
+                if (MODE != GLA_LOCAL) q_raw[u] = *reinterpret_cast<const float4*>(row + a.q_offset);
+                k_raw[u] = *reinterpret_cast<const float4*>(row + a.k_offset);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kWideEach; ++u) {
+            const int e = threadIdx.x + u * VDIM, t = e / (kTileDim / 4), i = e % (kTileDim / 4) * 4;
+            if (e < kWide && t < count) z_raw[u] = *reinterpret_cast<const float4*>(a.z + ((size_t)(first + t) * a.heads + head) * kTileDim + i);
+        }
+#pragma unroll
+        for (int u = 0; u < kValuesEach; ++u) {
+            const int e = threadIdx.x + u * VDIM, t = e / (VDIM / 8), j = e % (VDIM / 8) * 8;
+            if (t < count) v_raw[u] = *reinterpret_cast<const float4*>(proj + (size_t)(first + t) * a.row_width + a.v_offset + head * VDIM + j);
+        }
+#pragma unroll
+        for (int u = 0; u < kNarrowEach; ++u) {
+            const int e = threadIdx.x + u * VDIM;
+            if (e < kNarrow && e / (kTileDim / 8) < count) {
+                if (MODE != GLA_LOCAL) spread8(q_raw[u], a.q_scale, q_s + e * 8);
+                spread8(k_raw[u], 1.0f, k_s + e * 8);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kWideEach; ++u) {
+            const int e = threadIdx.x + u * VDIM, i = e % (kTileDim / 4) * 4;
+            if (e < kWide && e / (kTileDim / 4) < count) {
+                float zz[4] = {z_raw[u].x, z_raw[u].y, z_raw[u].z, z_raw[u].w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (a.z_bias) zz[c] += a.z_bias[head * kTileDim + i + c];
+                    // log sigmoid(zz) = -softplus(-zz), stable on both sides
+                    const float log_sigmoid = zz[c] >= 0.0f ? -log1pf(expf(-zz[c])) : zz[c] - log1pf(expf(zz[c]));
+                    zz[c] = expf(log_sigmoid * a.inverse_tau);
+                }
+                *reinterpret_cast<float4*>(alpha_s + e * 4) = make_float4(zz[0], zz[1], zz[2], zz[3]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kValuesEach; ++u) {
+            const int e = threadIdx.x + u * VDIM;
+            if (e / (VDIM / 8) < count) spread8(v_raw[u], 1.0f, v_s + e * 8);
+        }
+        __syncthreads();
+        for (int t = 0; t < count; ++t) {
+            const int at = t * kTileDim + 4 * row_group;
+            const ulonglong2 k_low = *reinterpret_cast<const ulonglong2*>(k_s + at), k_high = *reinterpret_cast<const ulonglong2*>(k_s + at + 32);
+            const ulonglong2 a_low = *reinterpret_cast<const ulonglong2*>(alpha_s + at), a_high = *reinterpret_cast<const ulonglong2*>(alpha_s + at + 32);
+            const uint64_t k[4] = {k_low.x, k_low.y, k_high.x, k_high.y}, alpha[4] = {a_low.x, a_low.y, a_high.x, a_high.y};
+            const float4 v_low = *reinterpret_cast<const float4*>(v_s + t * VDIM + column0), v_high = *reinterpret_cast<const float4*>(v_s + t * VDIM + column0 + 4);
+            const float v[8] = {v_low.x, v_low.y, v_low.z, v_low.w, v_high.x, v_high.y, v_high.z, v_high.w};
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint64_t vv = tc5::pair_of(v[c], v[c]);
+#pragma unroll
+                for (int pair = 0; pair < 4; ++pair) S[pair][c] = tc5::fma_pair(alpha[pair], S[pair][c], tc5::mul_pair(k[pair], vv));
+            }
+            if (MODE == GLA_LOCAL) {
+#pragma unroll
+                for (int pair = 0; pair < 4; ++pair) decay[pair] = tc5::mul_pair(decay[pair], alpha[pair]);
+                continue;
+            }
+            const ulonglong2 q_low = *reinterpret_cast<const ulonglong2*>(q_s + at), q_high = *reinterpret_cast<const ulonglong2*>(q_s + at + 32);
+            const uint64_t q[4] = {q_low.x, q_low.y, q_high.x, q_high.y};
+            float o[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                uint64_t sum = tc5::mul_pair(S[0][c], q[0]);
+#pragma unroll
+                for (int pair = 1; pair < 4; ++pair) sum = tc5::fma_pair(S[pair][c], q[pair], sum);
+                float low, high;
+                tc5::halves_of(sum, low, high);
+                o[c] = low + high;
+            }
+#pragma unroll
+            for (int held = 4; held > 0; held >>= 1) {      // of 2 * held columns a lane keeps the half that its row group names
+                const bool upper = row_group & held;
+#pragma unroll
+                for (int c = 0; c < held; ++c) {
+                    const float mine = upper ? o[c + held] : o[c], other = upper ? o[c] : o[c + held];
+                    o[c] = mine + __shfl_xor_sync(0xffffffffu, other, held);
+                }
+            }
+            o_s[t * VDIM + my_column] = o[0];
+        }
+        if (MODE == GLA_LOCAL) continue;
+        __syncthreads();
+        constexpr int kEach = VDIM / 32;      // neighbouring columns of a lane
+        for (int t = warp; t < count; t += kWarps) {
+            const T* g_row = proj + (size_t)(first + t) * a.row_width + a.g_offset + head * VDIM + lane * kEach;
+            T* dst = (T*)a.out + (size_t)(first + t) * a.heads * VDIM + head * VDIM + lane * kEach;
+            float o[kEach], g[kEach], sum_squares = 0.0f;
+#pragma unroll
+            for (int j = 0; j < kEach; ++j) {
+                g[j] = Num<T>::load(g_row + j);
+                o[j] = o_s[t * VDIM + lane * kEach + j];
+                sum_squares += o[j] * o[j];
+            }
+            const float inverse = rsqrtf(warp_sum(sum_squares) / (float)VDIM + a.eps);
+#pragma unroll
+            for (int j = 0; j < kEach; ++j) {
+                const float gate = g[j] / (1.0f + expf(-g[j]));
+                Num<T>::store(dst + j, o[j] * inverse * Num<W>::load((const W*)a.weight + lane * kEach + j) * gate);
+            }
+        }
+    }
+    if (MODE == GLA_LOCAL || last_segment) {
+        float* target = MODE == GLA_LOCAL ? segment_state : state;
+#pragma unroll
+        for (int pair = 0; pair < 4; ++pair) {
+            float* to = target + (size_t)row_of(pair) * VDIM + column0;
+#pragma unroll
+            for (int c = 0; c < 8; c += 4) {
+                float4 low, high;
+                tc5::halves_of(S[pair][c], low.x, high.x);
+                tc5::halves_of(S[pair][c + 1], low.y, high.y);
+                tc5::halves_of(S[pair][c + 2], low.z, high.z);
+                tc5::halves_of(S[pair][c + 3], low.w, high.w);
+                *reinterpret_cast<float4*>(to + c) = low;
+                *reinterpret_cast<float4*>(to + VDIM + c) = high;
+            }
+            if (MODE == GLA_LOCAL && warp == 0 && lane < 8) {
+                float low, high;
+                tc5::halves_of(decay[pair], low, high);
+                a.segment_decay[segment_index * kTileDim + row_of(pair)] = low;
+                a.segment_decay[segment_index * kTileDim + row_of(pair) + 1] = high;
+            }
+        }
+    }
+}
+
 // The scan between the passes: per (sequence, head), S_in(0) is the slot's state and S_in(k + 1) = D_k S_in(k) + S_local(k);
 // S_in(k) takes S_local(k)'s place in the scratch.  One thread per cell of S: the cells are independent, and the
 // segments' values are loaded a few ahead of the chain of multiply-adds that needs them.
@@ -239,6 +464,21 @@ LLM_EXPORT int llm_gla_supports(int dim, int vdim) {
     return gla_rows_per_thread(dim, (vdim + 31) / 32 * 32) != 0;
 }
 
+// bfloat16 steps of heads with 64 key channels and 64 or 128 value channels: the tiled kernel.
+template <typename W, int VDIM>
+int gla_tiles_launch(const GlaArgs& a, int n_seqs, bool segmented, cudaStream_t stream) {
+    const size_t shared = ((size_t)3 * GLA_TOKENS * kTileDim + (size_t)2 * GLA_TOKENS * VDIM) * sizeof(float);
+    const dim3 grid(n_seqs, a.heads, segmented ? a.max_segments : 1);
+    if (!segmented) {
+        llm_launch(gla_tiles_kernel<W, VDIM, GLA_ONE_PASS>, grid, VDIM, shared, stream, a);
+    } else {
+        llm_launch(gla_tiles_kernel<W, VDIM, GLA_LOCAL>, grid, VDIM, shared, stream, a);
+        llm_launch(gla_scan_kernel, dim3(n_seqs, a.heads, (a.dim * a.vdim + 255) / 256), 256, 0, stream, a);
+        llm_launch(gla_tiles_kernel<W, VDIM, GLA_OUTPUT>, grid, VDIM, shared, stream, a);
+    }
+    return llm_check_launch("gla_recurrent");
+}
+
 LLM_EXPORT int llm_gla_recurrent(const void* proj, int row_width, int q_offset, int k_offset, int v_offset, int g_offset,
                                  const float* z, const float* z_bias, const void* weight, float* state, const int* state_slots,
                                  const int* q_start, void* out, int n_seqs, int heads, int dim, int vdim, float inverse_tau,
@@ -264,6 +504,13 @@ LLM_EXPORT int llm_gla_recurrent(const void* proj, int row_width, int q_offset, 
     if (segmented && (max_segments <= 0 || !segment_state || !segment_decay)) {
         llm_set_error("gla_recurrent: the segmented form needs its scratch");
         return LLM_REFUSED;
+    }
+    // the tiled kernel reads rows and states in 16-byte pieces
+    const bool pieces = aligned16(proj) && row_width % 8 == 0 && q_offset % 8 == 0 && k_offset % 8 == 0 && v_offset % 8 == 0 && aligned16(z) &&
+                        aligned16(state) && (!segmented || (aligned16(segment_state) && aligned16(segment_decay)));
+    if (dtype == LLM_BF16 && (weight_dtype == LLM_F32 || weight_dtype == LLM_BF16) && dim == kTileDim && (vdim == 64 || vdim == 128) && pieces) {
+        if (vdim == 64) return weight_dtype == LLM_F32 ? gla_tiles_launch<float, 64>(a, n_seqs, segmented, stream) : gla_tiles_launch<__nv_bfloat16, 64>(a, n_seqs, segmented, stream);
+        return weight_dtype == LLM_F32 ? gla_tiles_launch<float, 128>(a, n_seqs, segmented, stream) : gla_tiles_launch<__nv_bfloat16, 128>(a, n_seqs, segmented, stream);
     }
     const int threads = a.partitions * a.column_threads;
     const size_t shared = ((size_t)3 * GLA_TOKENS * a.padded_dim + (size_t)GLA_TOKENS * vdim + (size_t)a.partitions * GLA_TOKENS * vdim) * sizeof(float);

@@ -441,6 +441,43 @@ def test_gated_linear_attention_kernel(dtype, heads, dim, vdim, tau):
         assert bool((state[1] == 7.0).all())
 
 
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("wide_weight,bias", [(False, True), (True, False)])
+@pytest.mark.parametrize("segment", [0, 16, 24, 64])
+def test_linear_attention_in_tiles(vdim, wide_weight, bias, segment):
+    """Heads of 64 key channels in bfloat16 with rows in whole 16-byte pieces, which run the tiled kernel: requests of lengths around
+    its batch of 16 tokens, each behind a state of its own, in one pass and in segments that are no multiple of a batch."""
+    from llmserver_b200 import ops
+    from llmserver_b200.engine.batch import SequenceSlice, build_batch
+    heads, dim, tau, eps, lengths = 3, 64, 16.0, 1e-5, [1, 15, 16, 17, 33, 130]
+    keys, values, count = heads * dim, heads * vdim, sum(lengths)
+    generator = torch.Generator().manual_seed(vdim + segment)
+    proj = torch.randn((count, 2 * keys + 2 * values + 8), generator=generator).to(torch.bfloat16)
+    z, z_bias = torch.randn((count, keys), generator=generator) * 2, torch.linspace(-2.0, 7.0, keys) if bias else None
+    weight = (1 + 0.2 * torch.randn((vdim,), generator=generator)).to(torch.float32 if wide_weight else torch.bfloat16)
+    before = torch.randn((len(lengths), heads, dim, vdim), generator=generator)
+    columns = (8, 8 + keys, 8 + 2 * keys, 8 + 2 * keys + values)
+    slots = list(reversed(range(len(lengths))))
+    state = before[torch.tensor(slots)].to(DEVICE)      # sequence s lies in slot slots[s]
+    batch = build_batch([SequenceSlice(s, [0] * n, 0, [], [[0]], slots[s]) for s, n in enumerate(lengths)], 1, DEVICE)
+    got = ops.gla_recurrent(proj.to(DEVICE), *columns, z.to(DEVICE), z_bias.to(DEVICE) if bias else None, weight.to(DEVICE), state, batch,
+                            heads, dim, vdim, tau, dim ** -0.5, eps, segment=segment).cpu().double()
+    alpha = (torch.sigmoid(z.double() + (z_bias.double() if bias else 0.0)) ** (1.0 / tau)).view(-1, heads, dim)
+    q, k, v, g = (proj.double()[:, at:at + size] for at, size in zip(columns, (keys, keys, values, values)))
+    q, k, v = q.view(-1, heads, dim) * dim ** -0.5, k.view(-1, heads, dim), v.view(-1, heads, vdim)
+    at = 0
+    for s, n in enumerate(lengths):
+        S, want = before[s].double(), torch.zeros((n, heads, vdim), dtype=F64)
+        for t in range(n):
+            S = alpha[at + t][:, :, None] * S + k[at + t][:, :, None] * v[at + t][:, None, :]
+            want[t] = torch.einsum("hdv,hd->hv", S, q[at + t])
+        want = plain.rms_norm(want, weight.double(), eps).reshape(n, values) * (g[at:at + n] * torch.sigmoid(g[at:at + n]))
+        # one rounding to bfloat16 of the result; the state is 32-bit: 130 steps of 2^-24 on sums of about 100
+        assert torch.allclose(got[at:at + n], want, atol=2.0 ** -8, rtol=2.0 ** -8), f"sequence {s}"
+        assert torch.allclose(state[slots[s]].cpu().double(), S, atol=2e-4, rtol=2e-5), f"state of sequence {s}"
+        at += n
+
+
 # ------------------------------------------------------------------------------------------------ whole models
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("name", NAMES)
