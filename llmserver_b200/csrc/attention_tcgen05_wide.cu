@@ -4,20 +4,25 @@
 //
 //   one CTA per SM takes 256 rows of one (sequence, kv head) as two halves A and B of 128 rows (rows are
 //   (token, head of the group) pairs) and walks the keys in tiles of 128.  Both halves read the same K and V
-//   tiles, so a tile is fetched once for 256 rows, and S = Q K^T is a 128 x 128 x 16 instruction, which the
-//   tensor core runs at full rate (the 128 x 64 x 16 form of the 128-row kernel is bound by shared-memory reads).
+//   tiles, so a tile is fetched once for 256 rows.
 //
 //   producer warp   TMA: Q of both halves once (4-D boxes), then per key tile the K and V pages (one 5-D box
 //                   per page) into rings of three and two stages
-//   MMA warp        one thread: S_A(0) S_B(0), then per tile  PV_A(j) S_A(j+1) PV_B(j) S_B(j+1): while the softmax
-//                   warps of one half work on their S, the tensor core runs the other half's P V and next S
-//   8 softmax warps four per half; thread r owns row r of its half: tcgen05.ld of S (two loads of 64 columns),
-//                   mask at the edges only, running maximum and sum in 32-bit, 2^x on the special-function unit,
-//                   P written as packed bfloat16 over columns 64..127 of the half's S; O is rescaled only when
-//                   a row's maximum has grown by more than 2^8 since its reference
+//   2 MMA warps     one thread per half: a tile's scores are two parts of 64 keys, S_low in columns 0..63 and S_high in columns
+//                   64..127 of the half's S.  Per tile: S_low(j+1) as soon as the softmax warps have S_low(j) in registers,
+//                   PV_low(j), PV_high(j), S_high(j+1)
+//   8 softmax warps four per half; thread r owns row r of its half: per part tcgen05.ld of 64 columns, mask at the edges only,
+//                   running maximum and sum in 32-bit, 2^x on the special-function unit, P written as packed bfloat16
+//                   over columns 64..127 of the half's S; O is rescaled only when a row's maximum has grown by more than
+//                   2^8 since its reference
 //
-// Tensor memory (all 512 columns): S_A | S_B | O_A | O_B, 128 columns each.  S_h(j+1) is issued behind PV_h(j) and the
-// tensor core works in order, so "S_h(j+1) is ready" also says that PV_h(j) has finished with O_h and P_h.
+// Tensor memory (all 512 columns): S_A | S_B | O_A | O_B, 128 columns each.  P takes the place of S_high, so with a tile's scores in
+// one piece the next ones could not be made before P V was done: softmax and tensor core waited for each other, 1846 of 3643
+// cycles a tile.  In two parts the softmax of S_low(j+1) runs while PV(j) and S_high(j+1) do; the parts wait 431 cycles, the
+// exponentials take 2353 of 3635 (the special-function unit half busy), although S of 64 keys costs 48 cycles an instruction against
+// 64 for 128 keys.  32 / 8 heads, TFLOP/s of one launch / repeated for 0.6 s, in one piece and in two parts: 8192 tokens behind
+// 8192 1010 / 986 and 1076 / 1017, 8192 alone 848 / 900 and 942 / 948, 4096 746 / 820 and 797 / 850.  S_high(j+1) is issued behind
+// PV_high(j) and the tensor core works in order, so "S_high(j+1) is ready" also says that PV(j) has finished with O and P.
 // Every mbarrier wait is bounded; a wait that runs out sets the error flag, and the CTA still releases its
 // tensor memory.  Takes head_dim 128, groups of 1 to 16 heads (floor(128 / G) tokens x G heads per half), pages of 8 to 128 tokens.
 #include "common.cuh"
@@ -39,7 +44,8 @@ constexpr int kKeys = 128;        // keys per tile (UMMA N of S, K of P V)
 constexpr int kDim = 128;         // head_dim
 constexpr int kKStages = 3;
 constexpr int kVStages = 2;
-constexpr int kThreads = 320;     // 8 softmax warps + producer warp + MMA warp
+constexpr int kPart = 64;         // keys per part of a tile (UMMA N of S)
+constexpr int kThreads = 352;     // 8 softmax warps + producer warp + an MMA warp per half
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleThreshold = 8.0f;   // log2 units
 
@@ -54,7 +60,8 @@ __device__ __forceinline__ uint32_t col_o(int half) { return half ? 384u : 256u;
 constexpr uint32_t kColP = 64;    // P of a half lies over columns 64..127 of its S
 
 struct Control {      // barriers and flags, at the end of the dynamic shared memory
-    uint64_t q_full, k_full[kKStages], k_free[kKStages], v_full[kVStages], v_free[kVStages], s_ready[2], p_ready[2], o_final[2];
+    uint64_t q_full, k_full[kKStages], k_free[kKStages], v_full[kVStages], v_free[kVStages];
+    uint64_t s_ready[2][2], s_read[2], p_ready[2][2], low_done[2], o_final[2];      // per half, those with two per part of a tile
     uint32_t tmem_slot;
     int failed;
 };
@@ -139,17 +146,22 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_wide_kernel(con
     // fresh barriers for every pass: at the end of a pass every copy has landed and every MMA has retired
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(&control.q_full), 1);
+        const uint32_t halves = has_b ? 2 : 1;              // a stage is free when every half has used it
         for (int s = 0; s < kKStages; ++s) {
             mbar_init(smem_u32(&control.k_full[s]), 1);
-            mbar_init(smem_u32(&control.k_free[s]), 1);
+            mbar_init(smem_u32(&control.k_free[s]), halves);
         }
         for (int s = 0; s < kVStages; ++s) {
             mbar_init(smem_u32(&control.v_full[s]), 1);
-            mbar_init(smem_u32(&control.v_free[s]), 1);
+            mbar_init(smem_u32(&control.v_free[s]), halves);
         }
         for (int h = 0; h < 2; ++h) {
-            mbar_init(smem_u32(&control.s_ready[h]), 1);
-            mbar_init(smem_u32(&control.p_ready[h]), 4);      // one arrival per softmax warp of the half
+            for (int part = 0; part < 2; ++part) {
+                mbar_init(smem_u32(&control.s_ready[h][part]), 1);
+                mbar_init(smem_u32(&control.p_ready[h][part]), 4);      // one arrival per softmax warp of the half
+            }
+            mbar_init(smem_u32(&control.s_read[h]), 4);
+            mbar_init(smem_u32(&control.low_done[h]), 1);
             mbar_init(smem_u32(&control.o_final[h]), 1);
         }
         tma::mbar_fence_init();
@@ -210,25 +222,27 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_wide_kernel(con
                 break;
             }
         }
-    } else if (warp == 9) {
-        // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc_s = instruction(kHalfRows, kKeys, false);
+    } else if (warp >= 9) {
+        // ---------------------------------------------------------------- MMA issuers, one per half
+        const int h = warp - 9;
+        if (lane == 0 && (h == 0 || has_b)) {
+            const uint32_t idesc_s = instruction(kHalfRows, kPart, false);
             const uint32_t idesc_o = instruction(kHalfRows, kDim, true);
             // descriptors are a base plus a byte offset / 16 in the low field (shared addresses stay below 2^18)
-            const uint64_t q_desc = desc_k_major(q_smem, 1024u), k_desc = desc_k_major(k_smem, 2048u);
+            const uint64_t q_desc = desc_k_major(q_smem + h * kQHalfBytes, 1024u), k_desc = desc_k_major(k_smem, 2048u);
             const uint64_t v_desc = desc_mn_major(v_smem, 1024u, 2048u);
-            auto issue_s = [&](int h, int stage) {          // S_h = Q_h K^T
+            auto issue_s = [&](int part, int stage) {          // S_h = Q_h K^T for 64 keys of the tile
 #pragma unroll
                 for (int ks = 0; ks < kDim / 16; ++ks) {
                     const uint32_t half = ks >> 2, within = (ks & 3) * 32;
-                    mma_ss(tmem + col_s(h), q_desc + ((h * kQHalfBytes + half * (kHalfRows * 128u) + within) >> 4),
-                           k_desc + ((stage * kKVBytes + half * 1024u + within) >> 4), idesc_s, ks > 0 ? 1u : 0u);
+                    mma_ss(tmem + col_s(h) + part * kPart, q_desc + ((half * (kHalfRows * 128u) + within) >> 4),
+                           k_desc + ((stage * kKVBytes + part * (kKVBytes / 2) + half * 1024u + within) >> 4), idesc_s, ks > 0 ? 1u : 0u);
                 }
+                mma_commit(smem_u32(&control.s_ready[h][part]));
             };
-            auto issue_pv = [&](int h, int stage, bool first) {     // O_h += P_h V
+            auto issue_pv = [&](int part, int stage, bool first) {     // O_h += P_h V for 64 keys
 #pragma unroll
-                for (int kk = 0; kk < kKeys / 16; ++kk)     // 16 keys = 8 packed columns of P, two 8-key groups of V
+                for (int kk = part * 4; kk < part * 4 + 4; ++kk)     // 16 keys = 8 packed columns of P, two 8-key groups of V
                     mma_ts(tmem + col_o(h), tmem + col_s(h) + kColP + kk * 8, v_desc + ((stage * kKVBytes + kk * 4096u) >> 4),
                            idesc_o, (first && kk == 0) ? 0u : 1u);
             };
@@ -236,41 +250,31 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_wide_kernel(con
             if (ok) {
                 fence_after();
                 issue_s(0, 0);
-                mma_commit(smem_u32(&control.s_ready[0]));
-                if (has_b) {
-                    issue_s(1, 0);
-                    mma_commit(smem_u32(&control.s_ready[1]));
-                }
+                issue_s(1, 0);
                 mma_commit(smem_u32(&control.k_free[0]));
             }
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const int vs = j % kVStages, ks = (j + 1) % kKStages;
                 const bool next = j + 1 < n_tiles;
-                ok = mbar_wait(smem_u32(&control.v_full[vs]), (j / kVStages) & 1) && mbar_wait(smem_u32(&control.p_ready[0]), j & 1);
-                if (!ok) break;
-                fence_after();
-                issue_pv(0, vs, j == 0);
-                if (!next) mma_commit(smem_u32(&control.o_final[0]));
-                if (next) {
-                    ok = mbar_wait(smem_u32(&control.k_full[ks]), ((j + 1) / kKStages) & 1);
+                if (next) {          // the low scores of this tile are in registers: those of the next tile take their place
+                    ok = mbar_wait(smem_u32(&control.k_full[ks]), ((j + 1) / kKStages) & 1) && mbar_wait(smem_u32(&control.s_read[h]), j & 1);
                     if (!ok) break;
                     fence_after();
                     issue_s(0, ks);
-                    mma_commit(smem_u32(&control.s_ready[0]));
                 }
-                if (has_b) {
-                    ok = mbar_wait(smem_u32(&control.p_ready[1]), j & 1);
-                    if (!ok) break;
-                    fence_after();
-                    issue_pv(1, vs, j == 0);
-                    if (!next) mma_commit(smem_u32(&control.o_final[1]));
-                }
+                ok = mbar_wait(smem_u32(&control.v_full[vs]), (j / kVStages) & 1) && mbar_wait(smem_u32(&control.p_ready[h][0]), j & 1);
+                if (!ok) break;
+                fence_after();
+                issue_pv(0, vs, j == 0);
+                mma_commit(smem_u32(&control.low_done[h]));
+                ok = mbar_wait(smem_u32(&control.p_ready[h][1]), j & 1);
+                if (!ok) break;
+                fence_after();
+                issue_pv(1, vs, false);
                 mma_commit(smem_u32(&control.v_free[vs]));
-                if (next) {
-                    if (has_b) {
-                        issue_s(1, ks);
-                        mma_commit(smem_u32(&control.s_ready[1]));
-                    }
+                if (!next) mma_commit(smem_u32(&control.o_final[h]));
+                if (next) {          // P lies over the high scores, so these follow behind its last product
+                    issue_s(1, ks);
                     mma_commit(smem_u32(&control.k_free[ks]));
                 }
             }
@@ -287,83 +291,109 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_wide_kernel(con
         const int low = (exists && p.window > 0) ? max(0, position - p.window + 1) : 0;
         const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const uint32_t s_address = lane_base + col_s(h), o_address = lane_base + col_o(h);
-        const uint32_t s_bar = smem_u32(&control.s_ready[h]), p_bar = smem_u32(&control.p_ready[h]);
         float reference = -INFINITY;     // what is subtracted in the exponent (a stale maximum)
         float row_sum = 0.0f;
         bool ok = true;
+        const uint64_t scale_pair = pair_of(p.scale_log2, p.scale_log2);
         for (int j = 0; j < n_tiles; ++j) {
-            if (ok && !mbar_wait(s_bar, j & 1)) ok = false;
-            fence_after();
             const int tile_key = first_tile_key + j * kKeys;
-            // only tiles that touch the diagonal, the window's edge or the end of the rows need the mask
-            const bool edge = tile_key + kKeys - 1 > position || tile_key < low;
-            // The exponentials are taken against the reference as it stands, so they do not wait for this tile's
-            // maximum; only when the maximum has outgrown the reference by the threshold (or nothing was seen yet) does
-            // the reference move, and the tile is done again: S stays readable until P is stored over columns 64..127.
-            // Maximum, exponential, sum and packing go element by element, so that the special-function unit and the
-            // arithmetic pipes of the one softmax warp a scheduler has at a time work side by side.
-            uint32_t packed_upper[32], packed_lower[32];
-            float sums[4], running[4];
-            auto half = [&](uint32_t (&packed)[32], int first_column, float subtract) {
-                uint32_t values[64];
-                tmem_load_64(s_address + first_column, values);
-                if (edge) {
+            uint32_t packed_low[32];
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                const int part_key = tile_key + part * kPart;
+                if (ok && !mbar_wait(smem_u32(&control.s_ready[h][part]), j & 1)) ok = false;
+                fence_after();
+                uint32_t scores[64];
+                tmem_load_64(s_address + part * kPart, scores);
+                if (part == 0) {
+                    // the low scores' place is free for the next tile's
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&control.s_read[h]));
+                } else {
+                    // all scores of the tile have been read: P of the low keys goes over the first high ones
+                    tmem_store_32(s_address + kColP, packed_low);
+                    tmem_wait_store();
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&control.p_ready[h][0]));
+                }
+                // only tiles that touch the diagonal, the window's edge or the end of the rows need the mask
+                if (part_key + kPart - 1 > position || part_key < low) {
 #pragma unroll
                     for (int c = 0; c < 64; ++c)
-                        if (!(tile_key + first_column + c >= low && tile_key + first_column + c <= position)) values[c] = 0xff800000u;   // -inf
+                        if (!(part_key + c >= low && part_key + c <= position)) scores[c] = 0xff800000u;   // -inf
                 }
+                // The exponentials are taken against the reference as it stands, so they do not wait for this part's
+                // maximum; only when the maximum has outgrown the reference by the threshold (or nothing was seen yet) does
+                // the reference move, and the part is done again.  Maximum, exponential, sum and packing go element by
+                // element, so that the special-function unit and the arithmetic pipes work side by side.
+                uint32_t packed[32];
+                uint64_t sums[2];
+                float running[2];
+                auto whole_part = [&]() -> float {
+                    const float subtract = reference == -INFINITY ? 0.0f : reference;
+                    const uint64_t minus_pair = pair_of(-subtract, -subtract);
 #pragma unroll
-                for (int c = 0; c < 64; c += 2) {
-                    const float x0 = __uint_as_float(values[c]), x1 = __uint_as_float(values[c + 1]);
-                    // the scale and the reference enter the exponent in one fused multiply-add
-                    const float e0 = exp2_approx(fmaf(x0, p.scale_log2, -subtract));
-                    const float e1 = exp2_approx(fmaf(x1, p.scale_log2, -subtract));
-                    running[(c >> 1) & 3] = fmaxf(running[(c >> 1) & 3], fmaxf(x0, x1));
-                    sums[(c >> 1) & 3] += e0 + e1;
-                    packed[c >> 1] = pack2(e0, e1);
-                }
-            };
-            auto whole_tile = [&]() -> float {
-                const float subtract = reference == -INFINITY ? 0.0f : reference;
+                    for (int c = 0; c < 2; ++c) {
+                        sums[c] = pair_of(0.0f, 0.0f);
+                        running[c] = -INFINITY;
+                    }
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    sums[c] = 0.0f;
-                    running[c] = -INFINITY;
-                }
-                half(packed_upper, 64, subtract);
-                half(packed_lower, 0, subtract);
-                // the maximum is taken over the raw scores (the scale is positive)
-                return fmaxf(fmaxf(running[0], running[1]), fmaxf(running[2], running[3])) * p.scale_log2;
-            };
-            const float tile_max = whole_tile();
-            float factor = 1.0f;
-            const bool moved = tile_max > reference + kRescaleThreshold || (reference == -INFINITY && tile_max > -INFINITY);
-            if (__any_sync(0xffffffffu, moved)) {
-                if (moved) {
-                    factor = reference == -INFINITY ? 0.0f : exp2_approx(reference - tile_max);
-                    reference = tile_max;
-                }
-                whole_tile();
-                // O is rescaled (by the whole warp, rows that need nothing use 1): P V of the tile before is done,
-                // since this tile's S was computed behind it
-                if (j > 0) {
+                    for (int c = 0; c < 32; ++c) {
+                        const float x0 = __uint_as_float(scores[2 * c]), x1 = __uint_as_float(scores[2 * c + 1]);
+                        // the scale and the reference enter the exponent in one fused multiply-add
+                        float e0, e1;
+                        halves_of(fma_pair(pair_of(x0, x1), scale_pair, minus_pair), e0, e1);
+                        e0 = exp2_approx(e0);
+                        e1 = exp2_approx(e1);
+                        running[c & 1] = max3(running[c & 1], x0, x1);
+                        sums[c & 1] = add_pair(sums[c & 1], pair_of(e0, e1));
+                        packed[c] = pack2(e0, e1);
+                    }
+                    // the maximum is taken over the raw scores (the scale is positive)
+                    return fmaxf(running[0], running[1]) * p.scale_log2;
+                };
+                const float part_max = whole_part();
+                float factor = 1.0f;
+                const bool moved = part_max > reference + kRescaleThreshold || (reference == -INFINITY && part_max > -INFINITY);
+                if (__any_sync(0xffffffffu, moved)) {
+                    if (moved) {
+                        factor = reference == -INFINITY ? 0.0f : exp2_approx(reference - part_max);
+                        reference = part_max;
+                    }
+                    whole_part();
+                    // O is rescaled (by the whole warp, rows that need nothing use 1) once the products into it are done: those of
+                    // the tile before when this tile's high scores are ready, which were issued behind them, and those of this
+                    // tile's low keys, which say so themselves
+                    if (j > 0 || part > 0) {
+                        if (ok && !mbar_wait(part == 0 ? smem_u32(&control.s_ready[h][1]) : smem_u32(&control.low_done[h]), j & 1)) ok = false;
+                        fence_after();
 #pragma unroll
-                    for (int chunk = 0; chunk < kDim / 32; ++chunk) {
-                        uint32_t o_raw[32];
-                        tmem_load_32(o_address + chunk * 32, o_raw);
+                        for (int chunk = 0; chunk < kDim / 32; ++chunk) {
+                            uint32_t o_raw[32];
+                            tmem_load_32(o_address + chunk * 32, o_raw);
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) o_raw[c] = __float_as_uint(__uint_as_float(o_raw[c]) * factor);
-                        tmem_store_32(o_address + chunk * 32, o_raw);
+                            for (int c = 0; c < 32; ++c) o_raw[c] = __float_as_uint(__uint_as_float(o_raw[c]) * factor);
+                            tmem_store_32(o_address + chunk * 32, o_raw);
+                        }
+                        tmem_wait_store();
                     }
                 }
+                float sum_low, sum_high;
+                halves_of(add_pair(sums[0], sums[1]), sum_low, sum_high);
+                row_sum = row_sum * factor + (sum_low + sum_high);
+                if (part == 0) {
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) packed_low[c] = packed[c];
+                } else {
+                    tmem_store_32(s_address + kColP + 32, packed);
+                    tmem_wait_store();
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&control.p_ready[h][1]));
+                }
             }
-            row_sum = row_sum * factor + ((sums[0] + sums[1]) + (sums[2] + sums[3]));
-            tmem_store_32(s_address + kColP, packed_lower);          // keys 0..63 of the tile
-            tmem_store_32(s_address + kColP + 32, packed_upper);     // keys 64..127
-            tmem_wait_store();
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(p_bar);
         }
         // the last P V, then O / sum
         if (ok && !mbar_wait(smem_u32(&control.o_final[h]), 0)) ok = false;
@@ -403,8 +433,12 @@ __global__ void __launch_bounds__(kThreads, 1) attention_prefill_wide_kernel(con
             tma::mbar_inval(smem_u32(&control.v_free[s]));
         }
         for (int h = 0; h < 2; ++h) {
-            tma::mbar_inval(smem_u32(&control.s_ready[h]));
-            tma::mbar_inval(smem_u32(&control.p_ready[h]));
+            for (int part = 0; part < 2; ++part) {
+                tma::mbar_inval(smem_u32(&control.s_ready[h][part]));
+                tma::mbar_inval(smem_u32(&control.p_ready[h][part]));
+            }
+            tma::mbar_inval(smem_u32(&control.s_read[h]));
+            tma::mbar_inval(smem_u32(&control.low_done[h]));
             tma::mbar_inval(smem_u32(&control.o_final[h]));
         }
     }

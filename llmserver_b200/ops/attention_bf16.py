@@ -36,11 +36,15 @@ UNEVEN_SPLITS, UNEVEN_SEQUENCES = 2, 128
 PREFILL_KERNEL = os.environ.get("LLMSERVER_B200_PREFILL_ATTENTION", "tcgen05")
 PREFILL_TILE = 128   # rows per block of the tcgen05 portions kernel
 WIDE_TILE = 256      # rows per block of the 256-row kernel
-# the 256-row kernel is used when the longest portion has this many rows (tokens x heads of a group), its request
-# holds this many tokens and the group divides 128: measured on the 8B, 14B and 32B head shapes, it wins from about
-# there (long key loops, enough row tiles; 8 % at 16384 tokens, 25 % at 32768), and not with groups of 5
+# The 256-row kernel is used when the longest portion has WIDE_MIN_ROWS rows (tokens x heads of a group), the group divides 128 and
+# its request holds WIDE_MIN_CONTEXT tokens, or half as many where its tiles are WIDE_WAVES waves of blocks, so that the last wave
+# does not count.  Attention alone, 32 / 8 heads, TFLOP/s repeated for 0.6 s, 128 rows / 256 rows: 722 / 705 at 2048 tokens, 838 /
+# 850 at 4096, 883 / 948 at 8192, 937 / 1017 for 8192 tokens behind 8192; whole prompts of the 8B shape, ms: 54.8 / 54.9 at 4096
+# tokens, 119.9 / 118.1 at 8192, 276.2 / 275.4 at 16384 (its first portion).  With groups of 5 (14B shape, a mixed step of 8192
+# tokens) 188.6 / 190.1.
 WIDE_MIN_ROWS = int(os.environ.get("LLMSERVER_B200_PREFILL_WIDE_ROWS", "8192"))
 WIDE_MIN_CONTEXT = int(os.environ.get("LLMSERVER_B200_PREFILL_WIDE_CONTEXT", "16384"))
+WIDE_WAVES = 4
 
 
 def prefill_tcgen05_supported(head_dim: int, n_q_heads: int, n_kv_heads: int, page_size: int) -> bool:
@@ -74,7 +78,10 @@ def prefill_wide_wanted(batch, group: int, head_dim: int, n_q_heads: int, n_kv_h
     if PREFILL_KERNEL == "tcgen05-256":
         return True
     length, context = max(zip(batch.q_lens, batch.context_lens))
-    return length * group >= WIDE_MIN_ROWS and context >= WIDE_MIN_CONTEXT and PREFILL_TILE % group == 0
+    if length * group < WIDE_MIN_ROWS or PREFILL_TILE % group:
+        return False
+    waves = length * group * n_kv_heads / (WIDE_TILE * _block_slots(batch.context_len.device, True))
+    return context >= WIDE_MIN_CONTEXT or (2 * context >= WIDE_MIN_CONTEXT and waves >= WIDE_WAVES)
 
 
 def supported(head_dim: int, n_q_heads: int, n_kv_heads: int) -> bool:
