@@ -1,7 +1,7 @@
 // Attention over the paged cache, any sizes, 32-bit arithmetic: the kernel of the true 32-bit path
 // and the fallback of the bfloat16 path for head sizes its tensor-core kernels refuse.
 //
-// One warp per (query token, query head).  The query at absolute position p sees keys
+// One block of four warps per (query token, query head).  The query at absolute position p sees keys
 // max(0, p - window + 1) .. p of its own sequence (window 0 = all), read through the sequence's
 // block table; the new tokens' keys are already in the cache when this runs.  Scores, the running
 // maximum, the normaliser and the output accumulate in 32-bit with the online-softmax recurrence
@@ -10,7 +10,8 @@
 // product (utils/architecture.py:105).
 //
 // Keys are visited 32 at a time from the first visible one, each lane owning one key's dot
-// product, so the order of every sum depends only on the query's position: the result for a token
+// product; warp w takes rounds w, w + 4, ... and the warps' results are merged in their order.  So the order of every sum
+// depends only on the query's position: the result for a token
 // is bit-identical however the prompt was cut into steps and whatever else is in the batch.
 //
 // Values may have another size than keys (`value_dim`; the output then has Hq * value_dim columns).  With `sinks`
@@ -69,7 +70,9 @@ __device__ __forceinline__ float row_dot(const float* q_row, const T* k_row, int
 // the chain of dependent loads per 32 keys (table entry, key row, value rows); so the value rows of a round are asked for,
 // kAhead at a time, before the weights that multiply them are known, and the table entry of the next round with them.  With
 // 150 keys, heads of 32 and 4 tokens a launch took 52 us when the loads were issued one by one and the accumulator had 16
-// columns for every size.
+// columns for every size, and added 11.3 us to a replayed step when one warp walked all five rounds; with the rounds dealt to four
+// warps it adds 8.6.
+constexpr int kRoundWarps = 4;
 template <typename T, int COLUMNS, bool VECTOR>
 __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_pages,
                                          const T* __restrict__ v_pages, const int* __restrict__ block_tables,
@@ -82,20 +85,17 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
     constexpr int kAhead = COLUMNS >= 16 ? 2 : 32 / COLUMNS;      // value rows in flight: 32 registers per lane
     pdl_trigger();   // let the next kernel start launching
     pdl_wait();      // everything before this kernel in the stream is complete and visible
-    extern __shared__ float q_shared[];  // [warps][head_dim]
+    extern __shared__ float q_shared[];  // [head_dim], then what warps 1 .. 3 leave: [3][maximum, normaliser, 32 * COLUMNS sums]
     const int token = blockIdx.x;
-    const int warps_per_block = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int head = blockIdx.y * warps_per_block + warp;
-    if (head >= n_q_heads) return;
+    const int head = blockIdx.y;
     const int kv_head = head / (n_q_heads / n_kv_heads);
     const int position = positions[token];
     const int* table = block_tables + (size_t)seq_of_token[token] * max_blocks;
 
-    float* q_row = q_shared + warp * head_dim;
+    float* q_row = q_shared;
     const T* q_src = q + (size_t)token * q_stride + (size_t)head * head_dim;
-    for (int i = lane; i < head_dim; i += 32) q_row[i] = Num<T>::load(q_src + i);
-    __syncwarp();
+    for (int i = threadIdx.x; i < head_dim; i += kRoundWarps * 32) q_row[i] = Num<T>::load(q_src + i);
 
     float accumulator[COLUMNS];
 #pragma unroll
@@ -107,13 +107,15 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
     const int kept = min(keep, first);      // keys 0 .. kept - 1, then first .. position
     const int count = kept + position - first + 1;
     auto key_of = [&](int index) { return index < kept ? index : first + index - kept; };
-    int next_page = lane < count ? table[key_of(lane) / page_size] : 0;
-    for (int base = 0; base < count; base += 32) {
+    const int mine = 32 * warp + lane;
+    int next_page = mine < count ? table[key_of(mine) / page_size] : 0;
+    __syncthreads();      // the query's row
+    for (int base = 32 * warp; base < count; base += 32 * kRoundWarps) {
         const int index = base + lane;
         const int key = key_of(index);
         const bool valid = index < count;
         int page = next_page;
-        if (index + 32 < count) next_page = table[key_of(index + 32) / page_size];
+        if (index + 32 * kRoundWarps < count) next_page = table[key_of(index + 32 * kRoundWarps) / page_size];
         if (valid && (unsigned)page >= (unsigned)num_pages) {      // no page of the pool: report it, read page 0 instead
             if (error_flag) atomicExch(error_flag, 5);
             page = 0;
@@ -142,8 +144,9 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
         }
         const float chunk_max = warp_max(score);
         const float new_max = fmaxf(running_max, chunk_max);
-        const float correction = expf(running_max - new_max);  // 0 on the first chunk
-        const float weight = valid ? expf(score - new_max) : 0.0f;
+        // (a round may hold nothing but scores of -inf, which a bias can give: no weight, nothing to correct)
+        const float correction = running_max == new_max ? 1.0f : expf(running_max - new_max);  // 0 on the first chunk
+        const float weight = valid && score != -INFINITY ? expf(score - new_max) : 0.0f;
         normaliser = normaliser * correction + warp_sum(weight);
 #pragma unroll
         for (int i = 0; i < COLUMNS; ++i) accumulator[i] *= correction;
@@ -160,6 +163,35 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
         }
         running_max = new_max;
     }
+    const int rounds = (count + 31) / 32;
+    if (rounds > 1) {      // warps 1 .. 3 leave what they have; warp 0 adds it in their order
+        float* parts = q_shared + head_dim;
+        constexpr int kPart = 2 + 32 * COLUMNS;
+        if (warp > 0) {
+            float* part = parts + (warp - 1) * kPart;
+            if (lane == 0) {
+                part[0] = running_max;
+                part[1] = normaliser;
+            }
+#pragma unroll
+            for (int i = 0; i < COLUMNS; ++i) part[2 + lane + 32 * i] = accumulator[i];
+        }
+        __syncthreads();
+        if (warp == 0) {
+            for (int other = 1; other < kRoundWarps && other < rounds; ++other) {
+                const float* part = parts + (other - 1) * kPart;
+                if (part[0] == -INFINITY && part[1] == 0.0f) continue;
+                const float new_max = fmaxf(running_max, part[0]);
+                const float correction = running_max == new_max ? 1.0f : expf(running_max - new_max);
+                const float weight = part[0] == new_max ? 1.0f : expf(part[0] - new_max);
+                normaliser = normaliser * correction + part[1] * weight;
+#pragma unroll
+                for (int i = 0; i < COLUMNS; ++i) accumulator[i] = accumulator[i] * correction + part[2 + lane + 32 * i] * weight;
+                running_max = new_max;
+            }
+        }
+    }
+    if (warp > 0) return;
     if (sinks) {      // one more term of the denominator; it has no value, so the sums only shrink
         const float sink = sinks[head];
         const float new_max = fmaxf(running_max, sink);
@@ -208,22 +240,26 @@ LLM_EXPORT int llm_attention_generic(const void* q, int q_stride, const void* k_
         llm_set_error("attention_generic: a chunk of %d positions, a bias of %d distances or %d kept positions", chunk, bias_len, keep);
         return LLM_REFUSED;
     }
-    const int warps = 4;
-    dim3 grid(n_tokens, (n_q_heads + warps - 1) / warps);
-    const size_t shared = (size_t)warps * head_dim * sizeof(float);
+    if (n_q_heads > 65535) {
+        llm_set_error("attention_generic: %d query heads are too many for one launch", n_q_heads);
+        return LLM_REFUSED;
+    }
+    dim3 grid(n_tokens, n_q_heads);
+    const int columns = value_dim <= 32 ? 1 : value_dim <= 64 ? 2 : value_dim <= 128 ? 4 : value_dim <= 256 ? 8 : 16;
+    const size_t shared = ((size_t)head_dim + (kRoundWarps - 1) * (2 + 32 * columns)) * sizeof(float);
     // key rows in 16-byte pieces where every row starts on such a boundary
     const int count = dtype == LLM_F32 ? 4 : 8;
     const bool vector = head_dim % count == 0 && aligned16(k_pages);
 #define LLM_GENERIC(COLUMNS)                                                                                                       \
     LLM_DISPATCH_DTYPE(dtype, llm_launch(vector ? attention_generic_kernel<T, COLUMNS, true> : attention_generic_kernel<T, COLUMNS, false>, \
-                                         grid, warps * 32, shared, stream, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages,     \
+                                         grid, kRoundWarps * 32, shared, stream, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages,     \
                                          block_tables, max_blocks, seq_of_token, positions, (T*)out, n_q_heads, n_kv_heads, head_dim,       \
                                          value_dim, page_size, num_pages, scale, window, sinks, chunk, bias, bias_len, keep,                \
                                          (const T*)gate, gate_stride, error_flag))
-    if (value_dim <= 32) LLM_GENERIC(1);
-    else if (value_dim <= 64) LLM_GENERIC(2);
-    else if (value_dim <= 128) LLM_GENERIC(4);
-    else if (value_dim <= 256) LLM_GENERIC(8);
+    if (columns == 1) LLM_GENERIC(1);
+    else if (columns == 2) LLM_GENERIC(2);
+    else if (columns == 4) LLM_GENERIC(4);
+    else if (columns == 8) LLM_GENERIC(8);
     else LLM_GENERIC(16);
 #undef LLM_GENERIC
     return llm_check_launch("attention_generic");
