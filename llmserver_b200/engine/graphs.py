@@ -4,8 +4,8 @@ A decode step launches a couple of hundred small kernels; issued one by one from
 more host time than the GPU needs to run them (the reference met the same wall and replays one graph
 per batch-size bucket: utils/cuda_graph.py:3-4,11-99).  Here a step's whole input is one packed int32
 buffer whose layout depends only on the batch size, so a graph is captured once per batch size over a
-fixed device buffer; a replayed step is: pack on the host (pinned) -> one copy -> replay -> read the
-sampled tokens (and the kernels' error flag) back in one copy.
+fixed device buffer; a replayed step is: pack on the host (pinned) -> replay, which begins with the copy of the buffer
+and ends with the copy of the sampled tokens (and the kernels' error flag) to the host -> wait for the stream.
 
 The captured attention launch is shaped for the longest context the runner was sized for; blocks
 beyond a sequence's real length exit at once.  Nothing is executed during capture, and the warm-up
@@ -13,6 +13,7 @@ that a capture needs is given by the eager steps of the same batch size that ran
 """
 from __future__ import annotations
 
+import operator
 import time
 from typing import Dict, List, Optional, Sequence
 
@@ -25,6 +26,10 @@ from .batch import BatchLayout, SequenceSlice, pack, views
 
 
 BUCKETS = (1, 2, 4, 8, 16, 32, 48, 64, 96, 128, 192, 256)   # batch sizes graphs are captured for
+
+
+_START, _STATE_SLOT = operator.attrgetter("start"), operator.attrgetter("state_slot")
+_TEMPERATURE, _STEP = operator.attrgetter("temperature"), operator.attrgetter("step")
 
 
 class _PadRow:
@@ -89,23 +94,24 @@ class DecodeRows:
         marks pages it gave back in its list; the buffer keeps their old ids, which the kernels mask and never
         write to.)"""
         host, off, count = self.host_view, self.layout.offsets, len(slices)
-        tokens = np.fromiter((piece.tokens[0] for piece in slices), dtype=np.int64, count=count)
-        if tokens.min() < 0 or tokens.max() >= self.vocab_size:
+        tokens = [piece.tokens[0] for piece in slices]
+        if min(tokens) < 0 or max(tokens) >= self.vocab_size:
             raise ValueError(f"a token id is outside the vocabulary of {self.vocab_size}")
-        starts = np.fromiter((piece.start for piece in slices), dtype=np.int32, count=count)
+        starts = np.fromiter(map(_START, slices), dtype=np.int32, count=count)
         host[off["token_ids"]:off["token_ids"] + count] = tokens
         host[off["positions"]:off["positions"] + count] = starts
         host[off["context_len"]:off["context_len"] + count] = starts + 1
         # a model without paged groups has no tables by which to recognise its rows: their state slots are rewritten
-        host[off["state_slots"]:off["state_slots"] + count] = np.fromiter((piece.state_slot for piece in slices), dtype=np.int32, count=count)
+        host[off["state_slots"]:off["state_slots"] + count] = np.fromiter(map(_STATE_SLOT, slices), dtype=np.int32, count=count)
         host[off["temperatures"]:off["temperatures"] + count] = np.fromiter(
-            (row.temperature for row in sampling), dtype=np.float32, count=count).view(np.int32)
-        host[off["seeds"]:off["seeds"] + 2 * count] = np.fromiter(
-            (row.seed & 0x7FFFFFFFFFFFFFFF for row in sampling), dtype=np.int64, count=count).view(np.int32)
-        host[off["sample_steps"]:off["sample_steps"] + count] = np.fromiter((row.step for row in sampling), dtype=np.int32, count=count)
+            map(_TEMPERATURE, sampling), dtype=np.float32, count=count).view(np.int32)
+        host[off["seeds"]:off["seeds"] + 2 * count] = np.asarray(
+            [row.seed & 0x7FFFFFFFFFFFFFFF for row in sampling], dtype=np.int64).view(np.int32)
+        host[off["sample_steps"]:off["sample_steps"] + count] = np.fromiter(map(_STEP, sampling), dtype=np.int32, count=count)
         host[off["error_flag"]] = 0
-        for row, piece in enumerate(slices):
-            lengths = self.table_lengths[row]
+        for row, (piece, lengths) in enumerate(zip(slices, self.table_lengths)):
+            if list(map(len, piece.tables)) == lengths:      # no page was added
+                continue
             for group, table in enumerate(piece.tables):
                 if len(table) != lengths[group]:
                     width, begin = self.layout.widths[group], self.layout.table_offsets[group] + row * self.layout.widths[group]
@@ -122,6 +128,8 @@ class DecodeGraph:
     sampled tokens are dropped, as the reference pads its buckets with copies of row 0
     (utils/cuda_graph.py:11-99)."""
 
+    meanwhile = None
+
     def __init__(self, model, batch_size: int, n_groups: int, table_width: int, max_context: int, vocab_size: int,
                  null_pages: Sequence[int], null_slot: int = 0):
         self.model, self.vocab_size, self.batch_size = model, vocab_size, batch_size
@@ -135,24 +143,33 @@ class DecodeGraph:
         shape_only = [SequenceSlice(index, [0], max_context - 1, [0], [[0] * table_width] * n_groups, 0)
                       for index in range(batch_size)]
         self.batch = views(self.buffer, self.layout, shape_only)
+        self.answer = torch.zeros(batch_size + 2, dtype=torch.int32, pin_memory=True)
+        self.answer_view = self.answer.numpy()
         self.graph = torch.cuda.CUDAGraph()
+        # the copies of the batch and of the result are part of the graph: a replay is one call, and the result lies on the host
+        # when the stream is done
         with torch.cuda.graph(self.graph, capture_error_mode="thread_local"):
+            self.buffer.copy_(self.host, non_blocking=True)
             logits = self.model.step(self.batch)
             self.logits = logits        # [batch_size, vocab] of the last replay (tests compare them with eager steps)
             tokens = ops.sample(logits, self.batch.temperatures, self.batch.seeds, self.batch.sample_steps)
             self.result = torch.cat([tokens, self.batch.error_flag, wait_error_flag(device)])
+            self.answer.copy_(self.result, non_blocking=True)
 
     def run(self, slices: List[SequenceSlice], sampling: Sequence, phases: Optional[dict] = None) -> List[int]:
         """Returns the sampled tokens of the real rows followed by the two error flags; ``phases`` receives the host
-        seconds spent packing and queueing the copy, replaying, and waiting for the result."""
+        seconds spent packing, replaying, and waiting for the result.  ``meanwhile``, when it is set, is called once the step is
+        queued: what the host has to do anyway is done while the GPU works."""
         clock = time.perf_counter
         self.began = clock()
         real = self.rows.fill(slices, sampling)
-        self.buffer.copy_(self.host, non_blocking=True)
         packed = clock()
         self.graph.replay()
         launched = clock()
-        result = self.result.tolist()
+        if self.meanwhile is not None:
+            self.meanwhile()
+        torch.cuda.current_stream(self.buffer.device).synchronize()
+        result = self.answer_view.tolist()
         if phases is not None:
             phases.update(pack_copy=packed - self.began, launch=launched - packed, read_back=clock() - launched)
         return result[:real] + result[-2:]

@@ -62,17 +62,18 @@ class StepFunction:
 
     def slices_for(self, entries: List[StepEntry]) -> List[SequenceSlice]:
         """Allocates the pages the step needs (all or nothing) and describes each request's share."""
+        computed, cache = self.computed, self.cache
         seen = set()
-        for request_id, tokens, _ in entries:
+        for request_id, _, _ in entries:
             if request_id in seen:
                 raise ValueError(f"request {request_id!r} appears twice in one step")
             seen.add(request_id)
-            if request_id not in self.computed:
+            if request_id not in computed:
                 raise KeyError(f"request {request_id!r} was not admitted")
         # check the whole step against what is available before allocating anything (entries that stay inside
         # their last page, as most decode tokens do, need nothing)
-        growing = [entry for entry in entries
-                   if not self.cache.has_room(entry[0], self.computed[entry[0]] + len(entry[1]))]
+        has_room = cache.has_room
+        growing = [entry for entry in entries if not has_room(entry[0], computed[entry[0]] + len(entry[1]))]
         if growing:
             totals = [0] * len(self.cache.groups)
             for request_id, tokens, _ in growing:
@@ -84,15 +85,13 @@ class StepFunction:
             for request_id, tokens, _ in growing:
                 self.cache.ensure(request_id, self.computed[request_id] + len(tokens))
         limit = self.model.spec.max_positions
-        slices = []
+        slices, tables = [], [group.tables for group in cache.groups]
         for request_id, tokens, want in entries:
-            start = self.computed[request_id]
+            start = computed[request_id]
             if limit is not None and start + len(tokens) > limit:
                 raise ValueError(f"request {request_id!r} would reach {start + len(tokens)} tokens; "
                                  f"the model's max_position_embeddings is {limit}")
-            slices.append(SequenceSlice(request_id, tokens, start, want,
-                                        [self.cache.table(request_id, group) for group in range(len(self.cache.groups))],
-                                        self.cache.slot_of(request_id)))
+            slices.append(SequenceSlice(request_id, tokens, start, want, [table[request_id] for table in tables], cache.slot_of(request_id)))
         return slices
 
     def prepare(self, entries: List[StepEntry], sampling: Optional[Sequence] = None) -> StepBatch:
@@ -130,8 +129,20 @@ class StepFunction:
         began = clock()
         slices = self.slices_for(entries)
         graph = self.graphs.ready_for(slices) if self.graphs is not None and sampling else None
+        advanced = False
+
+        def advance() -> None:      # once, while the GPU works where that can be done (pages given back go to later steps only)
+            nonlocal advanced
+            if not advanced:
+                advanced = True
+                self._advance(entries)
+
         if graph is not None:
-            result = graph.run(slices, sampling, self.last_phases)
+            graph.meanwhile = advance
+            try:
+                result = graph.run(slices, sampling, self.last_phases)
+            finally:
+                graph.meanwhile = None
             self.last_phases["pack_copy"] += graph.began - began
             self.last_batch_bytes = graph.layout.total * 4
             self.graph_steps += 1
@@ -148,9 +159,10 @@ class StepFunction:
             tokens = (sampler or self.sampler).from_batch(logits, batch)
             flags = torch.cat([tokens, batch.error_flag, wait_error_flag(self.device)])
             launched = clock()
+            advance()
             result = flags.tolist()
             self.last_phases.update(pack_copy=packed - began, launch=launched - packed, read_back=clock() - launched)
-        self._advance(entries)
+        advance()
         if result[-2] != 0:
             raise RuntimeError("a kernel met a block-table entry outside the page pool; the cache bookkeeping is corrupt")
         if result[-1] != 0:
