@@ -111,9 +111,10 @@ _flush_buffer = {}
 _ROUNDS = 4
 _empty_round = {}
 # Between two small kernels the candidates often lie within a few percent of each other, and whole steps decide
-# differently from that measurement at the two ends: up to 16 rows a step is faster with this package's kernel
+# differently from that measurement: a step is faster with this package's kernel
 # wherever the two are close (its weight stream starts before its predecessor ends, and it lets its successor launch
-# early), from 32 rows on with the library's.  So a candidate of the other kind has to win by this much.
+# early).  So the library's product has to win by this much, up to 16 rows and beyond (a step of 64 sequences of the Dikusun shape 1097 us
+# when this package's kernel had to win by 5 % there, 1082 this way).
 _CLOSE_FEW_ROWS = 0.10
 _CLOSE_MANY_ROWS = 0.05
 # Among the splits of this package's kernel, the ones within this much of the fastest count as equal, and the largest
@@ -235,8 +236,7 @@ def _plan_for(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, own
     def library_product():
         torch.matmul(x, weight.t(), out=out)
 
-    favour_library = key[0] > 16
-    best_time = _time_in_step(library_product, x.device) * ((1.0 - _CLOSE_MANY_ROWS) if favour_library else (1.0 + _CLOSE_FEW_ROWS))
+    best_time = _time_in_step(library_product, x.device) * (1.0 + (_CLOSE_MANY_ROWS if key[0] > 16 else _CLOSE_FEW_ROWS))
     timed = []
     tiles, k_blocks = -(-cols // 128), -(-inner // 128)
     for split in SPLITS:
