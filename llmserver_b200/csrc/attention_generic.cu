@@ -84,18 +84,17 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
                                          const T* __restrict__ gate, int gate_stride, int* __restrict__ error_flag) {
     constexpr int kAhead = COLUMNS >= 16 ? 2 : 32 / COLUMNS;      // value rows in flight: 32 registers per lane
     pdl_trigger();   // let the next kernel start launching
-    pdl_wait();      // everything before this kernel in the stream is complete and visible
     extern __shared__ float q_shared[];  // [head_dim], then what warps 1 .. 3 leave: [3][maximum, normaliser, 32 * COLUMNS sums]
     const int token = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int head = blockIdx.y;
     const int kv_head = head / (n_q_heads / n_kv_heads);
+    // A step's positions and block tables come from the host, or from a kernel that does not let its successors start early: they
+    // are complete when this kernel starts, and are asked for while the kernel in front still runs.
     const int position = positions[token];
     const int* table = block_tables + (size_t)seq_of_token[token] * max_blocks;
 
     float* q_row = q_shared;
-    const T* q_src = q + (size_t)token * q_stride + (size_t)head * head_dim;
-    for (int i = threadIdx.x; i < head_dim; i += kRoundWarps * 32) q_row[i] = Num<T>::load(q_src + i);
 
     float accumulator[COLUMNS];
 #pragma unroll
@@ -109,6 +108,9 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
     auto key_of = [&](int index) { return index < kept ? index : first + index - kept; };
     const int mine = 32 * warp + lane;
     int next_page = mine < count ? table[key_of(mine) / page_size] : 0;
+    pdl_wait();      // everything before this kernel in the stream is complete and visible
+    const T* q_src = q + (size_t)token * q_stride + (size_t)head * head_dim;
+    for (int i = threadIdx.x; i < head_dim; i += kRoundWarps * 32) q_row[i] = Num<T>::load(q_src + i);
     __syncthreads();      // the query's row
     for (int base = 32 * warp; base < count; base += 32 * kRoundWarps) {
         const int index = base + lane;

@@ -38,7 +38,6 @@ __global__ void qk_norm_rope_kv_write_kernel(T* __restrict__ qkv, const W* __res
                                              int write_cache, int* __restrict__ error_flag, int vector_form, int heads_per_block,
                                              int rotary_dim, int interleaved) {
     pdl_trigger();   // let the next kernel start launching
-    pdl_wait();      // everything before this kernel in the stream is complete and visible
     extern __shared__ float2 rotation[];   // (cos, sin) of angle = position * inv_freq[i], i < rotary_dim / 2
     const int token = blockIdx.x;
     const int warps_per_block = blockDim.x >> 5;
@@ -46,13 +45,17 @@ __global__ void qk_norm_rope_kv_write_kernel(T* __restrict__ qkv, const W* __res
     const int total_heads = n_q_heads + 2 * n_kv_heads;
     const int half = rotary_dim >> 1;      // the vector form below is used only when rotary_dim == head_dim
     const int position = positions[token];
-    // the angles depend on the token only: computed once per block, used by every head the block handles
+    // The angles depend on the token only: computed once per block, used by every head the block handles.  Positions and block tables
+    // come from the host, or from a kernel that does not let its successors start early: they are complete when this kernel
+    // starts, so angles and page are at hand when the kernel in front has ended.
     if (inv_freq) {
         for (int i = threadIdx.x; i < half; i += blockDim.x) {
             const float angle = (float)position * inv_freq[i];
             rotation[i] = make_float2(cosf(angle), sinf(angle));
         }
     }
+    const int page = write_cache ? block_tables[(size_t)seq_of_token[token] * max_blocks + position / page_size] : 0;
+    pdl_wait();      // everything before this kernel in the stream is complete and visible
     __syncthreads();
     const int first_head = blockIdx.y * heads_per_block;
     const int end_head = min(first_head + heads_per_block, total_heads);
@@ -66,7 +69,6 @@ __global__ void qk_norm_rope_kv_write_kernel(T* __restrict__ qkv, const W* __res
         } else {
             if (!write_cache) continue;
             const int kv_head = is_k ? head - n_q_heads : head - n_q_heads - n_kv_heads;
-            const int page = block_tables[(size_t)seq_of_token[token] * max_blocks + position / page_size];
             if (page < 0 || page >= num_pages) {
                 if (lane == 0) atomicExch(error_flag, 1 + token);  // host turns this into an exception
                 continue;
