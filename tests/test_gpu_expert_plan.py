@@ -31,3 +31,7 @@ def test_plan(experts, tokens, top, tile_rows):
             assert rows[pair] == -1
         else:
             assert offsets[expert] <= rows[pair] < offsets[expert + 1] and pairs[rows[pair]] == pair
+
+
+def test_plan_of_more_pairs_than_a_block_holds_in_registers():
+    test_plan(64, 6000, 3, 256)
