@@ -600,7 +600,7 @@ def gla_recurrent(proj: torch.Tensor, q_column: int, k_column: int, v_column: in
          z.data_ptr(), pointer(z_bias), weight.data_ptr(), state.data_ptr(), batch.state_slots.data_ptr(), batch.q_start.data_ptr(),
          out.data_ptr(), batch.n_seqs, int(heads), int(dim), int(value_dim), 1.0 / float(tau), float(q_scale), float(eps),
          dtype_code(proj.dtype), dtype_code(weight.dtype), int(segment), int(segments), pointer(segment_state), pointer(segment_decay),
-         stream_handle())
+         int(longest == 1), int(getattr(batch, "keys_settled", False)), stream_handle())
     return out
 
 

@@ -443,13 +443,15 @@ def test_gated_linear_attention_kernel(dtype, heads, dim, vdim, tau):
 
 @pytest.mark.parametrize("vdim", [64, 128])
 @pytest.mark.parametrize("wide_weight,bias", [(False, True), (True, False)])
-@pytest.mark.parametrize("segment", [0, 16, 24, 64])
-def test_linear_attention_in_tiles(vdim, wide_weight, bias, segment):
+@pytest.mark.parametrize("segment,lengths", [(0, [1, 15, 16, 17, 33, 130]), (16, [1, 15, 16, 17, 33, 130]), (24, [130, 1]), (64, [130, 1]),
+                                             (0, [1]), (0, [1] * 37)])
+def test_linear_attention_in_tiles(vdim, wide_weight, bias, segment, lengths):
     """Heads of 64 key channels in bfloat16 with rows in whole 16-byte pieces, which run the tiled kernel: requests of lengths around
-    its batch of 16 tokens, each behind a state of its own, in one pass and in segments that are no multiple of a batch."""
+    its batch of 16 tokens, each behind a state of its own, in one pass and in segments that are no multiple of a batch; and
+    single tokens alone, which run a kernel of their own."""
     from llmserver_b200 import ops
     from llmserver_b200.engine.batch import SequenceSlice, build_batch
-    heads, dim, tau, eps, lengths = 3, 64, 16.0, 1e-5, [1, 15, 16, 17, 33, 130]
+    heads, dim, tau, eps = 3, 64, 16.0, 1e-5
     keys, values, count = heads * dim, heads * vdim, sum(lengths)
     generator = torch.Generator().manual_seed(vdim + segment)
     proj = torch.randn((count, 2 * keys + 2 * values + 8), generator=generator).to(torch.bfloat16)
