@@ -32,12 +32,20 @@ __device__ __forceinline__ void take_better(float& best, int& best_index, float 
     }
 }
 
+// The words that a step's kernels report errors in, behind the tokens: what a step reads back is then one piece of memory (the
+// kernels in front are complete).
+__device__ __forceinline__ void leave_flags(int* behind, const int* flag_a, const int* flag_b) {
+    if (flag_a == nullptr || flag_b == nullptr) return;
+    behind[0] = *flag_a;
+    behind[1] = *flag_b;
+}
+
 // One block scans a slice of a row; grid (slices, rows).  With one slice the token goes straight to
 // `out`; with more, each block leaves its best (score, index) in `partial` and sample_merge_kernel picks.
 __global__ void sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
                               const uint64_t* __restrict__ seeds, const int* __restrict__ steps,
                               int* __restrict__ out, int vocab, float* __restrict__ partial_scores,
-                              int* __restrict__ partial_indices) {
+                              int* __restrict__ partial_indices, const int* __restrict__ flag_a, const int* __restrict__ flag_b) {
     pdl_trigger();   // let the next kernel start launching
     pdl_wait();      // everything before this kernel in the stream is complete and visible
     __shared__ float best_values[32];
@@ -99,6 +107,7 @@ __global__ void sample_kernel(const float* __restrict__ logits, const float* __r
         if (lane == 0) {
             if (slices == 1) {
                 out[row] = best_index == 0x7fffffff ? 0 : best_index;
+                if (row == 0) leave_flags(out + gridDim.y, flag_a, flag_b);
             } else {
                 partial_scores[row * slices + blockIdx.x] = best;
                 partial_indices[row * slices + blockIdx.x] = best_index;
@@ -108,7 +117,7 @@ __global__ void sample_kernel(const float* __restrict__ logits, const float* __r
 }
 
 __global__ void sample_merge_kernel(const float* __restrict__ partial_scores, const int* __restrict__ partial_indices,
-                                    int* __restrict__ out, int slices) {
+                                    int* __restrict__ out, int slices, const int* __restrict__ flag_a, const int* __restrict__ flag_b) {
     pdl_trigger();   // let the next kernel start launching
     pdl_wait();      // everything before this kernel in the stream is complete and visible
     const int row = blockIdx.x, lane = threadIdx.x;
@@ -121,7 +130,10 @@ __global__ void sample_merge_kernel(const float* __restrict__ partial_scores, co
         const int other_index = __shfl_xor_sync(0xffffffffu, best_index, offset);
         take_better(best, best_index, other, other_index);
     }
-    if (lane == 0) out[row] = best_index == 0x7fffffff ? 0 : best_index;
+    if (lane == 0) {
+        out[row] = best_index == 0x7fffffff ? 0 : best_index;
+        if (row == 0) leave_flags(out + gridDim.x, flag_a, flag_b);
+    }
 }
 
 // How many slices a row of `vocab` logits is scanned in (the caller sizes the scratch by it).
@@ -132,10 +144,11 @@ LLM_EXPORT int llm_sample_slices(int n_rows, int vocab) {
     return slices;
 }
 
-// partial_scores / partial_indices: [n_rows, slices] each, needed only when slices > 1.
+// partial_scores / partial_indices: [n_rows, slices] each, needed only when slices > 1.  With flag_a and flag_b their words follow the
+// tokens in `out` [n_rows + 2].
 LLM_EXPORT int llm_sample(const float* logits, const float* temperatures, const uint64_t* seeds, const int* steps,
                           int* out, int n_rows, int vocab, float* partial_scores, int* partial_indices,
-                          cudaStream_t stream) {
+                          const int* flag_a, const int* flag_b, cudaStream_t stream) {
     if (n_rows == 0) return LLM_OK;
     if (n_rows > 65535) {
         llm_set_error("sample: at most 65535 rows per launch, got %d", n_rows);
@@ -149,9 +162,9 @@ LLM_EXPORT int llm_sample(const float* logits, const float* temperatures, const 
     const int threads = vocab >= 4096 ? 512 : 256;
     dim3 grid(slices, n_rows);
     llm_launch(sample_kernel, grid, threads, 0, stream, logits, temperatures, seeds, steps, out, vocab, partial_scores,
-                                                partial_indices);
+                                                partial_indices, flag_a, flag_b);
     int status = llm_check_launch("sample");
     if (status != LLM_OK || slices == 1) return status;
-    llm_launch(sample_merge_kernel, n_rows, 32, 0, stream, partial_scores, partial_indices, out, slices);
+    llm_launch(sample_merge_kernel, n_rows, 32, 0, stream, partial_scores, partial_indices, out, slices, flag_a, flag_b);
     return llm_check_launch("sample_merge");
 }

@@ -152,8 +152,8 @@ class DecodeGraph:
             self.buffer.copy_(self.host, non_blocking=True)
             logits = self.model.step(self.batch)
             self.logits = logits        # [batch_size, vocab] of the last replay (tests compare them with eager steps)
-            tokens = ops.sample(logits, self.batch.temperatures, self.batch.seeds, self.batch.sample_steps)
-            self.result = torch.cat([tokens, self.batch.error_flag, wait_error_flag(device)])
+            self.result = ops.sample(logits, self.batch.temperatures, self.batch.seeds, self.batch.sample_steps,
+                                     flags=(self.batch.error_flag, wait_error_flag(device)))
             self.answer.copy_(self.result, non_blocking=True)
 
     def run(self, slices: List[SequenceSlice], sampling: Sequence, phases: Optional[dict] = None) -> List[int]:

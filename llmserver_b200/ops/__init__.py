@@ -164,9 +164,10 @@ def clamped_gate_up(x: torch.Tensor, weight: torch.Tensor, limit: float, alpha: 
 
 
 def sample(logits: torch.Tensor, temperatures: Optional[torch.Tensor] = None, seeds: Optional[torch.Tensor] = None,
-           steps: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+           steps: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, flags=None) -> torch.Tensor:
     """One token per row of float32 logits [R, V]: argmax where the temperature is 0, else the
-    Gumbel-max draw keyed by (seeds[r], steps[r]).  Returns int32 [R]."""
+    Gumbel-max draw keyed by (seeds[r], steps[r]).  Returns int32 [R].  ``flags``: two one-element int32 tensors whose
+    values follow the tokens; the result is then [R + 2]."""
     check(logits, "logits", torch.float32)
     rows, vocab = logits.shape
     if temperatures is not None:
@@ -176,15 +177,20 @@ def sample(logits: torch.Tensor, temperatures: Optional[torch.Tensor] = None, se
         check(seeds, "seeds", torch.int64)
         check(steps, "steps", torch.int32)
     if out is None:
-        out = torch.empty((rows,), dtype=torch.int32, device=logits.device)
+        out = torch.empty((rows + (2 if flags else 0),), dtype=torch.int32, device=logits.device)
     check(out, "sampled tokens", torch.int32)
+    if flags:
+        for flag in flags:
+            check(flag, "flag", torch.int32, 1)
+        if out.numel() != rows + 2 or rows == 0:
+            raise KernelError(f"{rows} tokens and two flags do not fit {out.numel()} elements")
     slices = library().llm_sample_slices(rows, vocab)
     scores = indices = None
     if slices > 1:      # large vocabularies are scanned by several blocks per row, merged by a second kernel
         scores = torch.empty((rows, slices), dtype=torch.float32, device=logits.device)
         indices = torch.empty((rows, slices), dtype=torch.int32, device=logits.device)
     call("llm_sample", logits.data_ptr(), pointer(temperatures), pointer(seeds), pointer(steps), out.data_ptr(), rows,
-         vocab, pointer(scores), pointer(indices), stream_handle())
+         vocab, pointer(scores), pointer(indices), *((flags[0].data_ptr(), flags[1].data_ptr()) if flags else (0, 0)), stream_handle())
     return out
 
 

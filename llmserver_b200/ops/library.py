@@ -26,7 +26,7 @@ SIGNATURES = {
     "llm_decay_recurrence_threads": [_I, _I],
     "llm_retention_recurrent": [_P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _S],
     "llm_ssd_recurrent": [_P, _I, _I, _P, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _S],
-    "llm_sample": [_P, _P, _P, _P, _P, _I, _I, _P, _P, _S],
+    "llm_sample": [_P, _P, _P, _P, _P, _I, _I, _P, _P, _P, _P, _S],
     "llm_sample_slices": [_I, _I],
     "llm_qk_norm_rope_kv_write": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P, _I, _I, _I, _I, _S],
     "llm_attention_generic": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _I, _P, _I, _I, _P, _I, _P, _I, _S],
