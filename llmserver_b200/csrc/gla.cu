@@ -191,7 +191,8 @@ __global__ void __launch_bounds__(RR == 128 ? 256 : 512, RR <= 16 ? 2 : 1) gla_r
 // bytes), and the row groups' parts of o are added by seven shuffles, each of which halves the columns that a lane still holds.
 // What bounds the kernel above for long portions is its staging: a thread's loads of a batch of tokens wait for one another (up to
 // 16 in a row).  Here all of a batch is asked for at once, 16 bytes at a time.  2048 tokens of 32 heads of 64 / 128, us, the
-// kernel above / this: states of the segments 153 / 76, outputs 232 / 156 (tiles with loads one after the other: 148 and 254).
+// kernel above / this: states of the segments 153 / 73, outputs 232 / 133 (tiles with loads one after the other: 148 and 254; outputs
+// with the gates read at a batch's end: 156; without two tokens in flight: 142, which would make the states' pass 82).
 constexpr int kTileDim = 64;
 
 // Eight bfloat16 numbers, times `scale`, as 32-bit numbers in shared memory.
@@ -264,6 +265,9 @@ __global__ void __launch_bounds__(VDIM) gla_tiles_kernel(GlaArgs a) {
             }
         }
     }
+    float weights[VDIM / 32];                        // of the norm, for the columns of a token that this lane finishes
+#pragma unroll
+    for (int j = 0; j < VDIM / 32; ++j) weights[j] = Num<W>::load((const W*)a.weight + lane * (VDIM / 32) + j);
     const int my_column = column0 + row_group;      // the one of its eight that a lane holds when the row groups' parts have been added
 
     for (int first = begin; first < end; first += GLA_TOKENS) {
@@ -291,6 +295,18 @@ __global__ void __launch_bounds__(VDIM) gla_tiles_kernel(GlaArgs a) {
         for (int u = 0; u < kValuesEach; ++u) {
             const int e = threadIdx.x + u * VDIM, t = e / (VDIM / 8), j = e % (VDIM / 8) * 8;
             if (t < count) v_raw[u] = *reinterpret_cast<const float4*>(proj + (size_t)(first + t) * a.row_width + a.v_offset + head * VDIM + j);
+        }
+        // (the gates of the tokens that this warp will finish, too)
+        constexpr int kEach = VDIM / 32, kMine = GLA_TOKENS / kWarps;      // neighbouring columns of a lane, tokens of a warp
+        uint32_t g_raw[MODE == GLA_LOCAL ? 1 : kMine][kEach / 2];
+        if (MODE != GLA_LOCAL) {
+#pragma unroll
+            for (int u = 0; u < kMine; ++u) {
+                const int t = warp + u * kWarps;
+                const uint32_t* g_row = reinterpret_cast<const uint32_t*>(proj + (size_t)(first + t) * a.row_width + a.g_offset + head * VDIM + lane * kEach);
+#pragma unroll
+                for (int j = 0; j < kEach / 2; ++j) g_raw[u][j] = t < count ? g_row[j] : 0u;
+            }
         }
 #pragma unroll
         for (int u = 0; u < kNarrowEach; ++u) {
@@ -321,6 +337,7 @@ __global__ void __launch_bounds__(VDIM) gla_tiles_kernel(GlaArgs a) {
             if (e / (VDIM / 8) < count) spread8(v_raw[u], 1.0f, v_s + e * 8);
         }
         __syncthreads();
+#pragma unroll(MODE == GLA_LOCAL ? 1 : 2)
         for (int t = 0; t < count; ++t) {
             const int at = t * kTileDim + 4 * row_group;
             const ulonglong2 k_low = *reinterpret_cast<const ulonglong2*>(k_s + at), k_high = *reinterpret_cast<const ulonglong2*>(k_s + at + 32);
@@ -364,22 +381,24 @@ __global__ void __launch_bounds__(VDIM) gla_tiles_kernel(GlaArgs a) {
         }
         if (MODE == GLA_LOCAL) continue;
         __syncthreads();
-        constexpr int kEach = VDIM / 32;      // neighbouring columns of a lane
-        for (int t = warp; t < count; t += kWarps) {
-            const T* g_row = proj + (size_t)(first + t) * a.row_width + a.g_offset + head * VDIM + lane * kEach;
+#pragma unroll
+        for (int u = 0; u < kMine; ++u) {
+            const int t = warp + u * kWarps;
+            if (t >= count) break;
             T* dst = (T*)a.out + (size_t)(first + t) * a.heads * VDIM + head * VDIM + lane * kEach;
-            float o[kEach], g[kEach], sum_squares = 0.0f;
+            float o[kEach], sum_squares = 0.0f;
 #pragma unroll
             for (int j = 0; j < kEach; ++j) {
-                g[j] = Num<T>::load(g_row + j);
                 o[j] = o_s[t * VDIM + lane * kEach + j];
                 sum_squares += o[j] * o[j];
             }
             const float inverse = rsqrtf(warp_sum(sum_squares) / (float)VDIM + a.eps);
 #pragma unroll
-            for (int j = 0; j < kEach; ++j) {
-                const float gate = g[j] / (1.0f + expf(-g[j]));
-                Num<T>::store(dst + j, o[j] * inverse * Num<W>::load((const W*)a.weight + lane * kEach + j) * gate);
+            for (int j = 0; j < kEach; j += 2) {
+                const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g_raw[u][j / 2]));
+                const float y0 = o[j] * inverse * weights[j] * (g.x / (1.0f + expf(-g.x)));
+                const float y1 = o[j + 1] * inverse * weights[j + 1] * (g.y / (1.0f + expf(-g.y)));
+                *reinterpret_cast<__nv_bfloat162*>(dst + j) = __floats2bfloat162_rn(y0, y1);
             }
         }
     }
@@ -597,7 +616,7 @@ LLM_EXPORT int llm_gla_recurrent(const void* proj, int row_width, int q_offset, 
         return LLM_REFUSED;
     }
     // the tiled kernel reads rows and states in 16-byte pieces
-    const bool pieces = aligned16(proj) && row_width % 8 == 0 && q_offset % 8 == 0 && k_offset % 8 == 0 && v_offset % 8 == 0 && aligned16(z) &&
+    const bool pieces = aligned16(proj) && row_width % 8 == 0 && q_offset % 8 == 0 && k_offset % 8 == 0 && v_offset % 8 == 0 && g_offset % 8 == 0 && aligned16(z) && aligned16(out) &&
                         aligned16(state) && (!segmented || (aligned16(segment_state) && aligned16(segment_decay)));
     if (dtype == LLM_BF16 && (weight_dtype == LLM_F32 || weight_dtype == LLM_BF16) && dim == kTileDim && (vdim == 64 || vdim == 128) && pieces) {
         if (vdim == 64) return weight_dtype == LLM_F32 ? gla_tiles_launch<float, 64>(a, n_seqs, segmented, singles, settled, stream) : gla_tiles_launch<__nv_bfloat16, 64>(a, n_seqs, segmented, singles, settled, stream);
