@@ -40,6 +40,7 @@
 #include "common.cuh"
 #include "tma.cuh"
 
+#include <atomic>
 #include <stdlib.h>
 
 namespace {
@@ -47,9 +48,11 @@ namespace {
 constexpr int kBlockRows = 128;     // rows of W per CTA (UMMA M)
 constexpr int kAtomK = 64;          // one 128-byte swizzle atom of bfloat16
 constexpr int kMaxRows = 128;       // tokens per launch
-constexpr int kTwoAtomRows = 64;    // up to this many tokens a pipeline stage holds two atoms of K, beyond (where a token atom is as
-                                    // large as a weight atom) one: three stages of 32 KiB then leave room for two blocks per SM
+constexpr int kTwoAtomRows = 64;    // up to this many tokens a stage of a block that shares its SM holds two atoms of K, beyond (where a token
+                                    // atom is as large as a weight atom) one: three stages of 32 KiB then leave room for two blocks per SM
 constexpr int kThreeBlocksKib = 74; // ring of a block that shares its SM with two others
+constexpr int kOneBlockKib = 200;   // ring of a block that has its SM to itself
+constexpr int kTurn = 7;            // blocks of K from where a tile begins to where the next one does (odd: shares are often a power of two)
 constexpr int kThreads = 256;       // at most: four warps up to 16 tokens, eight beyond (two have a role in the main
                                     // loop, all work in the epilogue, whose time per token is instruction issue)
 constexpr int kMaxStages = 12;
@@ -489,8 +492,18 @@ __device__ __forceinline__ void stream_finish8(const GemmParams& p, int m, bool 
 // PER_SM (MANY): how many blocks share an SM.  Two have room for a ring of 100 KiB and for registers that hold the parts of eight
 // ranks at once.  Where a launch has more than two blocks per SM, three of them with a shorter ring of single atoms (and 80 registers)
 // are faster than a second wave: gate/up projection of the 8B shape in two parts (384 blocks), one behind the other with weights
-// from HBM, at 24 / 61 / 119 tokens 33.9 / 35.6 / 40.0 us against 40.3 / 43.8 / 50.0 with two an SM and 35.8 / 37.4 / 41.5 unsplit; output
-// head of 151936 rows at 20 / 64 tokens 190 / 199 us against 206 / 218 (190 is what its bytes take).
+// from HBM, at 24 / 61 / 119 tokens 33.9 / 35.6 / 39.1 us against 40.3 / 43.8 / 49.7 with two an SM and 35.8 / 37.4 / 40.1 unsplit; output
+// head of 151936 rows at 20 / 64 / 119 tokens 190 / 199 / 222 us against 206 / 218 / 237 (190 is what its bytes take).
+//
+// Where every block can have an SM to itself (no more clusters than the device holds one block per SM), it takes 200 KiB: stages of two
+// atoms at any number of tokens, and clusters of four or fewer instead of eight.  Two things make that faster beyond 16 tokens.  The
+// parts that cross distributed shared memory are (split - 1) / split of every rank's tile, and that network brings some 20 bytes a
+// nanosecond to an SM: eight ranks of 119 tokens take 4.5 us where four take 2.  And a stage costs a block some 0.3 us of waits, copies
+// and commits whatever it holds: unsplit, one block per SM, the down projection takes 80.6 us at 119 tokens with six stages of one
+// atom, 60.3 with three of two.  8B shape, us, two blocks per SM in the best split / one: at 61 tokens q/k/v 14.1 / 14.0, output
+// projection 11.7 / 10.8, down projection 22.3 / 21.1; at 119 17.0 / 16.2, 15.0 / 12.6 and 26.2 / 23.8.  With 150 KiB (room for a block of the
+// next kernel) the same at 61 tokens and slower at 119 (18.2, 13.2 and 26.1).  Clusters that do not all fit cost a second wave
+// (48 tiles in three parts 27 us against 18), so the device is asked how many do.
 //
 // What bounds a product of 17 to 128 tokens beside its weights' bytes is the epilogue.  Leaving the token tiles out after the first
 // ring changes nothing up to 128 tokens (48.7 against 48.8 us for gate/up at 119), finishing 16 tokens only takes a warp-per-token
@@ -533,6 +546,11 @@ __global__ void __launch_bounds__(kThreads, PER_SM) gemm_small_m_kernel(const __
     const int kb_begin = (int)((long long)total_kb * rank / p.split);
     const int kb_end = (int)((long long)total_kb * (rank + 1) / p.split);
     const int n_kb = kb_end - kb_begin;
+    // Every tile begins at another place of its share of K and comes back to the share's start: blocks that walk K in step read the
+    // same columns of thousands of rows at a time, which lie on few of the memory's channels (q/k/v of the 8B shape in four parts, us,
+    // in step / turned: 11.8 / 11.3 at 8 tokens, 14.3 / 13.8 at 61, 17.1 / 16.6 at 119; gate/up unsplit at 119 42.0 / 40.7).
+    const int turn = n_kb > 0 ? tile * kTurn % n_kb : 0;
+    auto turned = [&](int i) { const int kb = i + turn; return kb >= n_kb ? kb - n_kb : kb; };
 
     if (threadIdx.x == 0) {
         failed = 0;
@@ -550,7 +568,7 @@ __global__ void __launch_bounds__(kThreads, PER_SM) gemm_small_m_kernel(const __
             mbar_expect_tx(bar, kAtoms * (a_bytes + b_bytes));
 #pragma unroll
             for (int atom = 0; atom < kAtoms; ++atom)
-                tma_load_2d(base + i * stage_bytes + atom * a_bytes, &map_w, bar, (kb_begin + i) * kBlockK + atom * kAtomK, n0);
+                tma_load_2d(base + i * stage_bytes + atom * a_bytes, &map_w, bar, (kb_begin + turned(i)) * kBlockK + atom * kAtomK, n0);
         }
     }
     const uint32_t tmem_cols = p.token_pad > 64 ? 128 : 64;      // one column of floats per token
@@ -573,7 +591,7 @@ __global__ void __launch_bounds__(kThreads, PER_SM) gemm_small_m_kernel(const __
 #pragma unroll
             for (int atom = 0; atom < kAtoms; ++atom)
                 tma_load_2d(base + i * stage_bytes + b_offset + atom * b_pitch, &map_x, smem_u32(&full_bar[i]),
-                            (kb_begin + i) * kBlockK + atom * kAtomK, 0);
+                            (kb_begin + turned(i)) * kBlockK + atom * kAtomK, 0);
         for (int i = first; i < n_kb; ++i) {
             const int s = i % p.stages;
             if (!mbar_wait(smem_u32(&empty_bar[s]), ((i / p.stages) - 1) & 1)) {
@@ -585,8 +603,8 @@ __global__ void __launch_bounds__(kThreads, PER_SM) gemm_small_m_kernel(const __
             mbar_expect_tx(bar, kAtoms * (a_bytes + b_bytes));
 #pragma unroll
             for (int atom = 0; atom < kAtoms; ++atom) {
-                tma_load_2d(stage + atom * a_bytes, &map_w, bar, (kb_begin + i) * kBlockK + atom * kAtomK, n0);
-                tma_load_2d(stage + b_offset + atom * b_pitch, &map_x, bar, (kb_begin + i) * kBlockK + atom * kAtomK, 0);
+                tma_load_2d(stage + atom * a_bytes, &map_w, bar, (kb_begin + turned(i)) * kBlockK + atom * kAtomK, n0);
+                tma_load_2d(stage + b_offset + atom * b_pitch, &map_x, bar, (kb_begin + turned(i)) * kBlockK + atom * kAtomK, 0);
             }
         }
     } else if (warp == 1 && lane == 0) {
@@ -856,6 +874,41 @@ static RowScale row_scale_of(const float* parts, int n_parts, int stride, float 
     return scale;
 }
 
+// How many clusters of `split` blocks that each fill an SM's shared memory the device holds at a time (a cluster lies within a group of
+// SMs, so that it can be fewer than SMs / split), 0 where it cannot say.  Asked once per size of cluster.
+static int lone_clusters(int split) {
+    static std::atomic<int> known[kMaxSplit + 1];      // 1 + answer
+    if (const int answer = known[split].load(std::memory_order_relaxed)) return answer - 1;
+    void (*kernel)(CUtensorMap, CUtensorMap, GemmParams) = gemm_small_m_kernel<2, true, 2>;
+    const size_t shared = (size_t)kOneBlockKib * 1024 + 1024;
+    int clusters = 0;
+    if (split == 1) {
+        clusters = llm_sm_count();
+    } else if (llm_raise_shared_limit(reinterpret_cast<const void*>(kernel), (size_t)226 * 1024, "gemm_small_m") == LLM_OK) {
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3((unsigned)(llm_sm_count() / split * split), 1, 1);
+        config.blockDim = dim3(kThreads, 1, 1);
+        config.dynamicSmemBytes = shared;
+        cudaLaunchAttribute attribute;
+        attribute.id = cudaLaunchAttributeClusterDimension;
+        attribute.val.clusterDim.x = (unsigned)split;
+        attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+        config.attrs = &attribute;
+        config.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+            cudaGetLastError();
+            clusters = 0;
+        }
+    }
+    known[split].store(1 + clusters, std::memory_order_relaxed);
+    return clusters;
+}
+
+// 1 when a product of n columns in `split` parts runs as one block per SM beyond 16 tokens.
+LLM_EXPORT int llm_gemm_small_m_one_per_sm(int n, int split) {
+    return split >= 1 && split <= kMaxSplit && (n + kBlockRows - 1) / kBlockRows <= lone_clusters(split);
+}
+
 static int small_m_launch(const void* x, const void* w, void* out, int m, int n, int k, int ldc, int out_is_f32,
                           int requested_split, int* error_flag, const RopeEpilogue* rope, cudaStream_t stream,
                           int silu_gate, const RowScale& scale, const StreamEpilogue* stream_out = nullptr) {
@@ -904,11 +957,12 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
     if (split > total_kb / 2) split = total_kb / 2;
     if (split > kMaxSplit) split = kMaxSplit;
     if (split < 1) split = 1;
-    // more than two blocks per SM: three, of single atoms (see gemm_small_m_kernel)
-    const bool three = many && m <= kTwoAtomRows && (long long)tiles * split > 2 * llm_sm_count();
-    if (three) {
-        atoms = 1;
-        total_kb = (k + kAtomK - 1) / kAtomK;
+    // more than two blocks per SM: three, of single atoms; no more than one: that one, with stages of two atoms (see gemm_small_m_kernel)
+    const bool three = many && (long long)tiles * split > 2 * llm_sm_count();
+    const bool alone = many && tiles <= lone_clusters(split);
+    if (three || alone) {
+        atoms = three ? 1 : 2;
+        total_kb = (k + kAtomK * atoms - 1) / (kAtomK * atoms);
     }
     p.split = split;
     const size_t a_bytes = (size_t)kBlockRows * kAtomK * 2;
@@ -923,7 +977,8 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
         if (ring_kib < 32) ring_kib = 32;
         if (ring_kib > 200) ring_kib = 200;
     }
-    int stages = (int)(((size_t)(three && ring_kib > kThreeBlocksKib ? kThreeBlocksKib : ring_kib) * 1024) / stage_bytes);
+    const int my_kib = three && ring_kib > kThreeBlocksKib ? kThreeBlocksKib : alone ? kOneBlockKib : ring_kib;
+    int stages = (int)((size_t)my_kib * 1024 / stage_bytes);
     if (stages < 1) stages = 1;
     if (stages > kMaxStages) stages = kMaxStages;
     const int my_kb = (total_kb + split - 1) / split;

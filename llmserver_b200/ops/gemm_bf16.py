@@ -120,15 +120,18 @@ _CLOSE_MANY_ROWS = 0.05
 # Among the splits of this package's kernel, the ones within this much of the fastest count as equal, and the largest
 # of them is taken: measured one product at a time, 6 and 8 parts of the 8B shape's q/k/v and output projections lie
 # within 1 to 3.5 % of each other and the choice went either way from process to process, while whole steps are 1 to
-# 2 % faster with 8 (more blocks keep more bytes in flight where one kernel hands over to the next).
+# 2 % faster with 8 (more blocks keep more bytes in flight where one kernel hands over to the next).  That is so up to 16 rows; beyond,
+# where fewer parts that have an SM to themselves are often the fastest, the fastest is taken (a step of 61 sequences of the 8B
+# shape 6523 us with the margin, 6466 without, of 64 of the Dikusun shape 957 and 945).
 _CLOSE_SPLITS = float(os.environ.get("LLMSERVER_B200_GEMM_CLOSE_SPLITS", "0.04"))
 
 
-def _fastest_split(timed: list) -> int:
-    """``timed``: (split, milliseconds) of this package's kernel; the largest split among the (nearly) fastest."""
+def _fastest_split(timed: list, rows: int) -> int:
+    """``timed``: (split, milliseconds) of this package's kernel for so many rows; up to 16, the largest split among the (nearly) fastest."""
     fastest = min(elapsed for _, elapsed in timed)
     # (a profiler that serialises launches can report times of zero or below: the margin must not turn negative)
-    return max(split for split, elapsed in timed if elapsed <= fastest + abs(fastest) * _CLOSE_SPLITS)
+    margin = abs(fastest) * _CLOSE_SPLITS if rows <= 16 else 0.0
+    return max(split for split, elapsed in timed if elapsed <= fastest + margin)
 
 
 def _time_in_step(run, device, repeats: int = 10) -> float:
@@ -181,12 +184,14 @@ def _small_m(x, weight, out, split: int, scale: tuple = NO_SCALE) -> None:
 
 
 def _split_beyond_64_rows(cols: int) -> int:
-    """The split of K beyond 64 rows, where only prompts run this package's kernel: the most parts that make clusters of a power of two
-    and at most two blocks per SM.  Measuring it stopped the first such prompt for 0.15 to 0.2 s and found no better one (8B shape, ms,
-    measured / this: 4.61 / 4.63 at 70 tokens, 4.83 / 4.82 at 100, 5.08 / 5.10 at 128; with clusters of 6 for q/k/v 5.29 at 100, with one
-    block per SM 5.11)."""
-    blocks = 2 * library().llm_sm_count()
-    return max([split for split in (1, 2, 4, 8) if -(-cols // 128) * split <= blocks], default=1)
+    """The split of K beyond 64 rows, where only prompts run this package's kernel: the most parts, of at most four, that run as one block
+    per SM; with more tiles than SMs two parts if three blocks per SM hold them (see gemm_small_m_kernel).  Measuring it stopped the first
+    such prompt for 0.15 to 0.2 s and found no better one."""
+    lib = library()
+    split = max([split for split in (1, 2, 3, 4) if lib.llm_gemm_small_m_one_per_sm(cols, split)], default=0)
+    if split == 0:
+        split = 2 if -(-cols // 128) * 2 <= 3 * lib.llm_sm_count() else 1
+    return split
 
 
 def _plan_for(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, own_kernel_only: bool = False) -> int:
@@ -225,7 +230,7 @@ def _plan_for(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, own
             if split > 1 and (tiles * split > 600 or k_blocks // split < 2):
                 continue
             timed.append((split, _time_in_step(lambda: _small_m(x, weight, out, split), x.device)))
-        best = _fastest_split(timed)
+        best = _fastest_split(timed, rows)
         _choice[key] = best
         _tunings += 1
         if PLAN_FILE:
@@ -243,7 +248,7 @@ def _plan_for(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, own
         if split > 1 and (tiles * split > 600 or k_blocks // split < 2):
             continue
         timed.append((split, _time_in_step(lambda: _small_m(x, weight, out, split), x.device)))
-    best = _fastest_split(timed) if min(elapsed for _, elapsed in timed) < best_time else 0
+    best = _fastest_split(timed, rows) if min(elapsed for _, elapsed in timed) < best_time else 0
     _choice[key] = best
     _tunings += 1
     if PLAN_FILE:
@@ -367,7 +372,7 @@ def _plan_fused(kind: str, rows: int, cols: int, inner: int, fused, apart, devic
         if split > 1 and (tiles * split > 600 or k_blocks // split < 2):
             continue
         timed.append((split, _time_in_step(lambda: fused(split), device)))
-    best = _fastest_split(timed) if min(elapsed for _, elapsed in timed) < apart_time else 0
+    best = _fastest_split(timed, rows) if min(elapsed for _, elapsed in timed) < apart_time else 0
     _choice[key] = best
     _tunings += 1
     if PLAN_FILE:

@@ -53,6 +53,27 @@ def test_three_blocks_an_sm(rows, tiles, inner, split):
     close(parts[:, :rows].sum(0), (want * want).sum(-1), torch.float32, "sums of squares", factor=4.0)
 
 
+@pytest.mark.parametrize("rows", [16, 17, 64, 65, 128])
+@pytest.mark.parametrize("tiles,inner,split", [(148, 136, 1), (149, 136, 1), (33, 1032, 4), (34, 1032, 4), (3, 200, 2), (22, 520, 6)])
+def test_one_block_an_sm(rows, tiles, inner, split):
+    """Launches around one block per SM, which run a long ring of two-atom stages beyond 16 rows; every tile begins at another place of
+    its share of K."""
+    from llmserver_b200.ops import gemm_bf16
+    from llmserver_b200.ops.library import call, check_wait_errors, stream_handle
+    cols = tiles * 128 - 126
+    x, w = rand((rows, inner), torch.bfloat16, 1), rand((cols, inner), torch.bfloat16, 2, inner ** -0.5)
+    flag, exact = gemm_bf16.error_flag(DEVICE).data_ptr(), x.double() @ w.double().T
+    out = torch.full((rows, cols), float("nan"), dtype=torch.float32, device=DEVICE)
+    call("llm_gemm_small_m", x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, cols, inner, cols, 1, split, *gemm_bf16.NO_SCALE, flag, stream_handle())
+    stream = rand((rows, cols), torch.float32, 3)
+    want = stream.double() + exact
+    call("llm_gemm_into_stream", x.data_ptr(), w.data_ptr(), stream.data_ptr(), rows, cols, inner, split, 0, 0, 0, 0, 0, flag, stream_handle())
+    torch.cuda.synchronize()
+    check_wait_errors()
+    close(out, exact, torch.float32, "sums", factor=4.0)
+    close(stream, want, torch.float32, "stream", factor=4.0)
+
+
 @pytest.mark.parametrize("rows", [16, 17, 33, 64, 65, 119, 128])
 def test_stream_and_scaled_rows(rows):
     """x W^T added to the stream, the sums of squares it leaves, and the gated product that divides by them: against the same in 64
