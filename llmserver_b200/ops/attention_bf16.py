@@ -30,7 +30,6 @@ WIDE_CLUSTER_SPLITS = 16
 UNEVEN_SPLITS, UNEVEN_SEQUENCES = 2, 128
 
 
-
 # "tcgen05": the 256-row kernel for long portions and the 128-row kernel otherwise; "tcgen05-128" / "tcgen05-256":
 # always that kernel; "mma": the mma.sync kernel
 PREFILL_KERNEL = os.environ.get("LLMSERVER_B200_PREFILL_ATTENTION", "tcgen05")
