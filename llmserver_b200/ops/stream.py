@@ -32,8 +32,9 @@ def stream_rows(width: int, decode: bool) -> int:
     replayed decode steps, contexts of 301 to 2000: width 2048 2.33 / 2.24 at 24 rows, 2.94 / 2.95 at 64, 3.93 / 4.07 at 96, 4.72 / 4.98
     at 128; 8B shape 4.75 / 4.70 at 24, 5.55 / 5.43 at 48, 5.63 / 5.40 at 61, 7.04 / 7.23 at 96, 8.09 / 8.51 at 128; 14B shape (5120) 6.68 /
     6.42 at 24, 7.91 / 7.94 at 64, 9.90 / 9.76 at 96, 11.19 / 11.43 at 128; 32B shape (5120) 15.66 / 15.50 at 64.  Prompts: width 2048 4.33 /
-    3.16 at 128 tokens; 8B 5.38 / 3.92 at 20, 6.18 / 4.38 at 64, 5.39 / 4.83 at 100, 5.34 / 5.13 at 128; 14B 6.02 / 5.61 at 20, 6.52 / 6.31
-    at 64, 6.94 / 6.95 at 100, 7.13 / 7.21 at 128; 32B 13.6 / 13.1 at 40, 14.4 / 14.1 at 64, 15.2 / 16.0 at 100, 15.8 / 16.9 at 128."""
+    3.16 at 128 tokens; 8B 5.38 / 3.92 at 20, 6.18 / 4.38 at 64, 5.39 / 4.11 at 100, 5.34 / 4.21 at 128; 14B 6.02 / 5.61 at 20, 6.52 / 6.31
+    at 64, 6.93 / 6.38 at 70, 6.88 / 6.82 at 100, 7.01 / 7.08 at 128; 32B 13.6 / 13.1 at 40, 14.4 / 14.1 at 64, 15.2 / 16.0 at 100, 15.8 / 16.9 at 128
+    (the 8B prompts of 100 and 128 tokens and the 14B ones from 70 on with blocks that have an SM to themselves, the others beyond 64 rows before)."""
     if STREAM_MANY_ROWS <= STREAM_ROWS:
         return STREAM_MANY_ROWS
     return STREAM_DEVICE_ROWS if decode or width > STREAM_LAUNCH_WIDTH else STREAM_MANY_ROWS
