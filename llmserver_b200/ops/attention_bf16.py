@@ -159,6 +159,19 @@ def _part_counters(batch, n_kv_heads: int, split_len: int, max_splits: int, devi
     return counters.data_ptr()
 
 
+def _split_scratch(batch, n_q_heads: int, value_dim: int, split_len: int, max_splits: int, device):
+    """Where the parts of single tokens leave their results, shared by the step's layers of one launch shape.  Parts by length have a
+    place per sequence, equal parts one per token of the step (single tokens may lie behind prompt portions): a layer of the
+    one kind must not get what a layer of the other kind left."""
+    rows = batch.n_seqs if 0 < -split_len < max_splits else batch.n_tokens
+    key = ("attention_mma_scratch", rows, n_q_heads, value_dim, max_splits)
+    scratch = batch.scratch.get(key)
+    if scratch is None:
+        scratch = batch.scratch[key] = (torch.empty((rows, n_q_heads, max_splits, value_dim), dtype=torch.float32, device=device),
+                                        torch.empty((rows, n_q_heads, max_splits, 2), dtype=torch.float32, device=device))
+    return scratch
+
+
 # A decode row's older keys were cached by earlier steps, which lie behind the step's batch copy; the decode kernel may
 # start copying them before the kernel in front of it (which writes the newest key) has ended.  Only batches that say
 # so (``keys_settled``, set where the engine packs a step) get this.
@@ -176,15 +189,7 @@ def try_attention(qkv, q_stride, batch, block_tables, k_pages, v_pages, n_q_head
     out = torch.empty((batch.n_tokens, n_q_heads * head_dim), dtype=torch.bfloat16, device=qkv.device)
     partial_out = partial_ml = None
     if run_decode and max_splits > 1:
-        # scratch of the split-KV decode, shared by every layer of the step
-        key = ("attention_mma_scratch", n_q_heads, head_dim, max_splits)
-        scratch = batch.scratch.get(key)
-        if scratch is None:
-            rows = batch.n_seqs if 0 < -split_len < max_splits else batch.n_tokens      # parts by length have a place per sequence
-            scratch = (torch.empty((rows, n_q_heads, max_splits, head_dim), dtype=torch.float32, device=qkv.device),
-                       torch.empty((rows, n_q_heads, max_splits, 2), dtype=torch.float32, device=qkv.device))
-            batch.scratch[key] = scratch
-        partial_out, partial_ml = scratch
+        partial_out, partial_ml = _split_scratch(batch, n_q_heads, head_dim, split_len, max_splits, qkv.device)
     page_size = k_pages.shape[2]
     flag = wait_error_flag(qkv.device).data_ptr()
     if run_portions and prefill_tcgen05_supported(head_dim, n_q_heads, n_kv_heads, page_size):
@@ -269,14 +274,7 @@ def try_attention_precise(qkv, q_stride, batch, block_tables, k_pages, v_pages, 
     out = torch.empty((batch.n_tokens, n_q_heads * value_dim), dtype=torch.bfloat16, device=qkv.device)
     partial_out = partial_ml = None
     if run_decode and max_splits > 1:
-        key = ("attention_mma_scratch", n_q_heads, value_dim, max_splits)
-        scratch = batch.scratch.get(key)
-        if scratch is None:
-            rows = batch.n_seqs if 0 < -split_len < max_splits else batch.n_tokens
-            scratch = (torch.empty((rows, n_q_heads, max_splits, value_dim), dtype=torch.float32, device=qkv.device),
-                       torch.empty((rows, n_q_heads, max_splits, 2), dtype=torch.float32, device=qkv.device))
-            batch.scratch[key] = scratch
-        partial_out, partial_ml = scratch
+        partial_out, partial_ml = _split_scratch(batch, n_q_heads, value_dim, split_len, max_splits, qkv.device)
     page_size = k_pages.shape[2]
     if run_portions and value_dim == head_dim and PRECISE_PREFILL_KERNEL == "tcgen05" and gate_pointer % 16 == 0 and gate_stride % 8 == 0 and \
             (bias_log2 is None or library().llm_attention_prefill_tcgen05_bias_fits(bias_log2.shape[1], n_q_heads // n_kv_heads)) and \

@@ -128,6 +128,31 @@ def test_parts_by_length(form, case, heads, dim):
     assert error.max() <= (2.0 ** -7 if form is not None else 2.0 ** -7 + 20 * 2.0 ** -9), f"{float(error.max()):.2e}"
 
 
+@pytest.mark.parametrize("q_lens,contexts,layers", [
+    ([100, 1, 1], [100, 1400, 1400], [(32, 8, 128, 128, 256), (32, 8, 64, 128, 0)]), ([512] + [1] * 13, [512] + [1500] * 13, [(32, 8, 64, 64, 0), (32, 4, 128, 64, 0)])])
+@pytest.mark.parametrize("turned", [False, True])
+def test_layers_of_other_kinds_in_one_step(q_lens, contexts, layers, turned):
+    """Two layers whose single tokens, behind a prompt portion, are divided by length in one and into equal parts of the cp.async kernel in
+    the other, with the same heads, value size and number of parts: each against the kernel for every size."""
+    from llmserver_b200 import ops
+    from llmserver_b200.ops.library import check_wait_errors
+    batch = HostBatch(q_lens, contexts)
+    batch.max_q_len = max(q_lens)
+    batch.seq_of_token = torch.repeat_interleave(torch.arange(len(q_lens), dtype=torch.int32), torch.tensor(q_lens)).to(DEVICE)
+    batch.positions = torch.cat([torch.arange(context - count, context) for context, count in zip(contexts, q_lens)]).to(torch.int32).to(DEVICE)
+    for seed, (heads, kv_heads, dim, value_dim, window) in enumerate(layers[::-1] if turned else layers):
+        qkv, q_stride, k_pages, _, tables = paged_case(seed, q_lens, contexts, heads, kv_heads, dim, 16, 2.0)
+        v_pages = torch.randn((*k_pages.shape[:3], value_dim), device=DEVICE).to(torch.bfloat16)
+        got = ops.attention(qkv, batch, tables, k_pages, v_pages, heads, kv_heads, dim, dim ** -0.5, window, value_dim, precise=True, q_stride=q_stride)
+        want = ops.attention_generic(qkv, q_stride, k_pages, v_pages, tables, batch.seq_of_token, batch.positions, heads, kv_heads, dim, dim ** -0.5,
+                                     window, value_dim=value_dim)
+        torch.cuda.synchronize()
+        check_wait_errors()
+        got, want = got.double(), want.double()
+        error = (got - want).abs() / torch.maximum(want.abs(), 0.05 * want.abs().amax(dim=-1, keepdim=True))
+        assert error.max() <= 2.0 ** -7, f"{float(error.max()):.2e}"      # as in the first test
+
+
 @pytest.mark.parametrize("dim", [64, 128])
 @pytest.mark.parametrize("precise", [False, True])
 @pytest.mark.parametrize("contexts", [[900], [3000, 700]])
