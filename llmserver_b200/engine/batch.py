@@ -97,6 +97,10 @@ class StepBatch:
     # kernel launched just before them.  True for every batch packed here; a hand-made batch that fills the cache and
     # reads it in the same breath must say False.
     keys_settled: bool = True
+    # The same of the recurrent states in the step's slots, which a layer does not add to but replaces: true only where every
+    # layer runs once on this batch, as the engine's steps do (they say so); whoever runs a layer or a kernel twice on one batch, and
+    # so reads what the first run wrote, does not.
+    states_settled: bool = False
 
 
 def layout_of(slices: List[SequenceSlice], n_groups: int, min_table_width: int = 1) -> BatchLayout:

@@ -143,6 +143,7 @@ class DecodeGraph:
         shape_only = [SequenceSlice(index, [0], max_context - 1, [0], [[0] * table_width] * n_groups, 0)
                       for index in range(batch_size)]
         self.batch = views(self.buffer, self.layout, shape_only)
+        self.batch.states_settled = True      # a replay begins with the batch's copy and runs every layer once
         self.answer = torch.zeros(batch_size + 2, dtype=torch.int32, pin_memory=True)
         self.answer_view = self.answer.numpy()
         self.graph = torch.cuda.CUDAGraph()

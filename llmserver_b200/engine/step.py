@@ -112,6 +112,7 @@ class StepFunction:
         """Runs one step; returns logits [wanted, vocab] (float32) in the order of the entries and of
         their wanted places."""
         batch = self.prepare(entries)
+        batch.states_settled = True      # this step is all that runs on the batch
         logits = self.model.step(batch)
         self.pending_flags.append(batch.error_flag)
         self._advance(entries)
@@ -150,6 +151,7 @@ class StepFunction:
             batch = build_batch(slices, len(self.cache.groups), self.device, self.model.spec.vocab_size, sampling=sampling)
             packed = clock()
             self.last_batch_bytes = batch.host_bytes
+            batch.states_settled = True
             logits = self.model.step(batch)
             if not sampling:
                 self.pending_flags.append(batch.error_flag)

@@ -562,7 +562,8 @@ def gla_supported(dim: int, value_dim: int) -> bool:
 
 def gla_recurrent(proj: torch.Tensor, q_column: int, k_column: int, v_column: int, g_column: int, z: torch.Tensor,
                   z_bias: Optional[torch.Tensor], weight: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: int,
-                  value_dim: int, tau: float, q_scale: float, eps: float, segment: Optional[int] = None) -> torch.Tensor:
+                  value_dim: int, tau: float, q_scale: float, eps: float, segment: Optional[int] = None,
+                  settled: bool = False) -> torch.Tensor:
     """The gated-linear-attention recurrence over a step's tokens, sequence by sequence, from and into each sequence's
     slot of ``state`` (float32 [slots, heads, dim, value_dim]):
 
@@ -574,7 +575,12 @@ def gla_recurrent(proj: torch.Tensor, q_column: int, k_column: int, v_column: in
 
     ``segment``: tokens per segment of the form that walks a long portion's segments in parallel (two passes and a scan
     between them; results equal to rounding).  None: chosen here, for bfloat16 steps whose longest portion spans several
-    segments; 0: always the one-pass form, which is also what the 32-bit path runs."""
+    segments; 0: always the one-pass form, which is also what the 32-bit path runs.
+
+    ``settled``: the caller vouches that everything that wrote ``state`` was complete when the copy of this batch to the device began
+    (a kernel launched just before this one lets it start early); single tokens then ask for it without waiting for that kernel.
+    LLMSERVER_B200_DECODE_EARLY_KEYS=0 switches it off, as it does for cached keys."""
+    from .attention_bf16 import EARLY_KEYS
     check(proj, "packed projection")
     tokens, row_width = proj.shape
     check(z, "decay projection", torch.float32, heads * dim)
@@ -606,7 +612,7 @@ def gla_recurrent(proj: torch.Tensor, q_column: int, k_column: int, v_column: in
          z.data_ptr(), pointer(z_bias), weight.data_ptr(), state.data_ptr(), batch.state_slots.data_ptr(), batch.q_start.data_ptr(),
          out.data_ptr(), batch.n_seqs, int(heads), int(dim), int(value_dim), 1.0 / float(tau), float(q_scale), float(eps),
          dtype_code(proj.dtype), dtype_code(weight.dtype), int(segment), int(segments), pointer(segment_state), pointer(segment_decay),
-         int(longest == 1), int(getattr(batch, "keys_settled", False)), stream_handle())
+         int(longest == 1), int(settled and EARLY_KEYS), stream_handle())
     return out
 
 

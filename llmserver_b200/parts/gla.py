@@ -77,5 +77,6 @@ class GatedLinearAttention(Mixer):
         z = ops.linear_wide(ops.linear(x, self.decay_in), self.decay_out)      # 32-bit sums, never rounded to the activation type
         q_column, k_column, v_column, g_column = self.columns
         mixed = ops.gla_recurrent(proj, q_column, k_column, v_column, g_column, z, self.decay_bias, self.norm, cache.state,
-                                  batch, self.heads, self.dim, self.value_dim, self.tau, self.dim ** -0.5, self.eps)
+                                  batch, self.heads, self.dim, self.value_dim, self.tau, self.dim ** -0.5, self.eps,
+                                  settled=getattr(batch, "states_settled", False))
         return ops.linear(mixed, self.out)

@@ -480,6 +480,30 @@ def test_linear_attention_in_tiles(vdim, wide_weight, bias, segment, lengths):
         at += n
 
 
+@pytest.mark.parametrize("vdim", [64, 128])
+def test_launches_one_after_the_other_on_one_state(vdim):
+    """Six launches of single tokens in a row on one batch and one state, with nothing between them: each reads what the one in front
+    has left."""
+    from llmserver_b200 import ops
+    from llmserver_b200.engine.batch import SequenceSlice, build_batch
+    heads, dim, count, rounds = 32, 64, 64, 6
+    keys, values = heads * dim, heads * vdim
+    generator = torch.Generator().manual_seed(vdim)
+    proj = [torch.randn((count, 2 * keys + 2 * values), generator=generator).to(torch.bfloat16) for _ in range(rounds)]
+    z, before = torch.randn((count, keys), generator=generator), torch.randn((count, heads, dim, vdim), generator=generator)
+    batch = build_batch([SequenceSlice(s, [0], 0, [], [[0]], s) for s in range(count)], 1, DEVICE)
+    given, z_given, state, weight = [rows.to(DEVICE) for rows in proj], z.to(DEVICE), before.to(DEVICE), torch.ones(vdim, device=DEVICE)
+    torch.cuda.synchronize()
+    for rows in given:
+        ops.gla_recurrent(rows, 0, keys, 2 * keys, 2 * keys + values, z_given, None, weight, state, batch, heads, dim, vdim, 16.0, 1.0, 1e-5)
+    alpha, want = (torch.sigmoid(z.double()) ** (1.0 / 16.0)).view(count, heads, dim), before.double()
+    for rows in proj:
+        k, v = rows[:, keys:2 * keys].double().view(count, heads, dim), rows[:, 2 * keys:2 * keys + values].double().view(count, heads, vdim)
+        want = alpha[..., None] * want + k[..., None] * v[:, :, None, :]
+    # the state is 32-bit: six steps of 2^-24 on sums of about 20
+    assert torch.allclose(state.cpu().double(), want, atol=2e-5, rtol=2e-6)
+
+
 # ------------------------------------------------------------------------------------------------ whole models
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("name", NAMES)
