@@ -167,9 +167,11 @@ class DecodeGraph:
         packed = clock()
         self.graph.replay()
         launched = clock()
-        if self.meanwhile is not None:
-            self.meanwhile()
-        torch.cuda.current_stream(self.buffer.device).synchronize()
+        try:
+            if self.meanwhile is not None:
+                self.meanwhile()
+        finally:      # whatever happened there: the graph may still be reading the buffer that the next step rewrites
+            torch.cuda.current_stream(self.buffer.device).synchronize()
         result = self.answer_view.tolist()
         if phases is not None:
             phases.update(pack_copy=packed - self.began, launch=launched - packed, read_back=clock() - launched)

@@ -3,13 +3,15 @@ name every row's real pages on every step, also after a request was preempted, r
 back into the same row under the same id."""
 import random
 import time
+from types import SimpleNamespace
 
 import numpy as np
+import pytest
 import torch
 
 from llmserver_b200.engine.batch import SequenceSlice
 from llmserver_b200.engine.engine import Engine
-from llmserver_b200.engine.graphs import DecodeGraphs, DecodeRows
+from llmserver_b200.engine.graphs import DecodeGraph, DecodeGraphs, DecodeRows
 from llmserver_b200.sampling import SamplingRow
 from stubs import VOCAB, StubModel, expected_generation
 
@@ -46,6 +48,28 @@ def test_same_id_with_other_pages_is_packed_again():
     off = rows.layout.offsets
     assert rows.host_view[off["positions"]:off["positions"] + 4].tolist() == [8, 8, 11, 0]
     assert rows.host_view[off["context_len"]:off["context_len"] + 4].tolist() == [9, 9, 12, 1]
+
+
+def test_a_replay_is_waited_for_whatever_happens_meanwhile(monkeypatch):
+    """The next step rewrites the buffer that the replayed copy reads: no way out of a replay leaves it running."""
+    order = []
+    stream = SimpleNamespace(synchronize=lambda: order.append("waited"))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: stream)
+    graph = object.__new__(DecodeGraph)
+    graph.rows = DecodeRows(batch_size=1, n_groups=1, table_width=2, vocab_size=10, null_pages=[3])
+    graph.graph = SimpleNamespace(replay=lambda: order.append("replayed"))
+    graph.buffer, graph.answer_view = torch.zeros(1), np.array([7, 0, 0], dtype=np.int32)
+    step = [SequenceSlice("A", [5], 1, [0], [[1]])]
+    graph.meanwhile = lambda: order.append("meanwhile")
+    assert graph.run(step, [SamplingRow()]) == [7, 0, 0] and order == ["replayed", "meanwhile", "waited"]
+
+    def fails():
+        raise ValueError("bookkeeping")
+
+    graph.meanwhile = fails
+    with pytest.raises(ValueError, match="bookkeeping"):
+        graph.run(step, [SamplingRow()])
+    assert order[3:] == ["replayed", "waited"]
 
 
 class HostStep:
