@@ -54,7 +54,11 @@ def _row_bucket(rows: int) -> int:
 # The choices can be kept in a file (LLMSERVER_B200_GEMM_PLAN): what is in the file is used as it is, what is
 # measured is added to it.  The choice fixes the order in which a product's partial sums are added, so two processes
 # that read the same file give bit-identical bfloat16 results; without a file each process measures for itself and a
-# close race may go either way.
+# close race may go either way.  The first line of a file that was written here names the revision of the kernels that its choices were
+# measured with: those of another revision are not read (and the file is written anew), since splits that were the fastest then
+# would stand in the way of the present ones for good.  A file without that line is somebody's own and is read.
+PLAN_REVISION = 2
+_PLAN_HEADER = "# row bucket,N,K,output,split of K (0: library product)"
 PLAN_FILE = os.environ.get("LLMSERVER_B200_GEMM_PLAN")
 _plan_loaded = False
 
@@ -69,7 +73,8 @@ def _key_text(key) -> str:
 
 
 def load_plan(path: Optional[str] = None) -> int:
-    """Reads choices from ``path`` (default: the file named by LLMSERVER_B200_GEMM_PLAN); returns how many."""
+    """Reads choices from ``path`` (default: the file named by LLMSERVER_B200_GEMM_PLAN); returns how many (none of a file that was
+    written for another revision of the kernels)."""
     global _plan_loaded
     _plan_loaded = True
     path = path or PLAN_FILE
@@ -79,6 +84,8 @@ def load_plan(path: Optional[str] = None) -> int:
     with open(path) as handle:
         for line in handle:
             line = line.strip()
+            if line.startswith(_PLAN_HEADER) and line != f"{_PLAN_HEADER}, revision {PLAN_REVISION}":
+                return 0
             if not line or line.startswith("#"):
                 continue
             try:
@@ -97,7 +104,7 @@ def save_plan(path: Optional[str] = None) -> None:
     path = path or PLAN_FILE
     if not path:
         raise KernelError("no plan file was named (LLMSERVER_B200_GEMM_PLAN)")
-    lines = ["# row bucket,N,K,output,split of K (0: library product)"]
+    lines = [f"{_PLAN_HEADER}, revision {PLAN_REVISION}"]
     lines += [f"{_key_text(key)},{split}" for key, split in sorted(_choice.items(), key=lambda item: _key_text(item[0]))]
     temporary = f"{path}.{os.getpid()}.tmp"
     with open(temporary, "w") as handle:
