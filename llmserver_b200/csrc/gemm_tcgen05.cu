@@ -52,7 +52,9 @@ constexpr int kTwoAtomRows = 64;    // up to this many tokens a stage of a block
                                     // atom is as large as a weight atom) one: three stages of 32 KiB then leave room for two blocks per SM
 constexpr int kThreeBlocksKib = 74; // ring of a block that shares its SM with two others
 constexpr int kOneBlockKib = 200;   // ring of a block that has its SM to itself
-constexpr int kTurn = 7;            // blocks of K from where a tile begins to where the next one does (odd: shares are often a power of two)
+constexpr int kTurn = 7;            // beyond 16 tokens: blocks of K from where a tile begins to where the next one does (odd: shares are often
+                                    // a power of two)
+constexpr int kTurnTiles = 8;       // up to so many tiles all begin at the start
 constexpr int kThreads = 256;       // at most: four warps up to 16 tokens, eight beyond (two have a role in the main
                                     // loop, all work in the epilogue, whose time per token is instruction issue)
 constexpr int kMaxStages = 12;
@@ -546,10 +548,13 @@ __global__ void __launch_bounds__(kThreads, PER_SM) gemm_small_m_kernel(const __
     const int kb_begin = (int)((long long)total_kb * rank / p.split);
     const int kb_end = (int)((long long)total_kb * (rank + 1) / p.split);
     const int n_kb = kb_end - kb_begin;
-    // Every tile begins at another place of its share of K and comes back to the share's start: blocks that walk K in step read the
-    // same columns of thousands of rows at a time, which lie on few of the memory's channels (q/k/v of the 8B shape in four parts, us,
-    // in step / turned: 11.8 / 11.3 at 8 tokens, 14.3 / 13.8 at 61, 17.1 / 16.6 at 119; gate/up unsplit at 119 42.0 / 40.7).
-    const int turn = n_kb > 0 ? tile * kTurn % n_kb : 0;
+    // MANY: every tile begins at another place of its share of K and comes back to the share's start: blocks that walk K in step
+    // read the same columns of thousands of rows at a time, which lie on few of the memory's channels (q/k/v of the 8B shape in four
+    // parts, us, in step / turned: 14.3 / 13.8 at 61 tokens, 17.1 / 16.6 at 119; gate/up unsplit at 119 42.0 / 40.7; a step of 21
+    // sequences of the 14B shape 6168 / 6103, of 64 of the Dikusun shape 953 / 945).  A few tiles share nothing that matters.  Up to 16
+    // tokens all tiles add in the order of K: a step of one sequence of the 8B shape takes 3017 us that way and 3023 turned, of
+    // eight 3537 and 3530, which is as far as two runs differ.
+    const int turn = MANY && n_kb > 0 && (int)gridDim.x > kTurnTiles * p.split ? tile * kTurn % n_kb : 0;
     auto turned = [&](int i) { const int kb = i + turn; return kb >= n_kb ? kb - n_kb : kb; };
 
     if (threadIdx.x == 0) {

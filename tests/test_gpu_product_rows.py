@@ -53,11 +53,28 @@ def test_three_blocks_an_sm(rows, tiles, inner, split):
     close(parts[:, :rows].sum(0), (want * want).sum(-1), torch.float32, "sums of squares", factor=4.0)
 
 
+@pytest.mark.parametrize("rows", [1, 8, 16])
+@pytest.mark.parametrize("split", [1, 3, 8])
+def test_few_rows_add_in_the_order_of_k(rows, split):
+    """Up to 16 rows a feature's sum does not depend on the tile that it lies in: tiles of equal weights give equal bits."""
+    from llmserver_b200.ops import gemm_bf16
+    from llmserver_b200.ops.library import call, check_wait_errors, stream_handle
+    tiles, inner = 9, 4096
+    x, w = rand((rows, inner), torch.bfloat16, 1), rand((128, inner), torch.bfloat16, 2, inner ** -0.5).repeat(tiles, 1)
+    out = torch.full((rows, tiles * 128), float("nan"), dtype=torch.float32, device=DEVICE)
+    call("llm_gemm_small_m", x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, tiles * 128, inner, tiles * 128, 1, split, *gemm_bf16.NO_SCALE,
+         gemm_bf16.error_flag(DEVICE).data_ptr(), stream_handle())
+    torch.cuda.synchronize()
+    check_wait_errors()
+    for tile in range(1, tiles):
+        assert torch.equal(out[:, tile * 128:(tile + 1) * 128], out[:, :128])
+
+
 @pytest.mark.parametrize("rows", [16, 17, 64, 65, 128])
 @pytest.mark.parametrize("tiles,inner,split", [(148, 136, 1), (149, 136, 1), (33, 1032, 4), (34, 1032, 4), (3, 200, 2), (22, 520, 6)])
 def test_one_block_an_sm(rows, tiles, inner, split):
-    """Launches around one block per SM, which run a long ring of two-atom stages beyond 16 rows; every tile begins at another place of
-    its share of K."""
+    """Launches around one block per SM, which run a long ring of two-atom stages beyond 16 rows, where the
+    tiles begin at different places of their shares of K."""
     from llmserver_b200.ops import gemm_bf16
     from llmserver_b200.ops.library import call, check_wait_errors, stream_handle
     cols = tiles * 128 - 126
