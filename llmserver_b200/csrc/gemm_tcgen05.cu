@@ -880,10 +880,19 @@ static RowScale row_scale_of(const float* parts, int n_parts, int stride, float 
 }
 
 // How many clusters of `split` blocks that each fill an SM's shared memory the device holds at a time (a cluster lies within a group of
-// SMs, so that it can be fewer than SMs / split), 0 where it cannot say.  Asked once per size of cluster.
+// SMs, so that it can be fewer than SMs / split), 0 where it cannot say.  Asked once per device and size of cluster; what could not be
+// said is asked again.
 static int lone_clusters(int split) {
-    static std::atomic<int> known[kMaxSplit + 1];      // 1 + answer
-    if (const int answer = known[split].load(std::memory_order_relaxed)) return answer - 1;
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices][kMaxSplit + 1];      // the answer; 0: none yet
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    const bool kept = device < kDevices;
+    if (kept)
+        if (const int answer = known[device][split].load(std::memory_order_relaxed)) return answer;
     void (*kernel)(CUtensorMap, CUtensorMap, GemmParams) = gemm_small_m_kernel<2, true, 2>;
     const size_t shared = (size_t)kOneBlockKib * 1024 + 1024;
     int clusters = 0;
@@ -905,7 +914,8 @@ static int lone_clusters(int split) {
             clusters = 0;
         }
     }
-    known[split].store(1 + clusters, std::memory_order_relaxed);
+    if (clusters < 0) clusters = 0;
+    if (kept) known[device][split].store(clusters, std::memory_order_relaxed);
     return clusters;
 }
 
