@@ -51,6 +51,7 @@ constexpr int kMaxRows = 128;       // tokens per launch
 constexpr int kTwoAtomRows = 64;    // up to this many tokens a stage of a block that shares its SM holds two atoms of K, beyond (where a token
                                     // atom is as large as a weight atom) one: three stages of 32 KiB then leave room for two blocks per SM
 constexpr int kThreeBlocksKib = 74; // ring of a block that shares its SM with two others
+constexpr int kTwoBlocksKib = 100;  // of one that shares it with one other
 constexpr int kOneBlockKib = 200;   // ring of a block that has its SM to itself
 constexpr int kTurn = 7;            // beyond 16 tokens: blocks of K from where a tile begins to where the next one does (odd: shares are often
                                     // a power of two)
@@ -924,6 +925,18 @@ LLM_EXPORT int llm_gemm_small_m_one_per_sm(int n, int split) {
     return split >= 1 && split <= kMaxSplit && (n + kBlockRows - 1) / kBlockRows <= lone_clusters(split);
 }
 
+// KiB of a block's ring of stages when `per_sm` blocks share an SM: LLMSERVER_B200_GEMM_RING_KIB where it is set (three blocks an SM: no
+// more than fits).
+LLM_EXPORT int llm_gemm_small_m_ring_kib(int per_sm) {
+    static const int asked = [] {
+        const char* value = getenv("LLMSERVER_B200_GEMM_RING_KIB");
+        const int kib = value ? atoi(value) : 0;
+        return value == nullptr ? 0 : kib < 32 ? 32 : kib > kOneBlockKib ? kOneBlockKib : kib;
+    }();
+    const int own = per_sm >= 3 ? kThreeBlocksKib : per_sm == 2 ? kTwoBlocksKib : kOneBlockKib;
+    return asked == 0 || (per_sm >= 3 && asked > own) ? own : asked;
+}
+
 static int small_m_launch(const void* x, const void* w, void* out, int m, int n, int k, int ldc, int out_is_f32,
                           int requested_split, int* error_flag, const RopeEpilogue* rope, cudaStream_t stream,
                           int silu_gate, const RowScale& scale, const StreamEpilogue* stream_out = nullptr) {
@@ -983,16 +996,9 @@ static int small_m_launch(const void* x, const void* w, void* out, int m, int n,
     const size_t a_bytes = (size_t)kBlockRows * kAtomK * 2;
     const size_t b_bytes = ((size_t)p.token_pad * kAtomK * 2 + 1023) & ~(size_t)1023;
     const size_t stage_bytes = atoms * (a_bytes + b_bytes);
-    // The ring of stages (about 100 KiB: two CTAs fit on an SM) lets a CTA that was launched early, while the kernels
+    // The ring of stages (about 100 KiB where two CTAs share an SM) lets a CTA that was launched early, while the kernels
     // before it still run, request that many bytes of weights before it has to wait for its input.
-    static int ring_kib = -1;
-    if (ring_kib < 0) {
-        const char* value = getenv("LLMSERVER_B200_GEMM_RING_KIB");
-        ring_kib = value ? atoi(value) : 100;
-        if (ring_kib < 32) ring_kib = 32;
-        if (ring_kib > 200) ring_kib = 200;
-    }
-    const int my_kib = three && ring_kib > kThreeBlocksKib ? kThreeBlocksKib : alone ? kOneBlockKib : ring_kib;
+    const int my_kib = llm_gemm_small_m_ring_kib(three ? 3 : alone ? 1 : 2);
     int stages = (int)((size_t)my_kib * 1024 / stage_bytes);
     if (stages < 1) stages = 1;
     if (stages > kMaxStages) stages = kMaxStages;

@@ -75,6 +75,7 @@ SIGNATURES = {
     "llm_attention_prefill_tcgen05_precise": [_P, _I, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _I, _P, _P, _I, _P, _I, _I, _P, _I, _S],
     "llm_attention_prefill_wide_supports": [_I, _I, _I, _I],
     "llm_attention_prefill_wide": [_P, _I, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _I, _P, _S],
+    "llm_gemm_small_m_ring_kib": [_I],
     "llm_gemm_small_m_supports": [_I, _I, _I],
     "llm_gemm_small_m": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _F, _P, _S],
     "llm_gemm_into_stream_parts": [_I],

@@ -1,4 +1,7 @@
-"""Saved choices of the matrix products, without a GPU."""
+"""Saved choices of the matrix products and the size of their kernel's ring, without a GPU."""
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -38,3 +41,17 @@ def test_lines_that_are_no_choices_are_refused(choices, tmp_path):
     path.write_text("8,4096,4096\n")
     with pytest.raises(KernelError):
         gemm_bf16.load_plan(str(path))
+
+
+@pytest.mark.parametrize("asked,want", [(None, [200, 100, 74]), ("64", [64, 64, 64]), ("120", [120, 120, 74]), ("8", [32, 32, 32]), ("999", [200, 200, 74])])
+def test_ring_size_that_was_asked_for(asked, want):
+    """LLMSERVER_B200_GEMM_RING_KIB holds for blocks that have an SM to themselves, share it with one other, and with two (as far as
+    three fit)."""
+    script = "from llmserver_b200.ops.library import library; print([library().llm_gemm_small_m_ring_kib(n) for n in (1, 2, 3)])"
+    env = {key: value for key, value in os.environ.items() if key != "LLMSERVER_B200_GEMM_RING_KIB"}
+    if asked is not None:
+        env["LLMSERVER_B200_GEMM_RING_KIB"] = asked
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, cwd=root, env=dict(env, PYTHONPATH=root), timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
+    assert done.stdout.split("\n")[-2] == str(want)
