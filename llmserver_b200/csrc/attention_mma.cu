@@ -85,7 +85,7 @@ struct AttnParams {
     int by_length = 0;              // TMA decode kernel: blocks take the sequences longest first (up to kThreads of them)
     int balance = 0;                // TMA decode kernel: > 0: long sequences are divided into more parts than short ones, so that no
                                     // more than this many parts per kv head are made (see part_of_block)
-    int* part_counters = nullptr;   // balance: [S, Hkv], zero before and after: parts of a sequence that have left their result
+    int* part_counters = nullptr;   // balance: [S, Hkv, 4], zero before and after: parts of which a warp has left its heads' results
 };
 
 // The first key that the query at `position` may see.
@@ -1110,50 +1110,64 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
         }
     }
     if constexpr (BALANCE) {
-        if (n_splits == 1) return;
-        // The part that comes last adds all of them, in their order and with the merge kernel's arithmetic: what the others left
-        // lies in L2.  (Clusters with a rank for every part that there could be keep the places of ranks without a part
-        // until the whole cluster ends: 32 sequences of 3072 keys in clusters of two, one rank idle, 6.86 ms a step against 5.56.)
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        int* counter = p.part_counters + (size_t)seq * p.n_kv_heads + kv_head;
-        if (threadIdx.x == 0)      // releases what the barrier has put in front of it, acquires what the other parts released
-            asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(place_of) : "l"(counter) : "memory");
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (place_of != n_splits - 1) return;
-        if (threadIdx.x == 0) *counter = 0;
-        constexpr int kMaxParts = 8;
-        for (int index = 2 * threadIdx.x; index < group * D; index += 2 * kThreads) {
-            const int r = index / D, d = index % D, head = kv_head * group + r;
+        if (n_splits == 1 || warp >= group) return;
+        // What the parts have left for a warp's heads is added, in their order and with the merge kernel's arithmetic, by that warp of
+        // the part whose warp comes last; the others' results lie in L2.  A warp counts for itself and asks for a head's parts at
+        // once: a step of the 8B shape at equal contexts of 3072 keys, us, when the block's four warps waited for one another and
+        // asked twice / this way: 24 sequences 5097 / 5043, 32 sequences 5549 / 5461.  (Clusters with a rank for every part that
+        // there could be keep the places of ranks without a part until the whole cluster ends: 32 sequences of 3072
+        // keys in clusters of two, one rank idle, 6.86 ms a step against 5.56.)
+        __syncwarp();
+        int* counter = p.part_counters + ((size_t)seq * p.n_kv_heads + kv_head) * 4 + warp;
+        int before = 0;
+        if (lane == 0)      // releases what the warp has written, acquires what the other parts' warps released
+            asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+        before = __shfl_sync(0xffffffffu, before, 0);
+        __syncwarp();
+        if (before != n_splits - 1) return;
+        if (lane == 0) *counter = 0;
+        constexpr int kMaxParts = 8, kPairs = D / 64;      // pairs of neighbouring elements that a lane adds
+        for (int r = warp; r < group; r += 4) {
+            const int head = kv_head * group + r;
             const size_t slot0 = ((size_t)(p.slot_by_seq ? seq : token) * p.n_q_heads + head) * p.max_splits;
-            float2 statistics[kMaxParts], outputs[kMaxParts];
+            float2 statistics[kMaxParts], outputs[kMaxParts][kPairs];
 #pragma unroll
             for (int s = 0; s < kMaxParts; ++s) {
                 statistics[s] = s < n_splits ? __ldcg(reinterpret_cast<const float2*>(p.partial_ml + (slot0 + s) * 2)) : make_float2(-INFINITY, 0.0f);
-                outputs[s] = s < n_splits ? __ldcg(reinterpret_cast<const float2*>(p.partial_out + (slot0 + s) * D + d)) : make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int i = 0; i < kPairs; ++i)
+                    outputs[s][i] = s < n_splits ? __ldcg(reinterpret_cast<const float2*>(p.partial_out + (slot0 + s) * D + 2 * lane + 64 * i)) : make_float2(0.0f, 0.0f);
             }
             float best = -INFINITY;
 #pragma unroll
             for (int s = 0; s < kMaxParts; ++s) best = fmaxf(best, statistics[s].x);
-            float numerator[2] = {0.0f, 0.0f}, denominator = 0.0f;
+            float numerator[kPairs][2] = {}, denominator = 0.0f;
 #pragma unroll
             for (int s = 0; s < kMaxParts; ++s) {
                 if (s < n_splits) {
                     const float weight = statistics[s].y * exp2f(statistics[s].x - best);
-                    numerator[0] += outputs[s].x * weight;
-                    numerator[1] += outputs[s].y * weight;
+#pragma unroll
+                    for (int i = 0; i < kPairs; ++i) {
+                        numerator[i][0] += outputs[s][i].x * weight;
+                        numerator[i][1] += outputs[s][i].y * weight;
+                    }
                     denominator += weight;
                 }
             }
-            float result[2] = {numerator[0] / denominator, numerator[1] / denominator};
-            if constexpr (PRECISE) {
-                if (p.gate) {
-                    result[0] = gated(p, result[0], token, head * D + d);
-                    result[1] = gated(p, result[1], token, head * D + d + 1);
+#pragma unroll
+            for (int i = 0; i < kPairs; ++i) {
+                const int d = 2 * lane + 64 * i;
+                float result[2] = {numerator[i][0] / denominator, numerator[i][1] / denominator};
+                if constexpr (PRECISE) {
+                    if (p.gate) {
+                        result[0] = gated(p, result[0], token, head * D + d);
+                        result[1] = gated(p, result[1], token, head * D + d + 1);
+                    }
                 }
+                const size_t at = (size_t)token * p.n_q_heads * D + (size_t)head * D + d;
+                if constexpr (DIFF) *reinterpret_cast<float2*>(p.maps_out + at) = make_float2(result[0], result[1]);
+                else *reinterpret_cast<__nv_bfloat162*>(p.out + at) = __floats2bfloat162_rn(result[0], result[1]);
             }
-            const size_t at = (size_t)token * p.n_q_heads * D + (size_t)head * D + d;
-            if constexpr (DIFF) *reinterpret_cast<float2*>(p.maps_out + at) = make_float2(result[0], result[1]);
-            else *reinterpret_cast<__nv_bfloat162*>(p.out + at) = __floats2bfloat162_rn(result[0], result[1]);
         }
         return;
     }

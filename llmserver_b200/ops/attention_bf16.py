@@ -148,14 +148,14 @@ def plan(batch, group: int, n_kv_heads: int, device=None, blocks_per_sm: int = D
 
 
 def _part_counters(batch, n_kv_heads: int, split_len: int, max_splits: int, device) -> int:
-    """Where the parts of a (sequence, kv head) pair are counted when sequences are divided by their lengths: zero before and after
-    every launch, shared by the layers of a step.  0 when parts are equal."""
+    """Where the parts of a (sequence, kv head) pair are counted, by each of a block's four warps, when sequences are divided by their
+    lengths: zero before and after every launch, shared by the layers of a step.  0 when parts are equal."""
     if not 0 < -split_len < max_splits:
         return 0
     key = ("attention_part_counters", n_kv_heads)
     counters = batch.scratch.get(key)
     if counters is None:
-        counters = batch.scratch[key] = torch.zeros(batch.n_seqs * n_kv_heads, dtype=torch.int32, device=device)
+        counters = batch.scratch[key] = torch.zeros(4 * batch.n_seqs * n_kv_heads, dtype=torch.int32, device=device)
     return counters.data_ptr()
 
 
