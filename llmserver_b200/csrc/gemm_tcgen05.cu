@@ -6,14 +6,16 @@
 // So the roles of the operands are swapped for the hardware: a CTA owns 128 rows of W as the MMA's
 // M = 128 dimension and the (padded) token rows as its N dimension (16..128), walks its share of K in
 // blocks of 64 through a ring of shared-memory stages, and ends with a 128 x M tile of y^T in tensor
-// memory, which the epilogue writes transposed.  When N / 128 tiles are too few to fill 148 SMs, K is
+// memory, which the epilogue writes transposed.  (Beyond 16 tokens and a few tiles, each tile begins its walk at another place
+// of its share of K.)  When N / 128 tiles are too few to fill 148 SMs, K is
 // split across a thread-block cluster; the partial tiles are added through distributed shared memory in
 // a fixed order (rank 0, 1, ...), so results do not depend on timing.
 //
-// The epilogue moves the tile through shared memory as [token][128 rows] and hands whole token rows to warps: a
+// The epilogue moves the tile through shared memory as [token][128 rows] and hands whole token rows to warps, up to 16 tokens: a
 // token's 128 elements are four per lane, so per-head and per-row reductions are warp reductions, rotation partners
 // and gate/up pairs a shuffle away, stores 8 or 16 bytes per lane, and the warps work on different tokens
-// without a block barrier (per-token block barriers cost 9 to 14 us of a q/k/v product at 32 to 64 tokens).
+// without a block barrier (per-token block barriers cost 9 to 14 us of a q/k/v product at 32 to 64 tokens).  Beyond 16 tokens half
+// a warp takes a token, eight elements a lane, with rotation partners and gate/up pairs in one lane.
 //
 // One elected thread issues the TMA copies, one issues the MMAs; mbarriers carry "stage full" (TMA
 // transaction bytes), "stage free" and "accumulator ready" (tcgen05.commit).  The thread that initialises the
