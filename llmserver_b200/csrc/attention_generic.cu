@@ -1,7 +1,7 @@
 // Attention over the paged cache, any sizes, 32-bit arithmetic: the kernel of the true 32-bit path
 // and the fallback of the bfloat16 path for head sizes its tensor-core kernels refuse.
 //
-// One block of four warps per (query token, query head).  The query at absolute position p sees keys
+// A block of four warps per (query token, query head), or a warp where there are many.  The query at absolute position p sees keys
 // max(0, p - window + 1) .. p of its own sequence (window 0 = all), read through the sequence's
 // block table; the new tokens' keys are already in the cache when this runs.  Scores, the running
 // maximum, the normaliser and the output accumulate in 32-bit with the online-softmax recurrence
@@ -10,8 +10,8 @@
 // product (utils/architecture.py:105).
 //
 // Keys are visited 32 at a time from the first visible one, each lane owning one key's dot
-// product; warp w takes rounds w, w + 4, ... and the warps' results are merged in their order.  So the order of every sum
-// depends only on the query's position: the result for a token
+// product; part w of four takes rounds w, w + 4, ... and the parts are merged in their order, whether four warps make them or one.
+// So the order of every sum depends only on the query's position: the result for a token
 // is bit-identical however the prompt was cut into steps and whatever else is in the batch.
 //
 // Values may have another size than keys (`value_dim`; the output then has Hq * value_dim columns).  With `sinks`
@@ -72,9 +72,23 @@ __device__ __forceinline__ float row_dot(const float* q_row, const T* k_row, int
 // 150 keys, heads of 32 and 4 tokens a launch took 52 us when the loads were issued one by one and the accumulator had 16
 // columns for every size, and added 11.3 us to a replayed step when one warp walked all five rounds; with the rounds dealt to four
 // warps it adds 8.6.
-constexpr int kRoundWarps = 4;
-template <typename T, int COLUMNS, bool VECTOR>
-__global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_pages,
+//
+// LONE: a warp makes all four parts of its (token, head), round after round, and keeps each part's sums.  Four warps per pair only help
+// while the GPU has room for them and a pair has rounds for all: with many pairs they crowd each other out of the L1 cache (the more,
+// the wider the values) and merge through shared memory for nothing, and at a prompt's first positions most have no round.  us a
+// launch, four warps / one; 32-bit prompts of 6 heads of 32: 128 tokens 8.7 / 11.8, 683 95 / 105, 2048 722 / 703, 4096 2823 / 2594,
+// 2048 behind a window of 64 keys 74 / 44; 16 heads of 64: 128 tokens 24 / 35, 512 222 / 232, 2048 3187 / 2961; 32 heads of 128: 32
+// tokens 17.7 / 11.3, 32 behind 1000 278 / 372, 96 behind 1000 717 / 605, 512 879 / 773; 8 heads of 192: 2048 tokens 8096 / 4755;
+// bfloat16, 32 heads of 96: 32 tokens behind 4000 688 / 1054, 64 1362 / 1283, 1024 2192 / 1448.  Held to six blocks an SM (with values
+// of up to 128) the one-warp form is 2 to 20 % faster than left alone.
+constexpr int kParts = 4;
+constexpr int kManySums = 8192;       // pairs x columns from which a warp makes all parts
+constexpr int kFewKeys = 64, kManyShortPairs = 2048;      // the same with no more than two rounds: from so many pairs; with one: always
+// Two parts' sums, each times what the common maximum makes of its own.
+__device__ __forceinline__ float merged(float a, float a_weight, float b, float b_weight) { return fmaf(a, a_weight, b * b_weight); }
+
+template <typename T, int COLUMNS, bool VECTOR, bool LONE>
+__global__ void __launch_bounds__(kParts * 32, !LONE ? 1 : COLUMNS <= 4 ? 6 : COLUMNS == 8 ? 4 : 3) attention_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_pages,
                                          const T* __restrict__ v_pages, const int* __restrict__ block_tables,
                                          int max_blocks, const int* __restrict__ seq_of_token,
                                          const int* __restrict__ positions, T* __restrict__ out, int n_q_heads,
@@ -84,40 +98,66 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
                                          const T* __restrict__ gate, int gate_stride, int* __restrict__ error_flag) {
     constexpr int kAhead = COLUMNS >= 16 ? 2 : 32 / COLUMNS;      // value rows in flight: 32 registers per lane
     pdl_trigger();   // let the next kernel start launching
-    extern __shared__ float q_shared[];  // [head_dim], then what warps 1 .. 3 leave: [3][maximum, normaliser, 32 * COLUMNS sums]
+    // LONE: [4][head_dim]; else [head_dim], then what warps 1 .. 3 leave: [3][maximum, normaliser, 32 * COLUMNS sums]
+    extern __shared__ float q_shared[];
     const int token = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int head = blockIdx.y;
+    const int head = LONE ? blockIdx.y * kParts + warp : blockIdx.y;
+    if (LONE && head >= n_q_heads) return;
     const int kv_head = head / (n_q_heads / n_kv_heads);
     // A step's positions and block tables come from the host, or from a kernel that does not let its successors start early: they
     // are complete when this kernel starts, and are asked for while the kernel in front still runs.
     const int position = positions[token];
     const int* table = block_tables + (size_t)seq_of_token[token] * max_blocks;
 
-    float* q_row = q_shared;
+    float* q_row = q_shared + (LONE ? warp * head_dim : 0);
 
-    float accumulator[COLUMNS];
+    // of the parts that this warp makes; the part whose round comes next is in front
+    constexpr int kHeld = LONE ? kParts : 1;
+    float accumulators[kHeld][COLUMNS], maxima[kHeld], normalisers[kHeld];
 #pragma unroll
-    for (int i = 0; i < COLUMNS; ++i) accumulator[i] = 0.0f;
-    float running_max = -INFINITY, normaliser = 0.0f;
+    for (int h = 0; h < kHeld; ++h) {
+        maxima[h] = -INFINITY, normalisers[h] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < COLUMNS; ++i) accumulators[h][i] = 0.0f;
+    }
+    float (&accumulator)[COLUMNS] = accumulators[0];
+    float &running_max = maxima[0], &normaliser = normalisers[0];
+    auto next_part = [&] {
+        if constexpr (LONE) {
+            const float front_max = maxima[0], front_normaliser = normalisers[0];
+#pragma unroll
+            for (int h = 0; h + 1 < kHeld; ++h) maxima[h] = maxima[h + 1], normalisers[h] = normalisers[h + 1];
+            maxima[kHeld - 1] = front_max, normalisers[kHeld - 1] = front_normaliser;
+#pragma unroll
+            for (int i = 0; i < COLUMNS; ++i) {
+                const float front = accumulators[0][i];
+#pragma unroll
+                for (int h = 0; h + 1 < kHeld; ++h) accumulators[h][i] = accumulators[h + 1][i];
+                accumulators[kHeld - 1][i] = front;
+            }
+        }
+    };
 
     int first = (window > 0 && position - window + 1 > 0) ? position - window + 1 : 0;
     if (chunk > 0) first = max(first, position / chunk * chunk);
     const int kept = min(keep, first);      // keys 0 .. kept - 1, then first .. position
     const int count = kept + position - first + 1;
     auto key_of = [&](int index) { return index < kept ? index : first + index - kept; };
-    const int mine = 32 * warp + lane;
-    int next_page = mine < count ? table[key_of(mine) / page_size] : 0;
+    constexpr int kStride = LONE ? 32 : 32 * kParts;
+    const int first_base = LONE ? 0 : 32 * warp;
+    int next_page = first_base + lane < count ? table[key_of(first_base + lane) / page_size] : 0;
     pdl_wait();      // everything before this kernel in the stream is complete and visible
     const T* q_src = q + (size_t)token * q_stride + (size_t)head * head_dim;
-    for (int i = threadIdx.x; i < head_dim; i += kRoundWarps * 32) q_row[i] = Num<T>::load(q_src + i);
-    __syncthreads();      // the query's row
-    for (int base = 32 * warp; base < count; base += 32 * kRoundWarps) {
+    for (int i = LONE ? lane : threadIdx.x; i < head_dim; i += kStride) q_row[i] = Num<T>::load(q_src + i);
+    if (LONE) __syncwarp();      // the query's row
+    else __syncthreads();
+    for (int base = first_base; base < count; base += kStride) {
         const int index = base + lane;
         const int key = key_of(index);
         const bool valid = index < count;
         int page = next_page;
-        if (index + 32 * kRoundWarps < count) next_page = table[key_of(index + 32 * kRoundWarps) / page_size];
+        if (index + kStride < count) next_page = table[key_of(index + kStride) / page_size];
         if (valid && (unsigned)page >= (unsigned)num_pages) {      // no page of the pool: report it, read page 0 instead
             if (error_flag) atomicExch(error_flag, 5);
             page = 0;
@@ -164,9 +204,23 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
             }
         }
         running_max = new_max;
+        next_part();
     }
     const int rounds = (count + 31) / 32;
-    if (rounds > 1) {      // warps 1 .. 3 leave what they have; warp 0 adds it in their order
+    if constexpr (LONE) {
+        for (int turn = rounds; turn % kParts != 0; ++turn) next_part();      // part 0 is in front again
+#pragma unroll
+        for (int other = 1; other < kParts; ++other) {
+            if (other >= rounds || (maxima[other] == -INFINITY && normalisers[other] == 0.0f)) continue;
+            const float new_max = fmaxf(running_max, maxima[other]);
+            const float correction = running_max == new_max ? 1.0f : expf(running_max - new_max);
+            const float weight = maxima[other] == new_max ? 1.0f : expf(maxima[other] - new_max);
+            normaliser = merged(normaliser, correction, normalisers[other], weight);
+#pragma unroll
+            for (int i = 0; i < COLUMNS; ++i) accumulator[i] = merged(accumulator[i], correction, accumulators[other][i], weight);
+            running_max = new_max;
+        }
+    } else if (rounds > 1) {      // warps 1 .. 3 leave what they have; warp 0 adds it in their order
         float* parts = q_shared + head_dim;
         constexpr int kPart = 2 + 32 * COLUMNS;
         if (warp > 0) {
@@ -180,20 +234,20 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
         }
         __syncthreads();
         if (warp == 0) {
-            for (int other = 1; other < kRoundWarps && other < rounds; ++other) {
+            for (int other = 1; other < kParts && other < rounds; ++other) {
                 const float* part = parts + (other - 1) * kPart;
                 if (part[0] == -INFINITY && part[1] == 0.0f) continue;
                 const float new_max = fmaxf(running_max, part[0]);
                 const float correction = running_max == new_max ? 1.0f : expf(running_max - new_max);
                 const float weight = part[0] == new_max ? 1.0f : expf(part[0] - new_max);
-                normaliser = normaliser * correction + part[1] * weight;
+                normaliser = merged(normaliser, correction, part[1], weight);
 #pragma unroll
-                for (int i = 0; i < COLUMNS; ++i) accumulator[i] = accumulator[i] * correction + part[2 + lane + 32 * i] * weight;
+                for (int i = 0; i < COLUMNS; ++i) accumulator[i] = merged(accumulator[i], correction, part[2 + lane + 32 * i], weight);
                 running_max = new_max;
             }
         }
     }
-    if (warp > 0) return;
+    if (!LONE && warp > 0) return;
     if (sinks) {      // one more term of the denominator; it has no value, so the sums only shrink
         const float sink = sinks[head];
         const float new_max = fmaxf(running_max, sink);
@@ -215,12 +269,13 @@ __global__ void attention_generic_kernel(const T* __restrict__ q, int q_stride, 
     }
 }
 
+// max_keys: no token has more keys than this (0: not known); it only decides between forms that give the same bits.
 LLM_EXPORT int llm_attention_generic(const void* q, int q_stride, const void* k_pages, const void* v_pages,
                                      const int* block_tables, int max_blocks, const int* seq_of_token,
                                      const int* positions, void* out, int n_tokens, int n_q_heads, int n_kv_heads,
                                      int head_dim, int value_dim, int page_size, int num_pages, float scale, int window,
                                      const float* sinks, int chunk, const float* bias, int bias_len, int keep, const void* gate, int gate_stride,
-                                     int* error_flag, int dtype, cudaStream_t stream) {
+                                     int max_keys, int* error_flag, int dtype, cudaStream_t stream) {
     if (n_tokens == 0) return LLM_OK;
     if (head_dim > ATTN_MAX_D || head_dim <= 0) {
         llm_set_error("attention_generic: head_dim %d is outside 1..%d", head_dim, ATTN_MAX_D);
@@ -242,19 +297,25 @@ LLM_EXPORT int llm_attention_generic(const void* q, int q_stride, const void* k_
         llm_set_error("attention_generic: a chunk of %d positions, a bias of %d distances or %d kept positions", chunk, bias_len, keep);
         return LLM_REFUSED;
     }
-    if (n_q_heads > 65535) {
+    if (n_q_heads > kParts * 65535) {
         llm_set_error("attention_generic: %d query heads are too many for one launch", n_q_heads);
         return LLM_REFUSED;
     }
-    dim3 grid(n_tokens, n_q_heads);
     const int columns = value_dim <= 32 ? 1 : value_dim <= 64 ? 2 : value_dim <= 128 ? 4 : value_dim <= 256 ? 8 : 16;
-    const size_t shared = ((size_t)head_dim + (kRoundWarps - 1) * (2 + 32 * columns)) * sizeof(float);
+    long long keys = max_keys > 0 ? max_keys : 1LL << 40;
+    if (window > 0) keys = min(keys, (long long)window + keep);
+    if (chunk > 0) keys = min(keys, (long long)chunk);
+    const long long pairs = (long long)n_tokens * n_q_heads;
+    const bool lone = pairs * columns >= kManySums || keys <= 32 || (keys <= kFewKeys && pairs >= kManyShortPairs) || n_q_heads > 65535;
+    const dim3 grid(n_tokens, lone ? (n_q_heads + kParts - 1) / kParts : n_q_heads);
+    const size_t shared = (lone ? (size_t)kParts * head_dim : (size_t)head_dim + (kParts - 1) * (2 + 32 * columns)) * sizeof(float);
     // key rows in 16-byte pieces where every row starts on such a boundary
     const int count = dtype == LLM_F32 ? 4 : 8;
     const bool vector = head_dim % count == 0 && aligned16(k_pages);
 #define LLM_GENERIC(COLUMNS)                                                                                                       \
-    LLM_DISPATCH_DTYPE(dtype, llm_launch(vector ? attention_generic_kernel<T, COLUMNS, true> : attention_generic_kernel<T, COLUMNS, false>, \
-                                         grid, kRoundWarps * 32, shared, stream, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages,     \
+    LLM_DISPATCH_DTYPE(dtype, llm_launch(lone ? (vector ? attention_generic_kernel<T, COLUMNS, true, true> : attention_generic_kernel<T, COLUMNS, false, true>) : \
+                                                vector ? attention_generic_kernel<T, COLUMNS, true, false> : attention_generic_kernel<T, COLUMNS, false, false>, \
+                                         grid, kParts * 32, shared, stream, (const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages,     \
                                          block_tables, max_blocks, seq_of_token, positions, (T*)out, n_q_heads, n_kv_heads, head_dim,       \
                                          value_dim, page_size, num_pages, scale, window, sinks, chunk, bias, bias_len, keep,                \
                                          (const T*)gate, gate_stride, error_flag))

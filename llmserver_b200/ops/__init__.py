@@ -242,7 +242,7 @@ def attention_generic(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_p
                       out: Optional[torch.Tensor] = None, error_flag: Optional[torch.Tensor] = None,
                       value_dim: Optional[int] = None, sinks: Optional[torch.Tensor] = None, chunk: int = 0,
                       bias: Optional[torch.Tensor] = None, keep: int = 0, gate: Optional[torch.Tensor] = None,
-                      gate_column: int = 0) -> torch.Tensor:
+                      gate_column: int = 0, max_keys: Optional[int] = None) -> torch.Tensor:
     """Causal (optionally windowed) attention of every token over its sequence's pages, 32-bit
     arithmetic.  ``q`` holds head h of token n at q[n * q_stride + h * D]; returns [N, Hq * Dv], Dv = ``value_dim``
     (default D).  ``sinks`` (float32 [Hq]): one more term exp(sinks[h]) in each head's softmax denominator.  ``chunk`` > 0:
@@ -250,7 +250,8 @@ def attention_generic(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_p
     is added to the scaled score of the key n positions back.  ``keep`` > 0: a windowed query also sees the sequence's first
     ``keep`` positions.  ``gate`` ([N, row], q's type): the result's element c of token n is multiplied by
     sigmoid(gate[n, gate_column + c]).  A block-table entry that names no page of the pool is not followed: page 0 is read instead and ``error_flag``
-    (default: the device's shared flag) is set to 5."""
+    (default: the device's shared flag) is set to 5.  ``max_keys``: no token's sequence is longer, where the caller knows; results do
+    not depend on it."""
     check(q, "q")
     tokens = positions.numel()
     value_dim = head_dim if value_dim is None else int(value_dim)
@@ -274,7 +275,7 @@ def attention_generic(q: torch.Tensor, q_stride: int, k_pages: torch.Tensor, v_p
          block_tables.data_ptr(), block_tables.shape[-1], seq_of_token.data_ptr(), positions.data_ptr(),
          out.data_ptr(), tokens, n_q_heads, n_kv_heads, head_dim, value_dim, k_pages.shape[2], k_pages.shape[0],
          float(scale), int(window), pointer(sinks), int(chunk), pointer(bias), 0 if bias is None else bias.shape[1],
-         int(keep) if window else 0, gate_pointer, gate_stride, (error_flag if error_flag is not None else wait_error_flag(q.device)).data_ptr(), dtype_code(q.dtype),
+         int(keep) if window else 0, gate_pointer, gate_stride, int(max_keys or 0), (error_flag if error_flag is not None else wait_error_flag(q.device)).data_ptr(), dtype_code(q.dtype),
          stream_handle())
     return out
 
@@ -1448,7 +1449,7 @@ def attention(qkv: torch.Tensor, batch, block_tables: torch.Tensor, k_pages: tor
             return result
     return attention_generic(qkv, q_stride, k_pages, v_pages, block_tables, batch.seq_of_token, batch.positions,
                              n_q_heads, n_kv_heads, head_dim, scale, window, value_dim=value_dim, sinks=sinks, chunk=chunk, bias=bias,
-                             keep=keep, gate=gate, gate_column=gate_column)
+                             keep=keep, gate=gate, gate_column=gate_column, max_keys=getattr(batch, "max_context", None))
 
 
 LOG2E = 1.4426950408889634

@@ -51,3 +51,39 @@ def test_attention_by_value_size(dtype, dim, value_dim):
 
     want = torch.cat([plain(q, k, v, c - n) for q, k, v, c, n in zip(queries, dense_k, dense_v, contexts, q_lens)])
     close(out, want, dtype, f"attention {dim, value_dim}")
+
+
+OPTIONS = [dict(), dict(window=70, keep=9), dict(chunk=50), dict(sinks=True, gate=True), dict(bias=True)]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim,value_dim", [(32, 32), (36, 33), (96, 128), (66, 257), (512, 512)])
+@pytest.mark.parametrize("options", OPTIONS, ids=lambda options: "-".join(options) or "plain")
+def test_many_tokens_give_the_bits_of_few(dtype, dim, value_dim, options):
+    """A launch of many (token, head) pairs, where a warp makes all parts of a pair, against launches of few, where four do: positions
+    with one round of 32 keys and with up to nine, scores of -inf (from a bias) in whole rounds."""
+    from llmserver_b200 import ops
+    heads, kv_heads, page_size, count, step = 36, 3, 8, 260, 14
+    assert count * heads >= 8192 > step * heads * 16      # as many columns as the widest values have
+    pages = -(-count // page_size)
+    k_pages, v_pages = rand((pages, kv_heads, page_size, dim), dtype, 1), rand((pages, kv_heads, page_size, value_dim), dtype, 2)
+    table = torch.randperm(pages, generator=torch.Generator().manual_seed(3)).to(torch.int32).view(1, -1).to(DEVICE)
+    q = rand((count, heads * dim), dtype, 4)
+    given = {key: value for key, value in options.items() if key in ("window", "keep", "chunk")}
+    if "sinks" in options:
+        given["sinks"] = torch.linspace(-2.0, 3.0, heads, device=DEVICE)
+    if "bias" in options:
+        given["bias"] = rand((heads, 200), torch.float32, 5)
+        given["bias"][:, 30:130] = -float("inf")
+    gate = rand((count, heads * value_dim), dtype, 6) if "gate" in options else None
+    positions, sequence = torch.arange(count, dtype=torch.int32, device=DEVICE), torch.zeros(count, dtype=torch.int32, device=DEVICE)
+
+    def run(first, last):
+        return ops.attention_generic(q[first:last].contiguous(), heads * dim, k_pages, v_pages, table, sequence[first:last].contiguous(),
+                                     positions[first:last].contiguous(), heads, kv_heads, dim, dim ** -0.5, value_dim=value_dim,
+                                     gate=None if gate is None else gate[first:last].contiguous(), **given)
+
+    many = run(0, count)
+    assert torch.isfinite(many).all()
+    for first in range(0, count, step):
+        assert torch.equal(run(first, min(count, first + step)), many[first:first + step])
