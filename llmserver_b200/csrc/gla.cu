@@ -16,7 +16,8 @@
 // and everything else that enters the recurrence in 32-bit; (2) every thread walks the sixteen tokens on its registers
 // and leaves its partial o; (3) the warps add the partitions' parts in a fixed order, normalise, gate and store.  The
 // order of every sum depends on the sizes alone, so a token's result does not depend on how the prompt was cut or on
-// what else is in the batch.
+// what else is in the batch.  (In bfloat16 steps with heads of 64 key channels the kernels further down run: there the states have the
+// same bits whichever of them made them in one pass, but o's sums have one order in steps of single tokens alone and another in steps with portions.)
 //
 // Long portions can also be walked segment by segment in parallel (`llm_gla_recurrent` with a segment length): pass A
 // runs every segment but the last from a zero state and leaves its end state and the product of its decays; a scan adds
@@ -192,7 +193,9 @@ __global__ void __launch_bounds__(RR == 128 ? 256 : 512, RR <= 16 ? 2 : 1) gla_r
 // What bounds the kernel above for long portions is its staging: a thread's loads of a batch of tokens wait for one another (up to
 // 16 in a row).  Here all of a batch is asked for at once, 16 bytes at a time.  2048 tokens of 32 heads of 64 / 128, us, the
 // kernel above / this: states of the segments 153 / 73, outputs 232 / 133 (tiles with loads one after the other: 148 and 254; outputs
-// with the gates read at a batch's end: 156; without two tokens in flight: 142, which would make the states' pass 82).
+// with the gates read at a batch's end: 156; without two tokens in flight: 142, which would make the states' pass 82).  The sizes of
+// this layer in the package are 64 / 128; a tile per thread of heads of 128 key channels would take other registers and was not
+// built, so they stay with the kernel above.
 constexpr int kTileDim = 64;
 
 // Eight bfloat16 numbers, times `scale`, as 32-bit numbers in shared memory.
