@@ -84,19 +84,21 @@ UNEVEN = [([4000] + [1] * 20, 0), ([64 * k + k % 3 - 1 for k in range(1, 34)], 0
 @pytest.mark.parametrize("form", [None, dict(), dict(sinks=True, gate=True), dict(window=300, keep=70)], ids=["narrow", "precise", "sinks-gate", "window"])
 @pytest.mark.parametrize("case", range(len(UNEVEN)))
 @pytest.mark.parametrize("heads,dim", [(32, 128), (10, 64)])
-def test_parts_by_length(form, case, heads, dim):
+@pytest.mark.parametrize("settled", [False, True])
+def test_parts_by_length(form, case, heads, dim, settled):
     """Sequences of unequal length on up to a wave of blocks: the longer ones are divided into more parts, and the part that comes
-    last adds them.  Three launches on the same counters give the same bits, and what the kernel for every size gives but for
-    the rounding of weights."""
+    last adds them.  Launches on the same counters give the same bits, and what the kernel for every size gives but for
+    the rounding of weights.  Settled: as an engine's step says, the older keys are read before the kernel in front, which writes
+    the newest, has ended; the bits are those of the plain order."""
     from llmserver_b200 import ops
     from llmserver_b200.ops import attention_bf16
     from llmserver_b200.ops.library import check_wait_errors
     contexts, portion = UNEVEN[case]
     kv_heads, page_size = (2 if len(contexts) > 37 else 8) if dim == 128 else 2, 16
-    q_lens = [1] * len(contexts) + ([portion] if portion else [])
-    contexts = contexts + ([portion + 77] if portion else [])
+    q_lens = ([portion] if portion else []) + [1] * len(contexts)
+    contexts = ([portion + 77] if portion else []) + contexts
     batch = HostBatch(q_lens, contexts)
-    batch.max_q_len = max(q_lens)
+    batch.max_q_len, batch.keys_settled = max(q_lens), False
     batch.seq_of_token = torch.repeat_interleave(torch.arange(len(q_lens), dtype=torch.int32), torch.tensor(q_lens)).to(DEVICE)
     batch.positions = torch.cat([torch.arange(context - count, context) for context, count in zip(contexts, q_lens)]).clamp_min(0).to(torch.int32).to(DEVICE)
     qkv, q_stride, k_pages, v_pages, tables = paged_case(case, q_lens, [max(c, 1) for c in contexts], heads, kv_heads, dim, page_size, 2.0)
@@ -107,8 +109,17 @@ def test_parts_by_length(form, case, heads, dim):
                                   span=attention_bf16.key_span(given["window"], 0, given.get("keep", 0)))
     singles = sum(count == 1 for count in q_lens)
     assert (0 < -planned[3] < planned[4]) == (296 // (singles * kv_heads) <= attention_bf16.UNEVEN_SPLITS), planned
-    results = []
-    for _ in range(3):
+    results, page_error = [], torch.zeros(1, dtype=torch.int32, device=DEVICE)
+    newest = batch.positions.long()
+    places = tables[batch.seq_of_token.long(), newest // page_size].long(), newest % page_size
+    torch.cuda.synchronize()
+    for launch in range(5 if settled else 3):
+        if settled:
+            batch.keys_settled = launch > 0
+            for pages in (k_pages, v_pages):
+                pages[places[0], :, places[1]] = 99.0
+            ops.qk_norm_rope_kv_write(qkv, None, None, None, batch.positions, batch.seq_of_token, tables, k_pages, v_pages, heads, kv_heads, dim, 1e-6,
+                                      True, page_error)
         if form is None:
             results.append(attention_bf16.try_attention(qkv, q_stride, batch, tables, k_pages, v_pages, heads, kv_heads, dim, dim ** -0.5, 0))
         else:
@@ -116,9 +127,9 @@ def test_parts_by_length(form, case, heads, dim):
     want = ops.attention_generic(qkv, q_stride, k_pages, v_pages, tables, batch.seq_of_token, batch.positions, heads, kv_heads, dim, dim ** -0.5, **given)
     torch.cuda.synchronize()
     check_wait_errors()
-    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
+    assert int(page_error) == 0 and all(torch.equal(result, results[0]) for result in results)
     got, want = results[0].double(), want.double()
-    for row, context in enumerate(contexts[:singles]):
+    for context, row in zip(contexts, batch.q_start.tolist()):
         if context == 0:
             assert not got[row].any()
             want[row] = 0
