@@ -1113,8 +1113,8 @@ __global__ void __launch_bounds__(kDecodeThreads) attention_decode_tma_kernel(co
         if (n_splits == 1 || warp >= group) return;
         // What the parts have left for a warp's heads is added, in their order and with the merge kernel's arithmetic, by that warp of
         // the part whose warp comes last; the others' results lie in L2.  A warp counts for itself and asks for a head's parts at
-        // once: a step of the 8B shape at equal contexts of 3072 keys, us, when the block's four warps waited for one another and
-        // asked twice / this way: 24 sequences 5097 / 5043, 32 sequences 5549 / 5461.  (Clusters with a rank for every part that
+        // once: a step of the 8B shape at equal contexts, us, when the block's four warps waited for one another and asked twice /
+        // this way: 16 sequences of 3072 keys 4277 / 4262, of 800 3502 / 3493, 18 of 2000 4192 / 4182, 32 of 3072 5470 / 5458.  (Clusters with a rank for every part that
         // there could be keep the places of ranks without a part until the whole cluster ends: 32 sequences of 3072
         // keys in clusters of two, one rank idle, 6.86 ms a step against 5.56.)
         __syncwarp();

@@ -555,8 +555,8 @@ __global__ void __launch_bounds__(kThreads, PER_SM) gemm_small_m_kernel(const __
     // read the same columns of thousands of rows at a time, which lie on few of the memory's channels (q/k/v of the 8B shape in four
     // parts, us, in step / turned: 14.3 / 13.8 at 61 tokens, 17.1 / 16.6 at 119; gate/up unsplit at 119 42.0 / 40.7; a step of 21
     // sequences of the 14B shape 6168 / 6103, of 64 of the Dikusun shape 953 / 945).  A few tiles share nothing that matters.  Up to 16
-    // tokens all tiles add in the order of K: a step of one sequence of the 8B shape takes 3017 us that way and 3023 turned, of
-    // eight 3537 and 3530, which is as far as two runs differ.
+    // tokens all tiles add in the order of K: a step of one sequence of the 8B shape takes 3013 us that way and 3017 turned, of
+    // eight 3551 and 3542.
     const int turn = MANY && n_kb > 0 && (int)gridDim.x > kTurnTiles * p.split ? tile * kTurn % n_kb : 0;
     auto turned = [&](int i) { const int kb = i + turn; return kb >= n_kb ? kb - n_kb : kb; };
 
