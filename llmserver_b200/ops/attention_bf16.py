@@ -24,8 +24,8 @@ WIDE_CLUSTER_SPLITS = 16
 # Up to a wave of (sequence, kv head) pairs, and where equal parts would be at most two, the TMA kernel divides sequences by their
 # lengths (up to this many sequences, of up to MAX_CLUSTER_SPLITS parts each), on the device: a replayed step is planned for contexts
 # that it does not know.  Equal parts / by length, ms a step of the 8B shape: 24 sequences of 517 to 4003 keys 5.74 / 4.87, 12 of 100 to
-# 4000 4.13 / 3.75, 16 of 301 to 4077 4.20 / 4.03; equal contexts of 3072 keys, 32 sequences 5.55 / 5.51, 16 sequences 4.26 / 4.32 (merging
-# through L2 instead of a cluster).  With four equal parts the cluster stays ahead: 8 sequences of 3072 3.53 / 3.61, of 301 to 4077
+# 4000 4.13 / 3.75, 16 of 301 to 4077 4.23 / 4.00; equal contexts, 32 sequences of 3072 keys 5.67 / 5.46, 16 of 3072 4.24 / 4.26 and of 800 3.48 /
+# 3.49 (merging through L2 instead of a cluster).  With four equal parts the cluster stays ahead: 8 sequences of 3072 3.53 / 3.61, of 301 to 4077
 # 3.52 / 3.44.
 UNEVEN_SPLITS, UNEVEN_SEQUENCES = 2, 128
 

@@ -27,8 +27,9 @@ def stream_rows(width: int, decode: bool) -> int:
     is a step of single tokens, which graphs replay.
 
     Up to 64 rows every step: the products are level with the library's and four launches a layer fall away.  Beyond, a token tile is
-    as large as a weight tile and the library's products are faster on the device, which decides wherever launches are replayed or
-    the matrices are wide; only steps that the host's launches bound gain.  Stand-alone kernels from 17 rows on / none, ms:
+    as large as a weight tile and the library's products were faster on the device when these bounds were drawn, which decides wherever
+    launches are replayed or the matrices are wide; only steps that the host's launches bound gain.  (This package's product kernel has
+    since become 7 to 18 % faster there; replayed steps beyond 64 rows were not measured again.)  Stand-alone kernels from 17 rows on / none, ms:
     replayed decode steps, contexts of 301 to 2000: width 2048 2.33 / 2.24 at 24 rows, 2.94 / 2.95 at 64, 3.93 / 4.07 at 96, 4.72 / 4.98
     at 128; 8B shape 4.75 / 4.70 at 24, 5.55 / 5.43 at 48, 5.63 / 5.40 at 61, 7.04 / 7.23 at 96, 8.09 / 8.51 at 128; 14B shape (5120) 6.68 /
     6.42 at 24, 7.91 / 7.94 at 64, 9.90 / 9.76 at 96, 11.19 / 11.43 at 128; 32B shape (5120) 15.66 / 15.50 at 64.  Prompts: width 2048 4.33 /
